@@ -9,14 +9,13 @@ import torch
 
 import ctypes
 
-from ._lib import lib, check, FcHeadArgs, UpdateItem, DpItem, DpUpdateArgs, WgradItem
+from ._lib import lib, check, NitiError, FcHeadArgs, UpdateItem, DpItem, DpUpdateArgs, WgradItem
+from . import _torch_ops as native  # built together with the library (python -m niti_b200.build)
+
+native.set_error_type(NitiError)
 
 ROUND_NEAREST, ROUND_STOCHASTIC, ROUND_PSEUDO_STOCHASTIC = 0, 1, 2
 CALC_ACT, CALC_ERR, CALC_GRAD = 0, 1, 2
-
-_status = {}
-_scratch = {}
-_scratch_retired = []
 
 # Launch accounting.  LAUNCHES counts kernels of this library enqueued through this module.
 # PROFILE, when set to a list (eager execution only, never under graph capture), makes every
@@ -39,6 +38,21 @@ def _call(name, kernels, algo_ops, algo_bytes, fn, *args):
     PROFILE.append((name, algo_ops, algo_bytes, a, b))
 
 
+def _run(name, kernels, work, fn, *args):
+    """fn(*args), a native operation that allocates and returns its outputs; `work(result)` gives its algorithmic ops and
+    bytes and is asked only while a profile is taken."""
+    global LAUNCHES
+    LAUNCHES += kernels
+    if PROFILE is None:
+        return fn(*args)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
+    r = fn(*args)
+    b.record()
+    PROFILE.append((name, *work(r), a, b))
+    return r
+
+
 def _st():
     return torch.cuda.current_stream().cuda_stream
 
@@ -55,10 +69,7 @@ def _need_cuda(*ts):
 
 def status_word(device):
     """int32[4] the tensor-core kernels write if one of their bounded waits expires."""
-    key = torch.device(device).index
-    if key not in _status:
-        _status[key] = torch.zeros(4, dtype=torch.int32, device=device)
-    return _status[key]
+    return native.status_word(torch.cuda.current_device() if (i := torch.device(device).index) is None else i)
 
 
 def status_message(s):
@@ -77,19 +88,6 @@ def check_status(device):
         raise RuntimeError(status_message(s))
 
 
-def scratch(device, nbytes):
-    """Grow-only per-device scratch arena (stream-ordered reuse on the current stream).  An arena that is outgrown is
-    kept alive, not freed: a captured CUDA graph may still hold its address."""
-    key = torch.device(device).index
-    cur = _scratch.get(key)
-    if cur is None or cur.numel() < nbytes:
-        if cur is not None:
-            _scratch_retired.append(cur)
-        cur = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _scratch[key] = cur
-    return cur
-
-
 def seed_tensor(value, device):
     """uint64 seed word on the device (stored in an int64 tensor)."""
     return torch.tensor([int(value)], dtype=torch.int64, device=device)
@@ -97,19 +95,9 @@ def seed_tensor(value, device):
 
 # ------------------------------------------------------------------ contractions
 def conv_fprop_acc(x, w, pad=1, stride=1):
-    _need_cuda(x, w)
-    N, H, W, C = x.shape
-    K, R, S, C2 = w.shape
-    assert C == C2 and x.dtype == torch.int8 and w.dtype == torch.int8
-    P, Q = H + 2 * pad - R + 1, W + 2 * pad - S + 1
-    y32 = torch.empty((N, P, Q, K), dtype=torch.int32, device=x.device)
-    mx = torch.empty(1, dtype=torch.int32, device=x.device)
-    nbytes = lib.niti_conv_fprop_scratch_bytes(N, H, W, C, K, R, S)
-    sc = scratch(x.device, nbytes) if nbytes else None
-    _call("niti_conv_fprop_i8", 2 if nbytes else 1, 2 * N * P * Q * K * R * S * C, x.numel() + w.numel() + 4 * y32.numel(),
-          lib.niti_conv_fprop_i8, _p(x), _p(w), _p(y32), _p(mx), _p(sc), sc.numel() if nbytes else 0,
-          N, H, W, C, K, R, S, pad, stride, _p(status_word(x.device)), _st())
-    return y32, mx
+    def work(r):
+        return 2 * r[0].numel() * w[0].numel(), x.numel() + w.numel() + 4 * r[0].numel()
+    return _run("niti_conv_fprop_i8", 2 if w.numel() <= 32 * w.shape[0] else 1, work, native.conv_fprop_acc, x, w, pad, stride)
 
 
 def conv_fprop_i4(x4, w4, pad=1):
@@ -123,7 +111,7 @@ def conv_fprop_i4(x4, w4, pad=1):
     y32 = torch.empty((N, P, Q, K), dtype=torch.int32, device=x4.device)
     mx = torch.empty(1, dtype=torch.int32, device=x4.device)
     nbytes = lib.niti_conv_fprop_i4_scratch_bytes(N, H, W, C2, K, R, S)
-    sc = scratch(x4.device, nbytes)
+    sc = torch.empty(nbytes, dtype=torch.uint8, device=x4.device)
     _call("niti_conv_fprop_i4", 3, 2 * N * P * Q * K * R * S * 2 * C2, x4.numel() + w4.numel() + 4 * y32.numel(),
           lib.niti_conv_fprop_i4, _p(x4), _p(w4), _p(y32), _p(mx), _p(sc), sc.numel(), N, H, W, C2, K, R, S, pad,
           _p(status_word(x4.device)), _st())
@@ -161,16 +149,16 @@ def new_requant_state(device):
 
 
 def conv_fprop_fused_supported(C, K, R, S, pad):
-    return bool(lib.niti_conv_fprop_requant_supported(C, K, R, S, pad))
+    return native.conv_fprop_fused_supported(C, K, R, S, pad)
 
 
 def conv_dgrad_fused_supported(C, K, R, S, pad):
-    return bool(lib.niti_conv_dgrad_requant_supported(C, K, R, S, pad))
+    return native.conv_dgrad_fused_supported(C, K, R, S, pad)
 
 
 def conv_fprop_scratch_bytes(N, H, W, C, K, R, S):
     """Scratch bytes of a forward convolution (non-zero for thin layers: their patch matrix [N*H*W][32] + padded filters)."""
-    return int(lib.niti_conv_fprop_scratch_bytes(N, H, W, C, K, R, S))
+    return native.conv_fprop_scratch_bytes(N, H, W, C, K, R, S)
 
 
 def conv_fprop_fused(x, w, state, pad=1, mode=ROUND_NEAREST, seed=None, rng_stream=0, rng_offset=0, relu=False,
@@ -178,46 +166,29 @@ def conv_fprop_fused(x, w, state, pad=1, mode=ROUND_NEAREST, seed=None, rng_stre
     """Convolution + act_calc in one pass.  Returns (int8 [N,H,W,K], exp_out, shift).  scratch_buf: a uint8 tensor of
     conv_fprop_scratch_bytes() bytes owned by the caller instead of the shared scratch; a thin layer's patch matrix
     then survives in its first N*H*W*32 bytes for conv_wgrad_from_patches."""
-    _need_cuda(x, w, state, scratch_buf)
-    N, H, W, C = x.shape
-    K, R, S, _ = w.shape
-    y8 = torch.empty((N, H, W, K), dtype=torch.int8, device=x.device)
-    exp_out = torch.empty((), dtype=torch.int32, device=x.device)
-    shift_out = torch.empty((), dtype=torch.int32, device=x.device)
-    nbytes = lib.niti_conv_fprop_scratch_bytes(N, H, W, C, K, R, S)
-    sc = (scratch_buf if scratch_buf is not None else scratch(x.device, nbytes)) if nbytes else None
-    _call("niti_conv_fprop_requant_i8", 3 if nbytes else 2, 2 * N * H * W * K * R * S * C, x.numel() + w.numel() + y8.numel(),
-          lib.niti_conv_fprop_requant_i8, _p(x), _p(w), _p(y8), _p(state), _p(sc), sc.numel() if nbytes else 0,
-          N, H, W, C, K, R, S, pad, mode, _p(seed), rng_stream, rng_offset, int(relu), _p(exp_a), _p(exp_b),
-          _p(exp_out), _p(shift_out), _p(status_word(x.device)), _st())
-    return y8, exp_out, shift_out
+    def work(r):
+        return 2 * r[0].numel() * w[0].numel(), x.numel() + w.numel() + r[0].numel()
+    return _run("niti_conv_fprop_requant_i8", 2, work, native.conv_fprop_fused, x, w, state, pad, mode, seed, rng_stream, rng_offset,
+                relu, exp_a, exp_b, scratch_buf)
 
 
 def conv_fprop_pool_fused_supported(N, H, W, C, K, R, S, pad):
-    return bool(lib.niti_conv_fprop_requant_pool_supported(N, H, W, C, K, R, S, pad))
+    return native.conv_fprop_pool_fused_supported(N, H, W, C, K, R, S, pad)
 
 
 def conv_fprop_pool_fused(x, w, state, pad=1, mode=ROUND_NEAREST, seed=None, rng_stream=0, rng_offset=0, relu=False,
                           exp_a=None, exp_b=None):
     """Convolution + act_calc (+ ReLU) + 2x2 max pooling in one launch.  Returns (int8 [N,H,W,K], int8 [N,H/2,W/2,K],
     exp_out, shift)."""
-    _need_cuda(x, w, state)
-    N, H, W, C = x.shape
-    K, R, S, _ = w.shape
-    y8 = torch.empty((N, H, W, K), dtype=torch.int8, device=x.device)
-    yp = torch.empty((N, H // 2, W // 2, K), dtype=torch.int8, device=x.device)
-    exp_out = torch.empty((), dtype=torch.int32, device=x.device)
-    shift_out = torch.empty((), dtype=torch.int32, device=x.device)
-    _call("niti_conv_fprop_requant_pool_i8", 1, 2 * N * H * W * K * R * S * C, x.numel() + w.numel() + y8.numel() + yp.numel(),
-          lib.niti_conv_fprop_requant_pool_i8, _p(x), _p(w), _p(y8), _p(yp), _p(state),
-          N, H, W, C, K, R, S, pad, mode, _p(seed), rng_stream, rng_offset, int(relu), _p(exp_a), _p(exp_b),
-          _p(exp_out), _p(shift_out), _p(status_word(x.device)), _st())
-    return y8, yp, exp_out, shift_out
+    def work(r):
+        return 2 * r[0].numel() * w[0].numel(), x.numel() + w.numel() + r[0].numel() + r[1].numel()
+    return _run("niti_conv_fprop_requant_pool_i8", 1, work, native.conv_fprop_pool_fused, x, w, state, pad, mode, seed, rng_stream,
+                rng_offset, relu, exp_a, exp_b)
 
 
 def conv_dgrad_side_bytes(N, H, W, C, K, R, S, pad):
     """Bytes of per-layer side memory conv_dgrad_fused can use for this shape (0: the single-launch kernel serves it)."""
-    return int(lib.niti_conv_dgrad_requant_side_bytes(N, H, W, C, K, R, S, pad))
+    return native.conv_dgrad_side_bytes(N, H, W, C, K, R, S, pad)
 
 
 def conv_dgrad_fused(err, w, state, pad=1, mode=ROUND_NEAREST, seed=None, rng_stream=0, rng_offset=0, exp_a=None, exp_b=None,
@@ -226,78 +197,43 @@ def conv_dgrad_fused(err, w, state, pad=1, mode=ROUND_NEAREST, seed=None, rng_st
     relu_mask, the layer's forward input, is given).  side: optional uint8 tensor of conv_dgrad_side_bytes() bytes kept
     with the layer; with it a shift guessed one too high is repaired by a cheap pass instead of a second contraction.
     Returns (int8 [N,H,W,C], exp_out, shift)."""
-    _need_cuda(err, w, state, relu_mask, side)
-    N, H, W, K = err.shape
-    K2, R, S, C = w.shape
-    e8 = torch.empty((N, H, W, C), dtype=torch.int8, device=err.device)
-    exp_out = torch.empty((), dtype=torch.int32, device=err.device)
-    shift_out = torch.empty((), dtype=torch.int32, device=err.device)
-    _call("niti_conv_dgrad_requant_i8", 2, 2 * N * H * W * K * R * S * C, err.numel() + w.numel() + e8.numel(),
-          lib.niti_conv_dgrad_requant_side_i8, _p(err), _p(w), _p(e8), _p(state), _p(side), side.numel() if side is not None else 0,
-          N, H, W, C, K, R, S, pad, mode, _p(seed),
-          rng_stream, rng_offset, _p(exp_a), _p(exp_b), _p(exp_out), _p(shift_out), _p(relu_mask),
-          _p(status_word(err.device)), _st())
-    return e8, exp_out, shift_out
+    def work(r):
+        return 2 * err.numel() * w[0].numel(), err.numel() + w.numel() + r[0].numel()
+    return _run("niti_conv_dgrad_requant_i8", 2, work, native.conv_dgrad_fused, err, w, state, pad, mode, seed, rng_stream, rng_offset,
+                exp_a, exp_b, relu_mask, side)
 
 
 def conv_dgrad_acc(err, w, pad=1):
     """err [N,H,W,K] with the layer's own filters w [K,R,S,C] -> int32 [N,H,W,C] (error w.r.t. the input)."""
-    _need_cuda(err, w)
-    N, H, W, K = err.shape
-    K2, R, S, C = w.shape
-    assert K == K2
-    e32 = torch.empty((N, H, W, C), dtype=torch.int32, device=err.device)
-    mx = torch.empty(1, dtype=torch.int32, device=err.device)
-    _call("niti_conv_dgrad_i8", 1, 2 * N * H * W * K * R * S * C, err.numel() + w.numel() + 4 * e32.numel(),
-          lib.niti_conv_dgrad_i8, _p(err), _p(w), _p(e32), _p(mx), N, H, W, C, K, R, S, pad,
-          _p(status_word(err.device)), _st())
-    return e32, mx
+    def work(r):
+        return 2 * err.numel() * w[0].numel(), err.numel() + w.numel() + 4 * r[0].numel()
+    return _run("niti_conv_dgrad_i8", 1, work, native.conv_dgrad_acc, err, w, pad)
 
 
 def conv_wgrad_acc(x, err, R=3, S=3, pad=1, out=None, want_max=True):
     """Weight gradient accumulators and max|g32| (None when want_max is False: update_multi finds it)."""
-    _need_cuda(x, err, out)
-    N, H, W, C = x.shape
-    K = err.shape[3]
-    g32 = out if out is not None else torch.empty((K, R, S, C), dtype=torch.int32, device=x.device)
-    mx = torch.empty(1, dtype=torch.int32, device=x.device) if want_max else None
-    nbytes = lib.niti_conv_wgrad_scratch_bytes(N, H, W, C, K, R, S)
-    sc = scratch(x.device, nbytes)
-    _call("niti_conv_wgrad_i8", 2 if C % 16 == 0 else 3, 2 * N * H * W * K * R * S * C, x.numel() + err.numel() + 4 * g32.numel(),
-          lib.niti_conv_wgrad_i8, _p(x), _p(err), _p(g32), _p(mx), _p(sc), sc.numel(), N, H, W, C, K, R, S, pad,
-          _p(status_word(x.device)), _st())
-    return g32, mx
+    def work(r):
+        return 2 * err.numel() * R * S * x.shape[3], x.numel() + err.numel() + 4 * r[0].numel()
+    return _run("niti_conv_wgrad_i8", 2, work, native.conv_wgrad_acc, x, err, R, S, pad, out, want_max)
 
 
 def conv_wgrad_from_patches(patches, err, C, R=3, S=3, out=None, want_max=True):
     """Weight gradient of a thin layer (R*S*C <= 32) from the patch matrix its forward call left in `patches` (see
     conv_fprop_fused(scratch_buf=...)): same result as conv_wgrad_acc on the layer's input, without gathering again."""
-    _need_cuda(patches, err, out)
-    N, H, W, K = err.shape
-    g32 = out if out is not None else torch.empty((K, R, S, C), dtype=torch.int32, device=err.device)
-    mx = torch.empty(1, dtype=torch.int32, device=err.device) if want_max else None
-    nbytes = lib.niti_conv_wgrad_patches_scratch_bytes(N, H, W, C, K, R, S)
-    sc = scratch(err.device, nbytes)
-    _call("niti_conv_wgrad_patches_i8", 2, 2 * N * H * W * K * R * S * C, N * H * W * 32 + err.numel() + 4 * g32.numel(),
-          lib.niti_conv_wgrad_patches_i8, _p(patches), _p(err), _p(g32), _p(mx), _p(sc), sc.numel(), N, H, W, C, K, R, S,
-          _p(status_word(err.device)), _st())
-    return g32, mx
+    def work(r):
+        return 2 * err.numel() * R * S * C, 32 * err.numel() // err.shape[3] + err.numel() + 4 * r[0].numel()
+    return _run("niti_conv_wgrad_patches_i8", 2, work, native.conv_wgrad_from_patches, patches, err, C, R, S, out, want_max)
 
 
 def conv_wgrad_accumulate_supported(C, K, R, S, pad):
-    return bool(lib.niti_conv_wgrad_accumulate_supported(C, K, R, S, pad))
+    return native.conv_wgrad_accumulate_supported(C, K, R, S, pad)
 
 
 def conv_wgrad_accumulate(x, err, g32, R=3, S=3, pad=1):
     """g32 += weight gradient (no clearing pass: the caller keeps g32 zeroed between steps, see update_multi)."""
-    _need_cuda(x, err, g32)
-    N, H, W, C = x.shape
-    K = err.shape[3]
-    assert g32.dtype == torch.int32 and g32.numel() == K * R * S * C
-    _call("niti_conv_wgrad_accumulate_i8", 1, 2 * N * H * W * K * R * S * C, x.numel() + err.numel() + 4 * g32.numel(),
-          lib.niti_conv_wgrad_accumulate_i8, _p(x), _p(err), _p(g32), N, H, W, C, K, R, S, pad,
-          _p(status_word(x.device)), _st())
-    return g32
+    def work(r):
+        return 2 * err.numel() * R * S * x.shape[3], x.numel() + err.numel() + 4 * g32.numel()
+    return _run("niti_conv_wgrad_accumulate_i8", 1, work, native.conv_wgrad_accumulate, x, err, g32, R, S, pad)
 
 
 def conv_wgrad_accumulate_multi_max():
@@ -324,16 +260,9 @@ def conv_wgrad_accumulate_multi(jobs):
 
 def gemm_acc(a, b, trans_a=False, trans_b=False, out=None):
     """C32[M,N] = op(a) @ op(b); a is [M,K] ([K,M] if trans_a), b is [K,N] ([N,K] if trans_b)."""
-    _need_cuda(a, b, out)
-    M, K = (a.shape[1], a.shape[0]) if trans_a else a.shape
-    N = b.shape[0] if trans_b else b.shape[1]
-    assert (b.shape[1] if trans_b else b.shape[0]) == K
-    c32 = out if out is not None else torch.empty((M, N), dtype=torch.int32, device=a.device)
-    mx = torch.empty(1, dtype=torch.int32, device=a.device)
-    _call("niti_gemm_i8", 1, 2 * M * N * K, a.numel() + b.numel() + 4 * c32.numel(),
-          lib.niti_gemm_i8, _p(a), _p(b), _p(c32), _p(mx), M, N, K, int(trans_a), int(trans_b),
-          _p(status_word(a.device)), _st())
-    return c32, mx
+    def work(r):
+        return 2 * r[0].numel() * a.shape[0 if trans_a else 1], a.numel() + b.numel() + 4 * r[0].numel()
+    return _run("niti_gemm_i8", 1, work, native.gemm_acc, a, b, trans_a, trans_b, out)
 
 
 def group_conv1(inp, wt, pad):
@@ -354,70 +283,54 @@ def group_conv1(inp, wt, pad):
 def requant(acc, maxabs, kind, target_bits, mode=ROUND_NEAREST, seed=None, rng_stream=0, rng_offset=0, relu=False,
             exp_a=None, exp_b=None, want_shift=False):
     """int32 -> int8 by the tensor-wide shift.  Returns (out8, exp_out, shift_out)."""
-    _need_cuda(acc, maxabs)
-    out = torch.empty(acc.shape, dtype=torch.int8, device=acc.device)
-    exp_out = torch.empty((), dtype=torch.int32, device=acc.device)
-    shift_out = torch.empty((), dtype=torch.int32, device=acc.device) if want_shift else None
-    _call("niti_requant_i8", 1, 0, 5 * acc.numel(),
-          lib.niti_requant_i8, _p(acc), _p(out), _p(maxabs), acc.numel(), kind, target_bits, mode, _p(seed), rng_stream,
-          rng_offset, int(relu), _p(exp_a), _p(exp_b), _p(exp_out), _p(shift_out), _st())
-    return out, exp_out, shift_out
+    def work(r):
+        return 0, 5 * acc.numel()
+    return _run("niti_requant_i8", 1, work, native.requant, acc, maxabs, kind, target_bits, mode, seed, rng_stream, rng_offset, relu,
+                exp_a, exp_b, want_shift)
 
 
 def absmax(acc):
-    _need_cuda(acc)
-    mx = torch.empty(1, dtype=torch.int32, device=acc.device)
-    _call("niti_absmax_i32", 1, 0, 4 * acc.numel(), lib.niti_absmax_i32, _p(acc), acc.numel(), _p(mx), _st())
-    return mx
+    def work(r):
+        return 0, 4 * acc.numel()
+    return _run("niti_absmax_i32", 1, work, native.absmax, acc)
 
 
 # ------------------------------------------------------------------ memory-bound layers
 def maxpool_fwd(x, k=2, stride=2):
-    _need_cuda(x)
-    N, H, W, C = x.shape
-    y = torch.empty((N, (H - k) // stride + 1, (W - k) // stride + 1, C), dtype=torch.int8, device=x.device)
-    _call("niti_maxpool_fwd_i8", 1, 0, x.numel() + y.numel(), lib.niti_maxpool_fwd_i8, _p(x), _p(y), N, H, W, C, k, stride, _st())
-    return y
+    def work(y):
+        return 0, x.numel() + y.numel()
+    return _run("niti_maxpool_fwd_i8", 1, work, native.maxpool_fwd, x, k, stride)
 
 
 def maxpool_bwd(x, dy, k=2, stride=2, relu_mask=False):
     """dx of max pooling; relu_mask also applies the backward of the ReLU that produced x (zero where x <= 0)."""
-    _need_cuda(x, dy)
-    N, H, W, C = x.shape
-    dx = torch.empty_like(x)
-    _call("niti_maxpool_bwd_i8", 1, 0, 2 * x.numel() + dy.numel(), lib.niti_maxpool_bwd_i8, _p(x), _p(dy), _p(dx), N, H, W, C, k, stride, int(relu_mask), _st())
-    return dx
+    def work(dx):
+        return 0, 2 * x.numel() + dy.numel()
+    return _run("niti_maxpool_bwd_i8", 1, work, native.maxpool_bwd, x, dy, k, stride, relu_mask)
 
 
 def relu_fwd(x):
-    _need_cuda(x)
-    y = torch.empty_like(x)
-    _call("niti_relu_fwd_i8", 1, 0, 2 * x.numel(), lib.niti_relu_fwd_i8, _p(x), _p(y), x.numel(), _st())
-    return y
+    def work(y):
+        return 0, 2 * x.numel()
+    return _run("niti_relu_fwd_i8", 1, work, native.relu_fwd, x)
 
 
 def relu_bwd(act, err):
-    _need_cuda(act, err)
-    out = torch.empty_like(err)
-    _call("niti_relu_bwd_i8", 1, 0, 3 * err.numel(), lib.niti_relu_bwd_i8, _p(act), _p(err), _p(out), err.numel(), _st())
-    return out
+    def work(r):
+        return 0, 3 * err.numel()
+    return _run("niti_relu_bwd_i8", 1, work, native.relu_bwd, act, err)
 
 
 def dropout(x, seed, rng_stream):
-    _need_cuda(x, seed)
-    y = torch.empty_like(x)
-    _call("niti_dropout_i8", 1, 0, 2 * x.numel(), lib.niti_dropout_i8, _p(x), _p(y), x.shape[0], x.numel() // x.shape[0],
-          _p(seed), rng_stream, _st())
-    return y
+    def work(y):
+        return 0, 2 * x.numel()
+    return _run("niti_dropout_i8", 1, work, native.dropout, x, seed, rng_stream)
 
 
 def loss_err(out8, out_exp, target, seed, rng_stream=0xFFFF, sample_offset=0):
-    _need_cuda(out8, out_exp, target, seed)
-    assert target.dtype == torch.int64 and out_exp.dtype == torch.int32
-    err = torch.empty_like(out8)
-    _call("niti_loss_i8", 1, 0, 2 * out8.numel(), lib.niti_loss_i8, _p(out8), _p(out_exp), _p(target), _p(err),
-          out8.shape[0], out8.shape[1], _p(seed), rng_stream, sample_offset, _st())
-    return err
+    def work(r):
+        return 0, 2 * out8.numel()
+    return _run("niti_loss_i8", 1, work, native.loss_err, out8, out_exp, target, seed, rng_stream, sample_offset)
 
 
 def fc_head_supported(B, F, J):
@@ -454,9 +367,9 @@ def fc_head_train(x, exp_x, w, exp_w, target, seed, layer_stream, *, dropout=Tru
 
 def update(w, g32, maxabs, mu, mode=ROUND_PSEUDO_STOCHASTIC, seed=None, rng_stream=0):
     """In-place integer SGD update of the int8 weights from their int32 gradient accumulators."""
-    _need_cuda(w, g32, maxabs)
-    _call("niti_update_i8", 1, 0, 6 * w.numel(), lib.niti_update_i8, _p(w), _p(g32), _p(maxabs),
-          w.numel(), mu, mode, _p(seed), rng_stream, _st())
+    def work(r):
+        return 0, 6 * w.numel()
+    _run("niti_update_i8", 1, work, native.update, w, g32, maxabs, mu, mode, seed, rng_stream)
 
 
 def update_multi(ws, g32s, streams, mu, mode=ROUND_PSEUDO_STOCHASTIC, seed=None, want_max=False, clear=False):
@@ -510,17 +423,18 @@ def peer_copy(dst_ptr, src_ptr, nbytes):
 def quantize_input(x, reduce_max=None):
     """float32 NCHW -> (int8 NHWC, exponent).  ``reduce_max(t)``: optional hook that replaces the int32[1] word
     holding the bit pattern of max|x| by its maximum over a process group, in place."""
+    if reduce_max is None:
+        def work(r):
+            return 0, 9 * x.numel()
+        return _run("niti_quantize_input_f32", 2, work, native.quantize_input, x)
     _need_cuda(x)
     assert x.dtype == torch.float32
     N, C, H, W = x.shape
     x8 = torch.empty((N, H, W, C), dtype=torch.int8, device=x.device)
     e = torch.empty((), dtype=torch.int32, device=x.device)
     tmp = torch.empty(1, dtype=torch.int32, device=x.device)
-    if reduce_max is not None:
-        _call("niti_absmax_f32", 1, 0, 4 * x.numel(), lib.niti_absmax_f32, _p(x), x.numel(), _p(tmp), _st())
-        reduce_max(tmp)
-        _call("niti_quantize_input_with_max_f32", 1, 0, 5 * x.numel(), lib.niti_quantize_input_with_max_f32, _p(x), _p(x8), _p(e),
-              _p(tmp), N, C, H, W, _st())
-        return x8, e
-    _call("niti_quantize_input_f32", 2, 0, 9 * x.numel(), lib.niti_quantize_input_f32, _p(x), _p(x8), _p(e), _p(tmp), N, C, H, W, _st())
+    _call("niti_absmax_f32", 1, 0, 4 * x.numel(), lib.niti_absmax_f32, _p(x), x.numel(), _p(tmp), _st())
+    reduce_max(tmp)
+    _call("niti_quantize_input_with_max_f32", 1, 0, 5 * x.numel(), lib.niti_quantize_input_with_max_f32, _p(x), _p(x8), _p(e),
+          _p(tmp), N, C, H, W, _st())
     return x8, e

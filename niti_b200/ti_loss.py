@@ -13,7 +13,8 @@ class TiLoss(Module):
 
     def forward(self, out_val, out_exp, target):
         dev = out_val.device
-        self.out_grad = ops.loss_err(out_val.contiguous(), ti_torch.exp_tensor(out_exp, dev),
-                                     target.to(device=dev, dtype=torch.int64).contiguous(),
-                                     ti_torch.RNG_SEED(dev), 0xFFFF, ti_torch.SAMPLE_OFFSET)
-        return self.out_grad, torch.zeros((), dtype=torch.int32, device=dev)
+        out_grad = ops.loss_err(out_val.contiguous(), ti_torch.exp_tensor(out_exp, dev),
+                                target.to(device=dev, dtype=torch.int64).contiguous(),
+                                ti_torch.RNG_SEED(dev), 0xFFFF, ti_torch.SAMPLE_OFFSET)
+        self.__dict__.update(out_grad=out_grad)
+        return out_grad, torch.zeros((), dtype=torch.int32, device=dev)

@@ -31,8 +31,9 @@ class TiNet(Module):
 
     def forward(self, x):
         x = TiFloatToInt8(x)  # NCHW float -> NHWC int8 + exponent
-        self.out, self.out_exp = self.forward_layers(x)
-        return self.out, self.out_exp
+        out, out_exp = self.forward_layers(x)
+        self.__dict__.update(out=out, out_exp=out_exp)
+        return out, out_exp
 
     @property
     def out_bits(self):

@@ -22,7 +22,11 @@ from . import ops
 
 
 class UpdateWeight(Module):
-    """Parameter update shared by TiConv2d and TiLinear (:11-21)."""
+    """Parameter update shared by TiConv2d and TiLinear (:11-21).
+
+    The layers' per-call attributes (activations, gradients, exponents) are written with ``__dict__.update``:
+    ``Module.__setattr__`` first looks through parameters, buffers and submodules, about 1 us per attribute and three to
+    six attributes per layer and step, which the kernels of a small batch do not take."""
 
     layer_id = 0          # index among the weighted layers; selects the random-bit streams
     grad_buffer = None    # optional preallocated int32 view the weight gradient is written into
@@ -74,8 +78,11 @@ def PstoShift(input, shift):
     return _shift_with(ops.ROUND_PSEUDO_STOCHASTIC, input, shift)
 
 
+_MODES = {RoundShift: ops.ROUND_NEAREST, StoShift: ops.ROUND_STOCHASTIC, PstoShift: ops.ROUND_PSEUDO_STOCHASTIC}
+
+
 def _mode(method):
-    return {RoundShift: ops.ROUND_NEAREST, StoShift: ops.ROUND_STOCHASTIC, PstoShift: ops.ROUND_PSEUDO_STOCHASTIC}[method]
+    return _MODES[method]
 
 
 def int8_clip(input, clip_val=127):
@@ -92,6 +99,9 @@ def Int8zeros(size):
 
 def exp_tensor(e, device=None):
     """Exponent as a 0-dim int32 tensor on the device (accepts ints, floats, tensors)."""
+    if isinstance(e, torch.Tensor):
+        if e.dtype is torch.int32 and e.dim() == 0 and e.is_cuda and (device is None or e.device == device):
+            return e  # what every layer of a network hands on: nothing to convert
     device = device or GPU
     if isinstance(e, torch.Tensor):
         return e.to(device=device, dtype=torch.int32).reshape(())
@@ -192,7 +202,7 @@ class TiLinear(UpdateWeight):
 
     def forward(self, input):
         """(act int8 [B,in], exp) -> (act int8 [B,out], exp) (:241-253)"""
-        self.act_in = input
+        self.__dict__.update(act_in=input)
         act_in, exp_in = input
         acc, mx = ops.gemm_acc(act_in, self.weight, trans_b=True)
         per = acc.shape[1]
@@ -201,17 +211,18 @@ class TiLinear(UpdateWeight):
     def backward(self, input):
         """(err int8 [B,out], exp) -> (err int8 [B,in], exp); updates the weights (:255-266)"""
         err_in, err_exp = input
-        act, self.act_in_exp = self.act_in
+        act, act_in_exp = self.act_in
         acc, mx = ops.gemm_acc(err_in, self.weight)
-        err_out, self.err_exp, _ = _calc(acc, ops.CALC_ERR, BITWIDTH, ERROR_ROUND_METHOD, 16 * self.layer_id + 1,
-                                         exp_tensor(err_exp, acc.device), self.weight_exp, mx, False,
-                                         SAMPLE_OFFSET * acc.shape[1])
-        self.grad_int32acc, self.grad_maxabs = ops.gemm_acc(err_in, act, trans_a=True, out=self.grad_buffer)
+        err_out, err_exp, _ = _calc(acc, ops.CALC_ERR, BITWIDTH, ERROR_ROUND_METHOD, 16 * self.layer_id + 1,
+                                    exp_tensor(err_exp, acc.device), self.weight_exp, mx, False,
+                                    SAMPLE_OFFSET * acc.shape[1])
+        g32, g_max = ops.gemm_acc(err_in, act, trans_a=True, out=self.grad_buffer)
+        self.__dict__.update(act_in_exp=act_in_exp, err_exp=err_exp, grad_int32acc=g32, grad_maxabs=g_max)
         if self.grad_ready is not None:
             self.grad_ready(self)
         if not self.defer_update:
             self.weight_update()
-        return err_out, self.err_exp
+        return err_out, err_exp
 
 
 class TiReLU(Module):
@@ -229,7 +240,7 @@ class TiReLU(Module):
     def forward(self, input):
         act_in, exp_in = input
         act_out = act_in if self.fused else ops.relu_fwd(act_in)
-        self.act_in = (act_out if self.fused else act_in, exp_in)
+        self.__dict__.update(act_in=(act_out if self.fused else act_in, exp_in))
         return act_out, exp_in
 
     def backward(self, input):
@@ -257,13 +268,14 @@ class TiMaxpool2d(Module):
         self.precomputed = None
 
     def forward(self, input):
-        self.act_in, exp_in = input
-        pre, self.precomputed = self.precomputed, None
-        if pre is not None and pre[0] is self.act_in:
-            self.act_out = pre[1]
+        act_in, exp_in = input
+        pre = self.precomputed
+        if pre is not None and pre[0] is act_in:
+            act_out = pre[1]
         else:
-            self.act_out = ops.maxpool_fwd(self.act_in, self.kernel_size, self.stride)
-        return self.act_out, exp_in
+            act_out = ops.maxpool_fwd(act_in, self.kernel_size, self.stride)
+        self.__dict__.update(act_in=act_in, act_out=act_out, precomputed=None)
+        return act_out, exp_in
 
     def backward(self, input):
         err_in, err_exp = input
@@ -275,7 +287,7 @@ class TiFlat(Module):
     """Flatten everything but the batch dimension (:318-332)."""
 
     def forward(self, input):
-        self.act_in = input
+        self.__dict__.update(act_in=input)
         act_in, exp_in = input
         return act_in.view(-1, act_in.nelement() // act_in.size(0)), exp_in
 
@@ -363,43 +375,46 @@ class TiConv2d(UpdateWeight):
         self._patches, self._patches_of = None, None
 
     def forward(self, input):
-        self.act, self.act_in_exp = input
+        act, exp_in = input
+        self.__dict__.update(act=act, act_in_exp=exp_in)
         K, R, S, C = self.weight.shape
-        per = self.act.shape[1] * self.act.shape[2] * K
+        offset = SAMPLE_OFFSET * act.shape[1] * act.shape[2] * K
         if FUSE_REQUANT and GLOBAL_MAX_GROUP is None and self.stride == 1 and ops.conv_fprop_fused_supported(C, K, R, S, self.padding):
             # conv2d_int8 + act_calc (:393-395) in one kernel; see ops.conv_fprop_fused
+            dev = act.device
             if self._fwd_state is None:
-                self._fwd_state = ops.new_requant_state(self.act.device)
+                self._fwd_state = ops.new_requant_state(dev)
+            mode, seed, stream, exp_in = _mode(ACT_ROUND_METHOD), RNG_SEED(dev), 16 * self.layer_id, exp_tensor(exp_in, dev)
             pool = self.pool_layer
             if (pool is not None and FUSE_POOL and self.fuse_relu and pool.kernel_size == 2 and pool.stride == 2
-                    and ops.conv_fprop_pool_fused_supported(*self.act.shape, K, R, S, self.padding)):
+                    and ops.conv_fprop_pool_fused_supported(*act.shape, K, R, S, self.padding)):
                 # conv2d_int8 + act_calc + ReLU (:393-395, :268-277) and the pool's forward (:302-307) in one kernel
-                out, pooled, exp_out, _ = ops.conv_fprop_pool_fused(self.act, self.weight, self._fwd_state, self.padding,
-                                                                    _mode(ACT_ROUND_METHOD), RNG_SEED(self.act.device),
-                                                                    16 * self.layer_id, SAMPLE_OFFSET * per, True,
-                                                                    exp_tensor(self.act_in_exp, self.act.device), self.weight_exp)
-                pool.precomputed = (out, pooled)
+                out, pooled, exp_out, _ = ops.conv_fprop_pool_fused(act, self.weight, self._fwd_state, self.padding, mode, seed,
+                                                                    stream, offset, True, exp_in, self.weight_exp)
+                pool.__dict__.update(precomputed=(out, pooled))
                 return out, exp_out
-            self._patches_of = None
+            patches = None
             if TRAINING and KEEP_PATCHES and self.first_layer:
                 # a thin layer runs as a GEMM over a patch matrix; kept in memory of its own it also serves the weight
                 # gradient of this step (the reference gathers its first-layer operands twice, :412-428)
-                nbytes = ops.conv_fprop_scratch_bytes(*self.act.shape, K, R, S)
+                nbytes = ops.conv_fprop_scratch_bytes(*act.shape, K, R, S)
                 if nbytes:
-                    if self._patches is None or self._patches.numel() < nbytes or self._patches.device != self.act.device:
-                        self._patches = torch.empty(nbytes, dtype=torch.uint8, device=self.act.device)
-                    self._patches_of = self.act
-            out, exp_out, _ = ops.conv_fprop_fused(self.act, self.weight, self._fwd_state, self.padding, _mode(ACT_ROUND_METHOD),
-                                                   RNG_SEED(self.act.device), 16 * self.layer_id, SAMPLE_OFFSET * per,
-                                                   self.fuse_relu, exp_tensor(self.act_in_exp, self.act.device), self.weight_exp,
-                                                   scratch_buf=self._patches if self._patches_of is not None else None)
+                    patches = self._patches
+                    if patches is None or patches.numel() < nbytes or patches.device != dev:
+                        patches = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+                        self.__dict__.update(_patches=patches)
+            self.__dict__.update(_patches_of=act if patches is not None else None)
+            out, exp_out, _ = ops.conv_fprop_fused(act, self.weight, self._fwd_state, self.padding, mode, seed, stream, offset,
+                                                   self.fuse_relu, exp_in, self.weight_exp, scratch_buf=patches)
             return out, exp_out
-        acc, mx = ops.conv_fprop_acc(self.act, self.weight, self.padding, self.stride)
-        return act_calc(acc, self.act_in_exp, mx, 16 * self.layer_id, self.fuse_relu, SAMPLE_OFFSET * per, self.weight_exp)
+        acc, mx = ops.conv_fprop_acc(act, self.weight, self.padding, self.stride)
+        return act_calc(acc, exp_in, mx, 16 * self.layer_id, self.fuse_relu, offset, self.weight_exp)
 
     def backward(self, input):
-        err_in, self.err_exp = input
+        err_in, err_exp = input
         err_in = err_in.contiguous()
+        act, dev = self.act, err_in.device
+        K, R, S, C = self.weight.shape
         err_out = None
         fork = None
         if self.wgrad_stream is not None and not self.first_layer:
@@ -407,32 +422,27 @@ class TiConv2d(UpdateWeight):
             fork.record()  # the weight gradient needs only what has been enqueued up to here
         if not self.first_layer:
             # the reference builds flip(w).transpose(0,3) here (:404); the kernels read w in place
-            K, R, S, C = self.weight.shape
-            per = self.act[0].numel()
+            n, h, w_ = err_in.shape[:3]
+            offset = SAMPLE_OFFSET * h * w_ * C
             if FUSE_REQUANT and GLOBAL_MAX_GROUP is None and ops.conv_dgrad_fused_supported(C, K, R, S, self.padding):
                 if self._bwd_state is None:
-                    self._bwd_state = ops.new_requant_state(err_in.device)
-                n, h, w_ = err_in.shape[:3]
+                    self._bwd_state = ops.new_requant_state(dev)
                 if STEP_DOWN_CODES and (self._bwd_side is None or self._bwd_side_shape != (n, h, w_)):
                     # layers whose output does not fit in tensor memory guess their shift; two more bits per output
                     # make a guess one too high a cheap repair instead of a second contraction
                     nbytes = ops.conv_dgrad_side_bytes(n, h, w_, C, K, R, S, self.padding)
-                    self._bwd_side = torch.empty(nbytes, dtype=torch.uint8, device=err_in.device) if nbytes else None
+                    self._bwd_side = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
                     self._bwd_side_shape = (n, h, w_)
-                err_out, self.err_exp, _ = ops.conv_dgrad_fused(err_in, self.weight, self._bwd_state, self.padding,
-                                                                _mode(ERROR_ROUND_METHOD), RNG_SEED(err_in.device),
-                                                                16 * self.layer_id + 1, SAMPLE_OFFSET * per,
-                                                                exp_tensor(self.err_exp, err_in.device), self.weight_exp,
-                                                                relu_mask=self.act if self.relu_backward_fused else None,
-                                                                side=self._bwd_side if STEP_DOWN_CODES else None)
+                err_out, err_exp, _ = ops.conv_dgrad_fused(err_in, self.weight, self._bwd_state, self.padding, _mode(ERROR_ROUND_METHOD),
+                                                           RNG_SEED(dev), 16 * self.layer_id + 1, offset, exp_tensor(err_exp, dev),
+                                                           self.weight_exp, relu_mask=act if self.relu_backward_fused else None,
+                                                           side=self._bwd_side if STEP_DOWN_CODES else None)
             else:
                 acc, mx = ops.conv_dgrad_acc(err_in, self.weight, self.padding)
-                err_out, self.err_exp, _ = _calc(acc, ops.CALC_ERR, BITWIDTH, ERROR_ROUND_METHOD, 16 * self.layer_id + 1,
-                                                 exp_tensor(self.err_exp, acc.device), self.weight_exp, mx, False,
-                                                 SAMPLE_OFFSET * per)
+                err_out, err_exp, _ = _calc(acc, ops.CALC_ERR, BITWIDTH, ERROR_ROUND_METHOD, 16 * self.layer_id + 1,
+                                            exp_tensor(err_exp, dev), self.weight_exp, mx, False, offset)
                 if self.relu_backward_fused:
-                    err_out = ops.relu_bwd(self.act, err_out)
-        K, R, S, C = self.weight.shape
+                    err_out = ops.relu_bwd(act, err_out)
         if self.first_layer:
             flush_wgrad()
         if (self.grad_accumulate and self.defer_update and self.grad_buffer is not None
@@ -440,28 +450,28 @@ class TiConv2d(UpdateWeight):
             if fork is not None:
                 # error-backward and weight gradient are independent: on two streams the SMs one kernel leaves idle
                 # (its last wave, its epilogue) are taken by the other
-                self._wgrad_inputs = (self.act, err_in)  # referenced until the owner of the side stream has joined it
-                _WGRAD_PENDING.append((self.wgrad_stream, fork, (self.act, err_in, self.grad_buffer, R, S, self.padding), self))
+                self._wgrad_inputs = (act, err_in)  # referenced until the owner of the side stream has joined it
+                _WGRAD_PENDING.append((self.wgrad_stream, fork, (act, err_in, self.grad_buffer, R, S, self.padding), self))
                 if len(_WGRAD_PENDING) >= min(WGRAD_GROUP, ops.conv_wgrad_accumulate_multi_max()):
                     flush_wgrad(full_group=True)
-                self.grad_int32acc, self.grad_maxabs = self.grad_buffer, None
+                g32, g_max = self.grad_buffer, None
             else:
-                self.grad_int32acc, self.grad_maxabs = ops.conv_wgrad_accumulate(self.act, err_in, self.grad_buffer, R, S, self.padding), None
-        elif getattr(self, "_patches_of", None) is self.act and self._patches is not None:
+                g32, g_max = ops.conv_wgrad_accumulate(act, err_in, self.grad_buffer, R, S, self.padding), None
+        elif self._patches_of is act and self._patches is not None:
             # the patch matrix of this step's forward pass is still there
-            self.grad_int32acc, self.grad_maxabs = ops.conv_wgrad_from_patches(self._patches, err_in, C, R, S, out=self.grad_buffer,
-                                                                               want_max=not self.defer_update)
+            g32, g_max = ops.conv_wgrad_from_patches(self._patches, err_in, C, R, S, out=self.grad_buffer,
+                                                     want_max=not self.defer_update)
             self._patches_of = None
         else:
             # a deferred update finds max|g| itself (weight_update_all)
-            self.grad_int32acc, self.grad_maxabs = ops.conv_wgrad_acc(self.act, err_in, R, S, self.padding, out=self.grad_buffer,
-                                                                      want_max=not self.defer_update)
+            g32, g_max = ops.conv_wgrad_acc(act, err_in, R, S, self.padding, out=self.grad_buffer, want_max=not self.defer_update)
+        self.__dict__.update(err_exp=err_exp, grad_int32acc=g32, grad_maxabs=g_max)
         if self.grad_ready is not None:
             self.grad_ready(self)
         if not self.defer_update:
             self.weight_update()
         if not self.first_layer:
-            return err_out, self.err_exp
+            return err_out, err_exp
 
 
 class TiDropout(Module):
@@ -509,12 +519,13 @@ _seed_words = {}
 
 def RNG_SEED(device=None):
     """The device word (int64[1]) that keys the random bits on ``device``."""
-    dev = torch.device(device or GPU)
-    if dev.index is None:
-        dev = torch.device("cuda", torch.cuda.current_device())
-    if dev.index not in _seed_words:
-        _seed_words[dev.index] = torch.zeros(1, dtype=torch.int64, device=dev)
-    return _seed_words[dev.index]
+    index = device.index if type(device) is torch.device else torch.device(device or GPU).index
+    if index is None:
+        index = torch.cuda.current_device()
+    word = _seed_words.get(index)
+    if word is None:
+        word = _seed_words[index] = torch.zeros(1, dtype=torch.int64, device=torch.device("cuda", index))
+    return word
 
 
 def set_seed(value, device=None):
