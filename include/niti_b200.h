@@ -91,7 +91,7 @@ NITI_API const char* niti_last_cuda_error(void);
  * niti_conv_fprop_i8: cutlassconv_cuda.sp_conv_optimized / sp_conv (cutlassconv.cpp:57-73,
  * cutlassconv_kernel.cu:38-319) as called from conv2d_int8 (ti_torch.py:178-192).
  * x [N][H][W][C], w [K][R][S][C] -> y32 [N][P][Q][K], cross-correlation, stride 1, P = H+2*pad-R+1.
- * Unlike the reference no channel padding to 16 is needed (C = 3 is accepted).  *maxabs = max |y32|.
+ * Unlike the reference no channel padding to 16 is needed (C = 3 is accepted).  *maxabs = max |y32| (may be null).
  * Kernel choice: implicit GEMM on the tensor cores when C % 16 == 0 (and R = S = 2*pad+1, K % 4 == 0);
  * R*S*C <= 32 (3-channel first layer) goes through a patch matrix in `scratch`
  * (niti_conv_fprop_scratch_bytes, 0 for the other paths; scratch may then be NULL) and the
@@ -174,6 +174,15 @@ typedef struct niti_wgrad_item {
 } niti_wgrad_item;
 NITI_API int niti_conv_wgrad_accumulate_multi_max(void);
 NITI_API int niti_conv_wgrad_accumulate_multi_i8(const niti_wgrad_item* items, int count, int32_t* status, void* stream);
+
+/* The weight gradient in the arrangement in which the reference's Python asks for it (ti_torch.py:429-432: the activations
+ * with the batch innermost as input, the errors likewise as image-sized filters of sp_conv, cutlassconv.cpp:57-73):
+ * x_t [C][H][W][N], err_t [K][H][W][N] -> out [C][R][S][K] int32,
+ * out[c][r][s][k] = sum_{n,h,w} err_t[k][h][w][n] * x_t[c][h+r-pad][w+s-pad][n].  Nothing is transposed on the way.
+ * R = S = 2*pad+1 <= 3, N % 16 == 0, K % 4 == 0 (niti_conv_wgrad_batch_inner_supported); pointers 16-byte aligned. */
+NITI_API int niti_conv_wgrad_batch_inner_supported(int N, int C, int K, int R, int S, int pad);
+NITI_API int niti_conv_wgrad_batch_inner_i8(const int8_t* x_t, const int8_t* err_t, int32_t* out, int N, int H, int W, int C, int K,
+                       int R, int S, int pad, int32_t* status, void* stream);
 
 /* niti_conv_wgrad_i8 for callers that cannot hand over scratch memory.  This entry point has no
  * counterpart in the reference.  Some hosts of this library are not able to call cudaMalloc at all:
@@ -274,7 +283,7 @@ NITI_API int niti_conv_fprop_requant_pool_i8(const int8_t* x, const int8_t* w, i
 /* int8mm_cuda.int8_mm (int8mm.cpp:9-18, int8mm_kernel.cu:8-34) as used by TiLinear
  * (ti_torch.py:241-266), without the padding / .contiguous() copies around it:
  * C32[M][N] = op(A) * op(B); trans_a == 0: A is [M][K], else [K][M];
- * trans_b == 0: B is [K][N], else [N][K].  Forward a*W^T: (0,1); error e*W: (0,0);
+ * trans_b == 0: B is [K][N], else [N][K].  *maxabs = max |C32| (may be null).  Forward a*W^T: (0,1); error e*W: (0,0);
  * gradient e^T*a: (1,0).  Tensor-core path when every row pitch is a multiple of 16 bytes,
  * M >= 64 and N, K >= 32; otherwise a CUDA-core path (the 10-class FC layer).
  */
@@ -325,6 +334,10 @@ NITI_API int niti_group_conv1_i8(const int8_t* in, const int8_t* wt, int32_t* ou
 NITI_API int niti_maxpool_fwd_i8(const int8_t* x, int8_t* y, int N, int H, int W, int C, int k, int stride, void* stream);
 NITI_API int niti_maxpool_bwd_i8(const int8_t* x, const int8_t* dy, int8_t* dx, int N, int H, int W, int C, int k, int stride,
                         int relu_mask, void* stream);
+/* niti_maxpool_bwd_i8 on the fp16 copies that the reference's Python passes to int8_pool_backward (ti_torch.py:309-316):
+ * x, dy, dx IEEE half as raw 16-bit words, every value an int8; 2x2 windows with stride 2, H and W even, C % 8 == 0,
+ * pointers 16-byte aligned, else NITI_ERR_UNSUPPORTED. */
+NITI_API int niti_maxpool_bwd_f16(const void* x, const void* dy, void* dx, int N, int H, int W, int C, int k, int stride, void* stream);
 /* TiReLU.forward / backward (ti_torch.py:268-290) */
 NITI_API int niti_relu_fwd_i8(const int8_t* x, int8_t* y, int64_t n, void* stream);
 NITI_API int niti_relu_bwd_i8(const int8_t* act, const int8_t* err, int8_t* out, int64_t n, void* stream);

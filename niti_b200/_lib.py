@@ -41,6 +41,8 @@ SIGNATURES = {
     "niti_conv_wgrad_i8": (_i, [_p, _p, _p, _p, _p, _sz] + [_i] * 8 + [_p, _p]),
     "niti_conv_wgrad_accumulate_multi_max": (_i, []),
     "niti_conv_wgrad_accumulate_multi_i8": (_i, [_p, _i, _p, _p]),
+    "niti_conv_wgrad_batch_inner_supported": (_i, [_i] * 6),
+    "niti_conv_wgrad_batch_inner_i8": (_i, [_p, _p, _p] + [_i] * 8 + [_p, _p]),
     "niti_conv_wgrad_patches_scratch_bytes": (_sz, [_i] * 7),
     "niti_conv_wgrad_patches_i8": (_i, [_p, _p, _p, _p, _p, _sz] + [_i] * 7 + [_p, _p]),
     "niti_conv_wgrad_builtin_scratch_i8": (_i, [_p, _p, _p, _p] + [_i] * 8 + [_p, _p]),
@@ -50,6 +52,7 @@ SIGNATURES = {
     "niti_group_conv1_i8": (_i, [_p, _p, _p] + [_i] * 7 + [_p]),
     "niti_maxpool_fwd_i8": (_i, [_p, _p] + [_i] * 6 + [_p]),
     "niti_maxpool_bwd_i8": (_i, [_p, _p, _p] + [_i] * 7 + [_p]),
+    "niti_maxpool_bwd_f16": (_i, [_p, _p, _p] + [_i] * 6 + [_p]),
     "niti_relu_fwd_i8": (_i, [_p, _p, _i64, _p]),
     "niti_relu_bwd_i8": (_i, [_p, _p, _p, _i64, _p]),
     "niti_dropout_i8": (_i, [_p, _p, _i64, _i64, _p, _u32, _p]),

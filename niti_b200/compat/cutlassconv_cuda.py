@@ -25,12 +25,14 @@ def _conv(input, weight, stride, padding):
     if R > 2 * padding + 1 and S > 2 * padding + 1 and P * Q <= 49 and C % 16 == 0 and K % 16 == 0 and N % 16 == 0:
         # weight gradient in disguise: input = activations [C,H,W,N], filters = errors [K,P',Q',N] of the layer's
         # output size; out[c,p,q,k] = sum_{n,h,w} x[n,h+p-pad,w+q-pad,c] * err[n,h,w,k] = dW[k,p,q,c]
+        if tuple(weight.shape[1:3]) == (H, W) and ops.conv_wgrad_batch_inner_supported(N, C, K, P, Q, padding):
+            return ops.conv_wgrad_batch_inner(input, weight, P, Q, padding)  # reads both operands as they lie
         x = input.permute(3, 1, 2, 0).contiguous()
         err = weight.permute(3, 1, 2, 0).contiguous()
         if err.shape[1] + 2 * padding - P + 1 == H and P == Q:
             g32, _ = ops.conv_wgrad_acc(x, err, P, Q, padding)
             return g32.permute(3, 1, 2, 0).contiguous()
-    return ops.conv_fprop_acc(input, weight, padding, stride)[0]
+    return ops.conv_fprop_acc(input, weight, padding, stride, want_max=False)[0]
 
 
 def sp_conv(input, weight, stride, padding):

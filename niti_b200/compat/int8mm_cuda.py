@@ -11,4 +11,4 @@ def int8_mm(lhs, rhs):
     check_input(lhs, rhs)
     if lhs.dtype != torch.int8 or rhs.dtype != torch.int8 or lhs.dim() != 2 or rhs.dim() != 2 or lhs.shape[1] != rhs.shape[0]:
         raise RuntimeError("int8_mm: int8 [m,k] and [k,n] matrices expected")
-    return ops.gemm_acc(lhs, rhs)[0]
+    return ops.gemm_acc(lhs, rhs, want_max=False)[0]

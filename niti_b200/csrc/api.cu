@@ -92,7 +92,8 @@ extern "C" int niti_peer_arena_destroy(void* ptr) {
     return set_cuda_error(cudaFree(ptr));
 }
 
-static int clear_word(uint32_t* p, cudaStream_t st) { return set_cuda_error(cudaMemsetAsync(p, 0, 4, st)); }
+// null: the caller does not want the maximum, and there is nothing to clear (a memset of its own costs 2 us of host time)
+static int clear_word(uint32_t* p, cudaStream_t st) { return p == nullptr ? NITI_OK : set_cuda_error(cudaMemsetAsync(p, 0, 4, st)); }
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -125,7 +126,7 @@ extern "C" size_t niti_conv_fprop_scratch_bytes(int N, int H, int W, int C, int 
 extern "C" int niti_conv_fprop_i8(const int8_t* x, const int8_t* w, int32_t* y32, uint32_t* maxabs, void* scratch,
                                   size_t scratch_bytes, int N, int H, int W, int C, int K, int R, int S, int pad, int stride,
                                   int32_t* status, void* stream) {
-    NITI_REQUIRE(x && w && y32 && maxabs && N > 0 && H > 0 && W > 0 && C > 0 && K > 0 && R > 0 && S > 0 && pad >= 0);
+    NITI_REQUIRE(x && w && y32 && N > 0 && H > 0 && W > 0 && C > 0 && K > 0 && R > 0 && S > 0 && pad >= 0);
     if (stride != 1) return NITI_ERR_UNSUPPORTED;
     if (H + 2 * pad - R + 1 <= 0 || W + 2 * pad - S + 1 <= 0) return NITI_ERR_BAD_ARG;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -226,6 +227,19 @@ extern "C" int niti_conv_wgrad_i8(const int8_t* x, const int8_t* err, int32_t* g
     return reduce_rows32(partial, splits, K, R * S * C, g32, maxabs, st);
 }
 
+extern "C" int niti_conv_wgrad_batch_inner_supported(int N, int C, int K, int R, int S, int pad) {
+    return same_padding(R, S, pad) && S <= 3 && N % 16 == 0 && K % 4 == 0 ? 1 : 0;
+}
+extern "C" int niti_conv_wgrad_batch_inner_i8(const int8_t* x_t, const int8_t* err_t, int32_t* out, int N, int H, int W, int C, int K,
+                                              int R, int S, int pad, int32_t* status, void* stream) {
+    NITI_REQUIRE(x_t && err_t && out && N > 0 && H > 0 && W > 0 && C > 0 && K > 0 && R > 0 && S > 0 && pad >= 0);
+    NITI_REQUIRE(aligned16(x_t) && aligned16(err_t) && aligned16(out));
+    if (!niti_conv_wgrad_batch_inner_supported(N, C, K, R, S, pad)) return NITI_ERR_UNSUPPORTED;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (int e = set_cuda_error(cudaMemsetAsync(out, 0, static_cast<size_t>(C) * R * S * K * 4, st))) return e;
+    return umma_conv_wgrad_batch_inner(x_t, err_t, out, N, H, W, C, K, R, S, pad, status, st);
+}
+
 extern "C" size_t niti_conv_wgrad_patches_scratch_bytes(int N, int H, int W, int C, int K, int R, int S) {
     if (N <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0 || R <= 0 || S <= 0) return 0;
     if (wgrad_path(C, K, R, S, (R - 1) / 2) != CONV_THIN) return 0;
@@ -281,7 +295,7 @@ extern "C" int niti_conv_wgrad_accumulate_multi_i8(const niti_wgrad_item* items,
 
 extern "C" int niti_gemm_i8(const int8_t* A, const int8_t* B, int32_t* C32, uint32_t* maxabs, int M, int N, int K,
                             int trans_a, int trans_b, int32_t* status, void* stream) {
-    NITI_REQUIRE(A && B && C32 && maxabs && M > 0 && N > 0 && K > 0);
+    NITI_REQUIRE(A && B && C32 && M > 0 && N > 0 && K > 0);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int e = clear_word(maxabs, st)) return e;
     const int pitch_a = trans_a ? M : K, pitch_b = trans_b ? K : N;

@@ -45,6 +45,9 @@ size_t umma_wgrad_scratch_bytes(int Nimg, int H, int W, int C, int K, int R, int
 int umma_conv_wgrad_partials(const int8_t* x, const int8_t* err, int32_t* partial, int* splits_out, int max_splits,
                              int Nimg, int H, int W, int C, int K, int R, int S, int pad, int32_t* status, cudaStream_t st,
                              int direct = 0);
+// operands with the batch innermost ([channels][H][W][N]) -> out [C][R][S][K] (zeroed by the caller)
+int umma_conv_wgrad_batch_inner(const int8_t* x_t, const int8_t* err_t, int32_t* out, int Nimg, int H, int W, int C, int K, int R,
+                                int S, int pad, int32_t* status, cudaStream_t st);
 // several layers' weight gradients, each ADDED into its g32, in one launch (umma_kernels.cu)
 struct WgradJob { const int8_t* x; const int8_t* err; int32_t* g32; int N, H, W, C, K, R, S, pad; };
 int umma_wgrad_multi_max();

@@ -3,6 +3,7 @@
 // fill a tensor-core tile (3-channel first convolution, 10-class FC layer).
 // All of them are bandwidth- or latency-bound: 16-byte accesses along the channel axis, packed
 // byte SIMD (__vmaxs4, __vcmpeq4, __dp4a), warp shuffles for reductions, one atomic per warp.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -306,6 +307,38 @@ maxpool2_bwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, u
         route4(a.z, b.z, d.z, e.z, g.z, relu_mask, oa.z, ob.z, od.z, oe.z);
         route4(a.w, b.w, d.w, e.w, g.w, relu_mask, oa.w, ob.w, od.w, oe.w);
         dx[base] = oa; dx[base + C16] = ob; dx[base + row] = od; dx[base + row + C16] = oe;
+    }
+}
+
+// The same routing on fp16 copies of the int8 tensors (what the reference's Python hands to its pooling backward): eight
+// channels per 16-byte access, two per 32-bit word.  Bound by memory: 2 x 2.25 X bytes for a tensor of X values; narrowing
+// to int8 and widening again in passes of their own moved that three times (50 us against 7 us at 128 x 16 x 16 x 256).
+__device__ __forceinline__ void route2h(unsigned a, unsigned b, unsigned d, unsigned e, unsigned dy, unsigned& oa, unsigned& ob,
+                                        unsigned& od, unsigned& oe) {
+    auto h2 = [](unsigned v) { return *reinterpret_cast<const __half2*>(&v); };
+    const __half2 m = __hmax2(__hmax2(h2(a), h2(b)), __hmax2(h2(d), h2(e)));
+    const unsigned ha = __heq2_mask(h2(a), m), hb = __heq2_mask(h2(b), m) & ~ha, hd = __heq2_mask(h2(d), m) & ~(ha | hb);
+    oa = dy & ha; ob = dy & hb; od = dy & hd; oe = dy & ~(ha | hb | hd);
+}
+__global__ void __launch_bounds__(256)
+maxpool2_bwd_f16_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4* __restrict__ dx, int Nimg, int H, int W,
+                        int C8, int P, int Q) {
+    const long long total = static_cast<long long>(Nimg) * P * Q * C8;
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
+         i += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const long long px = i / C8;
+        const int c = static_cast<int>(i - px * C8);
+        const long long row_of = px / Q;
+        const int q = static_cast<int>(px - row_of * Q), p = static_cast<int>(row_of % P);
+        const long long n = row_of / P;
+        const long long row = static_cast<long long>(W) * C8, base = ((n * H + 2 * p) * W + 2 * q) * C8 + c;
+        const uint4 a = __ldg(x + base), b = __ldg(x + base + C8), d = __ldg(x + base + row), e = __ldg(x + base + row + C8), g = __ldg(dy + i);
+        uint4 oa, ob, od, oe;
+        route2h(a.x, b.x, d.x, e.x, g.x, oa.x, ob.x, od.x, oe.x);
+        route2h(a.y, b.y, d.y, e.y, g.y, oa.y, ob.y, od.y, oe.y);
+        route2h(a.z, b.z, d.z, e.z, g.z, oa.z, ob.z, od.z, oe.z);
+        route2h(a.w, b.w, d.w, e.w, g.w, oa.w, ob.w, od.w, oe.w);
+        dx[base] = oa; dx[base + C8] = ob; dx[base + row] = od; dx[base + row + C8] = oe;
     }
 }
 
@@ -1069,11 +1102,88 @@ gemm_bn4_kernel(const int8_t* __restrict__ A, const int8_t* __restrict__ B, int3
     }
     warp_atomic_max(maxabs, mx);
 }
+// GEMM with B stored [K][N] and at most 16 columns (N % 4 == 0), A [M][K]: the reference's classifier forward product,
+// int8_mm(activations, W^T contiguous), with N = 10 classes padded to 12 and K = thousands of features.
+// A block owns RB rows and all columns; a thread takes four consecutive reduction indices at a time: their 4 N bytes of B
+// are N / 4 16-byte loads, twelve byte permutes per four columns turn them into __dp4a operands that all RB rows share.
+// Bound by latency (a block per SM and L2-resident operands): K / 4 / 256 loads per thread, then one integer warp
+// reduction per output.  128 x 12 x 16384: 1090 us with one thread per four outputs walking K serially, 5 us like this.
+template <int NW, int RB>
+__global__ void __launch_bounds__(256)
+gemm_thin_kernel(const int8_t* __restrict__ A, const int8_t* __restrict__ B, int32_t* __restrict__ C32, unsigned* maxabs, int M, int K) {
+    constexpr int N = 4 * NW;
+    __shared__ int part[8][RB * N];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long m0 = static_cast<long long>(blockIdx.x) * RB;
+    int acc[RB][N];
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc[r][n] = 0;
+    const uint4* B4 = reinterpret_cast<const uint4*>(B);
+#pragma unroll 2
+    for (int g = threadIdx.x; g < (K >> 2); g += 256) {
+        uint32_t b[4 * NW];  // [k of the group][word of the row]
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            const uint4 v = __ldg(B4 + static_cast<long long>(g) * NW + i);
+            b[4 * i] = v.x; b[4 * i + 1] = v.y; b[4 * i + 2] = v.z; b[4 * i + 3] = v.w;
+        }
+        uint32_t a[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            a[r] = m0 + r < M ? __ldg(reinterpret_cast<const uint32_t*>(A + (m0 + r) * K) + g) : 0u;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const uint32_t x0 = b[w], x1 = b[NW + w], x2 = b[2 * NW + w], x3 = b[3 * NW + w];
+            const uint32_t lo01 = __byte_perm(x0, x1, 0x5140), hi01 = __byte_perm(x0, x1, 0x7362);  // columns 0,1 / 2,3 of k = 0, 1
+            const uint32_t lo23 = __byte_perm(x2, x3, 0x5140), hi23 = __byte_perm(x2, x3, 0x7362);
+            const uint32_t c[4] = {__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632),
+                                   __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632)};
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[r][4 * w + j] = __dp4a(static_cast<int>(a[r]), static_cast<int>(c[j]), acc[r][4 * w + j]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const int v = __reduce_add_sync(0xFFFFFFFFu, acc[r][n]);
+            if (lane == 0) part[warp][r * N + n] = v;
+        }
+    __syncthreads();
+    unsigned mx = 0;
+    if (static_cast<int>(threadIdx.x) < RB * N && m0 + threadIdx.x / N < M) {
+        int v = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += part[w][threadIdx.x];
+        for (int k = K & ~3; k < K; ++k)  // up to three reduction indices beyond the last group of four
+            v += static_cast<int>(A[(m0 + threadIdx.x / N) * K + k]) * static_cast<int>(B[static_cast<long long>(k) * N + threadIdx.x % N]);
+        C32[m0 * N + threadIdx.x] = v;
+        mx = iabs_u(v);
+    }
+    if (maxabs != nullptr) block_atomic_max(maxabs, mx);
+}
+template <int NW>
+static void launch_gemm_thin(const int8_t* A, const int8_t* B, int32_t* C32, unsigned* maxabs, int M, int K, cudaStream_t st) {
+    // one row per block while that does not exceed two waves of blocks (latency), else four rows share the B operand
+    if (M <= 2 * sm_count_simt()) gemm_thin_kernel<NW, 1><<<M, 256, 0, st>>>(A, B, C32, maxabs, M, K);
+    else gemm_thin_kernel<NW, 4><<<(M + 3) / 4, 256, 0, st>>>(A, B, C32, maxabs, M, K);
+}
 int simt_gemm(const int8_t* A, const int8_t* B, int32_t* C32, unsigned* maxabs, int M, int N, int K, int trans_a,
               int trans_b, cudaStream_t st) {
     const long long outs = static_cast<long long>(M) * N;
     if (!trans_a && trans_b && K >= 256)
         gemm_kk_kernel<<<blocks_for(outs * 32, 256, sm_count_simt() * 16), 256, 0, st>>>(A, B, C32, maxabs, M, N, K);
+    else if (!trans_a && !trans_b && N % 4 == 0 && N <= 16 && K >= 256 && (K % 4 == 0 || M == 1) && reinterpret_cast<uintptr_t>(A) % 4 == 0 &&
+             reinterpret_cast<uintptr_t>(B) % 16 == 0) {
+        if (N == 4) launch_gemm_thin<1>(A, B, C32, maxabs, M, K, st);
+        else if (N == 8) launch_gemm_thin<2>(A, B, C32, maxabs, M, K, st);
+        else if (N == 12) launch_gemm_thin<3>(A, B, C32, maxabs, M, K, st);
+        else launch_gemm_thin<4>(A, B, C32, maxabs, M, K, st);
+    }
     else if (!trans_b && N % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 4 == 0 && reinterpret_cast<uintptr_t>(C32) % 16 == 0)
         gemm_bn4_kernel<<<blocks_for(outs / 4, 128, sm_count_simt() * 32), 128, 0, st>>>(A, B, C32, maxabs, M, N, K, trans_a);
     else
@@ -1195,6 +1305,16 @@ extern "C" int niti_maxpool_bwd_i8(const int8_t* x, const int8_t* dy, int8_t* dx
         const long long total = static_cast<long long>(N) * H * W * C;
         maxpool_bwd_generic<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, st>>>(x, dy, dx, N, H, W, C, k, stride, P, Q, relu_mask);
     }
+    return set_cuda_error(cudaGetLastError());
+}
+
+extern "C" int niti_maxpool_bwd_f16(const void* x, const void* dy, void* dx, int N, int H, int W, int C, int k, int stride, void* stream) {
+    NITI_REQUIRE(x && dy && dx && N > 0 && H >= k && W >= k && C > 0 && k > 0 && stride > 0);
+    const bool al = (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) % 16 == 0;
+    if (!(k == 2 && stride == 2 && C % 8 == 0 && H % 2 == 0 && W % 2 == 0 && al)) return NITI_ERR_UNSUPPORTED;
+    const long long total = static_cast<long long>(N) * (H / 2) * (W / 2) * (C / 8);
+    maxpool2_bwd_f16_kernel<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<uint4*>(dx), N, H, W, C / 8, H / 2, W / 2);
     return set_cuda_error(cudaGetLastError());
 }
 

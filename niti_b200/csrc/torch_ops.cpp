@@ -197,6 +197,7 @@ PyObject* conv_dgrad_side_bytes(Args& a) {
 PyObject* conv_fprop_acc(Args& a) {
     const Tensor &x = a.tensor(), &w = a.tensor();
     const int pad = a.i32(), stride = a.i32();
+    const bool want_max = a.flag();
     need_cuda({&x, &w});
     const Conv s = conv_shape(x, w);
     require(w.size(3) == s.C && x.scalar_type() == at::kChar && w.scalar_type() == at::kChar);
@@ -204,10 +205,10 @@ PyObject* conv_fprop_acc(Args& a) {
     {
         Launch l(x);
         y32 = l.empty({s.N, s.H + 2 * pad - s.R + 1, s.W + 2 * pad - s.S + 1, s.K}, at::kInt);
-        mx = l.empty({1}, at::kInt);
+        if (want_max) mx = l.empty({1}, at::kInt);
         const size_t nb = niti_conv_fprop_scratch_bytes(s.N, s.H, s.W, s.C, s.K, s.R, s.S);
         if (nb) sc = l.bytes(nb);
-        check(niti_conv_fprop_i8(cptr<int8_t>(x), cptr<int8_t>(w), mptr<int32_t>(y32), mptr<uint32_t>(mx), nb ? mptr(sc) : nullptr, nb,
+        check(niti_conv_fprop_i8(cptr<int8_t>(x), cptr<int8_t>(w), mptr<int32_t>(y32), want_max ? mptr<uint32_t>(mx) : nullptr, nb ? mptr(sc) : nullptr, nb,
                                  s.N, s.H, s.W, s.C, s.K, s.R, s.S, pad, stride, l.status(), l.stream), "niti_conv_fprop_i8");
     }
     return tuple(y32, mx);
@@ -334,6 +335,26 @@ PyObject* conv_wgrad_acc(Args& a) {
     return tuple(g32, mx);
 }
 
+PyObject* conv_wgrad_batch_inner_supported(Args& a) {
+    const auto v = ints<6>(a);
+    return PyBool_FromLong(niti_conv_wgrad_batch_inner_supported(v[0], v[1], v[2], v[3], v[4], v[5]));
+}
+PyObject* conv_wgrad_batch_inner(Args& a) {
+    const Tensor &x = a.tensor(), &err = a.tensor();
+    const int R = a.i32(), S = a.i32(), pad = a.i32();
+    need_cuda({&x, &err});
+    require(x.dim() == 4 && err.dim() == 4 && x.size(1) == err.size(1) && x.size(2) == err.size(2) && x.size(3) == err.size(3));
+    const int C = x.size(0), H = x.size(1), W = x.size(2), N = x.size(3), K = err.size(0);
+    Tensor out;
+    {
+        Launch l(x);
+        out = l.empty({C, R, S, K}, at::kInt);
+        check(niti_conv_wgrad_batch_inner_i8(cptr<int8_t>(x), cptr<int8_t>(err), mptr<int32_t>(out), N, H, W, C, K, R, S, pad, l.status(),
+                                             l.stream), "niti_conv_wgrad_batch_inner_i8");
+    }
+    return wrap(out);
+}
+
 PyObject* conv_wgrad_from_patches(Args& a) {
     const Tensor &patches = a.tensor(), &err = a.tensor();
     const int C = a.i32(), R = a.i32(), S = a.i32();
@@ -374,6 +395,7 @@ PyObject* gemm_acc(Args& a) {
     const Tensor &A = a.tensor(), &B = a.tensor();
     const bool ta = a.flag(), tb = a.flag();
     const Tensor* out = a.maybe();
+    const bool want_max = a.flag();
     need_cuda({&A, &B, out});
     require(A.dim() == 2 && B.dim() == 2);
     const int M = A.size(ta ? 1 : 0), K = A.size(ta ? 0 : 1), N = B.size(tb ? 0 : 1);
@@ -382,8 +404,8 @@ PyObject* gemm_acc(Args& a) {
     {
         Launch l(A);
         c32 = out ? *out : l.empty({M, N}, at::kInt);
-        mx = l.empty({1}, at::kInt);
-        check(niti_gemm_i8(cptr<int8_t>(A), cptr<int8_t>(B), mptr<int32_t>(c32), mptr<uint32_t>(mx), M, N, K, ta, tb, l.status(), l.stream),
+        if (want_max) mx = l.empty({1}, at::kInt);
+        check(niti_gemm_i8(cptr<int8_t>(A), cptr<int8_t>(B), mptr<int32_t>(c32), want_max ? mptr<uint32_t>(mx) : nullptr, M, N, K, ta, tb, l.status(), l.stream),
               "niti_gemm_i8");
     }
     return tuple(c32, mx);
@@ -450,6 +472,20 @@ PyObject* maxpool_bwd(Args& a) {
         Launch l(x);
         dx = l.empty(x.sizes(), x.scalar_type());
         check(niti_maxpool_bwd_i8(cptr<int8_t>(x), cptr<int8_t>(dy), mptr<int8_t>(dx), N, H, W, C, k, stride, mask, l.stream), "niti_maxpool_bwd_i8");
+    }
+    return wrap(dx);
+}
+PyObject* maxpool_bwd_f16(Args& a) {
+    const Tensor &x = a.tensor(), &dy = a.tensor();
+    const int k = a.i32(), stride = a.i32();
+    need_cuda({&x, &dy});
+    require(x.dim() == 4 && x.scalar_type() == at::kHalf && dy.scalar_type() == at::kHalf);
+    const int N = x.size(0), H = x.size(1), W = x.size(2), C = x.size(3);
+    Tensor dx;
+    {
+        Launch l(x);
+        dx = l.empty(x.sizes(), at::kHalf);
+        check(niti_maxpool_bwd_f16(cptr(x), cptr(dy), mptr(dx), N, H, W, C, k, stride, l.stream), "niti_maxpool_bwd_f16");
     }
     return wrap(dx);
 }
@@ -540,6 +576,7 @@ PyMethodDef methods[] = {
     NITI_ENTRY(conv_fprop_scratch_bytes), NITI_ENTRY(conv_dgrad_side_bytes),
     NITI_ENTRY(conv_fprop_acc), NITI_ENTRY(conv_fprop_fused),
     NITI_ENTRY(conv_fprop_pool_fused), NITI_ENTRY(conv_dgrad_fused), NITI_ENTRY(conv_dgrad_acc), NITI_ENTRY(conv_wgrad_acc),
+    NITI_ENTRY(conv_wgrad_batch_inner_supported), NITI_ENTRY(conv_wgrad_batch_inner), NITI_ENTRY(maxpool_bwd_f16),
     NITI_ENTRY(conv_wgrad_from_patches), NITI_ENTRY(conv_wgrad_accumulate), NITI_ENTRY(gemm_acc), NITI_ENTRY(requant),
     NITI_ENTRY(absmax), NITI_ENTRY(maxpool_fwd), NITI_ENTRY(maxpool_bwd), NITI_ENTRY(relu_fwd), NITI_ENTRY(relu_bwd),
     NITI_ENTRY(dropout), NITI_ENTRY(loss_err), NITI_ENTRY(update), NITI_ENTRY(quantize_input),

@@ -1248,6 +1248,11 @@ namespace niti {
 // 128 c-channels x the same pixels).  One CTA owns (128 k) x (128 c) x (one filter row r, all S
 // taps) and a contiguous range of pixel chunks; its S accumulators live in TMEM side by side.
 // Partial sums are written to scratch[split] and folded by wgrad_reduce_kernel.
+//
+// KMAJ: the same contraction of operands that hold the batch innermost, [channels][H][W][N] (the arrangement in which the
+// reference writes a weight gradient as a convolution with image-sized filters): both operands are then K-major as they
+// lie, a chunk is one pixel x 128 images, and nothing has to be transposed.  Turning the two 8.4 MB tensors of a
+// 128 x 16 x 16 x 256 layer round first cost 72 us, more than three times the contraction itself.
 // ------------------------------------------------------------------------------------------------
 struct WgradParams {
     int H, W, C, K, R, S, pad, Nimg;
@@ -1260,6 +1265,7 @@ struct WgradParams {
     int32_t* partial;      // [splits][K*R*S*C]
     int32_t* status;
     int reduce_direct;     // 1: every CTA adds its tiles straight into the (zeroed) gradient with TMA reductions
+    int flip;              // KMAJ: 1 = the column operand is read at pixel - (tap - pad) instead of pixel + (tap - pad)
 };
 
 constexpr int WG_MAX_S = 3;
@@ -1270,6 +1276,7 @@ constexpr int WG_TMEM_COLS = 512;
 
 // One CTA's share of one layer's weight gradient: work item `item` (filter row, k tile, c tile) over the pixel chunks of
 // split `split`.  The tensor maps live in kernel parameter space (grid constants of the calling kernel).
+template <bool KMAJ>
 __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUtensorMap& tmX, const CUtensorMap& tmP,
                                            const WgradParams& p, const int split, const int item, const bool probe_cta) {
     if (threadIdx.x == 0 && probe_cta) PARK_STAMP(10);
@@ -1320,6 +1327,7 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUten
     const int S = keep_reg(p.S);
     if (warp == 0) {
         {
+            const int flip = KMAJ ? keep_reg(p.flip) : 0;
             const int pad = keep_reg(p.pad), BW = keep_reg(p.BW), BH = keep_reg(p.BH), BI = keep_reg(p.BI);
             const int tiles_w = keep_reg(p.tiles_w), tiles_h = keep_reg(p.tiles_h);
             const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg((1 + p.S) * p.box_bytes));
@@ -1332,9 +1340,16 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUten
                 const uint32_t sa = smem0 + static_cast<uint32_t>(s) * WG_STAGE_BYTES;
                 if (elect_one()) {
                     mbar_arrive_expect_tx(fb, tx_bytes);
-                    tma_load_4d(sa, &tmErr, fb, kt * 128, tw * BW, th * BH, tn * BI);
-                    for (int sx = 0; sx < S; ++sx)
-                        tma_load_4d(sa + (1 + sx) * PANEL_BYTES, &tmX, fb, ct * 128, tw * BW + sx - pad, th * BH + r - pad, tn * BI);
+                    if (KMAJ) {
+                        tma_load_4d(sa, &tmErr, fb, tn * 128, tw, th, kt * 128);
+                        const int y = flip ? th + pad - r : th + r - pad;
+                        for (int sx = 0; sx < S; ++sx)
+                            tma_load_4d(sa + (1 + sx) * PANEL_BYTES, &tmX, fb, tn * 128, flip ? tw + pad - sx : tw + sx - pad, y, ct * 128);
+                    } else {
+                        tma_load_4d(sa, &tmErr, fb, kt * 128, tw * BW, th * BH, tn * BI);
+                        for (int sx = 0; sx < S; ++sx)
+                            tma_load_4d(sa + (1 + sx) * PANEL_BYTES, &tmX, fb, ct * 128, tw * BW + sx - pad, th * BH + r - pad, tn * BI);
+                    }
                 }
                 if (++s == WG_STAGES) { s = 0; ph ^= 1u; }
                 if (++tw == tiles_w) { tw = 0; if (++th == tiles_h) { th = 0; ++tn; } }
@@ -1343,12 +1358,15 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUten
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         {
-            const uint32_t idesc = make_idesc_i8(BLOCK_M, 128, 1, 1);
-            const uint32_t idesc2 = make_idesc_i8(BLOCK_M, 256, 1, 1);
+            constexpr int MN = KMAJ ? 0 : 1;
+            const uint32_t idesc = make_idesc_i8(BLOCK_M, 128, MN, MN);
+            const uint32_t idesc2 = make_idesc_i8(BLOCK_M, 256, MN, MN);
             const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
             const int nmma = keep_reg(p.mma_per_chunk);
-            const uint64_t kstep = (32u * ROW_BYTES) >> 4;  // 32 reduction rows per MMA, in descriptor units
-            const uint64_t d0 = make_smem_desc(smem0, PANEL_BYTES, 1024, SWIZZLE_128B_CODE);
+            // 32 reduction rows (KMAJ: 32 bytes) per MMA, in descriptor units.  Adjacent panels are one operand of 256
+            // columns in either major: 128-column panels one leading offset apart, or simply 256 rows.
+            const uint64_t kstep = (KMAJ ? 32u : 32u * ROW_BYTES) >> 4;
+            const uint64_t d0 = make_smem_desc(smem0, KMAJ ? 16 : PANEL_BYTES, 1024, SWIZZLE_128B_CODE);
             int s = 0; uint32_t ph = 0; bool ok = true;
             bool ready = false;  // the stage's "full" phase was seen complete by the previous chunk's probe
             for (int ch = chunk_lo; ch < chunk_hi; ++ch) {
@@ -1441,7 +1459,12 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUten
 __global__ void __launch_bounds__(UMMA_THREADS, 1)
 umma_wgrad_kernel(const __grid_constant__ CUtensorMap tmErr, const __grid_constant__ CUtensorMap tmX,
                   const __grid_constant__ CUtensorMap tmP, const __grid_constant__ WgradParams p) {
-    wgrad_body(tmErr, tmX, tmP, p, blockIdx.x, blockIdx.y, blockIdx.y == 0);
+    wgrad_body<false>(tmErr, tmX, tmP, p, blockIdx.x, blockIdx.y, blockIdx.y == 0);
+}
+__global__ void __launch_bounds__(UMMA_THREADS, 1)
+umma_wgrad_kmajor_kernel(const __grid_constant__ CUtensorMap tmErr, const __grid_constant__ CUtensorMap tmX,
+                         const __grid_constant__ CUtensorMap tmP, const __grid_constant__ WgradParams p) {
+    wgrad_body<true>(tmErr, tmX, tmP, p, blockIdx.x, blockIdx.y, blockIdx.y == 0);
 }
 
 // Several layers' weight gradients in ONE launch: CTAs [first_cta[l], first_cta[l + 1]) belong to layer l, split-major
@@ -1457,7 +1480,7 @@ umma_wgrad_multi_kernel(const __grid_constant__ WgradMultiMaps maps, const __gri
     while (l + 1 < mp.count && static_cast<int>(blockIdx.x) >= mp.first_cta[l + 1]) ++l;
     const int local = static_cast<int>(blockIdx.x) - mp.first_cta[l];
     const WgradParams& p = mp.layer[l];
-    wgrad_body(maps.err[l], maps.x[l], maps.g[l], p, local % p.splits, local / p.splits, blockIdx.x == 0);
+    wgrad_body<false>(maps.err[l], maps.x[l], maps.g[l], p, local % p.splits, local / p.splits, blockIdx.x == 0);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1800,6 +1823,40 @@ int umma_conv_wgrad_partials(const int8_t* x, const int8_t* err, int32_t* partia
     if (e != cudaSuccess) return set_cuda_error(e);
     dim3 grid(p.splits, R * p.k_tiles * p.c_tiles);
     umma_wgrad_kernel<<<grid, UMMA_THREADS, WG_SMEM_BYTES, st>>>(me, mx, mp, p);
+    return set_cuda_error(cudaGetLastError());
+}
+
+// x_t [C][H][W][N], err_t [K][H][W][N] (batch innermost, N a multiple of 16) -> out [C][R][S][K], zeroed by the caller:
+// out[c][r][s][k] = sum err_t[k][pixel] * x_t[c][pixel + (r, s) - pad].  x's channels are the rows of the product, so that
+// the result needs no transposition either; the taps move the error instead, the other way.
+int umma_conv_wgrad_batch_inner(const int8_t* x_t, const int8_t* err_t, int32_t* out, int Nimg, int H, int W, int C, int K, int R,
+                                int S, int pad, int32_t* status, cudaStream_t st) {
+    WgradParams p{};
+    p.BW = p.BH = 1; p.BI = 128;
+    p.tiles_w = W; p.tiles_h = H; p.tiles_n = (Nimg + 127) / 128;
+    p.chunks = p.tiles_w * p.tiles_h * p.tiles_n;
+    p.k_tiles = (C + 127) / 128; p.c_tiles = (K + 127) / 128;
+    p.splits = sm_count() / (R * p.k_tiles * p.c_tiles);
+    if (p.splits < 1) p.splits = 1;
+    if (p.splits > p.chunks) p.splits = p.chunks;
+    p.reduce_direct = 1; p.flip = 1;
+    p.H = H; p.W = W; p.C = K; p.K = C; p.R = R; p.S = S; p.pad = pad; p.Nimg = Nimg;
+    p.box_bytes = PANEL_BYTES;  // a box is always written whole; images beyond the batch are zero fill
+    p.mma_per_chunk = Nimg < 128 ? (Nimg + 31) / 32 : 4;
+    p.partial = out; p.status = status;
+    CUtensorMap ma, mb, mc;
+    const uint32_t box[4] = {128, 1, 1, 128};
+    const uint64_t str[3] = {(uint64_t)Nimg, (uint64_t)W * Nimg, (uint64_t)H * W * Nimg};
+    const uint64_t da[4] = {(uint64_t)Nimg, (uint64_t)W, (uint64_t)H, (uint64_t)C}, db[4] = {(uint64_t)Nimg, (uint64_t)W, (uint64_t)H, (uint64_t)K};
+    if (int e = encode_map(&ma, x_t, false, 4, da, str, box)) return e;
+    if (int e = encode_map(&mb, err_t, false, 4, db, str, box)) return e;
+    const uint64_t dc[4] = {(uint64_t)K, (uint64_t)R * S, (uint64_t)C, 1};
+    const uint64_t sc[3] = {(uint64_t)K * 4, (uint64_t)R * S * K * 4, (uint64_t)C * R * S * K * 4};
+    const uint32_t bc[4] = {32, 1, 128, 1};
+    if (int e = encode_map(&mc, out, true, 4, dc, sc, bc)) return e;
+    cudaError_t e = cudaFuncSetAttribute(umma_wgrad_kmajor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM_BYTES);
+    if (e != cudaSuccess) return set_cuda_error(e);
+    umma_wgrad_kmajor_kernel<<<dim3(p.splits, R * p.k_tiles * p.c_tiles), UMMA_THREADS, WG_SMEM_BYTES, st>>>(ma, mb, mc, p);
     return set_cuda_error(cudaGetLastError());
 }
 

@@ -94,10 +94,10 @@ def seed_tensor(value, device):
 
 
 # ------------------------------------------------------------------ contractions
-def conv_fprop_acc(x, w, pad=1, stride=1):
+def conv_fprop_acc(x, w, pad=1, stride=1, want_max=True):
     def work(r):
         return 2 * r[0].numel() * w[0].numel(), x.numel() + w.numel() + 4 * r[0].numel()
-    return _run("niti_conv_fprop_i8", 2 if w.numel() <= 32 * w.shape[0] else 1, work, native.conv_fprop_acc, x, w, pad, stride)
+    return _run("niti_conv_fprop_i8", 2 if w.numel() <= 32 * w.shape[0] else 1, work, native.conv_fprop_acc, x, w, pad, stride, want_max)
 
 
 def conv_fprop_i4(x4, w4, pad=1):
@@ -217,6 +217,17 @@ def conv_wgrad_acc(x, err, R=3, S=3, pad=1, out=None, want_max=True):
     return _run("niti_conv_wgrad_i8", 2, work, native.conv_wgrad_acc, x, err, R, S, pad, out, want_max)
 
 
+def conv_wgrad_batch_inner_supported(N, C, K, R, S, pad):
+    return native.conv_wgrad_batch_inner_supported(N, C, K, R, S, pad)
+
+
+def conv_wgrad_batch_inner(x_t, err_t, R=3, S=3, pad=1):
+    """Weight gradient of operands with the batch innermost, x_t [C,H,W,N] and err_t [K,H,W,N], as int32 [C,R,S,K]."""
+    def work(r):
+        return 2 * x_t.numel() * R * S * err_t.shape[0], x_t.numel() + err_t.numel() + 4 * r.numel()
+    return _run("niti_conv_wgrad_batch_inner_i8", 1, work, native.conv_wgrad_batch_inner, x_t, err_t, R, S, pad)
+
+
 def conv_wgrad_from_patches(patches, err, C, R=3, S=3, out=None, want_max=True):
     """Weight gradient of a thin layer (R*S*C <= 32) from the patch matrix its forward call left in `patches` (see
     conv_fprop_fused(scratch_buf=...)): same result as conv_wgrad_acc on the layer's input, without gathering again."""
@@ -258,11 +269,11 @@ def conv_wgrad_accumulate_multi(jobs):
           _p(status_word(dev)), _st())
 
 
-def gemm_acc(a, b, trans_a=False, trans_b=False, out=None):
+def gemm_acc(a, b, trans_a=False, trans_b=False, out=None, want_max=True):
     """C32[M,N] = op(a) @ op(b); a is [M,K] ([K,M] if trans_a), b is [K,N] ([N,K] if trans_b)."""
     def work(r):
         return 2 * r[0].numel() * a.shape[0 if trans_a else 1], a.numel() + b.numel() + 4 * r[0].numel()
-    return _run("niti_gemm_i8", 1, work, native.gemm_acc, a, b, trans_a, trans_b, out)
+    return _run("niti_gemm_i8", 1, work, native.gemm_acc, a, b, trans_a, trans_b, out, want_max)
 
 
 def group_conv1(inp, wt, pad):
@@ -307,6 +318,13 @@ def maxpool_bwd(x, dy, k=2, stride=2, relu_mask=False):
     def work(dx):
         return 0, 2 * x.numel() + dy.numel()
     return _run("niti_maxpool_bwd_i8", 1, work, native.maxpool_bwd, x, dy, k, stride, relu_mask)
+
+
+def maxpool_bwd_f16(x, dy, k=2, stride=2):
+    """maxpool_bwd on fp16 copies of int8 tensors (2x2 windows, even maps, channels in multiples of 8)."""
+    def work(dx):
+        return 0, 2 * (2 * x.numel() + dy.numel())
+    return _run("niti_maxpool_bwd_f16", 1, work, native.maxpool_bwd_f16, x, dy, k, stride)
 
 
 def relu_fwd(x):
