@@ -52,6 +52,7 @@ constexpr int ROW_BYTES = 128;               // bytes per shared-memory row of a
 constexpr int PANEL_BYTES = 128 * ROW_BYTES; // one 128-row operand panel
 constexpr int UMMA_THREADS = 192;
 constexpr uint32_t SWIZZLE_128B_CODE = 2;
+constexpr uint32_t SWIZZLE_64B_CODE = 4;
 constexpr int EPI_CHUNK_BYTES = 128 * 32 * 4;  // 128 rows x 32 int32 columns, one TMA store box
 constexpr int EPI_BARRIER = 1;                 // named barrier of the 128 epilogue threads
 
@@ -126,12 +127,11 @@ struct GemmParams {
 constexpr int GEMM_THREADS = 320;  // producer warp, MMA warp, two epilogue warpgroups of 4 warps
 constexpr unsigned STEP_DOWN_RUN = 12;  // step-downs in a row after which the predicted shift is lowered (< 16)
 
-template <int BN, bool FUSED, bool TWO = false>
+template <int BN, bool TWO = false>
 struct GemmCfg {
     static constexpr int B_STAGE_BYTES = (TWO ? BN / 2 : BN) * ROW_BYTES;  // a CTA of a pair holds half of the B columns
     static constexpr int STAGE_BYTES = PANEL_BYTES + B_STAGE_BYTES;
-    // staging per epilogue warpgroup: one 128 x 128 int8 tile (fused) or two 128 x 32 int32 tiles
-    static constexpr int EPI_GROUP_BYTES = FUSED ? EPI_CHUNK_BYTES : 2 * EPI_CHUNK_BYTES;
+    static constexpr int EPI_GROUP_BYTES = 2 * EPI_CHUNK_BYTES;  // staging per epilogue warpgroup: two 128 x 32 int32 tiles
     static constexpr int EPI_BYTES = 2 * EPI_GROUP_BYTES;
     static constexpr int STAGES = (224 * 1024 - EPI_BYTES) / STAGE_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;  // two accumulators; 256 or 512 columns
@@ -343,7 +343,7 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
                     else     tma_load_4d(sa, tmA, fb, cb * ROW_BYTES, px + dx, py + dy, pn);
                     if (b_mn) {
 #pragma unroll
-                        for (int q = 0; q < BNH / 128; ++q) {
+                        for (int q = 0; q < (BNH + 127) / 128; ++q) {
                             if (TWO) tma_load_2d_pair(sb + q * PANEL_BYTES, tmB, fb, tap * tapstride + ncol + q * 128, cb * 128);
                             else     tma_load_2d(sb + q * PANEL_BYTES, tmB, fb, tap * tapstride + ncol + q * 128, cb * 128);
                         }
@@ -382,8 +382,8 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
 }
 
 // MMA issuer: the whole warp runs the loop with warp-uniform control flow (see the producer), one elected lane issues
-// the MMAs and the commits.  Streaming: two accumulators used alternately, each handed back by the
-// epilogue (tempty).  PARKED: tile i of this CTA accumulates into TMEM columns [i*BN, (i+1)*BN) and
+// the MMAs and the commits.  Streaming: NACC accumulators used in turn, each handed back by the
+// epilogue (tempty).  Parked (NACC = 0): tile i of this CTA accumulates into TMEM columns [i*BN, (i+1)*BN) and
 // stays there until the kernel ends, so no accumulator is ever waited for.
 // TWO: run by rank 0 of a CTA pair only; M = 256 MMAs over both CTAs' shared and tensor memory, and every
 // completion (stage free, accumulator full) is signalled to both CTAs.
@@ -391,9 +391,10 @@ template <bool TWO>
 __device__ __forceinline__ void umma_issue(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     if (TWO) umma_i8_pair(d_tmem, a, b, idesc, accumulate); else umma_i8(d_tmem, a, b, idesc, accumulate);
 }
-template <int BN, int STAGES, int STAGE_BYTES, bool PARKED, bool TWO>
+template <int BN, int STAGES, int STAGE_BYTES, int NACC, bool TWO>
 __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* tfull_bar,
                                          uint64_t* tempty_bar, uint32_t tmem_base_in, const GemmParams& p, volatile int* abort_flag) {
+    constexpr bool PARKED = NACC == 0;
     const int mn_tiles = p.m_tiles * p.n_tiles;
     const int total_tiles = mn_tiles * p.splits;
     const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, BN, p.a_mn, p.b_mn);
@@ -406,10 +407,12 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     // operand descriptors of stage 0 (a stage's are these advanced by the stage offset) and the K = 32 steps
     const uint32_t s0 = smem_u32(smem);
     const uint64_t a_base = p.a_mn ? make_smem_desc(s0, PANEL_BYTES, 1024, SWIZZLE_128B_CODE) : make_smem_desc(s0, 16, 1024, SWIZZLE_128B_CODE);
-    const uint64_t b_base = p.b_mn ? make_smem_desc(s0 + PANEL_BYTES, PANEL_BYTES, 1024, SWIZZLE_128B_CODE)
+    // a 64-column MN-major operand has rows of 64 bytes: 64-byte swizzle, 8-row groups of 512 bytes
+    const uint64_t b_base = p.b_mn ? (BN == 64 ? make_smem_desc(s0 + PANEL_BYTES, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
+                                               : make_smem_desc(s0 + PANEL_BYTES, PANEL_BYTES, 1024, SWIZZLE_128B_CODE))
                                    : make_smem_desc(s0 + PANEL_BYTES, 16, 1024, SWIZZLE_128B_CODE);
     const uint32_t a_step = static_cast<uint32_t>(keep_reg((p.a_mn ? 32 * ROW_BYTES : 32) >> 4));  // in descriptor units of 16 bytes
-    const uint32_t b_step = static_cast<uint32_t>(keep_reg((p.b_mn ? 32 * ROW_BYTES : 32) >> 4));
+    const uint32_t b_step = static_cast<uint32_t>(keep_reg((p.b_mn ? 32 * (BN == 64 ? 64 : ROW_BYTES) : 32) >> 4));
     const int conv = keep_reg(p.conv), red = keep_reg(p.red), cblocks = keep_reg(p.cblocks), num_kb = keep_reg(p.num_kb), splits = keep_reg(p.splits);
     int s = 0; uint32_t ph = 0; bool ok = true; int it = 0;
     // every reduction block has four MMAs unless a conv tap's channel count ends in a partial 128-byte block
@@ -423,9 +426,9 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     long long c_first = 0;
 #endif
     for (int tile = first; ok && tile < total_tiles; tile += step, ++it) {
-        const int acc = PARKED ? it : (it & 1);
+        const int acc = PARKED ? it : it % (PARKED ? 1 : NACC);
         if (!PARKED) {
-            const uint32_t aph = (it >> 1) & 1u;
+            const uint32_t aph = (it / (PARKED ? 1 : NACC)) & 1u;
             ok = mbar_wait_uniform(smem_u32(&tempty_bar[acc]), aph ^ 1u, abort_addr);
             if (!ok) { *abort_flag = 1; report_abort(p.status, 2, 1); break; }
             tc_fence_after();
@@ -472,49 +475,6 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     DBG_OUT(16);
 }
 
-// Output row of an epilogue thread: validity, TMA store coordinates of its tile, linear row index.
-struct RowInfo { bool valid; int cy, cz, cw; long long row_lin; long long pool_row; };
-__device__ __forceinline__ RowInfo row_info(const GemmParams& p, int m_t, int split, int row_in_tile) {
-    RowInfo r;
-    if (p.conv) {
-        const int tw = m_t % p.tiles_w, th = (m_t / p.tiles_w) % p.tiles_h, tn = m_t / (p.tiles_w * p.tiles_h);
-        const int w = tw * p.BW + row_in_tile % p.BW;
-        const int h = th * p.BH + (row_in_tile / p.BW) % p.BH;
-        const int n = tn * p.BI + row_in_tile / (p.BW * p.BH);
-        r.valid = row_in_tile < p.BW * p.BH * p.BI && w < p.W && h < p.H && n < p.Nimg;
-        r.cy = tw * p.BW; r.cz = th * p.BH; r.cw = tn * p.BI;
-        r.row_lin = (static_cast<long long>(n) * p.H + h) * p.W + w;
-        // row of the 2x2-pooled tensor this pixel's window goes to; only the window's top-left pixel writes it
-        r.pool_row = ((w | h) & 1) == 0 ? (static_cast<long long>(n) * (p.H >> 1) + (h >> 1)) * (p.W >> 1) + (w >> 1) : -1;
-    } else {
-        r.row_lin = static_cast<long long>(m_t) * BLOCK_M + row_in_tile;
-        r.valid = r.row_lin < p.M;
-        r.cy = m_t * BLOCK_M; r.cz = split; r.cw = 0;
-        r.pool_row = -1;
-    }
-    return r;
-}
-// max|x| = max(max x, -min x) over the first `lim` of 128 accumulators: short chains of 3-input min/max
-__device__ __forceinline__ void track_minmax(const uint32_t (&v)[4][32], int lim, int (&vmax)[4], int (&vmin)[4]) {
-    if (lim >= 128) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-                vmax[j] = __vimax3_s32(vmax[j], static_cast<int>(v[j][i]), static_cast<int>(v[j][i + 1]));
-                vmin[j] = __vimin3_s32(vmin[j], static_cast<int>(v[j][i]), static_cast<int>(v[j][i + 1]));
-            }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-                if (j * 32 + i < lim) {
-                    vmax[0] = max(vmax[0], static_cast<int>(v[j][i]));
-                    vmin[0] = min(vmin[0], static_cast<int>(v[j][i]));
-                }
-    }
-}
 __device__ __forceinline__ unsigned fold_minmax(const int (&vmax)[4], const int (&vmin)[4]) {
     const int hi = max(max(vmax[0], vmax[1]), max(vmax[2], vmax[3]));
     const int lo = min(min(vmin[0], vmin[1]), min(vmin[2], vmin[3]));
@@ -541,6 +501,25 @@ __device__ __forceinline__ void minmax32(const uint32_t (&v)[32], int lim, int (
             }
     }
 }
+// Every other case (pseudo-stochastic rounding, shift 0, ...): a call of its own on arrays in local memory, so that its
+// registers are not the epilogue's.
+__device__ __noinline__ void narrow32_general(const uint32_t* v, uint32_t* packed, int shift, int mode, int relu,
+                                              unsigned long long seed, unsigned rng_stream, unsigned long long e0) {
+    const bool stochastic = mode == ROUND_STOCHASTIC && shift > 0;
+#pragma unroll 1
+    for (int i = 0; i < 32; i += 4) {
+        uint32_t rnd[4] = {0, 0, 0, 0};
+        if (stochastic) {
+            const unsigned long long e = e0 + i;
+            if ((e & 3ull) == 0) random_block(seed, rng_stream, e >> 2, rnd);
+            else {
+#pragma unroll
+                for (int t = 0; t < 4; ++t) rnd[t] = random_word(seed, rng_stream, e + t);
+            }
+        }
+        packed[i >> 2] = narrow4(v + i, shift, mode, relu, rnd);
+    }
+}
 __device__ __forceinline__ void narrow32(const uint32_t (&v)[32], uint32_t (&packed)[8], int shift, int mode, int relu,
                                          unsigned long long seed, unsigned rng_stream, unsigned long long e0) {
     if (mode == ROUND_NEAREST && shift > 0) {
@@ -553,30 +532,12 @@ __device__ __forceinline__ void narrow32(const uint32_t (&v)[32], uint32_t (&pac
             for (int i = 0; i < 32; i += 4) packed[i >> 2] = narrow4_nearest<false>(&v[i], shift, half);
         }
     } else {
-        const bool stochastic = mode == ROUND_STOCHASTIC && shift > 0;
-#pragma unroll 1
-        for (int i = 0; i < 32; i += 4) {
-            uint32_t rnd[4] = {0, 0, 0, 0};
-            if (stochastic) {
-                const unsigned long long e = e0 + i;
-                if ((e & 3ull) == 0) random_block(seed, rng_stream, e >> 2, rnd);
-                else {
+        uint32_t in[32], out[8];
 #pragma unroll
-                    for (int t = 0; t < 4; ++t) rnd[t] = random_word(seed, rng_stream, e + t);
-                }
-            }
-            uint32_t x[4];
-            // select without dynamic register indexing
+        for (int i = 0; i < 32; ++i) in[i] = v[i];
+        narrow32_general(in, out, shift, mode, relu, seed, rng_stream, e0);
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                x[t] = v[t];
-#pragma unroll
-                for (int k = 4; k < 32; k += 4) x[t] = (i == k) ? v[k + t] : x[t];
-            }
-            const uint32_t w = narrow4(x, shift, mode, relu, rnd);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) if (i == 4 * k) packed[k] = w;
-        }
+        for (int i = 0; i < 8; ++i) packed[i] = out[i];
     }
 }
 // ReLU backward folded into an error-backward epilogue: zero the packed int8 outputs where the layer's forward input
@@ -617,69 +578,27 @@ __device__ __forceinline__ void pool_window(uint32_t (&w)[8], int bw) {
         w[i] = __vmaxs4(m, __shfl_xor_sync(0xFFFFFFFFu, m, bw));
     }
 }
-// 32 packed int8 of one output row to global memory, as two 16-byte stores; `row` is null for rows outside the tensor,
-// `off` the byte offset within the unit's columns of which `cols` exist (a multiple of 16)
-__device__ __forceinline__ void store_piece(int8_t* row, int off, int cols, const uint32_t (&w)[8]) {
-    if (row == nullptr) return;
-    if (off + 16 <= cols) *reinterpret_cast<uint4*>(row + off) = make_uint4(w[0], w[1], w[2], w[3]);
-    if (off + 32 <= cols) *reinterpret_cast<uint4*>(row + off + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-}
-// a 32-byte piece (chunk j of the row's 128 bytes) at its 128-byte-swizzled place in the staging tile
-__device__ __forceinline__ void stage_piece(uint32_t buf, int row, int j, const uint32_t (&w)[8]) {
-    const uint32_t base = buf + static_cast<uint32_t>(row) * 128u;
-    st_shared_v4(base + (static_cast<uint32_t>((2 * j) ^ (row & 7)) << 4), w[0], w[1], w[2], w[3]);
-    st_shared_v4(base + (static_cast<uint32_t>((2 * j + 1) ^ (row & 7)) << 4), w[4], w[5], w[6], w[7]);
-}
-// 128 accumulators of one row -> 32 words of packed int8
-__device__ __forceinline__ void narrow_row(const uint32_t (&v)[4][32], uint32_t (&packed)[32], int shift, int mode, int relu,
-                                           unsigned long long seed, unsigned rng_stream, unsigned long long e0) {
-    if (mode == ROUND_NEAREST && shift > 0) {
-        const int half = 1 << (shift - 1);
-        if (relu) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) packed[j * 8 + (i >> 2)] = narrow4_nearest<true>(&v[j][i], shift, half);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) packed[j * 8 + (i >> 2)] = narrow4_nearest<false>(&v[j][i], shift, half);
-        }
-    } else {
-        const bool stochastic = mode == ROUND_STOCHASTIC && shift > 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                uint32_t rnd[4] = {0, 0, 0, 0};
-                if (stochastic) {
-                    const unsigned long long e = e0 + j * 32 + i;
-                    if ((e & 3ull) == 0) random_block(seed, rng_stream, e >> 2, rnd);
-                    else {
-#pragma unroll
-                        for (int t = 0; t < 4; ++t) rnd[t] = random_word(seed, rng_stream, e + t);
-                    }
-                }
-                packed[j * 8 + (i >> 2)] = narrow4(&v[j][i], shift, mode, relu, rnd);
-            }
+// whether every 32-byte piece of a tensor of `n`-byte rows starts on a 32-byte boundary
+__device__ __forceinline__ bool rows_of_32(const int8_t* base, int n) { return ((reinterpret_cast<uintptr_t>(base) | static_cast<uintptr_t>(n)) & 31) == 0; }
+// 32 packed int8 of one output row to global memory: one 32-byte store (a whole L2 sector) or, where the rows are only
+// 16-byte aligned, two.  `at` is null for rows outside the tensor; `cols` (a multiple of 16) exist from there on.
+__device__ __forceinline__ void store_piece(int8_t* at, int cols, const uint32_t (&w)[8], bool wide) {
+    if (at == nullptr) return;
+    if (wide) {
+        st_global_v8(at, w);  // rows of a multiple of 32 bytes: a piece that starts inside the row ends inside it
+        return;
     }
+    if (cols >= 16) *reinterpret_cast<uint4*>(at) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (cols >= 32) *reinterpret_cast<uint4*>(at + 16) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-template <int BN, bool FUSED, bool TWO>
+// Plain products: int32 out (+ max|acc|).
+template <int BN, bool TWO>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)  // 10 warps: 3 on one scheduler -> at most 168 registers per thread
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
-    using Cfg = GemmCfg<BN, FUSED, TWO>;
+    using Cfg = GemmCfg<BN, TWO>;
     constexpr int STAGES = Cfg::STAGES;
-    if (FUSED && p.only_if_redo) {
-        const int verdict = p.state[2] & 3;
-        if (verdict == 0) return;  // the prediction was right: nothing to redo
-        if (verdict == 2) {        // one bit too many was shifted out and the side codes hold what is missing
-            requant_step_down(p.out8, p.side, p.mask, static_cast<long long>(p.M) * p.N / 16);
-            return;
-        }
-    }
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -728,7 +647,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         __syncwarp();
     } else if (warp == 1) {
         if (rank == 0)
-            mma_role<BN, STAGES, Cfg::STAGE_BYTES, false, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            mma_role<BN, STAGES, Cfg::STAGE_BYTES, 2, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue (2 x 4 warps)
@@ -739,24 +658,13 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // four tcgen05.ld and ONE wait, the accumulator is handed back as soon as the warpgroup's
         // last columns sit in registers, max|acc| is tracked in registers, rows go to swizzled
         // staging tiles and leave through TMA stores (which clip rows/columns outside the tensor).
-        //   plain kernels: int32 out, two rounds of two 128 x 32 staging tiles per column group;
-        //   FUSED kernels: int8 out, narrowed with the shift in state[0], one 128 x 128-byte tile.
+        // Two rounds of two 128 x 32 staging tiles per column group.
         const int grp = (warp - 2) >> 2;  // epilogue warpgroup 0 / 1
         const int q = warp & 3;           // TMEM lanes [32q, 32q+32) are the ones this warp may read
         const int row_in_tile = q * 32 + lane;
         const int bar_id = EPI_BARRIER + grp;
         const bool leader = (threadIdx.x == 64 + grp * 128);
         const uint32_t buf = smem_u32(epi_smem) + grp * Cfg::EPI_GROUP_BYTES;
-        int shift = 0;
-        unsigned long long seed = 0;
-        if (FUSED) {
-            shift = p.state[0];
-            if (p.mode == ROUND_STOCHASTIC && shift > 0) seed = *p.seed;
-        }
-        const bool fast = FUSED && p.mode == ROUND_NEAREST && shift > 0;
-        // a first launch also keeps what the next lower shift would need (see narrow16_nearest_codes)
-        const bool with_codes = fast && shift >= 2 && !p.relu && p.side != nullptr && !p.only_if_redo;
-        const int half = shift > 0 ? 1 << (shift - 1) : 0;
         int vmax[4] = {0, 0, 0, 0}, vmin[4] = {0, 0, 0, 0};
         const int tile_step = p.split_cols ? cta_step : 2 * cta_step;
         int it = p.split_cols ? 0 : grp;
@@ -776,19 +684,16 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             int m_pair, n_t;
             tile_coords(p, mn, &m_pair, &n_t);
             const int m_t = TWO ? 2 * m_pair + static_cast<int>(rank) : m_pair;
-            bool valid; int cy, cz, cw; long long row_lin;
+            bool valid; int cy, cz, cw;
             if (p.conv) {
                 const int q1 = fdiv(m_t, p.fd_tw), tw = m_t - q1 * p.tiles_w, tn = fdiv(q1, p.fd_th), th = q1 - tn * p.tiles_h;
                 cy = tw * p.BW; cz = th * p.BH; cw = tn * p.BI;
                 const int w = cy + row_w, h = cz + row_h, n = cw + row_n;
                 valid = row_in_box && w < p.W && h < p.H && n < p.Nimg;
-                row_lin = (static_cast<long long>(n) * p.H + h) * p.W + w;
             } else {
-                row_lin = static_cast<long long>(m_t) * BLOCK_M + row_in_tile;
-                valid = row_lin < p.M;
+                valid = m_t * BLOCK_M + row_in_tile < p.M;
                 cy = m_t * BLOCK_M; cz = split; cw = 0;
             }
-            if (FUSED && p.mask != nullptr && valid) prefetch_l2(p.mask + row_lin * p.N + n_t * BN);
             const uint32_t failed = mbar_wait(smem_u32(&tfull_bar[acc]), aph, abort_flag) ? 0u : 1u;
             if (barrier_or(bar_id, 128, failed)) {  // same verdict in all 128 threads of the warpgroup
                 if (failed) report_abort(p.status, 4, 2);
@@ -837,82 +742,19 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                                 }
                     }
                 }
-                if constexpr (FUSED) {
-                    uint32_t packed[32];
-                    if (with_codes) {
-                        uint32_t codes[8];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-#pragma unroll
-                            for (int i = 0; i < 32; i += 16)
-                                codes[j * 2 + (i >> 4)] = narrow16_nearest_codes(&v[j][i], shift - 2, half, &packed[j * 8 + (i >> 2)]);
-                        if (valid) {  // a row's codes are 32 consecutive bytes, the rows of a tile mostly consecutive: plain stores
-                            uint32_t* srow = p.side + ((row_lin * p.N + col0 + g0) >> 4);
-                            if (lim >= 128 && (p.N & 63) == 0) {  // rows of N / 4 bytes: 16-byte aligned when N is a multiple of 64
-                                reinterpret_cast<uint4*>(srow)[0] = make_uint4(codes[0], codes[1], codes[2], codes[3]);
-                                reinterpret_cast<uint4*>(srow)[1] = make_uint4(codes[4], codes[5], codes[6], codes[7]);
-                            } else {
-#pragma unroll
-                                for (int k = 0; k < 8; ++k)
-                                    if (16 * k + 16 <= lim) srow[k] = codes[k];
-                            }
-                        }
-                    } else if (fast) {
-                        if (p.relu) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                                for (int i = 0; i < 32; i += 4) packed[j * 8 + (i >> 2)] = narrow4_nearest<true>(&v[j][i], shift, half);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                                for (int i = 0; i < 32; i += 4) packed[j * 8 + (i >> 2)] = narrow4_nearest<false>(&v[j][i], shift, half);
-                        }
-                    } else {
-                        const unsigned long long e0 = p.rng_offset + static_cast<unsigned long long>(row_lin) * p.N + (col0 + g0);
-                        const bool stochastic = p.mode == ROUND_STOCHASTIC && shift > 0;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-#pragma unroll
-                            for (int i = 0; i < 32; i += 4) {
-                                uint32_t rnd[4] = {0, 0, 0, 0};
-                                if (stochastic) {
-                                    const unsigned long long e = e0 + j * 32 + i;
-                                    if ((e & 3ull) == 0) random_block(seed, p.rng_stream, e >> 2, rnd);
-                                    else {
-#pragma unroll
-                                        for (int t = 0; t < 4; ++t) rnd[t] = random_word(seed, p.rng_stream, e + t);
-                                    }
-                                }
-                                packed[j * 8 + (i >> 2)] = narrow4(&v[j][i], shift, p.mode, p.relu, rnd);
-                            }
-                    }
-                    // (fetching the mask ahead of the narrowing, as the parked kernel does, costs this kernel registers it
-                    // does not have: 32.2 / 36.0 us per 128x32x32 call against 29.5 / 33.4 with the loads here)
-                    if (p.mask != nullptr && valid) apply_relu_mask<32>(packed, p.mask + row_lin * p.N + col0 + g0, lim);
-                    if (leader) bulk_wait_read<0>();  // the previous store has read the staging tile
+                for (int half_i = 0; half_i < 2; ++half_i) {
+                    if (col0 + g0 + half_i * 64 >= p.N) break;
+                    if (leader) bulk_wait_read<0>();  // the stores of the pass before have read the staging tiles
                     named_barrier(bar_id, 128);
-                    stage_row(buf, row_in_tile, packed);
+                    stage_row(buf, row_in_tile, v[2 * half_i]);
+                    stage_row(buf + EPI_CHUNK_BYTES, row_in_tile, v[2 * half_i + 1]);
                     fence_proxy_async();
                     named_barrier(bar_id, 128);
-                    if (leader) { tma_store_4d(&tmC, buf, col0 + g0, cy, cz, cw); bulk_commit(); }
-
-                } else {
-#pragma unroll
-                    for (int half_i = 0; half_i < 2; ++half_i) {
-                        if (col0 + g0 + half_i * 64 >= p.N) break;
-                        if (leader) bulk_wait_read<0>();  // the stores of the pass before have read the staging tiles
-                        named_barrier(bar_id, 128);
-                        stage_row(buf, row_in_tile, v[2 * half_i]);
-                        stage_row(buf + EPI_CHUNK_BYTES, row_in_tile, v[2 * half_i + 1]);
-                        fence_proxy_async();
-                        named_barrier(bar_id, 128);
-                        if (leader) {
-                            tma_store_4d(&tmC, buf, col0 + g0 + half_i * 64, cy, cz, cw);
-                            if (col0 + g0 + half_i * 64 + 32 < p.N) tma_store_4d(&tmC, buf + EPI_CHUNK_BYTES, col0 + g0 + half_i * 64 + 32, cy, cz, cw);
-                            bulk_commit();
-                        }
+                    if (leader) {
+                        tma_store_4d(&tmC, buf, col0 + g0 + half_i * 64, cy, cz, cw);
+                        if (col0 + g0 + half_i * 64 + 32 < p.N) tma_store_4d(&tmC, buf + EPI_CHUNK_BYTES, col0 + g0 + half_i * 64 + 32, cy, cz, cw);
+                        bulk_commit();
                     }
                 }
             }
@@ -939,45 +781,6 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int i = 0; i < 8; ++i) m = max(m, warp_max[i]);
             if (m != 0 && p.maxabs != nullptr) atomicMax(p.maxabs, m);
         }
-        if (FUSED && !p.only_if_redo) {
-            // the CTA that finishes last turns max|acc| into the true shift and checks the prediction
-            if (threadIdx.x == 64) {
-                __threadfence();
-                int32_t* st = p.state;
-                if (atomicAdd(&st[4], 1) == static_cast<int>(gridDim.x) - 1) {
-                    __threadfence();
-                    bool zero_out;
-                    const unsigned m = static_cast<unsigned>(atomicMax(reinterpret_cast<unsigned*>(&st[1]), 0u));
-                    const int true_shift = shift_for(m, p.kind, p.target_bits, &zero_out);
-                    // st[2] = verdict (0 right, 1 launch again, 2 step the output down one shift from the side codes)
-                    //         | run of step-downs << 4 | step-downs so far << 8
-                    const int pred = st[0];
-                    const unsigned old = static_cast<unsigned>(st[2]);
-                    unsigned run = (old >> 4) & 15u, downs = old >> 8;
-                    int verdict = 0;
-                    if (true_shift == pred) {
-                        run = 0;
-                    } else if (p.side != nullptr && p.mode == ROUND_NEAREST && !p.relu && pred >= 2 && true_shift == pred - 1) {
-                        // the prediction stays: a layer whose maximum hovers around a power of two keeps the upper
-                        // shift as its guess and pays the cheap pass when the lower one applies; after
-                        // STEP_DOWN_RUN lower ones in a row the guess follows
-                        verdict = 2;
-                        ++downs;
-                        if (++run >= STEP_DOWN_RUN) { run = 0; st[0] = true_shift; }
-                    } else {
-                        verdict = 1;
-                        run = 0;
-                        st[3] += 1;
-                        st[0] = true_shift;
-                    }
-                    st[2] = static_cast<int>(static_cast<unsigned>(verdict) | (run << 4) | (downs << 8));
-                    st[1] = 0;  // ready for the next call
-                    st[4] = 0;
-                    if (p.exp_out) *p.exp_out = true_shift + (p.exp_a ? *p.exp_a : 0) + (p.exp_b ? *p.exp_b : 0);
-                    if (p.shift_out) *p.shift_out = true_shift;
-                }
-            }
-        }
     }
 
     // ---------------------------------------------------------------------- teardown
@@ -993,6 +796,239 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 // ------------------------------------------------------------------------------------------------
+// The epilogue of the kernels that narrow to int8: sixteen warps (four per scheduler) in four groups of four.  Group g
+// takes its own columns of EVERY tile, 32 at a time, so that the load of an accumulator chunk, the 32 dependent
+// integer sequences of its narrowing and its store overlap between the four warps of a scheduler.  Eight warps that
+// held whole 128-column rows had two warps per scheduler and ran at 2.4 times the bound of the integer pipe: a launch
+// was paced by its epilogue and not by the tensor pipe (first layer at batch 1024, one MMA step per tile: 120 us).
+//   BN = 128: one 32-column chunk per group and tile;   BN = 256: two;
+//   BN = 64:  two groups share a tile, the other two the next one.
+// 18 warps (five on one scheduler) leave 96 registers per thread, which 32 accumulators at a time fit into.
+// ------------------------------------------------------------------------------------------------
+constexpr int EPI_WARPS = 16;
+constexpr int REQUANT_THREADS = 64 + 32 * EPI_WARPS;  // producer warp, MMA warp, epilogue warps
+template <int BN>
+struct EpiSplit {
+    static constexpr int GROUPS = BN >= 128 ? 4 : BN / 32;  // warp groups that share a tile
+    static constexpr int TILES = 4 / GROUPS;                // tiles worked on side by side
+    static constexpr int COLS = BN / GROUPS;                // columns of a group
+    static constexpr int CHUNKS = COLS / 32;
+};
+// Operand ring and accumulators of the kernels that narrow.  BN = 64 serves layers of up to 64 output channels: with
+// 128-column tiles half of the tensor work, of the accumulator reads and of the weight traffic was padding.
+template <int BN, bool TWO>
+struct RequantCfg {
+    static constexpr int B_STAGE_BYTES = (TWO ? BN / 2 : BN) * ROW_BYTES;
+    static constexpr int STAGE_BYTES = PANEL_BYTES + B_STAGE_BYTES;
+    static constexpr int STAGES = 216 * 1024 / STAGE_BYTES;
+    static constexpr int NACC = BN == 256 ? 2 : 4;  // streaming: accumulators in flight
+    static constexpr int TABLE_BYTES = 2 * 4 * 128 * 4;  // parked: output row and pooled row of every row of the CTA's tiles
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TABLE_BYTES + 1024 /*alignment slack*/ + 512 /*barriers*/;
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a CTA");
+};
+
+// Streaming kernel: narrows with the shift in state[0]; the last CTA derives the true one from max|acc|.
+template <int BN, bool TWO>
+__global__ void __launch_bounds__(REQUANT_THREADS, 1)
+umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+    using Cfg = RequantCfg<BN, TWO>;
+    using Split = EpiSplit<BN>;
+    constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC;
+    if (p.only_if_redo) {
+        const int verdict = p.state[2] & 3;
+        if (verdict == 0) return;  // the prediction was right: nothing to redo
+        if (verdict == 2) {        // one bit too many was shifted out and the side codes hold what is missing
+            requant_step_down(p.out8, p.side, p.mask, static_cast<long long>(p.M) * p.N / 16);
+            return;
+        }
+    }
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+    uint64_t* full_bar = bars;
+    uint64_t* empty_bar = bars + STAGES;
+    uint64_t* tfull_bar = bars + 2 * STAGES;
+    uint64_t* tempty_bar = bars + 2 * STAGES + NACC;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * NACC);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile unsigned* warp_max = reinterpret_cast<volatile unsigned*>(tmem_slot + 4);  // one word per epilogue warp
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t rank = TWO ? cluster_ctarank() : 0u;  // rank 0 of a pair issues the MMAs and owns the barriers the MMA thread waits on
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; ++i) { mbar_init(smem_u32(&full_bar[i]), 1); mbar_init(smem_u32(&empty_bar[i]), 1); }
+        for (int i = 0; i < NACC; ++i) { mbar_init(smem_u32(&tfull_bar[i]), 1); mbar_init(smem_u32(&tempty_bar[i]), 4 * Split::GROUPS * (TWO ? 2 : 1)); }
+        *abort_flag = 0;
+        fence_barrier_init();
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+    }
+    if (warp == 1) {
+        if (TWO) { tmem_alloc_pair(smem_u32(tmem_slot), NACC * BN); tmem_relinquish_pair(); }
+        else     { tmem_alloc(smem_u32(tmem_slot), NACC * BN); tmem_relinquish(); }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (TWO) cluster_sync_all();  // the partner's barriers exist before anything is signalled across the pair
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int total_tiles = p.m_tiles * p.n_tiles;  // TWO: m_tiles counts 256-row tiles of the pair; the reduction is never split here
+    const int cta_first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
+    const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+
+    if (warp == 0) {
+        producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
+    } else if (warp == 1) {
+        if (rank == 0)
+            mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+        __syncwarp();
+    } else {
+        const int grp = (warp - 2) >> 2;
+        const int q = warp & 3;  // TMEM lanes [32q, 32q+32) are the ones this warp may read
+        const int row_in_tile = q * 32 + lane;
+        const int cg = (grp % Split::GROUPS) * Split::COLS;
+        const int shift = p.state[0];
+        const unsigned long long seed = (p.mode == ROUND_STOCHASTIC && shift > 0) ? *p.seed : 0ull;
+        // a first launch also keeps what the next lower shift would need (see narrow16_nearest_codes)
+        const bool with_codes = p.mode == ROUND_NEAREST && shift >= 2 && !p.relu && p.side != nullptr && !p.only_if_redo;
+        const int half = shift > 0 ? 1 << (shift - 1) : 0;
+        const bool wide = rows_of_32(p.out8, p.N);
+        int vmax[4] = {0, 0, 0, 0}, vmin[4] = {0, 0, 0, 0};
+        // this thread's row inside a tile never changes: pixel offsets within the tile's box
+        int row_w = 0, row_h = 0, row_n = 0;
+        bool row_in_box = true;
+        if (p.conv) {
+            const int t_ = row_in_tile / p.BW;
+            row_w = row_in_tile - t_ * p.BW; row_n = t_ / p.BH; row_h = t_ - row_n * p.BH;
+            row_in_box = row_in_tile < p.BW * p.BH * p.BI;
+        }
+        int it = grp / Split::GROUPS;
+        for (int tile = cta_first + it * cta_step; tile < total_tiles; tile += Split::TILES * cta_step, it += Split::TILES) {
+            const int acc = it & (NACC - 1); const uint32_t aph = (it / NACC) & 1u;
+            // where the tile lies, and the mask of the first chunk, before waiting for its accumulator
+            int m_pair, n_t;
+            tile_coords(p, tile, &m_pair, &n_t);
+            const int m_t = TWO ? 2 * m_pair + static_cast<int>(rank) : m_pair;
+            bool valid; int row;  // row of the output tensor
+            if (p.conv) {
+                const int q1 = fdiv(m_t, p.fd_tw), tw = m_t - q1 * p.tiles_w, tn = fdiv(q1, p.fd_th), th = q1 - tn * p.tiles_h;
+                const int w = tw * p.BW + row_w, h = th * p.BH + row_h, n = tn * p.BI + row_n;
+                valid = row_in_box && w < p.W && h < p.H && n < p.Nimg;
+                row = (n * p.H + h) * p.W + w;
+            } else {
+                row = m_t * BLOCK_M + row_in_tile;
+                valid = row < p.M;
+            }
+            const int col0 = n_t * BN + cg;
+            const long long off = static_cast<long long>(row) * p.N + col0;  // of this thread's first output
+            const int8_t* mrow = (p.mask != nullptr && valid && col0 < p.N) ? p.mask + off : nullptr;
+            uint4 mk[2];
+            mask_load<2>(mrow, p.N - col0, mk);
+            const bool up = mbar_wait(smem_u32(&tfull_bar[acc]), aph, abort_flag);
+            if (!__all_sync(0xFFFFFFFFu, up)) { if (!up) report_abort(p.status, 4, 2); break; }
+            tc_fence_after();
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN + cg);
+#pragma unroll 1
+            for (int c = 0; c < Split::CHUNKS; ++c) {
+                const int cols = p.N - col0 - 32 * c;  // columns of the tensor from here on
+                uint32_t v[32], packed[8];
+                tmem_ld_32x32(taddr + 32 * c, v);
+                if (c > 0) mask_load<2>(mrow == nullptr ? nullptr : mrow + 32 * c, cols, mk);
+                tmem_ld_wait();
+                if (c == Split::CHUNKS - 1) {  // this warp's last columns sit in registers: hand the accumulator back
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (TWO) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty_bar[acc]), 0));
+                        else     mbar_arrive(smem_u32(&tempty_bar[acc]));
+                    }
+                }
+                if (cols <= 0) continue;
+                if (valid) minmax32(v, cols, vmax, vmin);
+                if (with_codes) {
+                    uint32_t codes[2];
+#pragma unroll
+                    for (int i = 0; i < 32; i += 16) codes[i >> 4] = narrow16_nearest_codes(&v[i], shift - 2, half, &packed[i >> 2]);
+                    if (valid) {  // 16 outputs per word, rows of N / 4 bytes
+                        uint32_t* srow = p.side + ((off + 32 * c) >> 4);
+                        srow[0] = codes[0];
+                        if (cols >= 32) srow[1] = codes[1];
+                    }
+                } else {
+                    narrow32(v, packed, shift, p.mode, p.relu, seed, p.rng_stream, p.rng_offset + static_cast<unsigned long long>(off) + 32 * c);
+                }
+                mask_apply<2>(packed, mrow, cols, mk);
+                store_piece(valid ? p.out8 + off + 32 * c : nullptr, cols, packed, wide);
+            }
+        }
+        const unsigned local_max = __reduce_max_sync(0xFFFFFFFFu, fold_minmax(vmax, vmin));
+        // one atomic per CTA: atomics on one address serialise at the L2, and there are 16 warps x 148 CTAs
+        if (lane == 0) warp_max[warp - 2] = local_max;
+        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
+        if (threadIdx.x == 64) {
+            unsigned m = 0;
+#pragma unroll
+            for (int i = 0; i < EPI_WARPS; ++i) m = max(m, warp_max[i]);
+            if (m != 0 && p.maxabs != nullptr) atomicMax(p.maxabs, m);
+        }
+        // the CTA that finishes last turns max|acc| into the true shift and checks the prediction
+        if (!p.only_if_redo && threadIdx.x == 64) {
+            __threadfence();
+            int32_t* st = p.state;
+            if (atomicAdd(&st[4], 1) == static_cast<int>(gridDim.x) - 1) {
+                __threadfence();
+                bool zero_out;
+                const unsigned m = static_cast<unsigned>(atomicMax(reinterpret_cast<unsigned*>(&st[1]), 0u));
+                const int true_shift = shift_for(m, p.kind, p.target_bits, &zero_out);
+                // st[2] = verdict (0 right, 1 launch again, 2 step the output down one shift from the side codes)
+                //         | run of step-downs << 4 | step-downs so far << 8
+                const int pred = st[0];
+                const unsigned old = static_cast<unsigned>(st[2]);
+                unsigned run = (old >> 4) & 15u, downs = old >> 8;
+                int verdict = 0;
+                if (true_shift == pred) {
+                    run = 0;
+                } else if (p.side != nullptr && p.mode == ROUND_NEAREST && !p.relu && pred >= 2 && true_shift == pred - 1) {
+                    // the prediction stays: a layer whose maximum hovers around a power of two keeps the upper
+                    // shift as its guess and pays the cheap pass when the lower one applies; after
+                    // STEP_DOWN_RUN lower ones in a row the guess follows
+                    verdict = 2;
+                    ++downs;
+                    if (++run >= STEP_DOWN_RUN) { run = 0; st[0] = true_shift; }
+                } else {
+                    verdict = 1;
+                    run = 0;
+                    st[3] += 1;
+                    st[0] = true_shift;
+                }
+                st[2] = static_cast<int>(static_cast<unsigned>(verdict) | (run << 4) | (downs << 8));
+                st[1] = 0;  // ready for the next call
+                st[4] = 0;
+                if (p.exp_out) *p.exp_out = true_shift + (p.exp_a ? *p.exp_a : 0) + (p.exp_b ? *p.exp_b : 0);
+                if (p.shift_out) *p.shift_out = true_shift;
+            }
+        }
+    }
+
+    // ---------------------------------------------------------------------- teardown
+    tc_fence_before();
+    __syncthreads();
+    if (TWO) cluster_sync_all();  // the partner may still signal this CTA's barriers / have MMAs reading its memory
+    if (warp == 1) {
+        if (*abort_flag) __nanosleep(200000);  // let copies and MMAs already in flight land
+        tc_fence_after();
+        __syncwarp();
+        if (TWO) tmem_dealloc_pair(tmem_base, NACC * BN); else tmem_dealloc(tmem_base, NACC * BN);
+    }
+}
+
+
+// ------------------------------------------------------------------------------------------------
 // Exact single-pass requantisation for problems whose accumulators all fit in tensor memory:
 // every CTA owns at most 512 / BN output tiles and PARKS their int32 accumulators in TMEM.  After
 // its main loops a CTA reduces max|acc| of its tiles into the global word, all CTAs meet at a grid
@@ -1001,29 +1037,21 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // no int32 in memory.  state = {shift out, max|acc|, redo flag (cleared), redo count, exit ticket,
 // -, max|acc| and barrier arrivals (adjacent: read with one 64-bit load)}; words 1, 4, 5, 6 and 7 are zero between calls.
 // ------------------------------------------------------------------------------------------------
-template <int BN, bool TWO = false>
-struct ParkedCfg {
-    static constexpr int STAGE_BYTES = PANEL_BYTES + (TWO ? BN / 2 : BN) * ROW_BYTES;
-    static constexpr int EPI_GROUP_BYTES = EPI_CHUNK_BYTES;  // one 128 x 128 int8 staging tile per warpgroup
-    static constexpr int EPI_BYTES = 2 * EPI_GROUP_BYTES;
-    static constexpr int STAGES = (224 * 1024 - EPI_BYTES) / STAGE_BYTES;
-    static constexpr int MAX_TILES = 512 / BN;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 256;
-};
-
 constexpr unsigned long long GRID_BARRIER_LIMIT_NS = 500000000ull;  // 0.5 s
 
 template <int BN, bool TWO>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
-    using Cfg = ParkedCfg<BN, TWO>;
+__global__ void __launch_bounds__(REQUANT_THREADS, 1)
+umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+    using Cfg = RequantCfg<BN, TWO>;
+    using Split = EpiSplit<BN>;
     constexpr int STAGES = Cfg::STAGES;
+    static_assert(BN >= 128 && 512 / BN <= 4, "all four warp groups share every tile; tables of four tiles");
     if (threadIdx.x == 0) PARK_STAMP(0);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(epi_smem + Cfg::EPI_BYTES);
+    int32_t* out_row = reinterpret_cast<int32_t*>(smem + STAGES * Cfg::STAGE_BYTES);  // [tile][row of the tile]; -1: outside the tensor
+    int32_t* pool_row = out_row + 4 * 128;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(pool_row + 4 * 128);
     uint64_t* full_bar = bars;
     uint64_t* empty_bar = bars + STAGES;
     uint64_t* tfull_bar = bars + 2 * STAGES;  // one per parked tile (up to 4)
@@ -1043,7 +1071,6 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         fence_barrier_init();
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        tma_prefetch_desc(&tmC);
     }
     if (warp == 1) {
         if (TWO) { tmem_alloc_pair(smem_u32(tmem_slot), 512); tmem_relinquish_pair(); }
@@ -1056,8 +1083,7 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const uint32_t tmem_base = *tmem_slot;
     if (threadIdx.x == 0) PARK_STAMP(1);
 
-    const int mn_tiles = p.m_tiles * p.n_tiles;  // TWO: m_tiles counts 256-row tiles of the pair
-    const int total_tiles = mn_tiles * p.splits;
+    const int total_tiles = p.m_tiles * p.n_tiles;  // TWO: m_tiles counts 256-row tiles of the pair
     const int cta_first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
@@ -1066,80 +1092,71 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if (rank == 0)
-            mma_role<BN, STAGES, Cfg::STAGE_BYTES, true, TWO>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
+            mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
         __syncwarp();
     } else {
-        // Work units of the epilogue: (tile of this CTA, 128-column group); the two warpgroups take
-        // alternate units, the same ones in both passes.
         const int grp = (warp - 2) >> 2;
         const int q = warp & 3;
         const int row_in_tile = q * 32 + lane;
-        const int bar_id = EPI_BARRIER + grp;
-        constexpr int CG = BN / 128;
+        const int cg = grp * Split::COLS;
         int my_tiles = 0;
         for (int tile = cta_first; tile < total_tiles; tile += cta_step) ++my_tiles;
-        const int units = my_tiles * CG;
 
-        // Everything about this warpgroup's (at most two) units that does not depend on the accumulators is worked out
-        // now, while the main loop runs: tile coordinates, the row this thread owns, tensor-memory address.
-        constexpr int MAX_UNITS = 2;  // tiles per CTA <= 512 / BN, 128-column groups per tile = BN / 128, two warpgroups
-        RowInfo u_ri[MAX_UNITS]; int u_col[MAX_UNITS], u_it[MAX_UNITS]; uint32_t u_taddr[MAX_UNITS]; bool u_live[MAX_UNITS];
-#pragma unroll
-        for (int k = 0; k < MAX_UNITS; ++k) {
-            const int u = grp + 2 * k;
-            u_live[k] = u < units;
-            u_it[k] = 0; u_col[k] = 0; u_taddr[k] = 0; u_ri[k] = RowInfo{false, 0, 0, 0, 0, -1};
-            if (u_live[k]) {
-                const int it = u / CG, g0 = (u % CG) * 128;
-                const int tile = cta_first + it * cta_step;
-                const int mn = tile % mn_tiles, n_t = mn % p.n_tiles;
-                const int m_t = TWO ? 2 * (mn / p.n_tiles) + static_cast<int>(rank) : mn / p.n_tiles;
-                u_ri[k] = row_info(p, m_t, tile / mn_tiles, row_in_tile);
-                u_it[k] = it;
-                u_col[k] = n_t * BN + g0;
-                // the ReLU mask this row will be gated with after the main loop: start moving it towards the L2 now
-                if (p.mask != nullptr && u_ri[k].valid && u_col[k] < p.N) prefetch_l2(p.mask + u_ri[k].row_lin * p.N + u_col[k]);
-                u_taddr[k] = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + it * BN + g0;
-            }
+        // Where the rows of the CTA's tiles go is worked out while the main loop runs: group g fills the table of tile g.
+        if (grp < my_tiles) {
+            int m_pair, n_t;
+            tile_coords(p, cta_first + grp * cta_step, &m_pair, &n_t);
+            const int m_t = TWO ? 2 * m_pair + static_cast<int>(rank) : m_pair;
+            const int q1 = fdiv(m_t, p.fd_tw), tw = m_t - q1 * p.tiles_w, tn = fdiv(q1, p.fd_th), th = q1 - tn * p.tiles_h;
+            const int w = tw * p.BW + row_in_tile % p.BW;
+            const int h = th * p.BH + (row_in_tile / p.BW) % p.BH;
+            const int n = tn * p.BI + row_in_tile / (p.BW * p.BH);
+            const bool valid = row_in_tile < p.BW * p.BH * p.BI && w < p.W && h < p.H && n < p.Nimg;
+            const int row = valid ? (n * p.H + h) * p.W + w : -1;
+            out_row[grp * 128 + row_in_tile] = row;
+            // row of the 2x2-pooled tensor this pixel's window goes to; only the window's top-left pixel writes it
+            pool_row[grp * 128 + row_in_tile] = (valid && ((w | h) & 1) == 0) ? (n * (p.H >> 1) + (h >> 1)) * (p.W >> 1) + (w >> 1) : -1;
+            // the ReLU mask this row will be gated with after the main loop: start moving it towards the L2 now
+            if (p.mask != nullptr && valid)
+                for (int c = n_t * BN; c < p.N && c < n_t * BN + BN; c += 128) prefetch_l2(p.mask + static_cast<long long>(row) * p.N + c);
         }
+        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
 
-        // ---- pass 1: max|acc| of this CTA's tiles (the load of the next 32-column chunk is in flight while this one is reduced)
+        // ---- pass 1: max|acc| of this CTA's tiles.  Rolled loops in both passes: code that runs a few times per launch is
+        //      bound by instruction fetch, and the four warps of a scheduler hide each other's latencies
         int vmax[4] = {0, 0, 0, 0}, vmin[4] = {0, 0, 0, 0};
         bool ok = true;
-#pragma unroll
-        for (int k = 0; k < MAX_UNITS; ++k) {
-            if (!u_live[k] || !ok) continue;
-            const uint32_t failed = mbar_wait(smem_u32(&tfull_bar[u_it[k]]), 0, abort_flag) ? 0u : 1u;
-            if (barrier_or(bar_id, 128, failed)) { if (failed) report_abort(p.status, 4, 2); ok = false; continue; }
-            if (threadIdx.x == 64 && k == 0) PARK_STAMP(4);
-            tc_fence_after();
-            const int cols = p.N - u_col[k];
-            if (cols <= 0) continue;
-            const int nch = cols >= 128 ? 4 : (cols + 31) >> 5;
-            uint32_t va[32], vb[32];
-            tmem_ld_32x32(u_taddr[k], va);
 #pragma unroll 1
-            for (int j = 0; j < nch; j += 2) {
+        for (int it = 0; it < my_tiles; ++it) {
+            const bool up = mbar_wait(smem_u32(&tfull_bar[it]), 0, abort_flag);
+            if (!__all_sync(0xFFFFFFFFu, up)) { if (!up) report_abort(p.status, 4, 2); ok = false; break; }
+            if (threadIdx.x == 64 && it == 0) PARK_STAMP(4);
+            tc_fence_after();
+            const int tile = cta_first + it * cta_step, col0 = (tile - fdiv(tile, p.fd_n) * p.n_tiles) * BN + cg;
+            const bool valid = out_row[it * 128 + row_in_tile] >= 0;
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(it * BN + cg);
+#pragma unroll 1
+            for (int c = 0; c < Split::CHUNKS; ++c) {
+                const int cols = p.N - col0 - 32 * c;
+                if (cols <= 0) break;
+                uint32_t v[32];
+                tmem_ld_32x32(taddr + 32 * c, v);
                 tmem_ld_wait();
-                if (j + 1 < nch) tmem_ld_32x32(u_taddr[k] + (j + 1) * 32, vb);
-                if (u_ri[k].valid) minmax32(va, cols - 32 * j, vmax, vmin);
-                tmem_ld_wait();
-                if (j + 2 < nch) tmem_ld_32x32(u_taddr[k] + (j + 2) * 32, va);
-                if (j + 1 < nch && u_ri[k].valid) minmax32(vb, cols - 32 * (j + 1), vmax, vmin);
+                if (valid) minmax32(v, cols, vmax, vmin);
             }
         }
-        unsigned local_max = __reduce_max_sync(0xFFFFFFFFu, fold_minmax(vmax, vmin));
+        const unsigned local_max = __reduce_max_sync(0xFFFFFFFFu, fold_minmax(vmax, vmin));
         int32_t* st = p.state;
         if (lane == 0) warp_max[warp - 2] = local_max;
         if (threadIdx.x == 64) PARK_STAMP(5);
 
         // ---- grid barrier: every CTA has contributed its maximum (one atomic each: atomics on one address
         //      serialise at the L2; the waiters poll with plain acquire loads for the same reason)
-        named_barrier(EPI_BARRIER + 2, 256);
+        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
         if (threadIdx.x == 64) {
             unsigned cta_max = 0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) cta_max = max(cta_max, warp_max[i]);
+            for (int i = 0; i < EPI_WARPS; ++i) cta_max = max(cta_max, warp_max[i]);
             // The maximum and the arrival count sit side by side (st[6], st[7]): two fire-and-forget reductions on the
             // way in (the count's release orders the maximum before it), ONE 64-bit acquire load per poll that returns
             // both -- a fence + atomicAdd + atomicMax read-back would add three round trips to the L2.
@@ -1159,59 +1176,49 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             *shift_slot = arrived ? shift_for(m, p.kind, p.target_bits, &zero_out) : -1;
             if (!arrived) { *abort_flag = 1; report_abort(p.status, 5, 2); }
         }
-        named_barrier(EPI_BARRIER + 2, 256);
+        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
         const int shift = *shift_slot;
         if (threadIdx.x == 64) PARK_STAMP(6);
 
         // ---- pass 2: narrow the parked accumulators with the true shift
         if (ok && shift >= 0) {
-            unsigned long long seed = 0;
-            if (p.mode == ROUND_STOCHASTIC && shift > 0) seed = *p.seed;
-#pragma unroll
-            for (int k = 0; k < MAX_UNITS; ++k) {
-                const int cols = p.N - u_col[k];
-                if (!u_live[k] || cols <= 0) continue;
-                const RowInfo ri = u_ri[k];
-                const int col = u_col[k];
-                const uint32_t taddr = u_taddr[k];
-                const int nch = cols >= 128 ? 4 : (cols + 31) >> 5;  // the store clips the columns beyond
-                const unsigned long long e0 = p.rng_offset + static_cast<unsigned long long>(ri.row_lin) * p.N + col;
-                const int8_t* mrow = (p.mask != nullptr && ri.valid) ? p.mask + ri.row_lin * p.N + col : nullptr;
-                // Each thread writes its own row straight from registers (32-byte pieces = whole L2 sectors): with one
-                // or two units per warpgroup there is nothing for a staged TMA store to overlap with, and its fence,
-                // barriers and the wait for the store engine at the end of the kernel cost more than the stores.
-                int8_t* orow = ri.valid ? p.out8 + ri.row_lin * p.N + col : nullptr;
-                // Max pooling in the same pass (TiMaxpool2d.forward): a warp's 32 rows are whole image rows of the tile
-                // (BW is a power of two <= 16, BH even), so the 2x2 window of lane l is lanes l, l^1, l^BW, l^BW^1:
-                // two shuffles and two byte-wise maxima per word, and the window's top-left lane stores the pooled piece.
-                const bool pooling = p.pool_out != nullptr;  // the same for the whole grid
-                int8_t* prow = (pooling && ri.valid && ri.pool_row >= 0) ? p.pool_out + ri.pool_row * p.N + col : nullptr;
-                uint32_t va[32], vb[32], packed[8];
-                uint4 ma[2], mb[2];  // the mask pieces of the chunk in va / vb, fetched one chunk ahead of their use
-                tmem_ld_32x32(taddr, va);
-                mask_load<2>(mrow, cols, ma);
+            const unsigned long long seed = (p.mode == ROUND_STOCHASTIC && shift > 0) ? *p.seed : 0ull;
+            const bool wide = rows_of_32(p.out8, p.N);
+            // Max pooling in the same pass (TiMaxpool2d.forward): a warp's 32 rows are whole image rows of the tile
+            // (BW is a power of two <= 16, BH even), so the 2x2 window of lane l is lanes l, l^1, l^BW, l^BW^1:
+            // two shuffles and two byte-wise maxima per word, and the window's top-left lane stores the pooled piece.
+            const bool pooling = p.pool_out != nullptr;  // the same for the whole grid
+            const bool wide_pool = pooling && rows_of_32(p.pool_out, p.N);
 #pragma unroll 1
-                for (int j = 0; j < nch; j += 2) {
+            for (int it = 0; it < my_tiles; ++it) {
+                const int tile = cta_first + it * cta_step, col0 = (tile - fdiv(tile, p.fd_n) * p.n_tiles) * BN + cg;
+                const int row = out_row[it * 128 + row_in_tile], prow = pool_row[it * 128 + row_in_tile];
+                const long long off = static_cast<long long>(row) * p.N + col0;
+                const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(it * BN + cg);
+#pragma unroll 1
+                for (int c = 0; c < Split::CHUNKS; ++c) {
+                    const int cols = p.N - col0 - 32 * c;  // columns of the tensor from here on; the same for the whole warp
+                    if (cols <= 0) break;
+                    const int8_t* mrow = (p.mask != nullptr && row >= 0) ? p.mask + off + 32 * c : nullptr;
+                    uint32_t v[32], packed[8];
+                    uint4 mk[2];
+                    tmem_ld_32x32(taddr + 32 * c, v);
+                    mask_load<2>(mrow, cols, mk);
                     tmem_ld_wait();
-                    if (j + 1 < nch) { tmem_ld_32x32(taddr + (j + 1) * 32, vb); mask_load<2>(mrow == nullptr ? nullptr : mrow + 32 * (j + 1), cols - 32 * (j + 1), mb); }
-                    narrow32(va, packed, shift, p.mode, p.relu, seed, p.rng_stream, e0 + 32 * j);
-                    mask_apply<2>(packed, mrow, cols - 32 * j, ma);
-                    store_piece(orow, 32 * j, cols, packed);
-                    if (pooling) { pool_window(packed, p.BW); store_piece(prow, 32 * j, cols, packed); }
-                    tmem_ld_wait();
-                    if (j + 2 < nch) { tmem_ld_32x32(taddr + (j + 2) * 32, va); mask_load<2>(mrow == nullptr ? nullptr : mrow + 32 * (j + 2), cols - 32 * (j + 2), ma); }
-                    if (j + 1 < nch) {
-                        narrow32(vb, packed, shift, p.mode, p.relu, seed, p.rng_stream, e0 + 32 * (j + 1));
-                        mask_apply<2>(packed, mrow, cols - 32 * (j + 1), mb);
-                        store_piece(orow, 32 * (j + 1), cols, packed);
-                        if (pooling) { pool_window(packed, p.BW); store_piece(prow, 32 * (j + 1), cols, packed); }
+                    narrow32(v, packed, shift, p.mode, p.relu, seed, p.rng_stream, p.rng_offset + static_cast<unsigned long long>(off) + 32 * c);
+                    mask_apply<2>(packed, mrow, cols, mk);
+                    // every thread writes its own row straight from registers (32-byte pieces = whole L2 sectors)
+                    store_piece(row >= 0 ? p.out8 + off + 32 * c : nullptr, cols, packed, wide);
+                    if (pooling) {
+                        pool_window(packed, p.BW);
+                        store_piece(prow >= 0 ? p.pool_out + static_cast<long long>(prow) * p.N + col0 + 32 * c : nullptr, cols, packed, wide_pool);
                     }
                 }
             }
         }
         if (threadIdx.x == 64) PARK_STAMP(7);
         // ---- the CTA that leaves last publishes the shift and clears the words for the next call
-        named_barrier(EPI_BARRIER + 2, 256);
+        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
         if (threadIdx.x == 64) {
             if (atomicAdd(&st[4], 1) == static_cast<int>(gridDim.x) - 1) {
                 __threadfence();
@@ -1234,6 +1241,7 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (TWO) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512);
     }
 }
+
 #ifdef NITI_PARKED_TIMING
 }  // namespace niti
 extern "C" __attribute__((visibility("default"))) int niti_debug_stamps(unsigned long long* out) {
@@ -1507,7 +1515,7 @@ static EncodeTiledFn get_encode() {
 // Tensor map with 128-byte swizzle over uint8 (operands) or int32 (outputs) elements; dims/box
 // innermost first, in elements; strides of dims 1.. in bytes.
 static int encode_map(CUtensorMap* map, const void* ptr, bool int32_elems, int rank, const uint64_t* dims,
-                      const uint64_t* strides, const uint32_t* box) {
+                      const uint64_t* strides, const uint32_t* box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     EncodeTiledFn enc = get_encode();
     if (!enc) return set_cuda_error_text("cuTensorMapEncodeTiled is not available from this driver");
     cuuint64_t gdim[4]; cuuint64_t gstr[3]; cuuint32_t bx[4]; cuuint32_t es[4];
@@ -1515,7 +1523,7 @@ static int encode_map(CUtensorMap* map, const void* ptr, bool int32_elems, int r
     for (int i = 0; i + 1 < rank; ++i) gstr[i] = strides[i];
     CUresult r = enc(map, int32_elems ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, rank,
                      const_cast<void*>(ptr), gdim, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         char buf[160];
         snprintf(buf, sizeof buf, "cuTensorMapEncodeTiled failed with CUresult %d (rank %d)", static_cast<int>(r), rank);
@@ -1535,41 +1543,25 @@ static int sm_count() {
     return n;
 }
 
-template <int BN, bool FUSED>
-static int launch_gemm_inst(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p,
-                            cudaStream_t st) {
-    using Cfg = GemmCfg<BN, FUSED, false>;
-    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN, FUSED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+// CTA pairs (TWO): clusters of two CTAs, p.m_tiles counts 256-row tiles
+template <int BN, bool TWO>
+static int launch_gemm_inst(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p, cudaStream_t st) {
+    using Cfg = GemmCfg<BN, TWO>;
+    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
-    int grid = p.m_tiles * p.n_tiles * p.splits;
-    if (grid > sm_count()) grid = sm_count();
-    umma_gemm_kernel<BN, FUSED, false><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(a, b, c, p);
-    return set_cuda_error(cudaGetLastError());
-}
-// CTA pairs: clusters of two CTAs, p.m_tiles counts 256-row tiles
-template <int BN, bool FUSED>
-static int launch_gemm_pair_inst(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p,
-                                 cudaStream_t st) {
-    using Cfg = GemmCfg<BN, FUSED, true>;
-    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN, FUSED, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-    if (e != cudaSuccess) return set_cuda_error(e);
-    int pairs = p.m_tiles * p.n_tiles * p.splits;
-    if (pairs > sm_count() / 2) pairs = sm_count() / 2;
+    int tiles = p.m_tiles * p.n_tiles * p.splits;
+    if (tiles > sm_count() / (TWO ? 2 : 1)) tiles = sm_count() / (TWO ? 2 : 1);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM_BYTES; cfg.stream = st;
+    cfg.gridDim = dim3(TWO ? 2 * tiles : tiles); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM_BYTES; cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BN, FUSED, true>, a, b, c, p));
+    cfg.attrs = attr; cfg.numAttrs = TWO ? 1 : 0;
+    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BN, TWO>, a, b, c, p));
 }
-static int launch_gemm(int bn, bool fused, bool pair, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c,
-                       const GemmParams& p, cudaStream_t st) {
-    if (pair) {
-        if (fused) return bn == 256 ? launch_gemm_pair_inst<256, true>(a, b, c, p, st) : launch_gemm_pair_inst<128, true>(a, b, c, p, st);
-        return bn == 256 ? launch_gemm_pair_inst<256, false>(a, b, c, p, st) : launch_gemm_pair_inst<128, false>(a, b, c, p, st);
-    }
-    if (fused) return bn == 256 ? launch_gemm_inst<256, true>(a, b, c, p, st) : launch_gemm_inst<128, true>(a, b, c, p, st);
+static int launch_gemm(int bn, bool pair, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p,
+                       cudaStream_t st) {
+    if (pair) return bn == 256 ? launch_gemm_inst<256, true>(a, b, c, p, st) : launch_gemm_inst<128, true>(a, b, c, p, st);
     return bn == 256 ? launch_gemm_inst<256, false>(a, b, c, p, st) : launch_gemm_inst<128, false>(a, b, c, p, st);
 }
 // CTA pairs (M = 256 MMAs, B operand split between the two CTAs): bit 0 enables them for GEMMs, bit 1 for
@@ -1580,24 +1572,36 @@ int g_two_cta = 1;
 static bool pair_ok(int m_tiles, int bn, int b_mn, int conv) {
     return (g_two_cta & (conv ? 2 : 1)) && m_tiles >= 2 && (!b_mn || bn == 256);
 }
-template <int BN, bool TWO>
-static int launch_parked_inst(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p,
-                              cudaStream_t st) {
-    using Cfg = ParkedCfg<BN, TWO>;
-    cudaError_t e = cudaFuncSetAttribute(umma_parked_kernel<BN, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+// PARKED: the kernel with the grid barrier (cooperative launch: every CTA must be resident at the same time)
+template <int BN, bool TWO, bool PARKED>
+static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
+    using Cfg = RequantCfg<BN, TWO>;
+    void (*kernel)(CUtensorMap, CUtensorMap, GemmParams);
+    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO>; else kernel = umma_requant_kernel<BN, TWO>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
-    int grid = p.m_tiles * p.n_tiles * p.splits;  // TWO: pairs
-    if (TWO) { if (grid > sm_count() / 2) grid = sm_count() / 2; grid *= 2; }
-    else if (grid > sm_count()) grid = sm_count();
-    // cooperative launch: the grid barrier inside needs every CTA resident at the same time
+    int tiles = p.m_tiles * p.n_tiles;
+    if (tiles > sm_count() / (TWO ? 2 : 1)) tiles = sm_count() / (TWO ? 2 : 1);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM_BYTES; cfg.stream = st;
+    cfg.gridDim = dim3(TWO ? 2 * tiles : tiles); cfg.blockDim = dim3(REQUANT_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM_BYTES; cfg.stream = st;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = TWO ? 2 : 1;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_parked_kernel<BN, TWO>, a, b, c, p));
+    int n = 0;
+    if (PARKED) { attr[n].id = cudaLaunchAttributeCooperative; attr[n].val.cooperative = g_cooperative; ++n; }
+    if (TWO) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = 2; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1; ++n;
+    }
+    cfg.attrs = attr; cfg.numAttrs = n;
+    return set_cuda_error(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
+}
+static int launch_requant(int bn, bool pair, bool parked, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
+    if (parked) {
+        if (pair) return bn == 256 ? launch_requant_inst<256, true, true>(a, b, p, st) : launch_requant_inst<128, true, true>(a, b, p, st);
+        return bn == 256 ? launch_requant_inst<256, false, true>(a, b, p, st) : launch_requant_inst<128, false, true>(a, b, p, st);
+    }
+    if (pair) return bn == 256 ? launch_requant_inst<256, true, false>(a, b, p, st) : launch_requant_inst<128, true, false>(a, b, p, st);
+    if (bn == 64) return launch_requant_inst<64, false, false>(a, b, p, st);
+    return bn == 256 ? launch_requant_inst<256, false, false>(a, b, p, st) : launch_requant_inst<128, false, false>(a, b, p, st);
 }
 // all accumulators of the problem fit in the tensor memory of one wave of CTAs (units: 128-row tiles,
 // or 256-row pair tiles on sm/2 pairs)
@@ -1610,6 +1614,9 @@ static int pick_bn(int m_tiles, int n_cols) {
     const int tiles256 = m_tiles * ((n_cols + 255) / 256);
     return tiles256 * 2 <= sm_count() ? 128 : 256;
 }
+
+// the streaming kernel that narrows also has 64-column tiles
+static int requant_bn(int n_cols, int m_tiles) { return n_cols <= 64 ? 64 : pick_bn(m_tiles, n_cols); }
 
 int g_stage_cap = 0;  // 0: use every compiled stage
 // 1: kernels with a grid barrier are launched cooperatively (the driver guarantees that all their blocks are
@@ -1664,19 +1671,18 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
               int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st) {
     CUtensorMap ma, mb, mc;
     const int a_mn = trans_a ? 1 : 0, b_mn = trans_b ? 0 : 1;
-    const int bn = (N > 128) ? 256 : 128;
-    const bool pair = pair_ok((M + 127) / 128, bn, b_mn, 0);
+    const int bn = fused ? requant_bn(N, 1 << 20) : (N > 128) ? 256 : 128;
+    const bool pair = !fused && pair_ok((M + 127) / 128, bn, b_mn, 0);  // fused: one reduction block, nothing to share
     {
         uint64_t dims[2], str[1]; uint32_t box[2] = {128, 128};
         if (a_mn) { dims[0] = M; dims[1] = K; str[0] = M; } else { dims[0] = K; dims[1] = M; str[0] = K; }
         if (int e = encode_map(&ma, A, false, 2, dims, str, box)) return e;
         if (b_mn) { dims[0] = N; dims[1] = K; str[0] = N; box[1] = 128; } else { dims[0] = K; dims[1] = N; str[0] = K; box[1] = pair ? bn / 2 : bn; }
         if (int e = encode_map(&mb, B, false, 2, dims, str, box)) return e;
-        const uint64_t es = fused ? 1 : 4;
         uint64_t dc[4] = {(uint64_t)N, (uint64_t)M, (uint64_t)splits, 1};
-        uint64_t sc[3] = {(uint64_t)N * es, (uint64_t)M * N * es, (uint64_t)splits * M * N * es};
-        uint32_t bc[4] = {fused ? 128u : 32u, 128, 1, 1};
-        if (int e = encode_map(&mc, out, !fused, 4, dc, sc, bc)) return e;
+        uint64_t sc[3] = {(uint64_t)N * 4, (uint64_t)M * N * 4, (uint64_t)splits * M * N * 4};
+        uint32_t bc[4] = {32, 128, 1, 1};
+        if (!fused) if (int e = encode_map(&mc, out, true, 4, dc, sc, bc)) return e;
     }
     GemmParams p{};
     p.conv = 0; p.M = M; p.N = N; p.num_kb = (K + 127) / 128; p.splits = splits;
@@ -1689,7 +1695,8 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.group_m = (static_cast<long long>(M) + N) * K > (48ll << 20) ? 8 : 0;
     set_fused(&p, fused);
     finish_params(&p);
-    return launch_gemm(bn, fused != nullptr, pair, ma, mb, mc, p, st);
+    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, pair, false, ma, mb, p, st); }
+    return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
 // Forward convolution (flip == 0: x [N,H,W,C] with w [K,R,S,C] -> [N,H,W,K]) or error-backward
@@ -1704,9 +1711,9 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     GemmParams p{};
     pick_pixel_box(Nimg, H, W, &p.BW, &p.BH, &p.BI);
     const int all_m_tiles = ((W + p.BW - 1) / p.BW) * ((H + p.BH - 1) / p.BH) * ((Nimg + p.BI - 1) / p.BI);
-    const int bn = pick_bn(all_m_tiles, outc);
     const bool parked = fused && fused->parked;
-    const bool pair = pair_ok(all_m_tiles, bn, flip ? 1 : 0, 1);
+    const int bn = fused && !parked ? requant_bn(outc, all_m_tiles) : pick_bn(all_m_tiles, outc);
+    const bool pair = bn != 64 && pair_ok(all_m_tiles, bn, flip ? 1 : 0, 1);
     {
         uint64_t dims[4] = {(uint64_t)red, (uint64_t)W, (uint64_t)H, (uint64_t)Nimg};
         uint64_t str[3] = {(uint64_t)red, (uint64_t)W * red, (uint64_t)H * W * red};
@@ -1714,13 +1721,13 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         if (int e = encode_map(&ma, x, false, 4, dims, str, box)) return e;
         uint64_t d2[2] = {(uint64_t)R * S * C, (uint64_t)K};
         uint64_t s2[1] = {(uint64_t)R * S * C};
-        uint32_t b2[2] = {128, flip ? 128u : (uint32_t)(pair ? bn / 2 : bn)};
-        if (int e = encode_map(&mb, w, false, 2, d2, s2, b2)) return e;
-        const uint64_t es = fused ? 1 : 4;
+        const bool narrow_b = flip && bn == 64;  // MN-major rows of 64 bytes
+        uint32_t b2[2] = {narrow_b ? 64u : 128u, flip ? 128u : (uint32_t)(pair ? bn / 2 : bn)};
+        if (int e = encode_map(&mb, w, false, 2, d2, s2, b2, narrow_b ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B)) return e;
         uint64_t dc[4] = {(uint64_t)outc, (uint64_t)W, (uint64_t)H, (uint64_t)Nimg};
-        uint64_t sc[3] = {(uint64_t)outc * es, (uint64_t)W * outc * es, (uint64_t)H * W * outc * es};
-        uint32_t bc[4] = {fused ? 128u : 32u, (uint32_t)p.BW, (uint32_t)p.BH, (uint32_t)p.BI};
-        if (int e = encode_map(&mc, out, !fused, 4, dc, sc, bc)) return e;
+        uint64_t sc[3] = {(uint64_t)outc * 4, (uint64_t)W * outc * 4, (uint64_t)H * W * outc * 4};
+        uint32_t bc[4] = {32, (uint32_t)p.BW, (uint32_t)p.BH, (uint32_t)p.BI};
+        if (!fused) if (int e = encode_map(&mc, out, true, 4, dc, sc, bc)) return e;
     }
     p.conv = 1; p.flip = flip; p.splits = 1;
     p.H = H; p.W = W; p.S = S; p.pad = pad; p.Nimg = Nimg; p.tapstride = C;
@@ -1740,12 +1747,9 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         if (!parked || flip || !pool_box_ok(H, W, p.BW, p.BH)) return NITI_ERR_UNSUPPORTED;
         p.pool_out = fused->pool_out;
     }
-    if (parked) {
-        if (!fits_parked(bn, p.m_tiles * p.n_tiles, pair)) return NITI_ERR_UNSUPPORTED;
-        if (pair) return bn == 256 ? launch_parked_inst<256, true>(ma, mb, mc, p, st) : launch_parked_inst<128, true>(ma, mb, mc, p, st);
-        return bn == 256 ? launch_parked_inst<256, false>(ma, mb, mc, p, st) : launch_parked_inst<128, false>(ma, mb, mc, p, st);
-    }
-    return launch_gemm(bn, fused != nullptr, pair, ma, mb, mc, p, st);
+    if (parked && !fits_parked(bn, p.m_tiles * p.n_tiles, pair)) return NITI_ERR_UNSUPPORTED;
+    if (fused) return launch_requant(bn, pair, parked, ma, mb, p, st);
+    return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
 // the parked kernel can pool 2x2 / stride 2 in its epilogue when every window lies inside one warp's 32 rows of a tile
