@@ -140,7 +140,7 @@ extern "C" int niti_conv_fprop_i8(const int8_t* x, const int8_t* w, int32_t* y32
         int8_t* xcol = static_cast<int8_t*>(scratch);
         int8_t* wp = xcol + align_up(m * 32, 1024);
         if (int e = im2col32(x, xcol, N, H, W, C, R, S, pad, st, w, wp, K)) return e;
-        return umma_gemm(xcol, wp, y32, maxabs, static_cast<int>(m), K, 32, 0, 1, 1, nullptr, status, st);
+        return umma_gemm(xcol, wp, y32, maxabs, static_cast<int>(m), K, 32, 0, 1, 1, nullptr, status, st, 1);
     }
     return simt_conv_fprop(x, w, y32, maxabs, N, H, W, C, K, R, S, pad, st);
 }
@@ -223,7 +223,7 @@ extern "C" int niti_conv_wgrad_i8(const int8_t* x, const int8_t* err, int32_t* g
     int32_t* partial = reinterpret_cast<int32_t*>(xcol + align_up(m * 32, 1024));
     const int splits = umma_gemm_splits(K, 32, static_cast<int>(m));
     if (int e = im2col32(x, xcol, N, H, W, C, R, S, pad, st)) return e;
-    if (int e = umma_gemm(err, xcol, partial, nullptr, K, 32, static_cast<int>(m), 1, 0, splits, nullptr, status, st)) return e;
+    if (int e = umma_gemm(err, xcol, partial, nullptr, K, 32, static_cast<int>(m), 1, 0, splits, nullptr, status, st, 2)) return e;
     return reduce_rows32(partial, splits, K, R * S * C, g32, maxabs, st);
 }
 
@@ -259,7 +259,7 @@ extern "C" int niti_conv_wgrad_patches_i8(const int8_t* patches, const int8_t* e
     const size_t m = static_cast<size_t>(N) * H * W;
     const int splits = umma_gemm_splits(K, 32, static_cast<int>(m));
     int32_t* partial = static_cast<int32_t*>(scratch);
-    if (int e = umma_gemm(err, patches, partial, nullptr, K, 32, static_cast<int>(m), 1, 0, splits, nullptr, status, st)) return e;
+    if (int e = umma_gemm(err, patches, partial, nullptr, K, 32, static_cast<int>(m), 1, 0, splits, nullptr, status, st, 2)) return e;
     return reduce_rows32(partial, splits, K, R * S * C, g32, maxabs, st);
 }
 
@@ -330,7 +330,7 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
     // first launch: narrow with the predicted shift, reduce max|acc|, verify; second launch: redo if it was wrong
     for (int pass = 0; pass < 2; ++pass) {
         f.only_if_redo = pass;
-        int rc = thin ? umma_gemm(xcol, wp, out8, nullptr, static_cast<int>(m), K, 32, 0, 1, 1, &f, status, st)
+        int rc = thin ? umma_gemm(xcol, wp, out8, nullptr, static_cast<int>(m), K, 32, 0, 1, 1, &f, status, st, 1)
                       : umma_conv(in, w, out8, nullptr, N, H, W, C, K, R, S, pad, flip, &f, status, st);
         if (rc) return rc;
     }
@@ -478,6 +478,6 @@ extern "C" int niti_conv_wgrad_builtin_scratch_i8(const int8_t* x, const int8_t*
     int splits = umma_gemm_splits(K, 32, static_cast<int>(m));
     if (splits > max_splits) splits = max_splits;
     if (int e = im2col32(x, xcol, N, H, W, C, R, S, pad, st)) return e;
-    if (int e = umma_gemm(err, xcol, partial, nullptr, K, 32, static_cast<int>(m), 1, 0, splits, nullptr, status, st)) return e;
+    if (int e = umma_gemm(err, xcol, partial, nullptr, K, 32, static_cast<int>(m), 1, 0, splits, nullptr, status, st, 2)) return e;
     return reduce_rows32(partial, splits, K, R * S * C, g32, maxabs, st);
 }

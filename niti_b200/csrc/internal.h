@@ -34,7 +34,7 @@ extern int g_stage_cap;  // experiments: cap on the shared-memory stages the GEM
 // tensor-core (tcgen05) paths, umma_kernels.cu; `out` is int32 (fused == null) or int8
 int umma_gemm_splits(int M, int N, int K);
 int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int M, int N, int K, int trans_a,
-              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st);
+              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st, int rows32 = 0);
 int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int Nimg, int H, int W, int C, int K,
               int R, int S, int pad, int flip, const FusedArgs* fused, int32_t* status, cudaStream_t st);
 bool umma_conv_fits_parked(int Nimg, int H, int W, int outc, int flip);
@@ -65,6 +65,7 @@ int simt_gemm(const int8_t* A, const int8_t* B, int32_t* C32, unsigned* maxabs, 
               int trans_b, cudaStream_t st);
 int reduce_partials(const int32_t* partial, int splits, long long n, int32_t* out, unsigned* maxabs, cudaStream_t st);
 int reduce_rows32(const int32_t* partial, int splits, int rows, int cols_out, int32_t* out, unsigned* maxabs, cudaStream_t st);
+// xcol[pixels][32] and wp[K][32] in the order the MMA reads 32-byte rows in (rows32 of umma_gemm).
 // w / wp / K: optionally the layer's filters w[K][R*S*C] are padded to wp[K][32] by the same launch
 int im2col32(const int8_t* x, int8_t* xcol, int Nimg, int H, int W, int C, int R, int S, int pad, cudaStream_t st,
              const int8_t* w = nullptr, int8_t* wp = nullptr, int K = 0);

@@ -203,7 +203,9 @@ int reduce_rows32(const int32_t* partial, int splits, int rows, int cols_out, in
 // Thin convolutions (R*S*C <= 32, the 3-channel first layer) run as GEMMs over an explicit patch
 // matrix: xcol[pixel][32] holds the R*S*C bytes of the pixel's receptive field, zero padded.
 // One thread per pixel: walks the receptive field in (r, s, c) order, packs the bytes into eight
-// words and writes the 32-byte row with two 16-byte stores.
+// words and writes the 32-byte row with two 16-byte stores.  Rows lie as the tensor cores read operands of 32-byte rows
+// (32-byte swizzle: the two 16-byte halves of rows 4..7 of every eight change places), so that a tile is one contiguous copy.
+__host__ __device__ inline int patch_half(long long row, int half) { return half ^ (static_cast<int>(row >> 2) & 1); }
 __global__ void __launch_bounds__(256)
 im2col32_kernel(const int8_t* __restrict__ x, uint4* __restrict__ xcol, int Nimg, int H, int W, int C, int R, int S, int pad,
                 const int8_t* __restrict__ w, int8_t* __restrict__ wp, int K) {
@@ -213,7 +215,7 @@ im2col32_kernel(const int8_t* __restrict__ x, uint4* __restrict__ xcol, int Nimg
     if (wp != nullptr)
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K * 32; i += gridDim.x * blockDim.x) {
             const int k = i >> 5, e = i & 31;
-            wp[i] = e < rsc ? w[k * rsc + e] : int8_t(0);
+            wp[k * 32 + 16 * patch_half(k, e >> 4) + (e & 15)] = e < rsc ? w[k * rsc + e] : int8_t(0);
         }
     for (long long pix = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; pix < pixels;
          pix += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -236,8 +238,8 @@ im2col32_kernel(const int8_t* __restrict__ x, uint4* __restrict__ xcol, int Nimg
             }
             word[t] = v;
         }
-        xcol[pix * 2] = make_uint4(word[0], word[1], word[2], word[3]);
-        xcol[pix * 2 + 1] = make_uint4(word[4], word[5], word[6], word[7]);
+        xcol[pix * 2 + patch_half(pix, 0)] = make_uint4(word[0], word[1], word[2], word[3]);
+        xcol[pix * 2 + patch_half(pix, 1)] = make_uint4(word[4], word[5], word[6], word[7]);
     }
 }
 int im2col32(const int8_t* x, int8_t* xcol, int Nimg, int H, int W, int C, int R, int S, int pad, cudaStream_t st,

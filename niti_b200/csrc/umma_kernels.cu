@@ -53,6 +53,7 @@ constexpr int PANEL_BYTES = 128 * ROW_BYTES; // one 128-row operand panel
 constexpr int UMMA_THREADS = 192;
 constexpr uint32_t SWIZZLE_128B_CODE = 2;
 constexpr uint32_t SWIZZLE_64B_CODE = 4;
+constexpr uint32_t SWIZZLE_32B_CODE = 6;
 constexpr int EPI_CHUNK_BYTES = 128 * 32 * 4;  // 128 rows x 32 int32 columns, one TMA store box
 constexpr int EPI_BARRIER = 1;                 // named barrier of the 128 epilogue threads
 
@@ -91,6 +92,12 @@ struct GemmParams {
     int m_tiles, n_tiles;
     int a_mn, b_mn;        // operand majors (0 = K-major, 1 = MN-major)
     int a_bytes;           // bytes one A stage receives from TMA
+    // Operands of 32-byte rows that lie in memory as the MMA reads them (32-byte swizzle: see patch_half), loaded with
+    // one untiled bulk copy instead of a box of 128 rows.  1: A [M][32] and B [N][32], one reduction block;
+    // 2: B [reduction][32] as 32 MN-major columns.
+    int rows32;
+    const int8_t* a32; const int8_t* b32;
+    int K;                 // rows32 == 2: reduction length
     // convolution geometry
     int H, W, S, pad, Nimg;
     int flip;              // 1: error-backward, taps are read mirrored (offset pad - r instead of r - pad)
@@ -299,7 +306,8 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
     const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
     const int conv = keep_reg(p.conv), flip = keep_reg(p.flip), pad = keep_reg(p.pad), S = keep_reg(p.S), cblocks = keep_reg(p.cblocks);
     const int tapstride = keep_reg(p.tapstride), b_mn = keep_reg(p.b_mn), a_mn = keep_reg(p.a_mn);
-    const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg(TWO ? 2 * (p.a_bytes + BNH * ROW_BYTES) : p.a_bytes + BN * ROW_BYTES));
+    const int rows32 = keep_reg(p.rows32);
+    const uint32_t tx_full = static_cast<uint32_t>(keep_reg(TWO ? 2 * (p.a_bytes + BNH * ROW_BYTES) : p.a_bytes + BN * ROW_BYTES));
     int s = 0; uint32_t ph = 0;
     uint32_t sa = smem0, fb_cur = full0, eb_cur = empty0;  // running stage pointers, wrapping with the ring
     DBG_DECL;
@@ -329,6 +337,12 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
             DBG_ACC(22, 1);
             const uint32_t sb = sa + PANEL_BYTES;
             uint32_t fb = fb_cur;
+            uint32_t tx_bytes = tx_full, tx_b = 0;
+            if (rows32 != 0) {  // the last rows of an operand may be fewer than a tile's; what they leave in the stage meets zeros or rows nobody stores
+                const int b_rows = rows32 == 1 ? min(BN, p.N - ncol) : min(128, p.K - kb * 128);
+                tx_b = static_cast<uint32_t>(b_rows) * 32u;
+                tx_bytes = tx_b + (rows32 == 1 ? static_cast<uint32_t>(min(BLOCK_M, p.M - m_t * BLOCK_M)) * 32u : static_cast<uint32_t>(PANEL_BYTES));
+            }
             if (elect_one()) {
                 if (TWO) {
                     if (rank == 0) mbar_arrive_expect_tx(fb, tx_bytes);
@@ -351,6 +365,12 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
                         if (TWO) tma_load_2d_pair(sb, tmB, fb, tap * tapstride + cb * ROW_BYTES, ncol);
                         else     tma_load_2d(sb, tmB, fb, tap * tapstride + cb * ROW_BYTES, ncol);
                     }
+                } else if (rows32 == 1) {
+                    bulk_load(sa, p.a32 + static_cast<long long>(m_t) * (BLOCK_M * 32), tx_bytes - tx_b, fb);
+                    bulk_load(sb, p.b32 + static_cast<long long>(ncol) * 32, tx_b, fb);
+                } else if (rows32 == 2) {
+                    tma_load_2d(sa, tmA, fb, m_t * BLOCK_M, kb * 128);
+                    bulk_load(sb, p.b32 + static_cast<long long>(kb) * (128 * 32), tx_b, fb);
                 } else {
                     if (TWO) {
                         if (a_mn) tma_load_2d_pair(sa, tmA, fb, m_t * BLOCK_M, kb * 128);
@@ -397,7 +417,7 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     constexpr bool PARKED = NACC == 0;
     const int mn_tiles = p.m_tiles * p.n_tiles;
     const int total_tiles = mn_tiles * p.splits;
-    const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, BN, p.a_mn, p.b_mn);
+    const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, p.rows32 == 2 ? 32 : BN, p.a_mn, p.b_mn);
     const int nst = (p.nstages > 0 && p.nstages < STAGES) ? p.nstages : STAGES;
     const int first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
@@ -406,17 +426,17 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
     // operand descriptors of stage 0 (a stage's are these advanced by the stage offset) and the K = 32 steps
     const uint32_t s0 = smem_u32(smem);
-    const uint64_t a_base = p.a_mn ? make_smem_desc(s0, PANEL_BYTES, 1024, SWIZZLE_128B_CODE) : make_smem_desc(s0, 16, 1024, SWIZZLE_128B_CODE);
+    const uint64_t a_base = p.rows32 == 1 ? make_smem_desc(s0, 16, 256, SWIZZLE_32B_CODE) : p.a_mn ? make_smem_desc(s0, PANEL_BYTES, 1024, SWIZZLE_128B_CODE) : make_smem_desc(s0, 16, 1024, SWIZZLE_128B_CODE);
     // a 64-column MN-major operand has rows of 64 bytes: 64-byte swizzle, 8-row groups of 512 bytes
-    const uint64_t b_base = p.b_mn ? (BN == 64 ? make_smem_desc(s0 + PANEL_BYTES, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
+    const uint64_t b_base = p.rows32 != 0 ? make_smem_desc(s0 + PANEL_BYTES, 1024, 256, SWIZZLE_32B_CODE) : p.b_mn ? (BN == 64 ? make_smem_desc(s0 + PANEL_BYTES, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
                                                : make_smem_desc(s0 + PANEL_BYTES, PANEL_BYTES, 1024, SWIZZLE_128B_CODE))
                                    : make_smem_desc(s0 + PANEL_BYTES, 16, 1024, SWIZZLE_128B_CODE);
     const uint32_t a_step = static_cast<uint32_t>(keep_reg((p.a_mn ? 32 * ROW_BYTES : 32) >> 4));  // in descriptor units of 16 bytes
-    const uint32_t b_step = static_cast<uint32_t>(keep_reg((p.b_mn ? 32 * (BN == 64 ? 64 : ROW_BYTES) : 32) >> 4));
+    const uint32_t b_step = static_cast<uint32_t>(keep_reg((p.rows32 == 2 ? 32 * 32 : p.b_mn ? 32 * (BN == 64 ? 64 : ROW_BYTES) : 32) >> 4));
     const int conv = keep_reg(p.conv), red = keep_reg(p.red), cblocks = keep_reg(p.cblocks), num_kb = keep_reg(p.num_kb), splits = keep_reg(p.splits);
     int s = 0; uint32_t ph = 0; bool ok = true; int it = 0;
     // every reduction block has four MMAs unless a conv tap's channel count ends in a partial 128-byte block
-    const bool all4 = !conv || (red & 127) == 0;
+    const bool all4 = conv ? (red & 127) == 0 : p.rows32 != 1;
     // running stage pointers: descriptors and barrier addresses advance by one stage per block and wrap with the ring
     const uint64_t stage_step = STAGE_BYTES >> 4;
     uint64_t a_cur = a_base, b_cur = b_base;
@@ -453,7 +473,7 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
             } else {
                 // a partial block: issue only the MMAs (K = 32 each) that cover real channels (the rest is TMA zero fill)
                 const int left = red - cb * 128;
-                const int nmma = left >= 128 ? 4 : (left + 31) >> 5;
+                const int nmma = !conv ? 1 : left >= 128 ? 4 : (left + 31) >> 5;  // rows32 == 1: the one block is 32 deep
                 if (++cb == cblocks) cb = 0;
                 mbar_wait_quiet(full_cur, ph, abort_addr);
                 if (elect_one()) {
@@ -1667,12 +1687,16 @@ int umma_gemm_splits(int M, int N, int K) {
 
 // out[splits][M][N] (splits == 1: the result itself) = op(A) * op(B) over disjoint reduction ranges.
 // `fused` == null: int32 out; otherwise int8 out narrowed by the shift in fused->state[0] (splits must be 1).
+// rows32: operands of 32-byte rows as im2col32 writes them (1: A and B, K = 32; 2: B only, N = 32).  As boxes of a
+// tensor map such rows cost the TMA unit about 18 cycles each, inner extent beyond the row and all: one 128 x 128 tile of
+// a first layer (256 rows) took 4600 cycles, whatever its epilogue did.  3 -> 128 channels, 500 images: 109 -> 68 us
+// with the gather, 3 -> 64, 1024 images: the product alone 110 -> 44 us.
 int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int M, int N, int K, int trans_a,
-              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st) {
+              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st, int rows32) {
     CUtensorMap ma, mb, mc;
     const int a_mn = trans_a ? 1 : 0, b_mn = trans_b ? 0 : 1;
     const int bn = fused ? requant_bn(N, 1 << 20) : (N > 128) ? 256 : 128;
-    const bool pair = !fused && pair_ok((M + 127) / 128, bn, b_mn, 0);  // fused: one reduction block, nothing to share
+    const bool pair = rows32 == 0 && !fused && pair_ok((M + 127) / 128, bn, b_mn, 0);
     {
         uint64_t dims[2], str[1]; uint32_t box[2] = {128, 128};
         if (a_mn) { dims[0] = M; dims[1] = K; str[0] = M; } else { dims[0] = K; dims[1] = M; str[0] = K; }
@@ -1689,6 +1713,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.m_tiles = (M + 127) / 128; p.n_tiles = (N + bn - 1) / bn;
     if (pair) p.m_tiles = (p.m_tiles + 1) / 2;
     p.a_mn = a_mn; p.b_mn = b_mn; p.a_bytes = PANEL_BYTES;
+    p.rows32 = rows32; p.a32 = A; p.b32 = B; p.K = K;
     p.maxabs = splits > 1 ? nullptr : maxabs; p.status = status;
     p.split_cols = (bn == 256 && p.m_tiles * p.n_tiles * splits <= 2 * (pair ? sm_count() / 2 : sm_count())) ? 1 : 0;
     // operands beyond ~half of the 126 MB L2: order the tiles in compact groups
