@@ -495,6 +495,109 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     DBG_OUT(16);
 }
 
+// ---- 3x3 convolutions whose tiles are 8 pixels wide: activations fetched once per filter COLUMN instead of once per tap
+// A stage holds, for one 128-byte channel block and one filter column, the activations of a tile and of the pixel rows
+// above and below it (a box of 8 x (BH + 2) pixels, 18 KB) and the weights of the column's three taps.  An image row of
+// the box is 8 shared-memory rows of 128 bytes, one swizzle atom, so the operand of tap (r, column) is the same panel
+// read from r atoms further on: a change of the descriptor's start address.  Against a box per tap (16 KB of activations
+// and 16 KB of weights for four 128-column MMAs, 550 cycles against 256 on the tensor pipe) a tile moves 199 instead of
+// 288 KB (64 columns: 127 instead of 216), and twelve MMAs instead of four ride on one hand-over between the roles.
+constexpr int HALO_ATOM = 8 * ROW_BYTES;          // one image row of the box
+constexpr int HALO_A_BYTES = 18 * HALO_ATOM;      // at most 16 + 2 image rows
+template <int BN, int STAGES, int STAGE_BYTES>
+__device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, const CUtensorMap* tmA,
+                                                   const CUtensorMap* tmB, const GemmParams& p, volatile int* abort_flag) {
+    const int total_tiles = p.m_tiles * p.n_tiles;
+    const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
+    const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+    const int flip = keep_reg(p.flip), cblocks = keep_reg(p.cblocks), tapstride = keep_reg(p.tapstride), b_mn = keep_reg(p.b_mn);
+    const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg(p.a_bytes + 3 * BN * ROW_BYTES));
+    int s = 0; uint32_t ph = 0;
+    uint32_t sa = smem0, fb = full0, eb = empty0;
+    for (int tile = static_cast<int>(blockIdx.x); tile < total_tiles; tile += static_cast<int>(gridDim.x)) {
+        const int m_t = fdiv(tile, p.fd_n), n_t = tile - m_t * p.n_tiles;
+        const int q1 = fdiv(m_t, p.fd_tw), tw = m_t - q1 * p.tiles_w, pn = fdiv(q1, p.fd_th), th = q1 - pn * p.tiles_h;
+        const int ncol = n_t * BN, px = tw * 8, py = th * p.BH - 1;
+        for (int cb = 0; cb < cblocks; ++cb)
+            for (int sx = 0; sx < 3; ++sx) {
+                mbar_wait_quiet(eb, ph ^ 1u, abort_addr);
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(fb, tx_bytes);
+                    tma_load_4d(sa, tmA, fb, cb * ROW_BYTES, px + (flip ? 1 - sx : sx - 1), py, pn);
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        const int x = (r * 3 + sx) * tapstride;
+                        if (b_mn) tma_load_2d(sa + HALO_A_BYTES + r * BN * ROW_BYTES, tmB, fb, x + ncol, cb * 128);
+                        else      tma_load_2d(sa + HALO_A_BYTES + r * BN * ROW_BYTES, tmB, fb, x + cb * ROW_BYTES, ncol);
+                    }
+                }
+                sa += STAGE_BYTES; fb += 8u; eb += 8u;
+                if (++s == STAGES) { s = 0; ph ^= 1u; sa = smem0; fb = full0; eb = empty0; }
+            }
+    }
+    if (*abort_flag) report_abort(p.status, 1, 0);
+}
+template <int BN, int STAGES, int STAGE_BYTES, int NACC>
+__device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* tfull_bar,
+                                              uint64_t* tempty_bar, uint32_t tmem_base_in, const GemmParams& p, volatile int* abort_flag) {
+    constexpr bool PARKED = NACC == 0;
+    constexpr int MOD = PARKED ? 1 : NACC;
+    const int total_tiles = p.m_tiles * p.n_tiles;
+    const uint32_t idesc = make_idesc_i8(BLOCK_M, BN, 0, p.b_mn);
+    const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_in, 0);
+    const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
+    const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), s0 = smem_u32(smem);
+    const uint64_t a_base = make_smem_desc(s0, 16, 1024, SWIZZLE_128B_CODE);
+    const uint64_t b_base = !p.b_mn ? make_smem_desc(s0 + HALO_A_BYTES, 16, 1024, SWIZZLE_128B_CODE)
+                            : BN == 64 ? make_smem_desc(s0 + HALO_A_BYTES, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
+                                       : make_smem_desc(s0 + HALO_A_BYTES, PANEL_BYTES, 1024, SWIZZLE_128B_CODE);
+    const uint32_t b_step = static_cast<uint32_t>(keep_reg((p.b_mn ? 32 * (BN == 64 ? 64 : ROW_BYTES) : 32) >> 4));
+    const int flip = keep_reg(p.flip), red = keep_reg(p.red), cblocks = keep_reg(p.cblocks);
+    // the panel of filter row r starts r image rows into the box (error-backward reads the taps mirrored)
+    const uint64_t a_first = flip ? (2 * HALO_ATOM) >> 4 : 0;
+    const uint64_t a_next = flip ? ~static_cast<uint64_t>(HALO_ATOM >> 4) + 1 : HALO_ATOM >> 4;
+    int s = 0, it = 0; uint32_t ph = 0;
+    uint64_t a_cur = a_base + a_first, b_cur = b_base;
+    uint32_t full_cur = full0, empty_cur = empty0;
+    for (int tile = static_cast<int>(blockIdx.x); tile < total_tiles; tile += static_cast<int>(gridDim.x), ++it) {
+        const int acc = PARKED ? it : it % MOD;
+        if (!PARKED) {
+            if (!mbar_wait_uniform(smem_u32(&tempty_bar[acc]), ((it / MOD) & 1u) ^ 1u, abort_addr)) { *abort_flag = 1; report_abort(p.status, 2, 1); break; }
+            tc_fence_after();
+        }
+        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+        uint32_t accumulate = 0;
+        for (int cb = 0; cb < cblocks; ++cb) {
+            const int left = red - cb * 128;
+            for (int sx = 0; sx < 3; ++sx) {
+                mbar_wait_quiet(full_cur, ph, abort_addr);
+                if (left >= 128) {
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        umma_seq4(d_tmem, a_cur + r * a_next, b_cur + static_cast<uint64_t>(r * BN * ROW_BYTES >> 4), 2, b_step, idesc, accumulate);
+                        accumulate = 1;
+                    }
+                    if (elect_one()) umma_commit(empty_cur);
+                } else {  // only the MMAs (K = 32 each) that cover real channels; the rest of the rows is TMA zero fill
+                    const int nmma = (left + 31) >> 5;
+                    if (elect_one()) {
+                        for (int r = 0; r < 3; ++r)
+                            for (int k = 0; k < nmma; ++k)
+                                umma_i8(d_tmem, a_cur + r * a_next + 2 * k, b_cur + static_cast<uint64_t>(r * BN * ROW_BYTES >> 4) + k * b_step, idesc,
+                                        accumulate | static_cast<uint32_t>(r + k != 0));
+                        umma_commit(empty_cur);
+                    }
+                    accumulate = 1;
+                }
+                a_cur += STAGE_BYTES >> 4; b_cur += STAGE_BYTES >> 4; full_cur += 8u; empty_cur += 8u;
+                if (++s == STAGES) { s = 0; ph ^= 1u; a_cur = a_base + a_first; b_cur = b_base; full_cur = full0; empty_cur = empty0; }
+            }
+        }
+        if (elect_one()) umma_commit(smem_u32(&tfull_bar[acc]));
+    }
+    if (*abort_flag) report_abort(p.status, 3, 1);
+}
+
 __device__ __forceinline__ unsigned fold_minmax(const int (&vmax)[4], const int (&vmin)[4]) {
     const int hi = max(max(vmax[0], vmax[1]), max(vmax[2], vmax[3]));
     const int lo = min(min(vmin[0], vmin[1]), min(vmin[2], vmin[3]));
@@ -836,10 +939,10 @@ struct EpiSplit {
 };
 // Operand ring and accumulators of the kernels that narrow.  BN = 64 serves layers of up to 64 output channels: with
 // 128-column tiles half of the tensor work, of the accumulator reads and of the weight traffic was padding.
-template <int BN, bool TWO>
+template <int BN, bool TWO, bool HALO>
 struct RequantCfg {
     static constexpr int B_STAGE_BYTES = (TWO ? BN / 2 : BN) * ROW_BYTES;
-    static constexpr int STAGE_BYTES = PANEL_BYTES + B_STAGE_BYTES;
+    static constexpr int STAGE_BYTES = HALO ? HALO_A_BYTES + 3 * B_STAGE_BYTES : PANEL_BYTES + B_STAGE_BYTES;
     static constexpr int STAGES = 216 * 1024 / STAGE_BYTES;
     static constexpr int NACC = BN == 256 ? 2 : 4;  // streaming: accumulators in flight
     static constexpr int TABLE_BYTES = 2 * 4 * 128 * 4;  // parked: output row and pooled row of every row of the CTA's tiles
@@ -848,10 +951,10 @@ struct RequantCfg {
 };
 
 // Streaming kernel: narrows with the shift in state[0]; the last CTA derives the true one from max|acc|.
-template <int BN, bool TWO>
+template <int BN, bool TWO, bool HALO>
 __global__ void __launch_bounds__(REQUANT_THREADS, 1)
 umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
-    using Cfg = RequantCfg<BN, TWO>;
+    using Cfg = RequantCfg<BN, TWO, HALO>;
     using Split = EpiSplit<BN>;
     constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC;
     if (p.only_if_redo) {
@@ -901,11 +1004,14 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (warp == 0) {
-        producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        if constexpr (HALO) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
-        if (rank == 0)
-            mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+        if (rank == 0) {
+            if constexpr (HALO) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+        }
         __syncwarp();
     } else {
         const int grp = (warp - 2) >> 2;
@@ -1059,10 +1165,10 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // ------------------------------------------------------------------------------------------------
 constexpr unsigned long long GRID_BARRIER_LIMIT_NS = 500000000ull;  // 0.5 s
 
-template <int BN, bool TWO>
+template <int BN, bool TWO, bool HALO>
 __global__ void __launch_bounds__(REQUANT_THREADS, 1)
 umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
-    using Cfg = RequantCfg<BN, TWO>;
+    using Cfg = RequantCfg<BN, TWO, HALO>;
     using Split = EpiSplit<BN>;
     constexpr int STAGES = Cfg::STAGES;
     static_assert(BN >= 128 && 512 / BN <= 4, "all four warp groups share every tile; tables of four tiles");
@@ -1108,11 +1214,14 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (warp == 0) {
-        producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        if constexpr (HALO) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
-        if (rank == 0)
-            mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
+        if (rank == 0) {
+            if constexpr (HALO) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, 0>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
+            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
+        }
         __syncwarp();
     } else {
         const int grp = (warp - 2) >> 2;
@@ -1593,11 +1702,11 @@ static bool pair_ok(int m_tiles, int bn, int b_mn, int conv) {
     return (g_two_cta & (conv ? 2 : 1)) && m_tiles >= 2 && (!b_mn || bn == 256);
 }
 // PARKED: the kernel with the grid barrier (cooperative launch: every CTA must be resident at the same time)
-template <int BN, bool TWO, bool PARKED>
+template <int BN, bool TWO, bool HALO, bool PARKED>
 static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
-    using Cfg = RequantCfg<BN, TWO>;
+    using Cfg = RequantCfg<BN, TWO, HALO>;
     void (*kernel)(CUtensorMap, CUtensorMap, GemmParams);
-    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO>; else kernel = umma_requant_kernel<BN, TWO>;
+    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, HALO>; else kernel = umma_requant_kernel<BN, TWO, HALO>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     int tiles = p.m_tiles * p.n_tiles;
@@ -1614,14 +1723,17 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
     cfg.attrs = attr; cfg.numAttrs = n;
     return set_cuda_error(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
 }
-static int launch_requant(int bn, bool pair, bool parked, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
+static int launch_requant(int bn, bool pair, bool halo, bool parked, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p,
+                          cudaStream_t st) {
     if (parked) {
-        if (pair) return bn == 256 ? launch_requant_inst<256, true, true>(a, b, p, st) : launch_requant_inst<128, true, true>(a, b, p, st);
-        return bn == 256 ? launch_requant_inst<256, false, true>(a, b, p, st) : launch_requant_inst<128, false, true>(a, b, p, st);
+        if (pair) return bn == 256 ? launch_requant_inst<256, true, false, true>(a, b, p, st) : launch_requant_inst<128, true, false, true>(a, b, p, st);
+        if (halo) return launch_requant_inst<128, false, true, true>(a, b, p, st);
+        return bn == 256 ? launch_requant_inst<256, false, false, true>(a, b, p, st) : launch_requant_inst<128, false, false, true>(a, b, p, st);
     }
-    if (pair) return bn == 256 ? launch_requant_inst<256, true, false>(a, b, p, st) : launch_requant_inst<128, true, false>(a, b, p, st);
-    if (bn == 64) return launch_requant_inst<64, false, false>(a, b, p, st);
-    return bn == 256 ? launch_requant_inst<256, false, false>(a, b, p, st) : launch_requant_inst<128, false, false>(a, b, p, st);
+    if (pair) return bn == 256 ? launch_requant_inst<256, true, false, false>(a, b, p, st) : launch_requant_inst<128, true, false, false>(a, b, p, st);
+    if (halo) return bn == 64 ? launch_requant_inst<64, false, true, false>(a, b, p, st) : launch_requant_inst<128, false, true, false>(a, b, p, st);
+    if (bn == 64) return launch_requant_inst<64, false, false, false>(a, b, p, st);
+    return bn == 256 ? launch_requant_inst<256, false, false, false>(a, b, p, st) : launch_requant_inst<128, false, false, false>(a, b, p, st);
 }
 // all accumulators of the problem fit in the tensor memory of one wave of CTAs (units: 128-row tiles,
 // or 256-row pair tiles on sm/2 pairs)
@@ -1675,6 +1787,30 @@ static void pick_pixel_box(int Nimg, int H, int W, int* BW, int* BH, int* BI) {
 
 static bool pool_box_ok(int H, int W, int bw, int bh);
 
+// Tiles of a convolution.  kernel: 0 = int32 out, 1 = streaming, 2 = parked.
+struct ConvPlan { int BW, BH, BI, tiles_w, tiles_h, m_tiles, bn; bool pair, halo; };
+static ConvPlan conv_plan(int Nimg, int H, int W, int outc, bool k3, int flip, int kernel) {
+    ConvPlan c{};
+    pick_pixel_box(Nimg, H, W, &c.BW, &c.BH, &c.BI);
+    c.tiles_w = (W + c.BW - 1) / c.BW; c.tiles_h = (H + c.BH - 1) / c.BH;
+    c.m_tiles = c.tiles_w * c.tiles_h * ((Nimg + c.BI - 1) / c.BI);
+    c.bn = kernel == 1 ? requant_bn(outc, c.m_tiles) : pick_bn(c.m_tiles, outc);
+    c.pair = c.bn != 64 && pair_ok(c.m_tiles, c.bn, flip, 1);
+    // 8-pixel-wide tiles of one image with the activations of three taps in one load (producer_halo_role): up to 128
+    // columns, where the loads and not the MMAs set the pace (128 -> 128 at 32x32, batch 128: 28.0 -> 19.5 us; 64 -> 64,
+    // batch 1024: 157 -> 119).  A tile so loaded takes about 0.7 of the time, so a quarter more of them (maps that 8 x 16
+    // pixels cover badly) is still a gain.
+    if (k3 && kernel != 0 && !c.pair && c.bn <= 128) {
+        const int th = (H + 15) / 16, bh = (H + th - 1) / th, tw = (W + 7) / 8;
+        const long long tiles = static_cast<long long>(tw) * th * Nimg;
+        if (4 * tiles <= 5ll * c.m_tiles && (kernel != 2 || fits_parked(c.bn, static_cast<int>(tiles) * ((outc + c.bn - 1) / c.bn), false))) {
+            c.halo = true;
+            c.BW = 8; c.BH = bh; c.BI = 1; c.tiles_w = tw; c.tiles_h = th; c.m_tiles = static_cast<int>(tiles);
+        }
+    }
+    return c;
+}
+
 int umma_gemm_splits(int M, int N, int K) {
     const int bn = (N > 128) ? 256 : 128;
     const int tiles = ((M + 127) / 128) * ((N + bn - 1) / bn);
@@ -1720,7 +1856,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.group_m = (static_cast<long long>(M) + N) * K > (48ll << 20) ? 8 : 0;
     set_fused(&p, fused);
     finish_params(&p);
-    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, pair, false, ma, mb, p, st); }
+    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, false, false, ma, mb, p, st); }
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
@@ -1734,15 +1870,15 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     const int red = flip ? K : C;   // reduction channels per tap
     const int outc = flip ? C : K;  // output channels
     GemmParams p{};
-    pick_pixel_box(Nimg, H, W, &p.BW, &p.BH, &p.BI);
-    const int all_m_tiles = ((W + p.BW - 1) / p.BW) * ((H + p.BH - 1) / p.BH) * ((Nimg + p.BI - 1) / p.BI);
     const bool parked = fused && fused->parked;
-    const int bn = fused && !parked ? requant_bn(outc, all_m_tiles) : pick_bn(all_m_tiles, outc);
-    const bool pair = bn != 64 && pair_ok(all_m_tiles, bn, flip ? 1 : 0, 1);
+    const ConvPlan plan = conv_plan(Nimg, H, W, outc, R == 3 && S == 3 && pad == 1, flip, !fused ? 0 : parked ? 2 : 1);
+    const int bn = plan.bn;
+    const bool pair = plan.pair;
+    p.BW = plan.BW; p.BH = plan.BH; p.BI = plan.BI;
     {
         uint64_t dims[4] = {(uint64_t)red, (uint64_t)W, (uint64_t)H, (uint64_t)Nimg};
         uint64_t str[3] = {(uint64_t)red, (uint64_t)W * red, (uint64_t)H * W * red};
-        uint32_t box[4] = {128, (uint32_t)p.BW, (uint32_t)p.BH, (uint32_t)p.BI};
+        uint32_t box[4] = {128, (uint32_t)p.BW, (uint32_t)(plan.halo ? p.BH + 2 : p.BH), (uint32_t)p.BI};
         if (int e = encode_map(&ma, x, false, 4, dims, str, box)) return e;
         uint64_t d2[2] = {(uint64_t)R * S * C, (uint64_t)K};
         uint64_t s2[1] = {(uint64_t)R * S * C};
@@ -1756,13 +1892,12 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     }
     p.conv = 1; p.flip = flip; p.splits = 1;
     p.H = H; p.W = W; p.S = S; p.pad = pad; p.Nimg = Nimg; p.tapstride = C;
-    p.tiles_w = (W + p.BW - 1) / p.BW; p.tiles_h = (H + p.BH - 1) / p.BH;
-    const int tiles_n = (Nimg + p.BI - 1) / p.BI;
+    p.tiles_w = plan.tiles_w; p.tiles_h = plan.tiles_h;
     p.cblocks = (red + 127) / 128; p.red = red;
     p.M = Nimg * H * W; p.N = outc; p.num_kb = R * S * p.cblocks;
-    p.m_tiles = p.tiles_w * p.tiles_h * tiles_n; p.n_tiles = (outc + bn - 1) / bn;
+    p.m_tiles = plan.m_tiles; p.n_tiles = (outc + bn - 1) / bn;
     if (pair) p.m_tiles = (p.m_tiles + 1) / 2;
-    p.a_mn = 0; p.b_mn = flip ? 1 : 0; p.a_bytes = p.BW * p.BH * p.BI * ROW_BYTES;
+    p.a_mn = 0; p.b_mn = flip ? 1 : 0; p.a_bytes = p.BW * (plan.halo ? p.BH + 2 : p.BH) * p.BI * ROW_BYTES;
     p.maxabs = maxabs; p.status = status;
     p.split_cols = (bn == 256 && p.m_tiles * p.n_tiles <= 2 * (pair ? sm_count() / 2 : sm_count())) ? 1 : 0;
     set_fused(&p, fused);
@@ -1773,7 +1908,7 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         p.pool_out = fused->pool_out;
     }
     if (parked && !fits_parked(bn, p.m_tiles * p.n_tiles, pair)) return NITI_ERR_UNSUPPORTED;
-    if (fused) return launch_requant(bn, pair, parked, ma, mb, p, st);
+    if (fused) return launch_requant(bn, pair, plan.halo, parked, ma, mb, p, st);
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
@@ -1781,19 +1916,14 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
 static bool pool_box_ok(int H, int W, int bw, int bh) {
     return H % 2 == 0 && W % 2 == 0 && bh % 2 == 0 && (bw == 2 || bw == 4 || bw == 8 || bw == 16);
 }
-bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc) {
-    int bw, bh, bi;
-    pick_pixel_box(Nimg, H, W, &bw, &bh, &bi);
-    return pool_box_ok(H, W, bw, bh) && umma_conv_fits_parked(Nimg, H, W, outc, 0);
+bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc, bool k3) {
+    const ConvPlan plain = conv_plan(Nimg, H, W, outc, false, 0, 2), c = conv_plan(Nimg, H, W, outc, k3, 0, 2);
+    return pool_box_ok(H, W, plain.BW, plain.BH) && pool_box_ok(H, W, c.BW, c.BH) && umma_conv_fits_parked(Nimg, H, W, outc, false, 0);
 }
 
-bool umma_conv_fits_parked(int Nimg, int H, int W, int outc, int flip) {
-    int bw, bh, bi;
-    pick_pixel_box(Nimg, H, W, &bw, &bh, &bi);
-    const int m_tiles = ((W + bw - 1) / bw) * ((H + bh - 1) / bh) * ((Nimg + bi - 1) / bi);
-    const int bn = pick_bn(m_tiles, outc);
-    const bool pair = pair_ok(m_tiles, bn, flip, 1);
-    return fits_parked(bn, (pair ? (m_tiles + 1) / 2 : m_tiles) * ((outc + bn - 1) / bn), pair);
+bool umma_conv_fits_parked(int Nimg, int H, int W, int outc, bool k3, int flip) {
+    const ConvPlan c = conv_plan(Nimg, H, W, outc, k3, flip, 2);
+    return fits_parked(c.bn, (c.pair ? (c.m_tiles + 1) / 2 : c.m_tiles) * ((outc + c.bn - 1) / c.bn), c.pair);
 }
 
 static void wgrad_plan(int Nimg, int H, int W, int C, int K, int R, int max_splits, WgradParams* p) {
