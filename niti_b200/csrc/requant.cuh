@@ -78,4 +78,56 @@ __device__ __forceinline__ int8_t narrow(int x, int shift, int mode, uint32_t rn
     return static_cast<int8_t>(clamp127(x < 0 ? -v : v));
 }
 
+// ---- four values at a time (shift > 0)
+// Two int32 -> two saturated bytes in the low half of the result, `upper` moved into the high half
+// (cvt.pack: d = upper << 16 | sat(hi) << 8 | sat(lo)).
+__device__ __forceinline__ uint32_t pack2_sat_s8(int hi, int lo, uint32_t upper) {
+    uint32_t d;
+    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(upper));
+    return d;
+}
+__device__ __forceinline__ uint32_t pack2_sat_u8(int hi, int lo, uint32_t upper) {
+    uint32_t d;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(upper));
+    return d;
+}
+// Round half away from zero is (x + half + (x >> 31)) >> shift with an arithmetic shift (for x < 0 that is
+// -((|x| + half) >> shift)); the saturating pack clamps to a byte and one packed min / max finishes the clamp to
+// +-127 (ReLU: the unsigned pack turns negatives into 0).  About 3 instructions per value.
+template <bool RELU>
+__device__ __forceinline__ uint32_t narrow4_nearest(const uint32_t* v, int shift, int half) {
+    int y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int x = static_cast<int>(v[j]);
+        y[j] = RELU ? (x + half) >> shift : (x + half + (x >> 31)) >> shift;
+    }
+    if (RELU) return __vminu4(pack2_sat_u8(y[1], y[0], pack2_sat_u8(y[3], y[2], 0u)), 0x7F7F7F7Fu);
+    return __vmaxs4(pack2_sat_s8(y[1], y[0], pack2_sat_s8(y[3], y[2], 0u)), 0x81818181u);
+}
+// Stochastic rounding: with lo the dropped bits of |x| and r the random word's, |x| is rounded up exactly
+// when lo > r, i.e. when lo + (mask - r) carries into bit `shift`: y = (|x| + (~r & mask)) >> shift.  For x < 0 the
+// negated quotient is the arithmetic shift (x + (r & mask)) >> shift (-floor(a / d) = floor((d - 1 - a) / d)), so both
+// signs are one add and one shift behind a three-input logic operation.  Shifts below 24 only: |x| is then below 2^31 - 2^shift.
+template <bool RELU>
+__device__ __forceinline__ uint32_t narrow4_stochastic(const uint32_t* v, int shift, uint32_t mask, const uint32_t (&rnd)[4]) {
+    int y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int x = static_cast<int>(v[j]);
+        y[j] = (x + static_cast<int>((rnd[j] ^ ~static_cast<uint32_t>(x >> 31)) & mask)) >> shift;
+    }
+    if (RELU) return __vminu4(pack2_sat_u8(y[1], y[0], pack2_sat_u8(y[3], y[2], 0u)), 0x7F7F7F7Fu);
+    return __vmaxs4(pack2_sat_s8(y[1], y[0], pack2_sat_s8(y[3], y[2], 0u)), 0x81818181u);
+}
+// Pseudo-stochastic rounding (the upper half of the dropped bits against their lower half), clamped to 127 in magnitude.
+__device__ __forceinline__ int narrow_pseudo(int x, int shift) {
+    const uint32_t a = static_cast<uint32_t>(x < 0 ? -x : x);
+    const int h = shift >> 1;
+    const uint32_t lo = a & ((1u << shift) - 1u);
+    const uint32_t up = (lo >> h) > ((lo & ((1u << h) - 1u)) << (shift & 1)) ? 1u : 0u;
+    const int v = static_cast<int>(min((a >> shift) + up, 127u));
+    return x < 0 ? -v : v;
+}
+
 }  // namespace niti

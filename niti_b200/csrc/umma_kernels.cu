@@ -152,34 +152,7 @@ __device__ __forceinline__ void report_abort(int32_t* status, int code, int role
     }
 }
 
-// Four accumulators of one row -> four int8 packed in a word (NITI's shift, see requant.cuh).
-// Round-to-nearest (the default of activations and errors) gets a short branch-free form, below.
-// Two int32 -> two saturated bytes in the low half of the result, `upper` moved into the high half
-// (cvt.pack: d = upper << 16 | sat(hi) << 8 | sat(lo)).
-__device__ __forceinline__ uint32_t pack2_sat_s8(int hi, int lo, uint32_t upper) {
-    uint32_t d;
-    asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(upper));
-    return d;
-}
-__device__ __forceinline__ uint32_t pack2_sat_u8(int hi, int lo, uint32_t upper) {
-    uint32_t d;
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(upper));
-    return d;
-}
-// Round half away from zero is (x + half + (x >> 31)) >> shift with an arithmetic shift (for x < 0 that is
-// -((|x| + half) >> shift)); the saturating pack clamps to a byte and one packed min / max finishes the clamp to
-// +-127 (ReLU: the unsigned pack turns negatives into 0).  About 3 instructions per value.
-template <bool RELU>
-__device__ __forceinline__ uint32_t narrow4_nearest(const uint32_t* v, int shift, int half) {
-    int y[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int x = static_cast<int>(v[j]);
-        y[j] = RELU ? (x + half) >> shift : (x + half + (x >> 31)) >> shift;
-    }
-    if (RELU) return __vminu4(pack2_sat_u8(y[1], y[0], pack2_sat_u8(y[3], y[2], 0u)), 0x7F7F7F7Fu);
-    return __vmaxs4(pack2_sat_s8(y[1], y[0], pack2_sat_s8(y[3], y[2], 0u)), 0x81818181u);
-}
+// Four accumulators of one row -> four int8 packed in a word, any rounding (the short forms are in requant.cuh).
 __device__ __forceinline__ uint32_t narrow4(const uint32_t* v, int shift, int mode, int relu, const uint32_t* rnd) {
     uint32_t w = 0;
 #pragma unroll
@@ -653,6 +626,16 @@ __device__ __forceinline__ void narrow32(const uint32_t (&v)[32], uint32_t (&pac
         } else {
 #pragma unroll
             for (int i = 0; i < 32; i += 4) packed[i >> 2] = narrow4_nearest<false>(&v[i], shift, half);
+        }
+    } else if (mode == ROUND_STOCHASTIC && shift > 0 && shift < 24 && (e0 & 3ull) == 0) {
+        // The random words of four neighbouring outputs come from one Philox block: ten rounds of two wide multiplications,
+        // which with the short narrowing is what a stochastic epilogue costs; the general form works value by value.
+        const uint32_t mask = (1u << shift) - 1u;
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+            uint32_t rnd[4];
+            random_block(seed, rng_stream, (e0 + i) >> 2, rnd);
+            packed[i >> 2] = relu ? narrow4_stochastic<true>(&v[i], shift, mask, rnd) : narrow4_stochastic<false>(&v[i], shift, mask, rnd);
         }
     } else {
         uint32_t in[32], out[8];
