@@ -477,14 +477,21 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
 // 288 KB (64 columns: 127 instead of 216), and twelve MMAs instead of four ride on one hand-over between the roles.
 constexpr int HALO_ATOM = 8 * ROW_BYTES;          // one image row of the box
 constexpr int HALO_A_BYTES = 18 * HALO_ATOM;      // at most 16 + 2 image rows
-template <int BN, int STAGES, int STAGE_BYTES>
-__device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, const CUtensorMap* tmA,
+// What a stage holds.  HALO_RESIDENT: layers of one channel block and one column tile keep their whole weights (nine taps,
+// 72 or 144 KB) in shared memory behind the ring; they arrive with the first tile, column by column (one barrier each),
+// and a stage is activations only.  The loads are paced by rows of 128 bytes (about 3 cycles each): 432 a tile instead
+// of 1008 (64 columns) or 1584 (128).
+enum LoadMode : int { LOAD_TAPS = 0, LOAD_HALO = 1, LOAD_HALO_RESIDENT = 2 };
+template <int BN, int STAGES, int STAGE_BYTES, bool RESIDENT>
+__device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint32_t weights0, const CUtensorMap* tmA,
                                                    const CUtensorMap* tmB, const GemmParams& p, volatile int* abort_flag) {
     const int total_tiles = p.m_tiles * p.n_tiles;
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
     const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
     const int flip = keep_reg(p.flip), cblocks = keep_reg(p.cblocks), tapstride = keep_reg(p.tapstride), b_mn = keep_reg(p.b_mn);
-    const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg(p.a_bytes + 3 * BN * ROW_BYTES));
+    const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg(p.a_bytes + (RESIDENT ? 0 : 3 * BN * ROW_BYTES)));
+    const uint32_t res0 = smem0 + STAGES * STAGE_BYTES;  // resident weights: [column][filter row]
+    bool weights_due = RESIDENT;
     int s = 0; uint32_t ph = 0;
     uint32_t sa = smem0, fb = full0, eb = empty0;
     for (int tile = static_cast<int>(blockIdx.x); tile < total_tiles; tile += static_cast<int>(gridDim.x)) {
@@ -497,21 +504,27 @@ __device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full
                 if (elect_one()) {
                     mbar_arrive_expect_tx(fb, tx_bytes);
                     tma_load_4d(sa, tmA, fb, cb * ROW_BYTES, px + (flip ? 1 - sx : sx - 1), py, pn);
+                    if (!RESIDENT || weights_due) {
+                        const uint32_t dst = RESIDENT ? res0 + sx * 3 * BN * ROW_BYTES : sa + HALO_A_BYTES;
+                        const uint32_t bar = RESIDENT ? weights0 + 8u * sx : fb;
+                        if (RESIDENT) mbar_arrive_expect_tx(bar, 3 * BN * ROW_BYTES);
 #pragma unroll
-                    for (int r = 0; r < 3; ++r) {
-                        const int x = (r * 3 + sx) * tapstride;
-                        if (b_mn) tma_load_2d(sa + HALO_A_BYTES + r * BN * ROW_BYTES, tmB, fb, x + ncol, cb * 128);
-                        else      tma_load_2d(sa + HALO_A_BYTES + r * BN * ROW_BYTES, tmB, fb, x + cb * ROW_BYTES, ncol);
+                        for (int r = 0; r < 3; ++r) {
+                            const int x = (r * 3 + sx) * tapstride;
+                            if (b_mn) tma_load_2d(dst + r * BN * ROW_BYTES, tmB, bar, x + ncol, cb * 128);
+                            else      tma_load_2d(dst + r * BN * ROW_BYTES, tmB, bar, x + cb * ROW_BYTES, ncol);
+                        }
                     }
                 }
                 sa += STAGE_BYTES; fb += 8u; eb += 8u;
                 if (++s == STAGES) { s = 0; ph ^= 1u; sa = smem0; fb = full0; eb = empty0; }
             }
+        weights_due = false;
     }
     if (*abort_flag) report_abort(p.status, 1, 0);
 }
-template <int BN, int STAGES, int STAGE_BYTES, int NACC>
-__device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* tfull_bar,
+template <int BN, int STAGES, int STAGE_BYTES, int NACC, bool RESIDENT>
+__device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint32_t weights0, uint64_t* tfull_bar,
                                               uint64_t* tempty_bar, uint32_t tmem_base_in, const GemmParams& p, volatile int* abort_flag) {
     constexpr bool PARKED = NACC == 0;
     constexpr int MOD = PARKED ? 1 : NACC;
@@ -521,9 +534,10 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
     const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), s0 = smem_u32(smem);
     const uint64_t a_base = make_smem_desc(s0, 16, 1024, SWIZZLE_128B_CODE);
-    const uint64_t b_base = !p.b_mn ? make_smem_desc(s0 + HALO_A_BYTES, 16, 1024, SWIZZLE_128B_CODE)
-                            : BN == 64 ? make_smem_desc(s0 + HALO_A_BYTES, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
-                                       : make_smem_desc(s0 + HALO_A_BYTES, PANEL_BYTES, 1024, SWIZZLE_128B_CODE);
+    const uint32_t b0 = RESIDENT ? s0 + STAGES * STAGE_BYTES : s0 + HALO_A_BYTES;
+    const uint64_t b_base = !p.b_mn ? make_smem_desc(b0, 16, 1024, SWIZZLE_128B_CODE)
+                            : BN == 64 ? make_smem_desc(b0, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
+                                       : make_smem_desc(b0, PANEL_BYTES, 1024, SWIZZLE_128B_CODE);
     const uint32_t b_step = static_cast<uint32_t>(keep_reg((p.b_mn ? 32 * (BN == 64 ? 64 : ROW_BYTES) : 32) >> 4));
     const int flip = keep_reg(p.flip), red = keep_reg(p.red), cblocks = keep_reg(p.cblocks);
     // the panel of filter row r starts r image rows into the box (error-backward reads the taps mirrored)
@@ -544,6 +558,10 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
             const int left = red - cb * 128;
             for (int sx = 0; sx < 3; ++sx) {
                 mbar_wait_quiet(full_cur, ph, abort_addr);
+                if (RESIDENT) {
+                    if (accumulate == 0) b_cur = b_base;
+                    if (it == 0) mbar_wait_quiet(weights0 + 8u * sx, 0, abort_addr);
+                }
                 if (left >= 128) {
 #pragma unroll
                     for (int r = 0; r < 3; ++r) {
@@ -562,8 +580,11 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
                     }
                     accumulate = 1;
                 }
-                a_cur += STAGE_BYTES >> 4; b_cur += STAGE_BYTES >> 4; full_cur += 8u; empty_cur += 8u;
-                if (++s == STAGES) { s = 0; ph ^= 1u; a_cur = a_base + a_first; b_cur = b_base; full_cur = full0; empty_cur = empty0; }
+                a_cur += STAGE_BYTES >> 4; b_cur += (RESIDENT ? 3 * BN * ROW_BYTES : STAGE_BYTES) >> 4; full_cur += 8u; empty_cur += 8u;
+                if (++s == STAGES) {
+                    s = 0; ph ^= 1u; a_cur = a_base + a_first; full_cur = full0; empty_cur = empty0;
+                    if (!RESIDENT) b_cur = b_base;
+                }
             }
         }
         if (elect_one()) umma_commit(smem_u32(&tfull_bar[acc]));
@@ -922,22 +943,24 @@ struct EpiSplit {
 };
 // Operand ring and accumulators of the kernels that narrow.  BN = 64 serves layers of up to 64 output channels: with
 // 128-column tiles half of the tensor work, of the accumulator reads and of the weight traffic was padding.
-template <int BN, bool TWO, bool HALO>
+template <int BN, bool TWO, int MODE>
 struct RequantCfg {
     static constexpr int B_STAGE_BYTES = (TWO ? BN / 2 : BN) * ROW_BYTES;
-    static constexpr int STAGE_BYTES = HALO ? HALO_A_BYTES + 3 * B_STAGE_BYTES : PANEL_BYTES + B_STAGE_BYTES;
-    static constexpr int STAGES = 216 * 1024 / STAGE_BYTES;
+    static constexpr int STAGE_BYTES = MODE == LOAD_HALO_RESIDENT ? HALO_A_BYTES
+                                       : MODE == LOAD_HALO ? HALO_A_BYTES + 3 * B_STAGE_BYTES : PANEL_BYTES + B_STAGE_BYTES;
+    static constexpr int RESIDENT_BYTES = MODE == LOAD_HALO_RESIDENT ? 9 * B_STAGE_BYTES : 0;
+    static constexpr int STAGES = (216 * 1024 - RESIDENT_BYTES) / STAGE_BYTES;
     static constexpr int NACC = BN == 256 ? 2 : 4;  // streaming: accumulators in flight
     static constexpr int TABLE_BYTES = 2 * 4 * 128 * 4;  // parked: output row and pooled row of every row of the CTA's tiles
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TABLE_BYTES + 1024 /*alignment slack*/ + 512 /*barriers*/;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + RESIDENT_BYTES + TABLE_BYTES + 1024 /*alignment slack*/ + 512 /*barriers*/;
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a CTA");
 };
 
 // Streaming kernel: narrows with the shift in state[0]; the last CTA derives the true one from max|acc|.
-template <int BN, bool TWO, bool HALO>
+template <int BN, bool TWO, int MODE>
 __global__ void __launch_bounds__(REQUANT_THREADS, 1)
 umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
-    using Cfg = RequantCfg<BN, TWO, HALO>;
+    using Cfg = RequantCfg<BN, TWO, MODE>;
     using Split = EpiSplit<BN>;
     constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC;
     if (p.only_if_redo) {
@@ -951,12 +974,13 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES + Cfg::RESIDENT_BYTES);
     uint64_t* full_bar = bars;
     uint64_t* empty_bar = bars + STAGES;
     uint64_t* tfull_bar = bars + 2 * STAGES;
     uint64_t* tempty_bar = bars + 2 * STAGES + NACC;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * NACC);
+    uint64_t* weights_bar = bars + 2 * STAGES + 2 * NACC;  // one per filter column (resident weights)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2 * NACC + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile unsigned* warp_max = reinterpret_cast<volatile unsigned*>(tmem_slot + 4);  // one word per epilogue warp
 
@@ -967,6 +991,7 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (threadIdx.x == 0) {
         for (int i = 0; i < STAGES; ++i) { mbar_init(smem_u32(&full_bar[i]), 1); mbar_init(smem_u32(&empty_bar[i]), 1); }
         for (int i = 0; i < NACC; ++i) { mbar_init(smem_u32(&tfull_bar[i]), 1); mbar_init(smem_u32(&tempty_bar[i]), 4 * Split::GROUPS * (TWO ? 2 : 1)); }
+        for (int i = 0; i < 3; ++i) mbar_init(smem_u32(&weights_bar[i]), 1);
         *abort_flag = 0;
         fence_barrier_init();
         tma_prefetch_desc(&tmA);
@@ -987,12 +1012,12 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (warp == 0) {
-        if constexpr (HALO) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        if constexpr (MODE != LOAD_TAPS) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
         else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if (rank == 0) {
-            if constexpr (HALO) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            if constexpr (MODE != LOAD_TAPS) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, tempty_bar, tmem_base, p, abort_flag);
             else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
         }
         __syncwarp();
@@ -1148,23 +1173,24 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // ------------------------------------------------------------------------------------------------
 constexpr unsigned long long GRID_BARRIER_LIMIT_NS = 500000000ull;  // 0.5 s
 
-template <int BN, bool TWO, bool HALO>
+template <int BN, bool TWO, int MODE>
 __global__ void __launch_bounds__(REQUANT_THREADS, 1)
 umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
-    using Cfg = RequantCfg<BN, TWO, HALO>;
+    using Cfg = RequantCfg<BN, TWO, MODE>;
     using Split = EpiSplit<BN>;
     constexpr int STAGES = Cfg::STAGES;
     static_assert(BN >= 128 && 512 / BN <= 4, "all four warp groups share every tile; tables of four tiles");
     if (threadIdx.x == 0) PARK_STAMP(0);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    int32_t* out_row = reinterpret_cast<int32_t*>(smem + STAGES * Cfg::STAGE_BYTES);  // [tile][row of the tile]; -1: outside the tensor
+    int32_t* out_row = reinterpret_cast<int32_t*>(smem + STAGES * Cfg::STAGE_BYTES + Cfg::RESIDENT_BYTES);  // [tile][row of the tile]; -1: outside the tensor
     int32_t* pool_row = out_row + 4 * 128;
     uint64_t* bars = reinterpret_cast<uint64_t*>(pool_row + 4 * 128);
     uint64_t* full_bar = bars;
     uint64_t* empty_bar = bars + STAGES;
     uint64_t* tfull_bar = bars + 2 * STAGES;  // one per parked tile (up to 4)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+    uint64_t* weights_bar = bars + 2 * STAGES + 4;  // one per filter column (resident weights)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* shift_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);
     volatile unsigned* warp_max = reinterpret_cast<volatile unsigned*>(tmem_slot + 4);  // one word per epilogue warp
@@ -1176,6 +1202,7 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     if (threadIdx.x == 0) {
         for (int i = 0; i < STAGES; ++i) { mbar_init(smem_u32(&full_bar[i]), 1); mbar_init(smem_u32(&empty_bar[i]), 1); }
         for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&tfull_bar[i]), 1);
+        for (int i = 0; i < 3; ++i) mbar_init(smem_u32(&weights_bar[i]), 1);
         *abort_flag = 0;
         fence_barrier_init();
         tma_prefetch_desc(&tmA);
@@ -1197,12 +1224,12 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (warp == 0) {
-        if constexpr (HALO) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        if constexpr (MODE != LOAD_TAPS) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
         else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if (rank == 0) {
-            if constexpr (HALO) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, 0>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
+            if constexpr (MODE != LOAD_TAPS) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, 0, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, nullptr, tmem_base, p, abort_flag);
             else mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
         }
         __syncwarp();
@@ -1685,11 +1712,11 @@ static bool pair_ok(int m_tiles, int bn, int b_mn, int conv) {
     return (g_two_cta & (conv ? 2 : 1)) && m_tiles >= 2 && (!b_mn || bn == 256);
 }
 // PARKED: the kernel with the grid barrier (cooperative launch: every CTA must be resident at the same time)
-template <int BN, bool TWO, bool HALO, bool PARKED>
+template <int BN, bool TWO, int MODE, bool PARKED>
 static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
-    using Cfg = RequantCfg<BN, TWO, HALO>;
+    using Cfg = RequantCfg<BN, TWO, MODE>;
     void (*kernel)(CUtensorMap, CUtensorMap, GemmParams);
-    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, HALO>; else kernel = umma_requant_kernel<BN, TWO, HALO>;
+    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, MODE>; else kernel = umma_requant_kernel<BN, TWO, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     int tiles = p.m_tiles * p.n_tiles;
@@ -1706,17 +1733,20 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
     cfg.attrs = attr; cfg.numAttrs = n;
     return set_cuda_error(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
 }
-static int launch_requant(int bn, bool pair, bool halo, bool parked, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p,
+static int launch_requant(int bn, bool pair, int mode, bool parked, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p,
                           cudaStream_t st) {
     if (parked) {
-        if (pair) return bn == 256 ? launch_requant_inst<256, true, false, true>(a, b, p, st) : launch_requant_inst<128, true, false, true>(a, b, p, st);
-        if (halo) return launch_requant_inst<128, false, true, true>(a, b, p, st);
-        return bn == 256 ? launch_requant_inst<256, false, false, true>(a, b, p, st) : launch_requant_inst<128, false, false, true>(a, b, p, st);
+        if (pair) return bn == 256 ? launch_requant_inst<256, true, LOAD_TAPS, true>(a, b, p, st) : launch_requant_inst<128, true, LOAD_TAPS, true>(a, b, p, st);
+        if (mode == LOAD_HALO_RESIDENT) return launch_requant_inst<128, false, LOAD_HALO_RESIDENT, true>(a, b, p, st);
+        if (mode == LOAD_HALO) return launch_requant_inst<128, false, LOAD_HALO, true>(a, b, p, st);
+        return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, true>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, true>(a, b, p, st);
     }
-    if (pair) return bn == 256 ? launch_requant_inst<256, true, false, false>(a, b, p, st) : launch_requant_inst<128, true, false, false>(a, b, p, st);
-    if (halo) return bn == 64 ? launch_requant_inst<64, false, true, false>(a, b, p, st) : launch_requant_inst<128, false, true, false>(a, b, p, st);
-    if (bn == 64) return launch_requant_inst<64, false, false, false>(a, b, p, st);
-    return bn == 256 ? launch_requant_inst<256, false, false, false>(a, b, p, st) : launch_requant_inst<128, false, false, false>(a, b, p, st);
+    if (pair) return bn == 256 ? launch_requant_inst<256, true, LOAD_TAPS, false>(a, b, p, st) : launch_requant_inst<128, true, LOAD_TAPS, false>(a, b, p, st);
+    if (mode == LOAD_HALO_RESIDENT)
+        return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO_RESIDENT, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO_RESIDENT, false>(a, b, p, st);
+    if (mode == LOAD_HALO) return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO, false>(a, b, p, st);
+    if (bn == 64) return launch_requant_inst<64, false, LOAD_TAPS, false>(a, b, p, st);
+    return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, false>(a, b, p, st);
 }
 // all accumulators of the problem fit in the tensor memory of one wave of CTAs (units: 128-row tiles,
 // or 256-row pair tiles on sm/2 pairs)
@@ -1839,7 +1869,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.group_m = (static_cast<long long>(M) + N) * K > (48ll << 20) ? 8 : 0;
     set_fused(&p, fused);
     finish_params(&p);
-    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, false, false, ma, mb, p, st); }
+    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, LOAD_TAPS, false, ma, mb, p, st); }
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
@@ -1891,7 +1921,8 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         p.pool_out = fused->pool_out;
     }
     if (parked && !fits_parked(bn, p.m_tiles * p.n_tiles, pair)) return NITI_ERR_UNSUPPORTED;
-    if (fused) return launch_requant(bn, pair, plan.halo, parked, ma, mb, p, st);
+    const int mode = !plan.halo ? LOAD_TAPS : p.cblocks == 1 && p.n_tiles == 1 ? LOAD_HALO_RESIDENT : LOAD_HALO;
+    if (fused) return launch_requant(bn, pair, mode, parked, ma, mb, p, st);
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
