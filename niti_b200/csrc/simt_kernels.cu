@@ -74,6 +74,43 @@ requant_kernel(const int32_t* __restrict__ acc, int8_t* __restrict__ out, const 
     const bool stochastic = (mode == ROUND_STOCHASTIC) && shift > 0;
     const unsigned long long seed = stochastic ? *seed_p : 0ull;
     const bool aligned_rng = (rng_offset & 3ull) == 0;
+    // Rounding to nearest and stochastic rounding, the modes of activations and errors: four neighbouring values per thread
+    // and load, so that a warp's loads and stores are whole lines, and two loads in flight.  Bound by HBM / L2 (5 bytes
+    // per value); the general loop below reads 64 bytes per thread at a 64-byte pitch and spends 15 instructions a value:
+    // 16.8 M values 21.4 us, this form 14.4.  Shifts of 24 and more (|x| up to 2^31) stay with the general form, whose sums cannot overflow.
+    if (shift > 0 && shift < 24 && !zero_out && (mode == ROUND_NEAREST || (stochastic && aligned_rng))) {
+        constexpr int U = 2;
+        const long long words = n >> 2, step = static_cast<long long>(gridDim.x) * blockDim.x;
+        const int near = blockDim.x;  // a block's U loads are neighbours
+        const int half = 1 << (shift - 1);
+        const uint32_t mask = (1u << shift) - 1u;
+        for (long long g0 = blockIdx.x * static_cast<long long>(U * blockDim.x) + threadIdx.x; g0 < words; g0 += U * step) {
+            int4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (g0 + u * near < words) v[u] = reinterpret_cast<const int4*>(acc)[g0 + u * near];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const long long g = g0 + u * near;
+                if (g >= words) continue;
+                const uint32_t x[4] = {static_cast<uint32_t>(v[u].x), static_cast<uint32_t>(v[u].y), static_cast<uint32_t>(v[u].z), static_cast<uint32_t>(v[u].w)};
+                uint32_t o;
+                if (stochastic) {
+                    uint32_t rnd[4];
+                    random_block(seed, rng_stream, (rng_offset >> 2) + static_cast<unsigned long long>(g), rnd);
+                    o = relu ? narrow4_stochastic<true>(x, shift, mask, rnd) : narrow4_stochastic<false>(x, shift, mask, rnd);
+                } else {
+                    o = relu ? narrow4_nearest<true>(x, shift, half) : narrow4_nearest<false>(x, shift, half);
+                }
+                reinterpret_cast<uint32_t*>(out)[g] = o;
+            }
+        }
+        for (long long i = (words << 2) + blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n; i += step) {
+            const int8_t r = narrow(acc[i], shift, mode, stochastic ? random_word(seed, rng_stream, rng_offset + i) : 0u);
+            out[i] = relu && r < 0 ? int8_t(0) : r;
+        }
+        return;
+    }
     for (long long g = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; g < groups;
          g += static_cast<long long>(gridDim.x) * blockDim.x) {
         const int4* src = reinterpret_cast<const int4*>(acc) + g * 4;
@@ -520,6 +557,18 @@ __global__ void loss_kernel(const int8_t* __restrict__ out8, const int32_t* __re
 // ------------------------------------------------------------------------------------------------
 // weight update and the flipped / transposed filter bank the error-backward convolution reads
 // ------------------------------------------------------------------------------------------------
+// Four weights less their narrowed gradients.  Pseudo-stochastic rounding, the gradients' own mode, has a short form.
+__device__ __forceinline__ uint32_t update_word(const int4 gv, const uint32_t wv, const uint32_t (&rnd)[4], int shift, int mode,
+                                                bool zero_out) {
+    const int gx[4] = {gv.x, gv.y, gv.z, gv.w};
+    int y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int g8 = zero_out ? 0 : mode == ROUND_PSEUDO_STOCHASTIC && shift > 0 ? narrow_pseudo(gx[j], shift) : narrow(gx[j], shift, mode, rnd[j]);
+        y[j] = static_cast<int8_t>(wv >> (8 * j)) - g8;
+    }
+    return __vmaxs4(pack2_sat_s8(y[1], y[0], pack2_sat_s8(y[3], y[2], 0u)), 0x81818181u);
+}
 __global__ void __launch_bounds__(256)
 update_kernel(int8_t* __restrict__ w, const int32_t* __restrict__ g32, const unsigned* __restrict__ maxabs, long long n,
               int mu, int mode, const unsigned long long* seed_p, unsigned rng_stream) {
@@ -534,15 +583,7 @@ update_kernel(int8_t* __restrict__ w, const int32_t* __restrict__ g32, const uns
         const uint32_t wv = reinterpret_cast<const uint32_t*>(w)[g];
         uint32_t rnd[4] = {0, 0, 0, 0};
         if (stochastic) random_block(seed, rng_stream, static_cast<unsigned long long>(g), rnd);
-        const int gx[4] = {gv.x, gv.y, gv.z, gv.w};
-        uint32_t o = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int g8 = zero_out ? 0 : narrow(gx[j], shift, mode, rnd[j]);
-            const int wj = static_cast<int8_t>(wv >> (8 * j));
-            o |= static_cast<uint32_t>(static_cast<uint8_t>(clamp127(wj - g8))) << (8 * j);
-        }
-        reinterpret_cast<uint32_t*>(w)[g] = o;
+        reinterpret_cast<uint32_t*>(w)[g] = update_word(gv, wv, rnd, shift, mode, zero_out);
     }
     for (long long i = (groups << 2) + blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -566,18 +607,6 @@ struct UpdateMultiParams {
 };
 __device__ __forceinline__ unsigned absmax4(const int4 v) {
     return max(max(iabs_u(v.x), iabs_u(v.y)), max(iabs_u(v.z), iabs_u(v.w)));
-}
-__device__ __forceinline__ uint32_t update_word(const int4 gv, const uint32_t wv, const uint32_t (&rnd)[4], int shift, int mode,
-                                                bool zero_out) {
-    const int gx[4] = {gv.x, gv.y, gv.z, gv.w};
-    uint32_t o = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int g8 = zero_out ? 0 : narrow(gx[j], shift, mode, rnd[j]);
-        const int wj = static_cast<int8_t>(wv >> (8 * j));
-        o |= static_cast<uint32_t>(static_cast<uint8_t>(clamp127(wj - g8))) << (8 * j);
-    }
-    return o;
 }
 // Every block works on ONE layer (blocks are dealt to the layers in proportion to their sizes on the host), so a
 // block has one chain of loads -> maximum -> atomic before the barrier and one read of its layer's maximum after it.
