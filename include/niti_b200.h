@@ -143,7 +143,8 @@ NITI_API int niti_conv_wgrad_i8(const int8_t* x, const int8_t* err, int32_t* g32
 
 /* The weight gradient of a thin layer (R*S*C <= 32: the 3-channel first layer) from the patch matrix that the
  * layer's forward call already built: niti_conv_fprop_i8 / niti_conv_fprop_requant_i8 leave it in the first
- * N*H*W*32 bytes of THEIR scratch ([pixel][32]: the R*S*C bytes of the pixel's receptive field, zero padded), so a
+ * N*H*W*32 bytes of THEIR scratch ([pixel][32]: the R*S*C bytes of the pixel's receptive field, zero padded, the two
+ * 16-byte halves exchanged in pixels 4..7 of every eight, which is how the tensor cores read rows of 32 bytes), so a
  * caller that gives the forward call a scratch buffer of its own and keeps it until the backward pass saves the
  * second gather (TiConv2d.backward's first-layer branch, ti_torch.py:412-428, rebuilds its operands from the input
  * every time).  Same result as niti_conv_wgrad_i8 on the layer's input.  scratch:
@@ -356,6 +357,14 @@ NITI_API int niti_loss_i8(const int8_t* out8, const int32_t* out_exp, const int6
  * *maxabs = max |g32| (from niti_conv_wgrad_i8 / niti_gemm_i8 / niti_absmax_i32). */
 NITI_API int niti_update_i8(int8_t* w, const int32_t* g32, const uint32_t* maxabs, int64_t n,
                    int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream, void* stream);
+
+/* Weight gradient and update of one convolution: what niti_conv_wgrad_i8 followed by niti_update_i8 leaves behind, in three
+ * launches.  g32 holds niti_conv_wgrad_update_elems() int32 (0: not a shape of this entry point): the gradient, padded to a
+ * multiple of 4, and a tail whose first word is max |g32| afterwards.  Nothing in it has to be zero. */
+NITI_API size_t niti_conv_wgrad_update_elems(int C, int K, int R, int S, int pad);
+NITI_API int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int32_t* g32, int8_t* w,
+                       int N, int H, int W, int C, int K, int R, int S, int pad,
+                       int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream, int32_t* status, void* stream);
 
 /* Every weighted layer's update in one (cooperative) launch: for each item max |g32| is found, written to
  * *maxabs when that is not null, and w updated exactly as niti_update_i8 would with that maximum and the

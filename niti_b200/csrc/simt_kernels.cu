@@ -5,6 +5,7 @@
 // byte SIMD (__vmaxs4, __vcmpeq4, __dp4a), warp shuffles for reductions, one atomic per warp.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 
 #include "../../include/niti_b200.h"
@@ -1397,6 +1398,38 @@ extern "C" int niti_update_i8(int8_t* w, const int32_t* g32, const uint32_t* max
 
 extern "C" size_t niti_update_multi_scratch_bytes(void) { return 2 * UPDATE_MULTI_MAX * sizeof(int32_t); }
 
+// One launch for the layers in p.item; p.state is zero.
+static int launch_update(UpdateMultiParams& p, cudaStream_t st) {
+    static std::atomic<int> known{0};
+    int blocks_per_sm = known.load(std::memory_order_relaxed);
+    if (blocks_per_sm == 0) {
+        int n = 0;
+        if (int e = set_cuda_error(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, update_multi_kernel, 256, 0))) return e;
+        blocks_per_sm = n < 1 ? 1 : (n > 8 ? 8 : n);
+        known.store(blocks_per_sm, std::memory_order_relaxed);
+    }
+    long long total = 0;
+    for (int i = 0; i < p.count; ++i) total += p.item[i].n;
+    // deal the blocks of one resident wave to the layers in proportion to their sizes (at least one each)
+    const int wave = sm_count_simt() * blocks_per_sm;
+    int grid = 0;
+    for (int i = 0; i < p.count; ++i) {
+        long long share = (static_cast<long long>(wave - p.count) * p.item[i].n) / (total > 0 ? total : 1);
+        const long long useful = (p.item[i].n / 4 + 255) / 256;  // a block per 256 word groups is as fine as it gets
+        if (share > useful - 1) share = useful - 1;
+        if (share < 0) share = 0;
+        p.first_block[i] = grid;
+        grid += 1 + static_cast<int>(share);
+    }
+    p.first_block[p.count] = grid;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;  // the grid fits in one wave
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return set_cuda_error(cudaLaunchKernelEx(&cfg, update_multi_kernel, p));
+}
+
 extern "C" int niti_update_multi_i8(const niti_update_item* items, int count, int mu, int round_mode, int clear_gradients,
                                     const uint64_t* seed, void* scratch, size_t scratch_bytes, int32_t* status, void* stream) {
     NITI_REQUIRE(items && count > 0 && round_mode >= 0 && round_mode <= 2 && scratch);
@@ -1407,46 +1440,47 @@ extern "C" int niti_update_multi_i8(const niti_update_item* items, int count, in
         NITI_REQUIRE(reinterpret_cast<uintptr_t>(items[i].w) % 4 == 0 && reinterpret_cast<uintptr_t>(items[i].g32) % 16 == 0);
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    static int blocks_per_sm = 0;
-    if (blocks_per_sm == 0) {
-        int n = 0;
-        if (int e = set_cuda_error(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, update_multi_kernel, 256, 0))) return e;
-        blocks_per_sm = n < 1 ? 1 : (n > 8 ? 8 : n);
-    }
     for (int first = 0; first < count; first += UPDATE_MULTI_MAX) {
         UpdateMultiParams p;
         p.count = count - first < UPDATE_MULTI_MAX ? count - first : UPDATE_MULTI_MAX;
-        long long total = 0;
         for (int i = 0; i < p.count; ++i) {
             const niti_update_item& it = items[first + i];
             p.item[i] = UpdateItem{it.w, it.g32, it.maxabs, it.n, it.rng_stream};
-            total += it.n;
         }
         p.mu = mu; p.mode = round_mode; p.clear = clear_gradients ? 1 : 0;
         p.seed = reinterpret_cast<const unsigned long long*>(seed);
         p.state = static_cast<int32_t*>(scratch);
         p.status = status;
         if (int e = set_cuda_error(cudaMemsetAsync(scratch, 0, niti_update_multi_scratch_bytes(), st))) return e;
-        // deal the blocks of one resident wave to the layers in proportion to their sizes (at least one each)
-        const int wave = sm_count_simt() * blocks_per_sm;
-        int grid = 0;
-        for (int i = 0; i < p.count; ++i) {
-            long long share = (static_cast<long long>(wave - p.count) * p.item[i].n) / (total > 0 ? total : 1);
-            const long long useful = (p.item[i].n / 4 + 255) / 256;  // a block per 256 word groups is as fine as it gets
-            if (share > useful - 1) share = useful - 1;
-            if (share < 0) share = 0;
-            p.first_block[i] = grid;
-            grid += 1 + static_cast<int>(share);
-        }
-        p.first_block[p.count] = grid;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0; cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;  // the grid fits in one wave
-        cfg.attrs = attr; cfg.numAttrs = 1;
-        if (int e = set_cuda_error(cudaLaunchKernelEx(&cfg, update_multi_kernel, p))) return e;
+        if (int e = launch_update(p, st)) return e;
     }
     return NITI_OK;
+}
+
+// The gradient's zeroing, its tail's and nothing else in front of the contraction; the maximum is found by the update
+// itself (grid barrier).  Per convolution that is three launches instead of the five of niti_conv_wgrad_i8 +
+// niti_update_i8 (two memsets, contraction, maximum, update), and a small layer's step is launches.
+extern "C" size_t niti_conv_wgrad_update_elems(int C, int K, int R, int S, int pad) {
+    if (C <= 0 || K <= 0 || R <= 0 || S <= 0 || !niti_conv_wgrad_accumulate_supported(C, K, R, S, pad)) return 0;
+    return (static_cast<size_t>(K) * R * S * C + 3) / 4 * 4 + niti_update_multi_scratch_bytes() / 4;
+}
+extern "C" int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int32_t* g32, int8_t* w, int N, int H, int W, int C, int K,
+                                         int R, int S, int pad, int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream,
+                                         int32_t* status, void* stream) {
+    NITI_REQUIRE(g32 && w && round_mode >= 0 && round_mode <= 2 && (seed || round_mode != NITI_ROUND_STOCHASTIC));
+    NITI_REQUIRE(reinterpret_cast<uintptr_t>(w) % 4 == 0 && reinterpret_cast<uintptr_t>(g32) % 16 == 0);
+    const size_t elems = niti_conv_wgrad_update_elems(C, K, R, S, pad);
+    if (elems == 0) return NITI_ERR_UNSUPPORTED;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (int e = set_cuda_error(cudaMemsetAsync(g32, 0, elems * 4, st))) return e;
+    if (int e = niti_conv_wgrad_accumulate_i8(x, err, g32, N, H, W, C, K, R, S, pad, status, stream)) return e;
+    UpdateMultiParams p;
+    p.count = 1; p.mu = mu; p.mode = round_mode; p.clear = 0;
+    p.item[0] = UpdateItem{w, g32, nullptr, static_cast<long long>(K) * R * S * C, rng_stream};
+    p.seed = reinterpret_cast<const unsigned long long*>(seed);
+    p.state = g32 + elems - niti_update_multi_scratch_bytes() / 4;  // its first word ends up as the maximum
+    p.status = status;
+    return launch_update(p, st);
 }
 
 extern "C" size_t niti_dp_exchange_bytes(void) { return DPX_WORDS * sizeof(int32_t); }

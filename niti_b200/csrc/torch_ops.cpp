@@ -335,6 +335,34 @@ PyObject* conv_wgrad_acc(Args& a) {
     return tuple(g32, mx);
 }
 
+// gradient [K,R,S,C] and its maximum, views of one allocation; w is updated in place
+PyObject* conv_wgrad_update(Args& a) {
+    const Tensor &x = a.tensor(), &err = a.tensor(), &w = a.tensor();
+    const int pad = a.i32(), mu = a.i32(), mode = a.i32();
+    const Tensor* seed = a.maybe();
+    const uint32_t stream = a.u32();
+    need_cuda({&x, &err, &w});
+    require(x.dim() == 4 && err.dim() == 4 && w.scalar_type() == at::kChar);
+    const Conv s = conv_shape(x, w);
+    require(w.size(3) == s.C && err.size(3) == s.K && err.size(0) == s.N && err.size(1) == s.H && err.size(2) == s.W);
+    Tensor g32, mx;
+    {
+        Launch l(x);
+        const int64_t elems = static_cast<int64_t>(niti_conv_wgrad_update_elems(s.C, s.K, s.R, s.S, pad));
+        const Tensor both = l.empty({elems}, at::kInt);
+        check(niti_conv_wgrad_update_i8(cptr<int8_t>(x), cptr<int8_t>(err), mptr<int32_t>(both), mptr<int8_t>(w), s.N, s.H, s.W, s.C, s.K, s.R,
+                                        s.S, pad, mu, mode, cptr<uint64_t>(seed), stream, l.status(), l.stream), "niti_conv_wgrad_update_i8");
+        auto view = [&](int64_t at_, at::IntArrayRef shape) {
+            Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(both.storage()), both.key_set(), both.dtype());
+            t.unsafeGetTensorImpl()->set_storage_offset(at_);
+            t.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
+            return t;
+        };
+        g32 = view(0, {s.K, s.R, s.S, s.C});
+        mx = view((static_cast<int64_t>(s.K) * s.R * s.S * s.C + 3) / 4 * 4, {1});
+    }
+    return tuple(g32, mx);
+}
 PyObject* conv_wgrad_batch_inner_supported(Args& a) {
     const auto v = ints<6>(a);
     return PyBool_FromLong(niti_conv_wgrad_batch_inner_supported(v[0], v[1], v[2], v[3], v[4], v[5]));
@@ -577,7 +605,7 @@ PyMethodDef methods[] = {
     NITI_ENTRY(conv_fprop_acc), NITI_ENTRY(conv_fprop_fused),
     NITI_ENTRY(conv_fprop_pool_fused), NITI_ENTRY(conv_dgrad_fused), NITI_ENTRY(conv_dgrad_acc), NITI_ENTRY(conv_wgrad_acc),
     NITI_ENTRY(conv_wgrad_batch_inner_supported), NITI_ENTRY(conv_wgrad_batch_inner), NITI_ENTRY(maxpool_bwd_f16),
-    NITI_ENTRY(conv_wgrad_from_patches), NITI_ENTRY(conv_wgrad_accumulate), NITI_ENTRY(gemm_acc), NITI_ENTRY(requant),
+    NITI_ENTRY(conv_wgrad_from_patches), NITI_ENTRY(conv_wgrad_update), NITI_ENTRY(conv_wgrad_accumulate), NITI_ENTRY(gemm_acc), NITI_ENTRY(requant),
     NITI_ENTRY(absmax), NITI_ENTRY(maxpool_fwd), NITI_ENTRY(maxpool_bwd), NITI_ENTRY(relu_fwd), NITI_ENTRY(relu_bwd),
     NITI_ENTRY(dropout), NITI_ENTRY(loss_err), NITI_ENTRY(update), NITI_ENTRY(quantize_input),
     {nullptr, nullptr, 0, nullptr}};

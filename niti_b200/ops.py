@@ -217,6 +217,14 @@ def conv_wgrad_acc(x, err, R=3, S=3, pad=1, out=None, want_max=True):
     return _run("niti_conv_wgrad_i8", 2, work, native.conv_wgrad_acc, x, err, R, S, pad, out, want_max)
 
 
+def conv_wgrad_update(x, err, w, pad=1, mu=5, mode=ROUND_PSEUDO_STOCHASTIC, seed=None, rng_stream=0):
+    """conv_wgrad_acc followed by update of the filters w, in fewer launches: (gradient int32, max|gradient|).  For the
+    shapes of conv_wgrad_accumulate_supported."""
+    def work(r):
+        return 2 * err.numel() * w[0].numel(), x.numel() + err.numel() + 10 * w.numel()
+    return _run("niti_conv_wgrad_update_i8", 2, work, native.conv_wgrad_update, x, err, w, pad, mu, mode, seed, rng_stream)
+
+
 def conv_wgrad_batch_inner_supported(N, C, K, R, S, pad):
     return native.conv_wgrad_batch_inner_supported(N, C, K, R, S, pad)
 

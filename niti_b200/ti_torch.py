@@ -417,6 +417,7 @@ class TiConv2d(UpdateWeight):
         K, R, S, C = self.weight.shape
         err_out = None
         fork = None
+        updated = False
         if self.wgrad_stream is not None and not self.first_layer:
             fork = torch.cuda.Event()
             fork.record()  # the weight gradient needs only what has been enqueued up to here
@@ -457,6 +458,12 @@ class TiConv2d(UpdateWeight):
                 g32, g_max = self.grad_buffer, None
             else:
                 g32, g_max = ops.conv_wgrad_accumulate(act, err_in, self.grad_buffer, R, S, self.padding), None
+        elif (not self.defer_update and self.grad_buffer is None and self.grad_ready is None
+                and type(self).weight_update is UpdateWeight.weight_update and ops.conv_wgrad_accumulate_supported(C, K, R, S, self.padding)):
+            # nobody looks at the gradient between its computation and the update: both in one call
+            g32, g_max = ops.conv_wgrad_update(act, err_in, self.weight, self.padding, GRAD_BITWIDTH, _mode(GRAD_ROUND_METHOD),
+                                               RNG_SEED(dev), 16 * self.layer_id + 2)
+            updated = True
         elif self._patches_of is act and self._patches is not None:
             # the patch matrix of this step's forward pass is still there
             g32, g_max = ops.conv_wgrad_from_patches(self._patches, err_in, C, R, S, out=self.grad_buffer,
@@ -468,7 +475,7 @@ class TiConv2d(UpdateWeight):
         self.__dict__.update(err_exp=err_exp, grad_int32acc=g32, grad_maxabs=g_max)
         if self.grad_ready is not None:
             self.grad_ready(self)
-        if not self.defer_update:
+        if not self.defer_update and not updated:
             self.weight_update()
         if not self.first_layer:
             return err_out, err_exp
