@@ -129,14 +129,18 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) fc_head_kernel(const HeadPara
     __syncthreads();
     HEAD_STAMP(1);
 
-    // ---- forward GEMM: out32[b][j] = sum_f drop(x)[b][f] * W[j][f], one sample per block at a time
+    // ---- forward GEMM: out32[b][j] = sum_f drop(x)[b][f] * W[j][f], one sample per block at a time; rows of up to 64
+    //      16-feature chunks, which would leave most of the block idle between two barriers a sample, one sample per warp
     unsigned fwd_max = 0;
-    for (int b = blockIdx.x; b < B; b += G) {
+    const bool per_warp = F16 <= 64;
+    const int c_first = per_warp ? lane : t, c_step = per_warp ? 32 : HEAD_THREADS;
+    const int b_step = per_warp ? G * (HEAD_THREADS / 32) : G;
+    for (int b = blockIdx.x + (per_warp ? warp * G : 0); b < B; b += b_step) {
         int acc[HEAD_MAX_CLASSES];
 #pragma unroll
         for (int j = 0; j < HEAD_MAX_CLASSES; ++j) acc[j] = 0;
         const uint4* x4 = reinterpret_cast<const uint4*>(p.x) + static_cast<size_t>(b) * F16;
-        for (int c = t; c < F16; c += HEAD_THREADS) {
+        for (int c = c_first; c < F16; c += c_step) {
             uint4 xv = __ldg(x4 + c);
             const unsigned bits = sMask[c];
             xv.x &= expand4(bits); xv.y &= expand4(bits >> 4); xv.z &= expand4(bits >> 8); xv.w &= expand4(bits >> 12);
@@ -152,12 +156,19 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) fc_head_kernel(const HeadPara
                     acc[j] = a;
                 }
         }
+        int mine = 0;  // lane j: the warp's sum of class j
 #pragma unroll
         for (int j = 0; j < HEAD_MAX_CLASSES; ++j)
             if (j < J) {
                 const int v = __reduce_add_sync(0xFFFFFFFFu, acc[j]);
-                if (lane == 0) sRed[warp * HEAD_MAX_CLASSES + j] = v;
+                if (lane == j) mine = v;
             }
+        if (per_warp) {
+            if (lane < J) p.out32[b * J + lane] = mine;
+            fwd_max = max(fwd_max, __reduce_max_sync(0xFFFFFFFFu, iabs32(mine)));
+            continue;
+        }
+        if (lane < J) sRed[warp * HEAD_MAX_CLASSES + lane] = mine;
         __syncthreads();
         if (warp == 0) {
             int v = 0;
@@ -170,7 +181,8 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) fc_head_kernel(const HeadPara
         }
         __syncthreads();
     }
-    if (t == 0 && fwd_max != 0) atomicMax(&umax[0], fwd_max);  // one atomic per block: they serialise at the L2
+    if (per_warp) block_max(&umax[0], fwd_max, sRed);
+    else if (t == 0 && fwd_max != 0) atomicMax(&umax[0], fwd_max);  // one atomic per block: they serialise at the L2
     HEAD_STAMP(2);
     if (!bounded_grid_barrier(&p.state[3], G, p.status, 6, sFlag)) return;
 
@@ -182,8 +194,8 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) fc_head_kernel(const HeadPara
         const int shift = shift_for(__ldcg(&umax[0]), CALC_ACT, p.bits, &z);
         const int out_exp = shift + *p.exp_x + (p.dropout ? 1 : 0) + exp_w;
         if (blockIdx.x == 0 && t == 0) *p.exp_out = out_exp;
-        if (warp == 0) {
-            for (int b = blockIdx.x; b < B; b += G) {
+        {   // the block's samples side by side on its warps: a sample's chain of double-precision steps takes about 3 us
+            for (int b = blockIdx.x + warp * G; b < B; b += G * (HEAD_THREADS / 32)) {
                 const bool on = lane < J;
                 const unsigned long long elem = (p.sample_offset + b) * static_cast<unsigned long long>(J) + lane;
                 int o8 = 0;
@@ -242,30 +254,30 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) fc_head_kernel(const HeadPara
     }
     __syncthreads();
 
-    // ---- error-backward GEMM, first pass: max|e32|.  The chunks of the block's FIRST sample (all there is when the
-    //      batch is not larger than the grid) stay in registers until the shift is known; the rest is recomputed then.
+    // ---- error-backward GEMM, first pass: max|e32|.  The block's (sample, 16-feature chunk) pairs are dealt to its threads
+    //      as one list; a thread's first ones (all there are for rows of 8192 features when the batch is not larger than
+    //      the grid) stay in registers until the shift is known, the rest is recomputed then.
+    const int items = static_cast<int>(blockIdx.x) < B ? (B - static_cast<int>(blockIdx.x) + G - 1) / G * F16 : 0;
+    const auto item_sample = [&](int i) { return static_cast<int>(blockIdx.x) + i / F16 * G; };
     constexpr int KEEP_CHUNKS = 2;
     int ekeep[KEEP_CHUNKS][16];
     {
         unsigned m = 0;
-        if (static_cast<int>(blockIdx.x) < B) {
 #pragma unroll
-            for (int k = 0; k < KEEP_CHUNKS; ++k) {
-                const int c = t + k * HEAD_THREADS;
-                if (c < F16) {
-                    dgrad_chunk(sW, sErr + blockIdx.x * J, J, F16, c, ekeep[k]);
+        for (int k = 0; k < KEEP_CHUNKS; ++k) {
+            const int i = t + k * HEAD_THREADS;
+            if (i < items) {
+                dgrad_chunk(sW, sErr + item_sample(i) * J, J, F16, i % F16, ekeep[k]);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) m = max(m, iabs32(ekeep[k][i]));
-                }
+                for (int q = 0; q < 16; ++q) m = max(m, iabs32(ekeep[k][q]));
             }
         }
-        for (int b = blockIdx.x; b < B; b += G)
-            for (int c = t + (b == static_cast<int>(blockIdx.x) ? KEEP_CHUNKS * HEAD_THREADS : 0); c < F16; c += HEAD_THREADS) {
-                int e[16];
-                dgrad_chunk(sW, sErr + b * J, J, F16, c, e);
+        for (int i = t + KEEP_CHUNKS * HEAD_THREADS; i < items; i += HEAD_THREADS) {
+            int e[16];
+            dgrad_chunk(sW, sErr + item_sample(i) * J, J, F16, i % F16, e);
 #pragma unroll
-                for (int k = 0; k < 16; ++k) m = max(m, iabs32(e[k]));
-            }
+            for (int q = 0; q < 16; ++q) m = max(m, iabs32(e[q]));
+        }
         block_max(&umax[1], m, sRed);
     }
     HEAD_STAMP(6);
@@ -351,19 +363,16 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) fc_head_kernel(const HeadPara
             o.z = packed[2] & expand4(bits >> 8); o.w = packed[3] & expand4(bits >> 12);
             reinterpret_cast<uint4*>(p.e8)[static_cast<size_t>(b) * F16 + c] = o;
         };
-        if (static_cast<int>(blockIdx.x) < B) {
 #pragma unroll
-            for (int k = 0; k < KEEP_CHUNKS; ++k) {
-                const int c = t + k * HEAD_THREADS;
-                if (c < F16) emit(blockIdx.x, c, ekeep[k]);
-            }
+        for (int k = 0; k < KEEP_CHUNKS; ++k) {
+            const int i = t + k * HEAD_THREADS;
+            if (i < items) emit(item_sample(i), i % F16, ekeep[k]);
         }
-        for (int b = blockIdx.x; b < B; b += G)
-            for (int c = t + (b == static_cast<int>(blockIdx.x) ? KEEP_CHUNKS * HEAD_THREADS : 0); c < F16; c += HEAD_THREADS) {
-                int e[16];
-                dgrad_chunk(sW, sErr + b * J, J, F16, c, e);
-                emit(b, c, e);
-            }
+        for (int i = t + KEEP_CHUNKS * HEAD_THREADS; i < items; i += HEAD_THREADS) {
+            int e[16];
+            dgrad_chunk(sW, sErr + item_sample(i) * J, J, F16, i % F16, e);
+            emit(item_sample(i), i % F16, e);
+        }
     }
     HEAD_STAMP(9);
     // ---- the update of the weights this block computed the gradient of
