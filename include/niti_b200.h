@@ -366,6 +366,12 @@ NITI_API int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int32
                        int N, int H, int W, int C, int K, int R, int S, int pad,
                        int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream, int32_t* status, void* stream);
 
+/* niti_gemm_i8 with scratch of niti_gemm_scratch_bytes() bytes (0: none needed): shapes whose row pitches the tensor-core
+ * kernels do not take (A rows that are not whole 16-byte groups, results of any width) then run on them all the same. */
+NITI_API size_t niti_gemm_scratch_bytes(int M, int N, int K, int trans_a, int trans_b);
+NITI_API int niti_gemm_scratch_i8(const int8_t* A, const int8_t* B, int32_t* C32, uint32_t* maxabs, void* scratch, size_t scratch_bytes,
+                         int M, int N, int K, int trans_a, int trans_b, int32_t* status, void* stream);
+
 /* Every weighted layer's update in one (cooperative) launch: for each item max |g32| is found, written to
  * *maxabs when that is not null, and w updated exactly as niti_update_i8 would with that maximum and the
  * item's rng_stream.  scratch: niti_update_multi_scratch_bytes() bytes.  status as in niti_fc_head_train_i8

@@ -307,6 +307,46 @@ extern "C" int niti_gemm_i8(const int8_t* A, const int8_t* B, int32_t* C32, uint
     return simt_gemm(A, B, C32, maxabs, M, N, K, trans_a, trans_b, st);
 }
 
+// Products that only their pitches keep off the tensor cores: a classifier of any number of classes (its errors are rows
+// of that many bytes, its result rows of that many words) on more than a handful of samples.  The A rows are copied to a
+// pitch of 16 bytes, a result whose rows are not whole 16-byte groups goes through a padded copy.  From 2^24 multiplications
+// on: the CUDA-core kernels reach 1.4-2 TMAC/s (500 x 1024 x 100, gradient: 26 us), the copies and the tensor product
+// about 10 us at such sizes.
+struct PaddedGemm { bool use; int lda, ldc; size_t a_bytes, c_bytes; };
+static PaddedGemm padded_gemm(int M, int N, int K, int trans_a, int trans_b) {
+    PaddedGemm g{};
+    const int pitch_a = trans_a ? M : K, rows_a = trans_a ? K : M, pitch_b = trans_b ? K : N;
+    const bool dense = pitch_a % 16 == 0 && N % 4 == 0 && M >= 64 && N >= 32 && K >= 32;
+    g.use = !dense && pitch_b % 16 == 0 && static_cast<long long>(M) * N * K >= (1ll << 24);
+    if (!g.use) return g;
+    g.lda = pitch_a % 16 == 0 ? 0 : (pitch_a + 15) / 16 * 16;
+    g.ldc = N % 4 == 0 ? 0 : (N + 3) / 4 * 4;
+    g.a_bytes = align_up(static_cast<size_t>(rows_a) * g.lda, 256);
+    g.c_bytes = static_cast<size_t>(M) * g.ldc * 4;
+    return g;
+}
+extern "C" size_t niti_gemm_scratch_bytes(int M, int N, int K, int trans_a, int trans_b) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const PaddedGemm g = padded_gemm(M, N, K, trans_a, trans_b);
+    return g.use ? g.a_bytes + g.c_bytes + 16 : 0;
+}
+extern "C" int niti_gemm_scratch_i8(const int8_t* A, const int8_t* B, int32_t* C32, uint32_t* maxabs, void* scratch, size_t scratch_bytes,
+                                    int M, int N, int K, int trans_a, int trans_b, int32_t* status, void* stream) {
+    NITI_REQUIRE(A && B && C32 && M > 0 && N > 0 && K > 0);
+    const PaddedGemm g = padded_gemm(M, N, K, trans_a, trans_b);
+    if (!g.use || scratch == nullptr || !aligned16(B) || !aligned16(A) || !aligned16(C32))
+        return niti_gemm_i8(A, B, C32, maxabs, M, N, K, trans_a, trans_b, status, stream);
+    if (!aligned16(scratch) || scratch_bytes < niti_gemm_scratch_bytes(M, N, K, trans_a, trans_b)) return NITI_ERR_SCRATCH;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (int e = clear_word(maxabs, st)) return e;
+    int8_t* a = static_cast<int8_t*>(scratch);
+    const int pitch_a = trans_a ? M : K, rows_a = trans_a ? K : M;
+    if (g.lda) if (int e = copy_rows(A, pitch_a, a, g.lda, pitch_a, rows_a, 1, st)) return e;
+    int32_t* c = g.ldc ? reinterpret_cast<int32_t*>(a + g.a_bytes) : C32;
+    if (int e = umma_gemm(g.lda ? a : A, B, c, maxabs, M, N, K, trans_a, trans_b, 1, nullptr, status, st, 0, g.lda, g.ldc)) return e;
+    return g.ldc ? copy_rows(c, 4ll * g.ldc, C32, 4ll * N, 4ll * N, M, 4, st) : NITI_OK;
+}
+
 // ---------------------------------------------------------------- contraction + requantisation in one pass
 static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* state, void* scratch, size_t scratch_bytes,
                       int N, int H, int W, int C, int K, int R, int S, int pad, int flip, int kind, int round_mode,

@@ -34,7 +34,8 @@ extern int g_stage_cap;  // experiments: cap on the shared-memory stages the GEM
 // tensor-core (tcgen05) paths, umma_kernels.cu; `out` is int32 (fused == null) or int8
 int umma_gemm_splits(int M, int N, int K);
 int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int M, int N, int K, int trans_a,
-              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st, int rows32 = 0);
+              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st, int rows32 = 0,
+              int lda = 0, int ldc = 0);  // row pitches of A and of an int32 result in elements (0: dense)
 int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int Nimg, int H, int W, int C, int K,
               int R, int S, int pad, int flip, const FusedArgs* fused, int32_t* status, cudaStream_t st);
 // k3: 3x3 filters, padding 1
@@ -70,6 +71,8 @@ int reduce_rows32(const int32_t* partial, int splits, int rows, int cols_out, in
 // w / wp / K: optionally the layer's filters w[K][R*S*C] are padded to wp[K][32] by the same launch
 int im2col32(const int8_t* x, int8_t* xcol, int Nimg, int H, int W, int C, int R, int S, int pad, cudaStream_t st,
              const int8_t* w = nullptr, int8_t* wp = nullptr, int K = 0);
+// rows of `bytes` bytes from one pitch (in bytes) to another; everything a multiple of `unit` (1 or 4)
+int copy_rows(const void* src, long long src_pitch, void* dst, long long dst_pitch, long long bytes, long long rows, int unit, cudaStream_t st);
 int unpack_i4(const uint8_t* in, int8_t* out, long long nbytes, cudaStream_t st);  // two int4 per byte (low nibble first) -> int8
 
 }  // namespace niti

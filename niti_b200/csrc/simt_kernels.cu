@@ -1338,6 +1338,23 @@ __global__ void __launch_bounds__(256) unpack_i4_kernel(const uint8_t* __restric
     }
 }
 namespace niti {
+template <class T>
+__global__ void __launch_bounds__(256) copy_rows_kernel(const T* __restrict__ src, long long src_pitch, T* __restrict__ dst, long long dst_pitch,
+                                                        int cols, long long rows) {
+    const long long total = rows * cols;
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const long long r = i / cols;
+        dst[r * dst_pitch + (i - r * cols)] = src[r * src_pitch + (i - r * cols)];
+    }
+}
+int copy_rows(const void* src, long long src_pitch, void* dst, long long dst_pitch, long long bytes, long long rows, int unit, cudaStream_t st) {
+    const int grid = blocks_for(rows * bytes / unit, 256, sm_count_simt() * 8);
+    if (unit == 4)
+        copy_rows_kernel<<<grid, 256, 0, st>>>(static_cast<const int32_t*>(src), src_pitch / 4, static_cast<int32_t*>(dst), dst_pitch / 4, static_cast<int>(bytes / 4), rows);
+    else
+        copy_rows_kernel<<<grid, 256, 0, st>>>(static_cast<const int8_t*>(src), src_pitch, static_cast<int8_t*>(dst), dst_pitch, static_cast<int>(bytes), rows);
+    return set_cuda_error(cudaGetLastError());
+}
 int unpack_i4(const uint8_t* in, int8_t* out, long long nbytes, cudaStream_t st) {
     unpack_i4_kernel<<<blocks_for(nbytes, 256, sm_count_simt() * 16), 256, 0, st>>>(in, out, nbytes);
     return set_cuda_error(cudaGetLastError());

@@ -433,8 +433,11 @@ PyObject* gemm_acc(Args& a) {
         Launch l(A);
         c32 = out ? *out : l.empty({M, N}, at::kInt);
         if (want_max) mx = l.empty({1}, at::kInt);
-        check(niti_gemm_i8(cptr<int8_t>(A), cptr<int8_t>(B), mptr<int32_t>(c32), want_max ? mptr<uint32_t>(mx) : nullptr, M, N, K, ta, tb, l.status(), l.stream),
-              "niti_gemm_i8");
+        const size_t nb = niti_gemm_scratch_bytes(M, N, K, ta, tb);
+        Tensor sc;
+        if (nb) sc = l.bytes(nb);
+        check(niti_gemm_scratch_i8(cptr<int8_t>(A), cptr<int8_t>(B), mptr<int32_t>(c32), want_max ? mptr<uint32_t>(mx) : nullptr,
+                                   nb ? mptr(sc) : nullptr, nb, M, N, K, ta, tb, l.status(), l.stream), "niti_gemm_i8");
     }
     return tuple(c32, mx);
 }

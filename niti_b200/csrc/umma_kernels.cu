@@ -1841,19 +1841,20 @@ int umma_gemm_splits(int M, int N, int K) {
 // a first layer (256 rows) took 4600 cycles, whatever its epilogue did.  3 -> 128 channels, 500 images: 109 -> 68 us
 // with the gather, 3 -> 64, 1024 images: the product alone 110 -> 44 us.
 int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int M, int N, int K, int trans_a,
-              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st, int rows32) {
+              int trans_b, int splits, const FusedArgs* fused, int32_t* status, cudaStream_t st, int rows32, int lda, int ldc) {
     CUtensorMap ma, mb, mc;
     const int a_mn = trans_a ? 1 : 0, b_mn = trans_b ? 0 : 1;
     const int bn = fused ? requant_bn(N, 1 << 20) : (N > 128) ? 256 : 128;
     const bool pair = rows32 == 0 && !fused && pair_ok((M + 127) / 128, bn, b_mn, 0);
     {
         uint64_t dims[2], str[1]; uint32_t box[2] = {128, 128};
-        if (a_mn) { dims[0] = M; dims[1] = K; str[0] = M; } else { dims[0] = K; dims[1] = M; str[0] = K; }
+        if (a_mn) { dims[0] = M; dims[1] = K; str[0] = lda > 0 ? lda : M; } else { dims[0] = K; dims[1] = M; str[0] = lda > 0 ? lda : K; }
         if (int e = encode_map(&ma, A, false, 2, dims, str, box)) return e;
         if (b_mn) { dims[0] = N; dims[1] = K; str[0] = N; box[1] = 128; } else { dims[0] = K; dims[1] = N; str[0] = K; box[1] = pair ? bn / 2 : bn; }
         if (int e = encode_map(&mb, B, false, 2, dims, str, box)) return e;
         uint64_t dc[4] = {(uint64_t)N, (uint64_t)M, (uint64_t)splits, 1};
-        uint64_t sc[3] = {(uint64_t)N * 4, (uint64_t)M * N * 4, (uint64_t)splits * M * N * 4};
+        const uint64_t pitch = ldc > 0 ? ldc : N;
+        uint64_t sc[3] = {pitch * 4, M * pitch * 4, splits * M * pitch * 4};
         uint32_t bc[4] = {32, 128, 1, 1};
         if (!fused) if (int e = encode_map(&mc, out, true, 4, dc, sc, bc)) return e;
     }
