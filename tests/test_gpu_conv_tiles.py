@@ -1,0 +1,118 @@
+"""The narrowing convolutions at the edges of their tiles, against the oracle: 8-pixel-wide tiles with shared rows (ragged
+maps, several channel blocks, weights resident or not, 64- and 128-column tiles, masks and side codes), the thin layer's
+operands of 32-byte rows, the gradient-and-update call, and the short roundings of the stand-alone kernels."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from niti_b200 import ops  # noqa: E402
+from oracle import niti_oracle as O  # noqa: E402
+from oracle import philox  # noqa: E402
+
+DEV = "cuda:0"
+
+
+def rnd8(rng, shape):
+    return rng.integers(-127, 128, size=shape).astype(np.int8)
+
+
+def cu(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+
+
+def same(got, want):
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("N,H,W,C,K", [
+    (1, 16, 8, 16, 16), (2, 17, 9, 48, 80), (1, 33, 31, 32, 64), (3, 15, 13, 144, 64), (2, 20, 24, 128, 48), (1, 32, 32, 272, 128),
+    (2, 12, 8, 64, 144), (5, 30, 16, 112, 112)])
+@pytest.mark.parametrize("parking", [False, True])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_tiles_that_share_rows(N, H, W, C, K, parking, mode):
+    rng = np.random.default_rng(N + H + 3 * W + C + K)
+    x, w, err = np.maximum(rnd8(rng, (N, H, W, C)), 0), rnd8(rng, (K, 3, 3, C)), rnd8(rng, (N, H, W, K))
+    seed, ea = ops.seed_tensor(9, DEV), torch.zeros((), dtype=torch.int32, device=DEV)
+    acc, back = O.conv_fprop(x, w), O.conv_dgrad(err, w)
+    want = O.relu_fwd(O.act_calc(acc, 0, mode, philox.random_u32_tensor(9, 3, acc.shape))[0])
+    want_e = np.where(x > 0, O.err_calc(back, mode, philox.random_u32_tensor(9, 4, back.shape))[0], 0).astype(np.int8)
+    old = ops.set_accumulator_parking(parking)
+    try:
+        fwd, bwd = ops.new_requant_state(DEV), ops.new_requant_state(DEV)
+        nbytes = ops.conv_dgrad_side_bytes(N, H, W, C, K, 3, 3, 1)
+        side = torch.empty(nbytes, dtype=torch.uint8, device=DEV) if nbytes else None
+        for _ in range(2):  # a streaming layer guesses wrong first and right afterwards
+            same(ops.conv_fprop_fused(cu(x), cu(w), fwd, 1, mode, seed, 3, 0, True, ea, ea)[0], want)
+            same(ops.conv_dgrad_fused(cu(err), cu(w), bwd, 1, mode, seed, 4, 0, ea, ea, relu_mask=cu(x), side=side)[0], want_e)
+    finally:
+        ops.set_accumulator_parking(old)
+    ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("N,H,W,K", [(1, 1, 1, 16), (1, 4, 4, 16), (3, 7, 12, 80), (2, 5, 9, 144), (9, 32, 32, 48), (1, 3, 260, 64)])
+def test_thin_layer(N, H, W, K):
+    """Rows of whole words take the staged gather, the others the general one; fewer pixels than a tile; 16 to 144 filters."""
+    rng = np.random.default_rng(N + H + W + K)
+    x, w, err = rnd8(rng, (N, H, W, 3)), rnd8(rng, (K, 3, 3, 3)), rnd8(rng, (N, H, W, K))
+    ea, st = torch.zeros((), dtype=torch.int32, device=DEV), ops.new_requant_state(DEV)
+    acc = O.conv_fprop(x, w)
+    for _ in range(2):
+        same(ops.conv_fprop_fused(cu(x), cu(w), st, 1, 0, None, 0, 0, False, ea, ea)[0], O.act_calc(acc, 0)[0])
+    same(ops.conv_fprop_acc(cu(x), cu(w))[0], acc)
+    same(ops.conv_wgrad_acc(cu(x), cu(err), 3, 3, 1)[0], O.conv_wgrad(x, err, 3, 3, 1))
+
+
+@pytest.mark.parametrize("N,H,W", [(1, 1, 4), (3, 6, 10), (2, 5, 7), (40, 32, 32)])
+def test_input_quantisation_of_three_planes(N, H, W):
+    x = np.random.default_rng(N + H + W).standard_normal((N, 3, H, W)).astype(np.float32)
+    want, want_e = O.float_to_int8(x)
+    got, e = ops.quantize_input(cu(x))
+    same(got, np.ascontiguousarray(want.transpose(0, 2, 3, 1)))
+    assert int(e) == want_e
+
+
+@pytest.mark.parametrize("N,H,W,C,K,mode", [(2, 5, 7, 16, 16, 2), (3, 8, 8, 48, 80, 2), (1, 4, 4, 144, 128, 1)])
+def test_gradient_and_update_in_one_call(N, H, W, C, K, mode):
+    rng = np.random.default_rng(N + C + K)
+    x, w, err = rnd8(rng, (N, H, W, C)), rnd8(rng, (K, 3, 3, C)), rnd8(rng, (N, H, W, K))
+    g = O.conv_wgrad(x, err, 3, 3, 1)
+    wd = cu(w)
+    g32, mx = ops.conv_wgrad_update(cu(x), cu(err), wd, 1, 5, mode, ops.seed_tensor(7, DEV), 18)
+    same(g32, g)
+    assert int(mx) == int(np.abs(g).max())
+    same(wd, O.weight_update(w, g, 5, mode, philox.random_u32_tensor(7, 18, g.shape))[0])
+
+
+@pytest.mark.parametrize("n", [1, 3, 16, 2055, 300001])
+@pytest.mark.parametrize("top", [0, 90, 129, 1 << 15, (1 << 30) - 1, (1 << 31) - 1])
+def test_roundings_of_the_stand_alone_kernels(n, top):
+    """All three roundings from no shift at all to accumulators that fill 31 bits (the short forms end at 30)."""
+    rng = np.random.default_rng(n + top % 97)
+    acc = rng.integers(-top, top + 1, size=n).astype(np.int32)
+    acc[rng.integers(n)] = top
+    mx, seed = ops.absmax(cu(acc)), ops.seed_tensor(5, DEV)
+    for mode in (0, 1, 2):
+        words = philox.random_u32_tensor(5, 2, acc.shape)
+        same(ops.requant(cu(acc), mx, ops.CALC_ACT, 7, mode, seed, 2)[0], O.act_calc(acc, 0, mode, words)[0])
+        w = rnd8(rng, (n,))
+        wd = cu(w)
+        ops.update(wd, cu(acc), mx, 5, mode, seed, 2)
+        same(wd, O.weight_update(w, acc, 5, mode, words)[0])
+
+
+@pytest.mark.parametrize("M,N,K,ta,tb", [
+    (4097, 50, 128, False, True), (700, 10, 2448, False, True), (1000, 101, 256, False, True), (513, 1024, 50, False, False),
+    (10, 2064, 1003, True, False), (99, 512, 500, True, False), (130, 4096, 33, True, False)])
+def test_products_of_any_row_pitch(M, N, K, ta, tb):
+    rng = np.random.default_rng(M + N + K)
+    a, b = rnd8(rng, (M, K)), rnd8(rng, (K, N))
+    want = O.int8_mm(a, b)
+    c, mx = ops.gemm_acc(cu(a.T if ta else a), cu(b.T if tb else b), ta, tb)
+    same(c, want)
+    assert int(mx) == int(np.abs(want).max())
+    ops.check_status(DEV)
