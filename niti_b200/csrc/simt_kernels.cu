@@ -1564,6 +1564,11 @@ extern "C" int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int
     NITI_REQUIRE(reinterpret_cast<uintptr_t>(w) % 4 == 0 && reinterpret_cast<uintptr_t>(g32) % 16 == 0);
     const size_t elems = niti_conv_wgrad_update_elems(C, K, R, S, pad);
     if (elems == 0) return NITI_ERR_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(err)) % 16 != 0) {  // not for the tensor cores: the separate calls
+        uint32_t* mx = reinterpret_cast<uint32_t*>(g32 + elems - niti_update_multi_scratch_bytes() / 4);
+        if (int e = niti_conv_wgrad_i8(x, err, g32, mx, nullptr, 0, N, H, W, C, K, R, S, pad, status, stream)) return e;
+        return niti_update_i8(w, g32, mx, static_cast<int64_t>(K) * R * S * C, mu, round_mode, seed, rng_stream, stream);
+    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int e = set_cuda_error(cudaMemsetAsync(g32, 0, elems * 4, st))) return e;
     if (int e = niti_conv_wgrad_accumulate_i8(x, err, g32, N, H, W, C, K, R, S, pad, status, stream)) return e;

@@ -86,6 +86,12 @@ def test_gradient_and_update_in_one_call(N, H, W, C, K, mode):
     same(g32, g)
     assert int(mx) == int(np.abs(g).max())
     same(wd, O.weight_update(w, g, 5, mode, philox.random_u32_tensor(7, 18, g.shape))[0])
+    # operands that do not start on a 16-byte boundary are served too, as by the separate calls
+    odd = torch.empty(x.size + 1, dtype=torch.int8, device=DEV)[1:].view(x.shape)
+    odd.copy_(cu(x))
+    w2 = cu(w)
+    same(ops.conv_wgrad_update(odd, cu(err), w2, 1, 5, mode, ops.seed_tensor(7, DEV), 18)[0], g)
+    assert torch.equal(w2, wd)
 
 
 @pytest.mark.parametrize("n", [1, 3, 16, 2055, 300001])
