@@ -1,10 +1,10 @@
 // int8 x int8 -> int32 contractions on the 5th-generation tensor cores (sm_100a):
 // GEMM, implicit-GEMM convolution forward / error-backward, and convolution weight gradient.
 //
-// Common structure (one CTA per SM, 192 threads):
+// Common structure (one CTA per SM):
 //   warp 0      TMA producer: cp.async.bulk.tensor into 128-byte-swizzled shared-memory stages
 //   warp 1      allocates tensor memory, issues tcgen05.mma.kind::i8 (one lane), frees TMEM
-//   warps 2..5  epilogue: tcgen05.ld the int32 accumulators, reduce max|acc|, store
+//   warps 2..   epilogue (4, 8 or 16 warps): tcgen05.ld the int32 accumulators, reduce max|acc|, store
 // Stages hand over through mbarriers (TMA complete_tx -> MMA, tcgen05.commit -> producer);
 // accumulators are double-buffered in TMEM so the epilogue of one tile overlaps the main loop
 // of the next.  All waits are bounded (ptx.cuh).
