@@ -108,7 +108,8 @@ __device__ __forceinline__ uint32_t narrow4_nearest(const uint32_t* v, int shift
 // Stochastic rounding: with lo the dropped bits of |x| and r the random word's, |x| is rounded up exactly
 // when lo > r, i.e. when lo + (mask - r) carries into bit `shift`: y = (|x| + (~r & mask)) >> shift.  For x < 0 the
 // negated quotient is the arithmetic shift (x + (r & mask)) >> shift (-floor(a / d) = floor((d - 1 - a) / d)), so both
-// signs are one add and one shift behind a three-input logic operation.  Shifts below 24 only: |x| is then below 2^31 - 2^shift.
+// signs are one add and one shift behind a three-input logic operation.  For shifts below 24 and x <= 2^31 - 2^shift, as
+// for the nearest form: negative sums only move towards zero, positive ones must not pass 2^31.
 template <bool RELU>
 __device__ __forceinline__ uint32_t narrow4_stochastic(const uint32_t* v, int shift, uint32_t mask, const uint32_t (&rnd)[4]) {
     int y[4];

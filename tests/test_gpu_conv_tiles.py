@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 if not torch.cuda.is_available():
     pytest.skip("needs a CUDA device", allow_module_level=True)
 
-from niti_b200 import ops  # noqa: E402
+from niti_b200 import ops, ti_torch  # noqa: E402
 from oracle import niti_oracle as O  # noqa: E402
 from oracle import philox  # noqa: E402
 
@@ -109,6 +109,23 @@ def test_roundings_of_the_stand_alone_kernels(n, top):
         wd = cu(w)
         ops.update(wd, cu(acc), mx, 5, mode, seed, 2)
         same(wd, O.weight_update(w, acc, 5, mode, words)[0])
+
+
+@pytest.mark.parametrize("n", [1, 4, 6, 1023, 4096])
+@pytest.mark.parametrize("shift", [1, 4, 10, 23])
+def test_roundings_by_a_shift_that_the_data_exceed(n, shift):
+    """RoundShift and StoShift take any shift, niti_requant_i8 any target width: int32 values whose rounded quotients (and
+    whose sums with half a unit) pass both ends of the range are clamped like all others, in whole words and in the tail."""
+    rng = np.random.default_rng(n + shift)
+    lim = np.iinfo(np.int32)
+    x = rng.choice(np.array([lim.max, lim.max - (1 << shift >> 1), lim.max - (1 << shift) + 2, (127 << shift) + 1, 127 << shift, 5, 0, -5,
+                             -(127 << shift) - 1, lim.min + (1 << shift), lim.min + 1, lim.min], dtype=np.int32), size=n)
+    words = philox.random_u32_tensor(3, 0, x.shape)
+    ti_torch.set_seed(3, DEV)
+    same(ti_torch.RoundShift(cu(x), shift), O.round_shift(x, shift))
+    same(ti_torch.StoShift(cu(x), shift), O.sto_shift(x, shift, words))
+    same(ti_torch.PstoShift(cu(x), shift), O.psto_shift(x, shift))
+    same(ops.requant(cu(x), cu(np.array([lim.max], np.int32)), ops.CALC_ACT, 31 - shift, 0, relu=True)[0], np.maximum(O.round_shift(x, shift), 0))
 
 
 @pytest.mark.parametrize("M,N,K,ta,tb", [
