@@ -40,6 +40,13 @@ class UpdateWeight(Module):
         ops.update(self.weight, self.grad_int32acc, self.grad_maxabs, GRAD_BITWIDTH, _mode(GRAD_ROUND_METHOD),
                    RNG_SEED(self.weight.device), 16 * self.layer_id + 2)
 
+    def plain_update(self):
+        """Whether weight_update is the one above: neither a subclass, nor the class, nor this object replaced it."""
+        return type(self).weight_update is _WEIGHT_UPDATE and 'weight_update' not in self.__dict__
+
+
+_WEIGHT_UPDATE = UpdateWeight.weight_update
+
 
 def weight_update_all(layers, clear=False):
     """The updates of all `layers` (UpdateWeight modules whose grad_int32acc is set) in one launch; each
@@ -459,7 +466,7 @@ class TiConv2d(UpdateWeight):
             else:
                 g32, g_max = ops.conv_wgrad_accumulate(act, err_in, self.grad_buffer, R, S, self.padding), None
         elif (not self.defer_update and self.grad_buffer is None and self.grad_ready is None
-                and type(self).weight_update is UpdateWeight.weight_update and ops.conv_wgrad_accumulate_supported(C, K, R, S, self.padding)):
+                and self.plain_update() and ops.conv_wgrad_accumulate_supported(C, K, R, S, self.padding)):
             # nobody looks at the gradient between its computation and the update: both in one call
             g32, g_max = ops.conv_wgrad_update(act, err_in, self.weight, self.padding, GRAD_BITWIDTH, _mode(GRAD_ROUND_METHOD),
                                                RNG_SEED(dev), 16 * self.layer_id + 2)

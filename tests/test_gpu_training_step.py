@@ -161,6 +161,36 @@ def test_reference_function_names_and_shift_helpers():
     assert np.array_equal(ti_torch.int8mm(torch.from_numpy(l).to(DEV), torch.from_numpy(r).to(DEV)).cpu().numpy(), O.int8_mm(l, r))
 
 
+@pytest.mark.parametrize("where", ["object", "class", "base class", "subclass"])
+@pytest.mark.parametrize("channels", [3, 16])
+def test_a_replaced_weight_update_is_the_one_that_runs(where, channels, monkeypatch):
+    """A layer frozen or wrapped on the object, the class or its base keeps its filters and sees its gradient, as the
+    reference's backward (which calls self.weight_update) would have it; the layers beside it are updated as ever."""
+    calls = []
+
+    def frozen(self=None):
+        calls.append((layer.grad_int32acc.clone(), layer.grad_maxabs.clone()))
+
+    cls = ti_torch.TiConv2d if where != "subclass" else type("Frozen", (ti_torch.TiConv2d,), {"weight_update": frozen})
+    layer, beside = cls(channels, 16, first_layer=channels == 3), ti_torch.TiConv2d(16, 16)
+    rng = np.random.default_rng(3)
+    act = rng.integers(-127, 128, size=(2, 6, 6, channels)).astype(np.int8)
+    err = rng.integers(-127, 128, size=(2, 6, 6, 16)).astype(np.int8)
+    exp = ti_torch.exp_tensor(-7, torch.device(DEV))
+    before = [layer.weight.clone(), beside.weight.clone()]
+    for l, x in ((layer, act), (beside, err)):
+        with monkeypatch.context() as m:
+            if l is layer and where == "object":
+                layer.weight_update = frozen
+            elif l is layer and where != "subclass":
+                m.setattr(ti_torch.TiConv2d if where == "class" else ti_torch.UpdateWeight, "weight_update", frozen)
+            l.forward((torch.from_numpy(x).to(DEV), exp))
+            l.backward((torch.from_numpy(err).to(DEV), exp))
+    want = O.conv_wgrad(act, err, 3, 3, 1)
+    assert len(calls) == 1 and np.array_equal(calls[0][0].cpu().numpy(), want) and int(calls[0][1]) == int(np.abs(want).max())
+    assert torch.equal(layer.weight, before[0]) and not torch.equal(beside.weight, before[1])
+
+
 def test_state_dict_roundtrip_reference_format():
     model, _, _ = build([16, "M", 32, "M", 512, "M"], 5, True, True, 5)
     sd = model.state_dict()
