@@ -25,7 +25,8 @@ def _conv(input, weight, stride, padding):
     if R > 2 * padding + 1 and S > 2 * padding + 1 and P * Q <= 49 and C % 16 == 0 and K % 16 == 0 and N % 16 == 0:
         # weight gradient in disguise: input = activations [C,H,W,N], filters = errors [K,P',Q',N] of the layer's
         # output size; out[c,p,q,k] = sum_{n,h,w} x[n,h+p-pad,w+q-pad,c] * err[n,h,w,k] = dW[k,p,q,c]
-        if tuple(weight.shape[1:3]) == (H, W) and ops.conv_wgrad_batch_inner_supported(N, C, K, P, Q, padding):
+        if tuple(weight.shape[1:3]) == (H, W) and ops.conv_wgrad_batch_inner_supported(N, C, K, P, Q, padding) \
+                and (input.data_ptr() | weight.data_ptr()) % 16 == 0:  # the tensor cores' loads; copies are aligned below
             return ops.conv_wgrad_batch_inner(input, weight, P, Q, padding)  # reads both operands as they lie
         x = input.permute(3, 1, 2, 0).contiguous()
         err = weight.permute(3, 1, 2, 0).contiguous()

@@ -24,6 +24,12 @@ def cu(a):
     return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
 
 
+def off_by_one(t):
+    """The same contiguous tensor, starting one element into its buffer."""
+    odd = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)[1:].view(t.shape)
+    return odd.copy_(t)
+
+
 @pytest.mark.parametrize("N,H,W,C,K", [
     (16, 4, 4, 16, 16), (48, 5, 7, 32, 144), (128, 3, 6, 144, 128), (144, 2, 2, 16, 272), (256, 8, 8, 128, 64)])
 def test_weight_gradient_with_the_batch_innermost(N, H, W, C, K):
@@ -33,6 +39,16 @@ def test_weight_gradient_with_the_batch_innermost(N, H, W, C, K):
     want = O.conv_wgrad(x, err, 3, 3, 1).transpose(3, 1, 2, 0)
     assert np.array_equal(got.cpu().numpy(), want)
     ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("which", ["input", "filters", "both"])
+def test_weight_gradient_of_operands_off_a_16_byte_boundary(which):
+    """A view that starts inside a buffer goes through aligned copies, as any operand did."""
+    rng = np.random.default_rng(4)
+    x, err = rnd8(rng, (16, 4, 6, 32)), rnd8(rng, (16, 4, 6, 16))
+    x_t, err_t = cu(x.transpose(3, 1, 2, 0)), cu(err.transpose(3, 1, 2, 0))
+    got = cutlassconv_cuda.sp_conv_optimized(x_t if which == "filters" else off_by_one(x_t), err_t if which == "input" else off_by_one(err_t), 1, 1)
+    assert np.array_equal(got.cpu().numpy(), O.conv_wgrad(x, err, 3, 3, 1).transpose(3, 1, 2, 0))
 
 
 @pytest.mark.parametrize("M,K,N", [(1, 256, 4), (128, 1028, 12), (77, 2048, 8), (296, 4096, 16), (299, 260, 12), (1, 259, 12)])
