@@ -70,3 +70,16 @@ def test_pool_backward_on_fp16_copies(N, H, W, C):
     dx = int8pool_cuda.int8_pool_backward(cu(y).half(), cu(dy).half(), cu(x).half(), 2, 2, 0)
     assert dx.dtype == torch.float16
     assert np.array_equal(dx.cpu().numpy(), O.maxpool_bwd(x, dy).astype(np.float16))
+
+
+@pytest.mark.parametrize("which", ["input", "error", "both"])
+def test_pool_backward_of_fp16_operands_off_a_16_byte_boundary(which):
+    """A view that starts inside a buffer is narrowed to int8 on the way, as any operand was."""
+    rng = np.random.default_rng(6)
+    x = rng.integers(-4, 5, size=(2, 6, 4, 16)).astype(np.int8)
+    dy = rnd8(rng, (2, 3, 2, 16))
+    xh, dyh = cu(x).half(), cu(dy).half()
+    dx = int8pool_cuda.int8_pool_backward(cu(O.maxpool_fwd(x)).half(), dyh if which == "input" else off_by_one(dyh),
+                                          xh if which == "error" else off_by_one(xh), 2, 2, 0)
+    assert dx.dtype == torch.float16
+    assert np.array_equal(dx.cpu().numpy(), O.maxpool_bwd(x, dy).astype(np.float16))
