@@ -139,3 +139,22 @@ def test_products_of_any_row_pitch(M, N, K, ta, tb):
     same(c, want)
     assert int(mx) == int(np.abs(want).max())
     ops.check_status(DEV)
+
+
+def test_launches_are_counted_by_shape():
+    """Gather, product and conditional second launch of a thin layer; row copies of a padded product and none of others."""
+    def counted(fn, *args):
+        before = ops.LAUNCHES
+        fn(*args)
+        return ops.LAUNCHES - before
+
+    rng = np.random.default_rng(0)
+    z = torch.zeros((), dtype=torch.int32, device=DEV)
+    for C, fused, grad in ((3, 3, 3), (16, 2, 2)):
+        x, w, err = cu(rnd8(rng, (2, 8, 8, C))), cu(rnd8(rng, (16, 3, 3, C))), cu(rnd8(rng, (2, 8, 8, 16)))
+        assert counted(ops.conv_fprop_fused, x, w, ops.new_requant_state(DEV), 1, 0, None, 0, 0, False, z, z) == fused
+        assert counted(ops.conv_wgrad_acc, x, err) == grad
+    for M, N, K, ta, tb, n in [(500, 1024, 100, False, False, 2), (1000, 101, 256, False, True, 2), (700, 33, 1000, False, True, 1),
+                               (99, 1024, 500, True, False, 2), (64, 64, 64, False, True, 1), (5, 3, 7, False, False, 1)]:
+        a, b = rnd8(rng, (K, M) if ta else (M, K)), rnd8(rng, (N, K) if tb else (K, N))
+        assert counted(ops.gemm_acc, cu(a), cu(b), ta, tb) == n, (M, N, K)
