@@ -106,8 +106,8 @@ def Int8zeros(size):
 
 def exp_tensor(e, device=None):
     """Exponent as a 0-dim int32 tensor on the device (accepts ints, floats, tensors)."""
-    if isinstance(e, torch.Tensor):
-        if e.dtype is torch.int32 and e.dim() == 0 and e.is_cuda and (device is None or e.device == device):
+    if device is not None and isinstance(e, torch.Tensor):
+        if e.dtype is torch.int32 and e.dim() == 0 and e.is_cuda and e.device == device:
             return e  # what every layer of a network hands on: nothing to convert
     device = device or GPU
     if isinstance(e, torch.Tensor):

@@ -191,6 +191,12 @@ def test_a_replaced_weight_update_is_the_one_that_runs(where, channels, monkeypa
     assert torch.equal(layer.weight, before[0]) and not torch.equal(beside.weight, before[1])
 
 
+def test_exponent_without_a_device_goes_to_the_default_one(monkeypatch):
+    monkeypatch.setattr(ti_torch, "GPU", "cpu")
+    e = torch.full((), -7, dtype=torch.int32, device=DEV)
+    assert ti_torch.exp_tensor(e).device.type == "cpu" and ti_torch.exp_tensor(e, e.device) is e
+
+
 def test_state_dict_roundtrip_reference_format():
     model, _, _ = build([16, "M", 32, "M", 512, "M"], 5, True, True, 5)
     sd = model.state_dict()
