@@ -9,6 +9,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+from importlib import metadata
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -51,10 +52,24 @@ def build(force=False, verbose=False):
     return LIB
 
 
+def ops_tag():
+    """What the front end is tied to besides its source: torch's C++ classes and the interpreter's ABI."""
+    return f"torch {metadata.version('torch')}, {sysconfig.get_config_var('SOABI')}"
+
+
+def ops_stale():
+    """Whether _torch_ops.so has to be built: no file, older than its sources, or built for another torch or interpreter (the
+    tag is compiled into the module's docstring, so a torch that was exchanged underneath is noticed without loading it)."""
+    if _stale(OPS, [os.path.join(CSRC, "torch_ops.cpp"), os.path.join(os.path.dirname(PKG), "include", "niti_b200.h")]):
+        return True
+    with open(OPS, "rb") as f:
+        return f"({ops_tag()})\0".encode() not in f.read()
+
+
 def build_ops(force=False):
     """The CPython module niti_b200._torch_ops: links against the library beside it (rpath $ORIGIN) and the installed torch."""
     src = os.path.join(CSRC, "torch_ops.cpp")
-    if not force and not _stale(OPS, [src, os.path.join(os.path.dirname(PKG), "include", "niti_b200.h")]):
+    if not force and not ops_stale():
         return OPS
     import torch
     base = os.path.dirname(torch.__file__)
@@ -62,7 +77,7 @@ def build_ops(force=False):
     incs = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
             sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-                    f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *["-I" + d for d in incs], src, "-o", OPS,
+                    f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DNITI_OPS_TAG="{ops_tag()}"', *["-I" + d for d in incs], src, "-o", OPS,
                     "-L" + PKG, "-l:libniti_b200.so", "-L" + os.path.join(base, "lib"), "-lc10", "-ltorch_cpu", "-ltorch_python",
                     "-lc10_cuda", "-ltorch_cuda", "-Wl,-rpath,$ORIGIN"], check=True)
     return OPS

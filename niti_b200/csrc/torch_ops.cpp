@@ -612,7 +612,7 @@ PyMethodDef methods[] = {
     NITI_ENTRY(absmax), NITI_ENTRY(maxpool_fwd), NITI_ENTRY(maxpool_bwd), NITI_ENTRY(relu_fwd), NITI_ENTRY(relu_bwd),
     NITI_ENTRY(dropout), NITI_ENTRY(loss_err), NITI_ENTRY(update), NITI_ENTRY(quantize_input),
     {nullptr, nullptr, 0, nullptr}};
-PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_torch_ops", "native torch front end of libniti_b200", -1, methods, nullptr, nullptr, nullptr, nullptr};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_torch_ops", "native torch front end of libniti_b200 (" NITI_OPS_TAG ")", -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 

@@ -38,3 +38,11 @@ def test_error_strings_and_argument_checks_need_no_gpu():
     assert L.niti_conv_wgrad_scratch_bytes(0, 8, 8, 128, 128, 3, 3) == 0
     assert L.niti_conv_fprop_requant_supported(128, 128, 3, 3, 1) == 1
     assert L.niti_conv_fprop_requant_supported(100, 128, 3, 3, 1) == 0
+
+
+def test_front_end_is_rebuilt_for_another_torch(monkeypatch):
+    from niti_b200 import build
+    build.build()
+    assert not build.ops_stale()
+    monkeypatch.setattr(build.metadata, "version", lambda name: "99.0")  # as after an upgrade of torch
+    assert build.ops_stale()
