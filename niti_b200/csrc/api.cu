@@ -363,7 +363,7 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
         if (!scratch || !aligned16(scratch) || scratch_bytes < niti_conv_fprop_scratch_bytes(N, H, W, C, K, R, S)) return NITI_ERR_SCRATCH;
         if (int e = im2col32(in, xcol, N, H, W, C, R, S, pad, st, w, wp, K)) return e;
     }
-    if (pool_out != nullptr && !(g_opt_parking && !thin && !flip && umma_conv_pool_fusable(N, H, W, K, k3(R, S, pad)))) return NITI_ERR_UNSUPPORTED;
+    if (pool_out != nullptr && !(g_opt_parking && !thin && !flip && umma_conv_pool_fusable(N, H, W, K))) return NITI_ERR_UNSUPPORTED;
     // Few enough output tiles for every accumulator to stay in tensor memory: one exact launch.
     if (g_opt_parking && !thin && umma_conv_fits_parked(N, H, W, flip ? C : K, k3(R, S, pad), flip)) {
         f.parked = 1;
@@ -402,7 +402,7 @@ extern "C" int niti_conv_fprop_requant_i8(const int8_t* x, const int8_t* w, int8
 
 extern "C" int niti_conv_fprop_requant_pool_supported(int N, int H, int W, int C, int K, int R, int S, int pad) {
     if (N <= 0 || H <= 0 || W <= 0 || !niti_conv_fprop_requant_supported(C, K, R, S, pad)) return 0;
-    return g_opt_parking && fprop_path(C, K, R, S, pad) == CONV_TC && umma_conv_pool_fusable(N, H, W, K, k3(R, S, pad)) ? 1 : 0;
+    return g_opt_parking && fprop_path(C, K, R, S, pad) == CONV_TC && umma_conv_pool_fusable(N, H, W, K) ? 1 : 0;
 }
 
 extern "C" int niti_conv_fprop_requant_pool_i8(const int8_t* x, const int8_t* w, int8_t* y8, int8_t* y8_pooled, int32_t* state, int N,

@@ -40,7 +40,7 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
               int R, int S, int pad, int flip, const FusedArgs* fused, int32_t* status, cudaStream_t st);
 // k3: 3x3 filters, padding 1
 bool umma_conv_fits_parked(int Nimg, int H, int W, int outc, bool k3, int flip);
-bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc, bool k3);  // the fused forward kernel can also emit the 2x2-pooled output
+bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc);  // the fused forward kernel can also emit the 2x2-pooled output
 size_t umma_wgrad_scratch_bytes(int Nimg, int H, int W, int C, int K, int R, int S);
 // max_splits > 0 caps the number of pixel-range splits (and with it the size of `partial`)
 // direct == 1: `partial` is the zeroed gradient and the CTAs add into it (TMA reduction) instead of storing partials

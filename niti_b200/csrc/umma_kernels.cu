@@ -1824,6 +1824,13 @@ static ConvPlan conv_plan(int Nimg, int H, int W, int outc, bool k3, int flip, i
     return c;
 }
 
+// The tiles of a call that pools too: with the shared activation rows unless that makes tiles of an odd number of rows
+// (18, 22, 26, 30, 38 image rows), which would tear pooling windows apart; those keep the box per tap.
+static ConvPlan pool_plan(int Nimg, int H, int W, int outc, bool k3) {
+    const ConvPlan c = conv_plan(Nimg, H, W, outc, k3, 0, 2);
+    return pool_box_ok(H, W, c.BW, c.BH) ? c : conv_plan(Nimg, H, W, outc, false, 0, 2);
+}
+
 int umma_gemm_splits(int M, int N, int K) {
     const int bn = (N > 128) ? 256 : 128;
     const int tiles = ((M + 127) / 128) * ((N + bn - 1) / bn);
@@ -1885,7 +1892,9 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     const int outc = flip ? C : K;  // output channels
     GemmParams p{};
     const bool parked = fused && fused->parked;
-    const ConvPlan plan = conv_plan(Nimg, H, W, outc, R == 3 && S == 3 && pad == 1, flip, !fused ? 0 : parked ? 2 : 1);
+    const bool k3 = R == 3 && S == 3 && pad == 1;
+    const ConvPlan plan = fused && fused->pool_out != nullptr ? pool_plan(Nimg, H, W, outc, k3)
+                                                              : conv_plan(Nimg, H, W, outc, k3, flip, !fused ? 0 : parked ? 2 : 1);
     const int bn = plan.bn;
     const bool pair = plan.pair;
     p.BW = plan.BW; p.BH = plan.BH; p.BI = plan.BI;
@@ -1931,9 +1940,9 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
 static bool pool_box_ok(int H, int W, int bw, int bh) {
     return H % 2 == 0 && W % 2 == 0 && bh % 2 == 0 && (bw == 2 || bw == 4 || bw == 8 || bw == 16);
 }
-bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc, bool k3) {
-    const ConvPlan plain = conv_plan(Nimg, H, W, outc, false, 0, 2), c = conv_plan(Nimg, H, W, outc, k3, 0, 2);
-    return pool_box_ok(H, W, plain.BW, plain.BH) && pool_box_ok(H, W, c.BW, c.BH) && umma_conv_fits_parked(Nimg, H, W, outc, false, 0);
+bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc) {
+    const ConvPlan c = conv_plan(Nimg, H, W, outc, false, 0, 2);
+    return pool_box_ok(H, W, c.BW, c.BH) && umma_conv_fits_parked(Nimg, H, W, outc, false, 0);
 }
 
 bool umma_conv_fits_parked(int Nimg, int H, int W, int outc, bool k3, int flip) {

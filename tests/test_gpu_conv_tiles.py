@@ -54,6 +54,23 @@ def test_tiles_that_share_rows(N, H, W, C, K, parking, mode):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("N,H,W,C,K", [(2, 18, 8, 16, 16), (1, 22, 16, 144, 64), (3, 26, 8, 48, 80), (2, 30, 4, 128, 128), (1, 38, 2, 32, 272),
+                                       (4, 20, 8, 64, 48)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_pooling_in_the_same_launch_on_maps_of_any_even_height(N, H, W, C, K, mode):
+    """Maps whose height does not split into tiles of an even number of rows (18, 22, 26, 30, 38) pool in the launch too."""
+    assert ops.conv_fprop_pool_fused_supported(N, H, W, C, K, 3, 3, 1)
+    rng = np.random.default_rng(N + H + W + C + K)
+    x, w = rnd8(rng, (N, H, W, C)), rnd8(rng, (K, 3, 3, C))
+    ea, st = torch.zeros((), dtype=torch.int32, device=DEV), ops.new_requant_state(DEV)
+    y8, yp, _, _ = ops.conv_fprop_pool_fused(cu(x), cu(w), st, 1, mode, ops.seed_tensor(9, DEV), 3, 0, True, ea, ea)
+    acc = O.conv_fprop(x, w)
+    want = O.relu_fwd(O.act_calc(acc, 0, mode, philox.random_u32_tensor(9, 3, acc.shape))[0])
+    same(y8, want)
+    same(yp, O.maxpool_fwd(want))
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("N,H,W,K", [(1, 1, 1, 16), (1, 4, 4, 16), (3, 7, 12, 80), (2, 5, 9, 144), (9, 32, 32, 48), (1, 3, 260, 64)])
 def test_thin_layer(N, H, W, K):
     """Rows of whole words take the staged gather, the others the general one; fewer pixels than a tile; 16 to 144 filters."""
