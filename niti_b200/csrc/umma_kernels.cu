@@ -1048,18 +1048,18 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             int m_pair, n_t;
             tile_coords(p, tile, &m_pair, &n_t);
             const int m_t = TWO ? 2 * m_pair + static_cast<int>(rank) : m_pair;
-            bool valid; int row;  // row of the output tensor
+            bool valid; long long row;  // row of the output tensor (there may be more than 2^31)
             if (p.conv) {
                 const int q1 = fdiv(m_t, p.fd_tw), tw = m_t - q1 * p.tiles_w, tn = fdiv(q1, p.fd_th), th = q1 - tn * p.tiles_h;
                 const int w = tw * p.BW + row_w, h = th * p.BH + row_h, n = tn * p.BI + row_n;
                 valid = row_in_box && w < p.W && h < p.H && n < p.Nimg;
-                row = (n * p.H + h) * p.W + w;
+                row = (static_cast<long long>(n) * p.H + h) * p.W + w;
             } else {
-                row = m_t * BLOCK_M + row_in_tile;
+                row = static_cast<long long>(m_t) * BLOCK_M + row_in_tile;
                 valid = row < p.M;
             }
             const int col0 = n_t * BN + cg;
-            const long long off = static_cast<long long>(row) * p.N + col0;  // of this thread's first output
+            const long long off = row * p.N + col0;  // of this thread's first output
             const int8_t* mrow = (p.mask != nullptr && valid && col0 < p.N) ? p.mask + off : nullptr;
             uint4 mk[2];
             mask_load<2>(mrow, p.N - col0, mk);

@@ -71,6 +71,27 @@ def test_pooling_in_the_same_launch_on_maps_of_any_even_height(N, H, W, C, K, mo
     ops.check_status(DEV)
 
 
+def test_more_than_2_to_the_31_output_rows():
+    """16 channels in and out, 34 GB each: images at both ends and in the middle come out as they do alone, the others stay zero."""
+    N, C = (1 << 21) + 5, 16
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < (80 << 30):
+        pytest.skip("needs 80 GB of device memory")
+    rng = np.random.default_rng(8)
+    few, w, at = cu(rnd8(rng, (4, 32, 32, C))), cu(rnd8(rng, (16, 3, 3, C))), [0, 1 << 20, N - 2, N - 1]
+    ea = torch.zeros((), dtype=torch.int32, device=DEV)
+    want = ops.conv_fprop_fused(few, w, ops.new_requant_state(DEV), 1, 0, None, 0, 0, False, ea, ea)[0]
+    x = torch.zeros((N, 32, 32, C), dtype=torch.int8, device=DEV)
+    x[at] = few
+    got = ops.conv_fprop_fused(x, w, ops.new_requant_state(DEV), 1, 0, None, 0, 0, False, ea, ea)[0]
+    ops.check_status(DEV)
+    assert torch.equal(got[at], want)
+    got[at] = 0
+    assert not any(bool(part.any()) for part in got.split(1 << 17))
+    del x, got
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("N,H,W,K", [(1, 1, 1, 16), (1, 4, 4, 16), (3, 7, 12, 80), (2, 5, 9, 144), (9, 32, 32, 48), (1, 3, 260, 64)])
 def test_thin_layer(N, H, W, K):
     """Rows of whole words take the staged gather, the others the general one; fewer pixels than a tile; 16 to 144 filters."""
