@@ -254,6 +254,9 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int mn, int* m_
 }
 
 // ---- warp roles shared by the streaming kernel and the accumulator-parking kernel -------------
+// stages of the ring in use (NITI_OPT_STAGE_CAP)
+__device__ __forceinline__ int ring_stages(const GemmParams& p, int compiled) { return keep_reg((p.nstages > 0 && p.nstages < compiled) ? p.nstages : compiled); }
+
 // TMA producer: fills the stage ring for every tile of this CTA, in tile order.  The WHOLE warp runs the loop and
 // an elected lane issues.  TMA and MMA instructions take their operands from uniform registers, and the compiler keeps
 // addresses, coordinates and descriptors there only while every branch around them is provably warp-uniform: waits
@@ -274,7 +277,7 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
     const int first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
     constexpr int BNH = TWO ? BN / 2 : BN;  // B columns this CTA loads
-    const int nst = (p.nstages > 0 && p.nstages < STAGES) ? p.nstages : STAGES;
+    const int nst = ring_stages(p, STAGES);
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
     const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
     const int conv = keep_reg(p.conv), flip = keep_reg(p.flip), pad = keep_reg(p.pad), S = keep_reg(p.S), cblocks = keep_reg(p.cblocks);
@@ -391,7 +394,7 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     const int mn_tiles = p.m_tiles * p.n_tiles;
     const int total_tiles = mn_tiles * p.splits;
     const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, p.rows32 == 2 ? 32 : BN, p.a_mn, p.b_mn);
-    const int nst = (p.nstages > 0 && p.nstages < STAGES) ? p.nstages : STAGES;
+    const int nst = ring_stages(p, STAGES);
     const int first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
     const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_in, 0);  // read from shared memory: make it provably uniform
@@ -492,6 +495,7 @@ __device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full
     const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg(p.a_bytes + (RESIDENT ? 0 : 3 * BN * ROW_BYTES)));
     const uint32_t res0 = smem0 + STAGES * STAGE_BYTES;  // resident weights: [column][filter row]
     bool weights_due = RESIDENT;
+    const int nst = ring_stages(p, STAGES);
     int s = 0; uint32_t ph = 0;
     uint32_t sa = smem0, fb = full0, eb = empty0;
     for (int tile = static_cast<int>(blockIdx.x); tile < total_tiles; tile += static_cast<int>(gridDim.x)) {
@@ -517,7 +521,7 @@ __device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full
                     }
                 }
                 sa += STAGE_BYTES; fb += 8u; eb += 8u;
-                if (++s == STAGES) { s = 0; ph ^= 1u; sa = smem0; fb = full0; eb = empty0; }
+                if (++s == nst) { s = 0; ph ^= 1u; sa = smem0; fb = full0; eb = empty0; }
             }
         weights_due = false;
     }
@@ -543,6 +547,7 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
     // the panel of filter row r starts r image rows into the box (error-backward reads the taps mirrored)
     const uint64_t a_first = flip ? (2 * HALO_ATOM) >> 4 : 0;
     const uint64_t a_next = flip ? ~static_cast<uint64_t>(HALO_ATOM >> 4) + 1 : HALO_ATOM >> 4;
+    const int nst = ring_stages(p, STAGES);
     int s = 0, it = 0; uint32_t ph = 0;
     uint64_t a_cur = a_base + a_first, b_cur = b_base;
     uint32_t full_cur = full0, empty_cur = empty0;
@@ -581,7 +586,7 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
                     accumulate = 1;
                 }
                 a_cur += STAGE_BYTES >> 4; b_cur += (RESIDENT ? 3 * BN * ROW_BYTES : STAGE_BYTES) >> 4; full_cur += 8u; empty_cur += 8u;
-                if (++s == STAGES) {
+                if (++s == nst) {
                     s = 0; ph ^= 1u; a_cur = a_base + a_first; full_cur = full0; empty_cur = empty0;
                     if (!RESIDENT) b_cur = b_base;
                 }

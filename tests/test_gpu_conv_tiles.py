@@ -11,6 +11,7 @@ if not torch.cuda.is_available():
     pytest.skip("needs a CUDA device", allow_module_level=True)
 
 from niti_b200 import ops, ti_torch  # noqa: E402
+from niti_b200._lib import lib  # noqa: E402
 from oracle import niti_oracle as O  # noqa: E402
 from oracle import philox  # noqa: E402
 
@@ -90,6 +91,34 @@ def test_more_than_2_to_the_31_output_rows():
     assert not any(bool(part.any()) for part in got.split(1 << 17))
     del x, got
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("C,K", [(128, 128), (64, 64), (256, 64), (144, 128)])  # weights resident, weights in the ring; two tile widths
+def test_stage_cap_reaches_the_kernels_that_share_rows(C, K):
+    """NITI_OPT_STAGE_CAP: the same bytes from a ring of one, two or all stages, and with one stage, where every load waits for
+    the products of the stage before it, a longer time (more than twice; a tenth is asserted)."""
+    rng = np.random.default_rng(C + K)
+    x, w, ea = cu(rnd8(rng, (40, 32, 32, C))), cu(rnd8(rng, (K, 3, 3, C))), torch.zeros((), dtype=torch.int32, device=DEV)
+    old, out, times = ops.set_accumulator_parking(False), [], []
+    try:
+        for cap in (0, 2, 1):
+            lib.niti_set_option(3, cap)
+            st = ops.new_requant_state(DEV)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            for i in range(60):
+                if i == 20:
+                    a.record()
+                y = ops.conv_fprop_fused(x, w, st, 1, 0, None, 0, 0, False, ea, ea)[0]
+            b.record()
+            b.synchronize()
+            out.append(y)
+            times.append(a.elapsed_time(b))
+    finally:
+        lib.niti_set_option(3, 0)
+        ops.set_accumulator_parking(old)
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+    assert times[2] > 1.1 * times[0], times
+    ops.check_status(DEV)
 
 
 @pytest.mark.parametrize("N,H,W,K", [(1, 1, 1, 16), (1, 4, 4, 16), (3, 7, 12, 80), (2, 5, 9, 144), (9, 32, 32, 48), (1, 3, 260, 64)])
