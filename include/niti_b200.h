@@ -65,7 +65,8 @@ extern "C" {
 #define NITI_OPT_ACCUMULATOR_PARKING 1
 /* NITI_OPT_WGRAD_TMA_REDUCE (default 1): the tensor-core weight gradient adds every thread block's tiles
  * straight into the zeroed gradient with TMA reductions at the L2; 0: partial sums per pixel range go to
- * scratch and a second kernel folds them.  Same integers either way. */
+ * scratch and a second kernel folds them (niti_conv_wgrad_i8; the entry points without scratch for partial sums that have a
+ * query, niti_conv_wgrad_update_i8 and niti_conv_wgrad_batch_inner_i8, then refuse every shape).  Same integers either way. */
 #define NITI_OPT_WGRAD_TMA_REDUCE 2
 /* NITI_OPT_STAGE_CAP (default 0 = all): use at most this many shared-memory stages in the GEMM / conv
  * main loops (measurement aid: separates latency-bound from bandwidth-bound behaviour). */
@@ -359,7 +360,8 @@ NITI_API int niti_update_i8(int8_t* w, const int32_t* g32, const uint32_t* maxab
                    int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream, void* stream);
 
 /* Weight gradient and update of one convolution: what niti_conv_wgrad_i8 followed by niti_update_i8 leaves behind, in three
- * launches.  g32 holds niti_conv_wgrad_update_elems() int32 (0: not a shape of this entry point): the gradient, padded to a
+ * launches.  g32 holds niti_conv_wgrad_update_elems() int32 (0: not a shape of this entry point, or NITI_OPT_WGRAD_TMA_REDUCE
+ * is 0): the gradient, padded to a
  * multiple of 4, and a tail whose first word is max |g32| afterwards.  Nothing in it has to be zero. */
 NITI_API size_t niti_conv_wgrad_update_elems(int C, int K, int R, int S, int pad);
 NITI_API int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int32_t* g32, int8_t* w,

@@ -48,7 +48,7 @@ extern "C" const char* niti_last_cuda_error(void) { return g_cuda_error; }
 
 // tuning switches (process-wide): see niti_set_option
 static int g_opt_parking = 1;
-static int g_opt_wgrad_reduce = 1;
+int niti::g_opt_wgrad_reduce = 1;
 
 extern "C" int niti_set_option(int option, int value) {
     if (option == NITI_OPT_ACCUMULATOR_PARKING) { const int old = g_opt_parking; g_opt_parking = value ? 1 : 0; return old; }
@@ -230,7 +230,7 @@ extern "C" int niti_conv_wgrad_i8(const int8_t* x, const int8_t* err, int32_t* g
 }
 
 extern "C" int niti_conv_wgrad_batch_inner_supported(int N, int C, int K, int R, int S, int pad) {
-    return same_padding(R, S, pad) && S <= 3 && N % 16 == 0 && K % 4 == 0 ? 1 : 0;
+    return g_opt_wgrad_reduce && same_padding(R, S, pad) && S <= 3 && N % 16 == 0 && K % 4 == 0 ? 1 : 0;  // it has no other way to sum
 }
 extern "C" int niti_conv_wgrad_batch_inner_i8(const int8_t* x_t, const int8_t* err_t, int32_t* out, int N, int H, int W, int C, int K,
                                               int R, int S, int pad, int32_t* status, void* stream) {

@@ -1560,7 +1560,7 @@ extern "C" int niti_update_multi_i8(const niti_update_item* items, int count, in
 // itself (grid barrier).  Per convolution that is three launches instead of the five of niti_conv_wgrad_i8 +
 // niti_update_i8 (two memsets, contraction, maximum, update), and a small layer's step is launches.
 extern "C" size_t niti_conv_wgrad_update_elems(int C, int K, int R, int S, int pad) {
-    if (C <= 0 || K <= 0 || R <= 0 || S <= 0 || !niti_conv_wgrad_accumulate_supported(C, K, R, S, pad)) return 0;
+    if (C <= 0 || K <= 0 || R <= 0 || S <= 0 || !g_opt_wgrad_reduce || !niti_conv_wgrad_accumulate_supported(C, K, R, S, pad)) return 0;
     return (static_cast<size_t>(K) * R * S * C + 3) / 4 * 4 + niti_update_multi_scratch_bytes() / 4;
 }
 extern "C" int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int32_t* g32, int8_t* w, int N, int H, int W, int C, int K,

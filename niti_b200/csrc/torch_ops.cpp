@@ -180,6 +180,10 @@ PyObject* conv_wgrad_accumulate_supported(Args& a) {
     const auto v = ints<5>(a);
     return PyBool_FromLong(niti_conv_wgrad_accumulate_supported(v[0], v[1], v[2], v[3], v[4]));
 }
+PyObject* conv_wgrad_update_supported(Args& a) {
+    const auto v = ints<5>(a);
+    return PyBool_FromLong(niti_conv_wgrad_update_elems(v[0], v[1], v[2], v[3], v[4]) != 0);
+}
 PyObject* conv_fprop_pool_fused_supported(Args& a) {
     const auto v = ints<8>(a);
     return PyBool_FromLong(niti_conv_fprop_requant_pool_supported(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]));
@@ -603,7 +607,7 @@ PyObject* quantize_input(Args& a) {
 #define NITI_ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<&name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     NITI_ENTRY(set_error_type), NITI_ENTRY(status_word), NITI_ENTRY(conv_fprop_fused_supported),
-    NITI_ENTRY(conv_dgrad_fused_supported), NITI_ENTRY(conv_wgrad_accumulate_supported), NITI_ENTRY(conv_fprop_pool_fused_supported),
+    NITI_ENTRY(conv_dgrad_fused_supported), NITI_ENTRY(conv_wgrad_accumulate_supported), NITI_ENTRY(conv_wgrad_update_supported), NITI_ENTRY(conv_fprop_pool_fused_supported),
     NITI_ENTRY(conv_fprop_scratch_bytes), NITI_ENTRY(conv_dgrad_side_bytes),
     NITI_ENTRY(conv_fprop_acc), NITI_ENTRY(conv_fprop_fused),
     NITI_ENTRY(conv_fprop_pool_fused), NITI_ENTRY(conv_dgrad_fused), NITI_ENTRY(conv_dgrad_acc), NITI_ENTRY(conv_wgrad_acc),

@@ -220,7 +220,13 @@ def conv_wgrad_acc(x, err, R=3, S=3, pad=1, out=None, want_max=True):
 
 def conv_wgrad_update(x, err, w, pad=1, mu=5, mode=ROUND_PSEUDO_STOCHASTIC, seed=None, rng_stream=0):
     """conv_wgrad_acc followed by update of the filters w, in fewer launches: (gradient int32, max|gradient|).  For the
-    shapes of conv_wgrad_accumulate_supported."""
+    shapes of conv_wgrad_accumulate_supported; with NITI_OPT_WGRAD_TMA_REDUCE off it is those two calls."""
+    K, R, S, C = w.shape
+    if not native.conv_wgrad_update_supported(C, K, R, S, pad):
+        g32, mx = conv_wgrad_acc(x, err, R, S, pad)
+        update(w, g32, mx, mu, mode, seed, rng_stream)
+        return g32, mx
+
     def work(r):
         return 2 * err.numel() * w[0].numel(), x.numel() + err.numel() + 10 * w.numel()
     return _run("niti_conv_wgrad_update_i8", 2, work, native.conv_wgrad_update, x, err, w, pad, mu, mode, seed, rng_stream)

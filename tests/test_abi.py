@@ -46,3 +46,13 @@ def test_front_end_is_rebuilt_for_another_torch(monkeypatch):
     assert not build.ops_stale()
     monkeypatch.setattr(build.metadata, "version", lambda name: "99.0")  # as after an upgrade of torch
     assert build.ops_stale()
+
+
+def test_entry_points_without_scratch_follow_the_reduction_switch():
+    from niti_b200._lib import lib
+    assert lib.niti_conv_wgrad_update_elems(16, 16, 3, 3, 1) > 0 and lib.niti_conv_wgrad_batch_inner_supported(16, 16, 16, 3, 3, 1) == 1
+    old = lib.niti_set_option(2, 0)
+    try:
+        assert lib.niti_conv_wgrad_update_elems(16, 16, 3, 3, 1) == 0 and lib.niti_conv_wgrad_batch_inner_supported(16, 16, 16, 3, 3, 1) == 0
+    finally:
+        lib.niti_set_option(2, old)

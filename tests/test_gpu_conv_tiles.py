@@ -12,6 +12,7 @@ if not torch.cuda.is_available():
 
 from niti_b200 import ops, ti_torch  # noqa: E402
 from niti_b200._lib import lib  # noqa: E402
+from niti_b200.compat import cutlassconv_cuda  # noqa: E402
 from oracle import niti_oracle as O  # noqa: E402
 from oracle import philox  # noqa: E402
 
@@ -225,3 +226,25 @@ def test_launches_are_counted_by_shape():
                                (99, 1024, 500, True, False, 2), (64, 64, 64, False, True, 1), (5, 3, 7, False, False, 1)]:
         a, b = rnd8(rng, (K, M) if ta else (M, K)), rnd8(rng, (N, K) if tb else (K, N))
         assert counted(ops.gemm_acc, cu(a), cu(b), ta, tb) == n, (M, N, K)
+
+
+@pytest.mark.parametrize("N,H,W,C,K", [(16, 5, 7, 32, 48), (32, 4, 4, 144, 128)])
+def test_partial_sums_instead_of_reductions_in_every_weight_gradient(N, H, W, C, K):
+    """NITI_OPT_WGRAD_TMA_REDUCE = 0 sends the update call and the batch-innermost form through niti_conv_wgrad_i8."""
+    rng = np.random.default_rng(N + C)
+    x, w, err = rnd8(rng, (N, H, W, C)), rnd8(rng, (K, 3, 3, C)), rnd8(rng, (N, H, W, K))
+    g, wd = O.conv_wgrad(x, err, 3, 3, 1), cu(w)
+    old = lib.niti_set_option(2, 0)
+    ops.PROFILE = []
+    try:
+        g32, mx = ops.conv_wgrad_update(cu(x), cu(err), wd, 1, 5, 2, None, 18)
+        dis = cutlassconv_cuda.sp_conv_optimized(cu(x.transpose(3, 1, 2, 0)), cu(err.transpose(3, 1, 2, 0)), 1, 1)
+        names = [p[0] for p in ops.PROFILE]
+    finally:
+        ops.PROFILE = None
+        lib.niti_set_option(2, old)
+    assert names == ["niti_conv_wgrad_i8", "niti_update_i8", "niti_conv_wgrad_i8"]
+    same(g32, g)
+    assert int(mx) == int(np.abs(g).max())
+    same(wd, O.weight_update(w, g, 5, 2)[0])
+    same(dis, g.transpose(3, 1, 2, 0))
