@@ -307,17 +307,29 @@ extern "C" int niti_gemm_i8(const int8_t* A, const int8_t* B, int32_t* C32, uint
     return simt_gemm(A, B, C32, maxabs, M, N, K, trans_a, trans_b, st);
 }
 
-// Products that only their pitches keep off the tensor cores: a classifier of any number of classes (its errors are rows
-// of that many bytes, its result rows of that many words) on more than a handful of samples.  The A rows are copied to a
-// pitch of 16 bytes, a result whose rows are not whole 16-byte groups goes through a padded copy.  From 2^24 multiplications
-// on: the CUDA-core kernels reach 1.4-2 TMAC/s (500 x 1024 x 100, gradient: 26 us), the copies and the tensor product
-// about 10 us at such sizes.
+// Products that only their pitches or a short side keep off the tensor cores: a classifier of any number of classes (its
+// errors are rows of that many bytes, its result rows of that many words), any layer on a handful of samples.  The A rows
+// are copied to a pitch of 16 bytes, a result whose rows are not whole 16-byte groups goes through a padded copy.
+// Where the line lies (780 random shapes of up to 16384 samples, both routes timed; us, CUDA cores / tensor cores):
+//   below 2^24 multiplications the CUDA cores;
+//   both operands along the reduction (x * W^T): the tensor route walks the reduction in series, about 0.36 us per 128 of it,
+//     the CUDA-core kernel puts a warp on every result.  10 x 259 x 8032: 8 / 31, 61 x 112 x 5472: 12 / 20, 245 x 127 x 640:
+//     19 / 13.  From M N >= 4 K + 4096 on the tensor cores win or lie within 1.3;
+//   W [K][N] with a reduction below 112, more than one row tile and fewer than 2^20 results: the copies cost more than the
+//     product until 2^25 multiplications (929 x 544 x 54: 10 / 14, 1204 x 224 x 74: 10 / 13, 1020 x 400 x 143: 18 / 14);
+//   every other product: 18 x 112 x 8886 (gradient): 389 / 36, 607 x 48 x 725: 37 / 13, 48 x 3024 x 119: 13 / 10.
+static bool padded_pays(int M, int N, int K, int trans_a, int trans_b) {
+    const long long outs = static_cast<long long>(M) * N, macs = outs * K;
+    if (macs < (1ll << 24)) return false;
+    if (!trans_a && trans_b) return outs >= 4ll * K + 4096;
+    return trans_b || K >= 112 || M <= 128 || outs >= (1ll << 20) || macs >= (1ll << 25);
+}
 struct PaddedGemm { bool use; int lda, ldc; size_t a_bytes, c_bytes; };
 static PaddedGemm padded_gemm(int M, int N, int K, int trans_a, int trans_b) {
     PaddedGemm g{};
     const int pitch_a = trans_a ? M : K, rows_a = trans_a ? K : M, pitch_b = trans_b ? K : N;
     const bool dense = pitch_a % 16 == 0 && N % 4 == 0 && M >= 64 && N >= 32 && K >= 32;
-    g.use = !dense && pitch_b % 16 == 0 && static_cast<long long>(M) * N * K >= (1ll << 24);
+    g.use = !dense && pitch_b % 16 == 0 && padded_pays(M, N, K, trans_a, trans_b);
     if (!g.use) return g;
     g.lda = pitch_a % 16 == 0 ? 0 : (pitch_a + 15) / 16 * 16;
     g.ldc = N % 4 == 0 ? 0 : (N + 3) / 4 * 4;

@@ -56,3 +56,12 @@ def test_entry_points_without_scratch_follow_the_reduction_switch():
         assert lib.niti_conv_wgrad_update_elems(16, 16, 3, 3, 1) == 0 and lib.niti_conv_wgrad_batch_inner_supported(16, 16, 16, 3, 3, 1) == 0
     finally:
         lib.niti_set_option(2, old)
+
+
+def test_padded_products_leave_deep_reductions_with_few_results_to_the_cuda_cores():
+    from niti_b200._lib import lib
+    padded = lambda *a: lib.niti_gemm_scratch_bytes(*a) > 0
+    for M, N, K in [(1, 2048, 8192), (10, 259, 8032), (61, 112, 5472), (498, 24, 8064), (2, 4096, 4096)]:
+        assert not padded(M, N, K, 0, 1)
+    assert padded(245, 127, 640, 0, 1) and padded(18, 112, 8886, 1, 0) and padded(607, 48, 725, 0, 0)
+    assert not padded(929, 544, 54, 1, 0) and padded(1020, 400, 143, 1, 0)
