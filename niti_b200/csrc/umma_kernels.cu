@@ -255,7 +255,7 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int mn, int* m_
 
 // ---- warp roles shared by the streaming kernel and the accumulator-parking kernel -------------
 // stages of the ring in use (NITI_OPT_STAGE_CAP)
-__device__ __forceinline__ int ring_stages(const GemmParams& p, int compiled) { return keep_reg((p.nstages > 0 && p.nstages < compiled) ? p.nstages : compiled); }
+__device__ __forceinline__ int ring_stages(const GemmParams& p, int compiled) { return (p.nstages > 0 && p.nstages < compiled) ? p.nstages : compiled; }
 
 // TMA producer: fills the stage ring for every tile of this CTA, in tile order.  The WHOLE warp runs the loop and
 // an elected lane issues.  TMA and MMA instructions take their operands from uniform registers, and the compiler keeps
@@ -268,7 +268,9 @@ __device__ __forceinline__ int ring_stages(const GemmParams& p, int compiled) { 
 // TWO: this CTA is half of a CTA pair (cluster ranks 0/1).  Tiles are 256 rows high: rank r owns rows
 // [128 r, 128 r + 128) of the pair's tile (m tile 2*pair_m + r) and columns [r BN/2, (r+1) BN/2) of the B
 // operand; all byte counts are reported to rank 0's "full" barrier, which its MMA thread waits on.
-template <int BN, int STAGES, int STAGE_BYTES, bool TWO>
+// ROWS32: operands of 32-byte rows (p.rows32).  A variant of its own: as a branch of the one loop its byte counts and
+// sources made every other product's issue slower (2048 x 128 x 4096: 20.5 us with the branch, 18.5 without; 8x8x8, 512 -> 256: 20.5, 18.5).
+template <int BN, int STAGES, int STAGE_BYTES, bool TWO, bool ROWS32>
 __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, const CUtensorMap* tmA,
                                               const CUtensorMap* tmB, const GemmParams& p, volatile int* abort_flag) {
     const int mn_tiles = p.m_tiles * p.n_tiles;
@@ -282,7 +284,7 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
     const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
     const int conv = keep_reg(p.conv), flip = keep_reg(p.flip), pad = keep_reg(p.pad), S = keep_reg(p.S), cblocks = keep_reg(p.cblocks);
     const int tapstride = keep_reg(p.tapstride), b_mn = keep_reg(p.b_mn), a_mn = keep_reg(p.a_mn);
-    const int rows32 = keep_reg(p.rows32);
+    const int rows32 = ROWS32 ? keep_reg(p.rows32) : 0;
     const uint32_t tx_full = static_cast<uint32_t>(keep_reg(TWO ? 2 * (p.a_bytes + BNH * ROW_BYTES) : p.a_bytes + BN * ROW_BYTES));
     int s = 0; uint32_t ph = 0;
     uint32_t sa = smem0, fb_cur = full0, eb_cur = empty0;  // running stage pointers, wrapping with the ring
@@ -314,7 +316,7 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
             const uint32_t sb = sa + PANEL_BYTES;
             uint32_t fb = fb_cur;
             uint32_t tx_bytes = tx_full, tx_b = 0;
-            if (rows32 != 0) {  // the last rows of an operand may be fewer than a tile's; what they leave in the stage meets zeros or rows nobody stores
+            if (ROWS32) {  // the last rows of an operand may be fewer than a tile's; what they leave in the stage meets zeros or rows nobody stores
                 const int b_rows = rows32 == 1 ? min(BN, p.N - ncol) : min(128, p.K - kb * 128);
                 tx_b = static_cast<uint32_t>(b_rows) * 32u;
                 tx_bytes = tx_b + (rows32 == 1 ? static_cast<uint32_t>(min(BLOCK_M, p.M - m_t * BLOCK_M)) * 32u : static_cast<uint32_t>(PANEL_BYTES));
@@ -341,10 +343,10 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
                         if (TWO) tma_load_2d_pair(sb, tmB, fb, tap * tapstride + cb * ROW_BYTES, ncol);
                         else     tma_load_2d(sb, tmB, fb, tap * tapstride + cb * ROW_BYTES, ncol);
                     }
-                } else if (rows32 == 1) {
+                } else if (ROWS32 && rows32 == 1) {
                     bulk_load(sa, p.a32 + static_cast<long long>(m_t) * (BLOCK_M * 32), tx_bytes - tx_b, fb);
                     bulk_load(sb, p.b32 + static_cast<long long>(ncol) * 32, tx_b, fb);
-                } else if (rows32 == 2) {
+                } else if (ROWS32) {
                     tma_load_2d(sa, tmA, fb, m_t * BLOCK_M, kb * 128);
                     bulk_load(sb, p.b32 + static_cast<long long>(kb) * (128 * 32), tx_b, fb);
                 } else {
@@ -387,13 +389,14 @@ template <bool TWO>
 __device__ __forceinline__ void umma_issue(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     if (TWO) umma_i8_pair(d_tmem, a, b, idesc, accumulate); else umma_i8(d_tmem, a, b, idesc, accumulate);
 }
-template <int BN, int STAGES, int STAGE_BYTES, int NACC, bool TWO>
+template <int BN, int STAGES, int STAGE_BYTES, int NACC, bool TWO, bool ROWS32>
 __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* tfull_bar,
                                          uint64_t* tempty_bar, uint32_t tmem_base_in, const GemmParams& p, volatile int* abort_flag) {
     constexpr bool PARKED = NACC == 0;
+    const int rows32 = ROWS32 ? keep_reg(p.rows32) : 0;
     const int mn_tiles = p.m_tiles * p.n_tiles;
     const int total_tiles = mn_tiles * p.splits;
-    const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, p.rows32 == 2 ? 32 : BN, p.a_mn, p.b_mn);
+    const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, rows32 == 2 ? 32 : BN, p.a_mn, p.b_mn);
     const int nst = ring_stages(p, STAGES);
     const int first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
@@ -402,17 +405,17 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
     // operand descriptors of stage 0 (a stage's are these advanced by the stage offset) and the K = 32 steps
     const uint32_t s0 = smem_u32(smem);
-    const uint64_t a_base = p.rows32 == 1 ? make_smem_desc(s0, 16, 256, SWIZZLE_32B_CODE) : p.a_mn ? make_smem_desc(s0, PANEL_BYTES, 1024, SWIZZLE_128B_CODE) : make_smem_desc(s0, 16, 1024, SWIZZLE_128B_CODE);
+    const uint64_t a_base = rows32 == 1 ? make_smem_desc(s0, 16, 256, SWIZZLE_32B_CODE) : p.a_mn ? make_smem_desc(s0, PANEL_BYTES, 1024, SWIZZLE_128B_CODE) : make_smem_desc(s0, 16, 1024, SWIZZLE_128B_CODE);
     // a 64-column MN-major operand has rows of 64 bytes: 64-byte swizzle, 8-row groups of 512 bytes
-    const uint64_t b_base = p.rows32 != 0 ? make_smem_desc(s0 + PANEL_BYTES, 1024, 256, SWIZZLE_32B_CODE) : p.b_mn ? (BN == 64 ? make_smem_desc(s0 + PANEL_BYTES, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
+    const uint64_t b_base = ROWS32 ? make_smem_desc(s0 + PANEL_BYTES, 1024, 256, SWIZZLE_32B_CODE) : p.b_mn ? (BN == 64 ? make_smem_desc(s0 + PANEL_BYTES, 64 * ROW_BYTES, 512, SWIZZLE_64B_CODE)
                                                : make_smem_desc(s0 + PANEL_BYTES, PANEL_BYTES, 1024, SWIZZLE_128B_CODE))
                                    : make_smem_desc(s0 + PANEL_BYTES, 16, 1024, SWIZZLE_128B_CODE);
     const uint32_t a_step = static_cast<uint32_t>(keep_reg((p.a_mn ? 32 * ROW_BYTES : 32) >> 4));  // in descriptor units of 16 bytes
-    const uint32_t b_step = static_cast<uint32_t>(keep_reg((p.rows32 == 2 ? 32 * 32 : p.b_mn ? 32 * (BN == 64 ? 64 : ROW_BYTES) : 32) >> 4));
+    const uint32_t b_step = static_cast<uint32_t>(keep_reg((rows32 == 2 ? 32 * 32 : p.b_mn ? 32 * (BN == 64 ? 64 : ROW_BYTES) : 32) >> 4));
     const int conv = keep_reg(p.conv), red = keep_reg(p.red), cblocks = keep_reg(p.cblocks), num_kb = keep_reg(p.num_kb), splits = keep_reg(p.splits);
     int s = 0; uint32_t ph = 0; bool ok = true; int it = 0;
     // every reduction block has four MMAs unless a conv tap's channel count ends in a partial 128-byte block
-    const bool all4 = conv ? (red & 127) == 0 : p.rows32 != 1;
+    const bool all4 = conv ? (red & 127) == 0 : rows32 != 1;
     // running stage pointers: descriptors and barrier addresses advance by one stage per block and wrap with the ring
     const uint64_t stage_step = STAGE_BYTES >> 4;
     uint64_t a_cur = a_base, b_cur = b_base;
@@ -484,7 +487,9 @@ constexpr int HALO_A_BYTES = 18 * HALO_ATOM;      // at most 16 + 2 image rows
 // 72 or 144 KB) in shared memory behind the ring; they arrive with the first tile, column by column (one barrier each),
 // and a stage is activations only.  The loads are paced by rows of 128 bytes (about 3 cycles each): 432 a tile instead
 // of 1008 (64 columns) or 1584 (128).
-enum LoadMode : int { LOAD_TAPS = 0, LOAD_HALO = 1, LOAD_HALO_RESIDENT = 2 };
+// LOAD_ROWS32: operands of 32-byte rows (the thin layer; streaming only).
+enum LoadMode : int { LOAD_TAPS = 0, LOAD_HALO = 1, LOAD_HALO_RESIDENT = 2, LOAD_ROWS32 = 3 };
+constexpr bool shares_rows(int mode) { return mode == LOAD_HALO || mode == LOAD_HALO_RESIDENT; }
 template <int BN, int STAGES, int STAGE_BYTES, bool RESIDENT>
 __device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint32_t weights0, const CUtensorMap* tmA,
                                                    const CUtensorMap* tmB, const GemmParams& p, volatile int* abort_flag) {
@@ -725,7 +730,7 @@ __device__ __forceinline__ void store_piece(int8_t* at, int cols, const uint32_t
 }
 
 // Plain products: int32 out (+ max|acc|).
-template <int BN, bool TWO>
+template <int BN, bool TWO, bool ROWS32>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)  // 10 warps: 3 on one scheduler -> at most 168 registers per thread
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const GemmParams p) {
@@ -775,11 +780,11 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // Only one lane of warps 0 and 1 works; the others wait at __syncwarp so that each warp reaches the
     // block-wide barrier of the teardown converged (an aligned barrier executed by a diverged warp is undefined).
     if (warp == 0) {
-        producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
         __syncwarp();
     } else if (warp == 1) {
         if (rank == 0)
-            mma_role<BN, STAGES, Cfg::STAGE_BYTES, 2, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            mma_role<BN, STAGES, Cfg::STAGE_BYTES, 2, TWO, ROWS32>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue (2 x 4 warps)
@@ -1017,13 +1022,13 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (warp == 0) {
-        if constexpr (MODE != LOAD_TAPS) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
-        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        if constexpr (shares_rows(MODE)) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if (rank == 0) {
-            if constexpr (MODE != LOAD_TAPS) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, tempty_bar, tmem_base, p, abort_flag);
-            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            if constexpr (shares_rows(MODE)) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
         }
         __syncwarp();
     } else {
@@ -1229,13 +1234,13 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const int cta_step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
     if (warp == 0) {
-        if constexpr (MODE != LOAD_TAPS) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
-        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        if constexpr (shares_rows(MODE)) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if (rank == 0) {
-            if constexpr (MODE != LOAD_TAPS) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, 0, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, nullptr, tmem_base, p, abort_flag);
-            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
+            if constexpr (shares_rows(MODE)) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, 0, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, nullptr, tmem_base, p, abort_flag);
+            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO, false>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
         }
         __syncwarp();
     } else {
@@ -1688,10 +1693,10 @@ static int sm_count() {
 }
 
 // CTA pairs (TWO): clusters of two CTAs, p.m_tiles counts 256-row tiles
-template <int BN, bool TWO>
+template <int BN, bool TWO, bool ROWS32 = false>
 static int launch_gemm_inst(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p, cudaStream_t st) {
     using Cfg = GemmCfg<BN, TWO>;
-    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN, TWO, ROWS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     int tiles = p.m_tiles * p.n_tiles * p.splits;
     if (tiles > sm_count() / (TWO ? 2 : 1)) tiles = sm_count() / (TWO ? 2 : 1);
@@ -1701,11 +1706,12 @@ static int launch_gemm_inst(const CUtensorMap& a, const CUtensorMap& b, const CU
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = TWO ? 1 : 0;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BN, TWO>, a, b, c, p));
+    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BN, TWO, ROWS32>, a, b, c, p));
 }
 static int launch_gemm(int bn, bool pair, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p,
                        cudaStream_t st) {
     if (pair) return bn == 256 ? launch_gemm_inst<256, true>(a, b, c, p, st) : launch_gemm_inst<128, true>(a, b, c, p, st);
+    if (p.rows32) return bn == 256 ? launch_gemm_inst<256, false, true>(a, b, c, p, st) : launch_gemm_inst<128, false, true>(a, b, c, p, st);
     return bn == 256 ? launch_gemm_inst<256, false>(a, b, c, p, st) : launch_gemm_inst<128, false>(a, b, c, p, st);
 }
 // CTA pairs (M = 256 MMAs, B operand split between the two CTAs): bit 0 enables them for GEMMs, bit 1 for
@@ -1750,6 +1756,10 @@ static int launch_requant(int bn, bool pair, int mode, bool parked, const CUtens
     if (mode == LOAD_HALO_RESIDENT)
         return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO_RESIDENT, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO_RESIDENT, false>(a, b, p, st);
     if (mode == LOAD_HALO) return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO, false>(a, b, p, st);
+    if (mode == LOAD_ROWS32)
+        return bn == 64    ? launch_requant_inst<64, false, LOAD_ROWS32, false>(a, b, p, st)
+               : bn == 256 ? launch_requant_inst<256, false, LOAD_ROWS32, false>(a, b, p, st)
+                           : launch_requant_inst<128, false, LOAD_ROWS32, false>(a, b, p, st);
     if (bn == 64) return launch_requant_inst<64, false, LOAD_TAPS, false>(a, b, p, st);
     return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, false>(a, b, p, st);
 }
@@ -1882,7 +1892,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.group_m = (static_cast<long long>(M) + N) * K > (48ll << 20) ? 8 : 0;
     set_fused(&p, fused);
     finish_params(&p);
-    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, LOAD_TAPS, false, ma, mb, p, st); }
+    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, rows32 ? LOAD_ROWS32 : LOAD_TAPS, false, ma, mb, p, st); }
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
