@@ -122,6 +122,31 @@ def test_stage_cap_reaches_the_kernels_that_share_rows(C, K):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("N,H,W,C,K", [(80, 32, 32, 144, 48), (90, 30, 28, 272, 64), (76, 32, 32, 160, 112), (90, 30, 28, 144, 128)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_tiles_that_share_rows_over_several_rounds_of_the_ring(N, H, W, C, K, mode):
+    """More than four tiles per thread block with the weights in the ring: accumulators and stages are used again, 64-column
+    tiles are dealt to two pairs of warp groups.  Against the int32 products, narrowed by the stand-alone kernel."""
+    rng = np.random.default_rng(N + C + K)
+    x, w, err = cu(np.maximum(rnd8(rng, (N, H, W, C)), 0)), cu(rnd8(rng, (K, 3, 3, C))), cu(rnd8(rng, (N, H, W, C)))
+    wb = cu(rnd8(rng, (C, 3, 3, K)))  # error-backward of a layer K -> C has K output columns
+    mask = cu(rnd8(rng, (N, H, W, K)))
+    seed, ea = ops.seed_tensor(9, DEV), torch.zeros((), dtype=torch.int32, device=DEV)
+    want, e, s = ops.requant(*ops.conv_fprop_acc(x, w), ops.CALC_ACT, 7, mode, seed, 3, relu=True, exp_a=ea, want_shift=True)
+    want_b = ops.relu_bwd(mask, ops.requant(*ops.conv_dgrad_acc(err, wb), ops.CALC_ERR, 7, mode, seed, 4)[0])
+    old = ops.set_accumulator_parking(False)
+    try:
+        fwd, bwd = ops.new_requant_state(DEV), ops.new_requant_state(DEV)
+        side = torch.empty(ops.conv_dgrad_side_bytes(N, H, W, K, C, 3, 3, 1), dtype=torch.uint8, device=DEV)
+        for _ in range(2):
+            y, ey, sy = ops.conv_fprop_fused(x, w, fwd, 1, mode, seed, 3, 0, True, ea, None)
+            assert torch.equal(y, want) and int(ey) == int(e) and int(sy) == int(s)
+            assert torch.equal(ops.conv_dgrad_fused(err, wb, bwd, 1, mode, seed, 4, 0, None, None, relu_mask=mask, side=side)[0], want_b)
+    finally:
+        ops.set_accumulator_parking(old)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("N,H,W,K", [(1, 1, 1, 16), (1, 4, 4, 16), (3, 7, 12, 80), (2, 5, 9, 144), (9, 32, 32, 48), (1, 3, 260, 64)])
 def test_thin_layer(N, H, W, K):
     """Rows of whole words take the staged gather, the others the general one; fewer pixels than a tile; 16 to 144 filters."""
