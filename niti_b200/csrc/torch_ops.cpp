@@ -423,6 +423,7 @@ PyObject* conv_wgrad_accumulate(Args& a) {
     return wrap(g32);
 }
 
+// result, maximum, and how many launches besides the product the call made (row copies around a padded product)
 PyObject* gemm_acc(Args& a) {
     const Tensor &A = a.tensor(), &B = a.tensor();
     const bool ta = a.flag(), tb = a.flag();
@@ -433,17 +434,25 @@ PyObject* gemm_acc(Args& a) {
     const int M = A.size(ta ? 1 : 0), K = A.size(ta ? 0 : 1), N = B.size(tb ? 0 : 1);
     require(B.size(tb ? 1 : 0) == K);
     Tensor c32, mx;
+    size_t nb = 0;
     {
         Launch l(A);
         c32 = out ? *out : l.empty({M, N}, at::kInt);
         if (want_max) mx = l.empty({1}, at::kInt);
-        const size_t nb = niti_gemm_scratch_bytes(M, N, K, ta, tb);
+        nb = niti_gemm_scratch_bytes(M, N, K, ta, tb);
         Tensor sc;
         if (nb) sc = l.bytes(nb);
         check(niti_gemm_scratch_i8(cptr<int8_t>(A), cptr<int8_t>(B), mptr<int32_t>(c32), want_max ? mptr<uint32_t>(mx) : nullptr,
                                    nb ? mptr(sc) : nullptr, nb, M, N, K, ta, tb, l.status(), l.stream), "niti_gemm_i8");
     }
-    return tuple(c32, mx);
+    const auto aligned = [](const Tensor& t) { return reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0; };
+    const bool padded = nb != 0 && aligned(A) && aligned(B) && aligned(c32);
+    PyObject* r = PyTuple_New(3);
+    if (r == nullptr) throw python_error();
+    PyTuple_SET_ITEM(r, 0, wrap(c32));
+    PyTuple_SET_ITEM(r, 1, wrap(mx));
+    PyTuple_SET_ITEM(r, 2, PyLong_FromLong(padded ? ((ta ? M : K) % 16 != 0) + (N % 4 != 0) : 0));
+    return r;
 }
 
 // ---------------------------------------------------------------------------------------------- requantisation, memory-bound layers

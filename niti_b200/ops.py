@@ -169,8 +169,8 @@ def conv_fprop_fused(x, w, state, pad=1, mode=ROUND_NEAREST, seed=None, rng_stre
     def work(r):
         return 2 * r[0].numel() * w[0].numel(), x.numel() + w.numel() + r[0].numel()
     # contraction and conditional second launch; a thin layer gathers its patches first
-    return _run("niti_conv_fprop_requant_i8", 3 if w.numel() <= 32 * w.shape[0] else 2, work, native.conv_fprop_fused, x, w, state, pad, mode, seed, rng_stream, rng_offset,
-                relu, exp_a, exp_b, scratch_buf)
+    return _run("niti_conv_fprop_requant_i8", 3 if w.numel() <= 32 * w.size(0) else 2, work, native.conv_fprop_fused, x, w, state, pad,
+                mode, seed, rng_stream, rng_offset, relu, exp_a, exp_b, scratch_buf)
 
 
 def conv_fprop_pool_fused_supported(N, H, W, C, K, R, S, pad):
@@ -215,7 +215,7 @@ def conv_wgrad_acc(x, err, R=3, S=3, pad=1, out=None, want_max=True):
     """Weight gradient accumulators and max|g32| (None when want_max is False: update_multi finds it)."""
     def work(r):
         return 2 * err.numel() * R * S * x.shape[3], x.numel() + err.numel() + 4 * r[0].numel()
-    return _run("niti_conv_wgrad_i8", 2 if x.shape[3] % 16 == 0 else 3, work, native.conv_wgrad_acc, x, err, R, S, pad, out, want_max)
+    return _run("niti_conv_wgrad_i8", 2 if x.size(3) % 16 == 0 else 3, work, native.conv_wgrad_acc, x, err, R, S, pad, out, want_max)
 
 
 def conv_wgrad_update(x, err, w, pad=1, mu=5, mode=ROUND_PSEUDO_STOCHASTIC, seed=None, rng_stream=0):
@@ -288,12 +288,10 @@ def gemm_acc(a, b, trans_a=False, trans_b=False, out=None, want_max=True):
     """C32[M,N] = op(a) @ op(b); a is [M,K] ([K,M] if trans_a), b is [K,N] ([N,K] if trans_b)."""
     def work(r):
         return 2 * r[0].numel() * a.shape[0 if trans_a else 1], a.numel() + b.numel() + 4 * r[0].numel()
-    # row copies around a product whose pitches the tensor cores do not take (see niti_gemm_scratch_i8)
-    copies = (a.shape[1] % 16 != 0) + ((b.shape[0] if trans_b else b.shape[1]) % 4 != 0)
-    if copies:
-        (k, m) = a.shape if trans_a else a.shape[::-1]
-        copies *= lib.niti_gemm_scratch_bytes(m, b.shape[0] if trans_b else b.shape[1], k, trans_a, trans_b) > 0
-    return _run("niti_gemm_i8", 1 + copies, work, native.gemm_acc, a, b, trans_a, trans_b, out, want_max)
+    global LAUNCHES
+    c32, mx, copies = _run("niti_gemm_i8", 1, work, native.gemm_acc, a, b, trans_a, trans_b, out, want_max)
+    LAUNCHES += copies  # of rows, around a product whose pitches the tensor cores do not take (see niti_gemm_scratch_i8)
+    return c32, mx
 
 
 def group_conv1(inp, wt, pad):
