@@ -65,3 +65,15 @@ def test_padded_products_leave_deep_reductions_with_few_results_to_the_cuda_core
         assert not padded(M, N, K, 0, 1)
     assert padded(245, 127, 640, 0, 1) and padded(18, 112, 8886, 1, 0) and padded(607, 48, 725, 0, 0)
     assert not padded(929, 544, 54, 1, 0) and padded(1020, 400, 143, 1, 0)
+
+
+def test_the_reference_arm_without_the_reference_says_so():
+    import json
+    import subprocess
+    import sys
+    import pytest
+    if os.path.isfile(os.path.join(ROOT, "oracle", "_ref", "ti_torch.py")):
+        pytest.skip("the reference's Python is here")
+    out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference"], capture_output=True, text=True, timeout=300, check=True)
+    line = json.loads(out.stdout.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
