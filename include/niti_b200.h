@@ -298,7 +298,8 @@ NITI_API int niti_gemm_i8(const int8_t* A, const int8_t* B, int32_t* C32, uint32
  * (ti_torch.py:23-72,103-147), with RangeEstimate (ti_torch.py:366-377) already reduced into
  * *maxabs by the producing kernel.  bits = 0 if max==0 else bit_length(max-1);
  * shift = max(bits - target_bits, 0); shift == 0 wraps (tensor.type(int8)), otherwise round
- * and clamp to +-127; kind GRAD with bits == 0 writes zeros.
+ * and clamp to +-127 (also where *maxabs does not bound the data: a caller may choose a shift by it); kind GRAD with
+ * bits == 0 writes zeros.
  * Random word of element i (stochastic mode): Philox4x32-10 keyed by *seed, stream `rng_stream`,
  * element index rng_offset + i.  If relu != 0, max(.,0) is applied after narrowing
  * (TiReLU.forward, ti_torch.py:272-279).
