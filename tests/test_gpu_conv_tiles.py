@@ -147,6 +147,37 @@ def test_tiles_that_share_rows_over_several_rounds_of_the_ring(N, H, W, C, K, mo
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("K", [16, 112, 272])  # one column tile of 64, of 128, two of 256
+@pytest.mark.parametrize("parking", [False, True])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_accumulators_that_need_no_shift(K, parking, mode):
+    """A maximum of 128 has 7 bits: the low bytes as they are, so that 128 wraps to -128 (and ends as 0 behind a ReLU)."""
+    rng = np.random.default_rng(K)
+    x, w = np.zeros((2, 9, 10, 16), np.int8), rng.integers(-2, 3, size=(K, 3, 3, 16)).astype(np.int8)
+    x[0, 2, 2, 0], x[1, 6, 7, 3], x[1, 1, 1, 5] = 64, -64, 9
+    acc = O.conv_fprop(x, w)
+    assert np.abs(acc).max() == 128 and O.act_calc(acc, 0)[2] == 0
+    err = np.zeros((2, 9, 10, K), np.int8)
+    err[0, 2, 2, 0], err[1, 6, 7, K - 1], err[1, 1, 1, 5] = 64, -64, 9
+    back = O.conv_dgrad(err, w)
+    assert np.abs(back).max() == 128
+    seed, z = ops.seed_tensor(9, DEV), torch.zeros((), dtype=torch.int32, device=DEV)
+    old = ops.set_accumulator_parking(parking)
+    try:
+        for relu in (False, True):
+            st = ops.new_requant_state(DEV)
+            for _ in range(2):
+                y, _, shift = ops.conv_fprop_fused(cu(x), cu(w), st, 1, mode, seed, 3, 0, relu, z, z)
+                same(y, np.maximum(O.wrap_int8(acc), 0) if relu else O.wrap_int8(acc))
+                assert int(shift) == 0
+        e, _, shift = ops.conv_dgrad_fused(cu(err), cu(w), ops.new_requant_state(DEV), 1, mode, seed, 4, 0, z, z)
+        same(e, O.wrap_int8(back))
+        assert int(shift) == 0
+    finally:
+        ops.set_accumulator_parking(old)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("N,H,W,K", [(1, 1, 1, 16), (1, 4, 4, 16), (3, 7, 12, 80), (2, 5, 9, 144), (9, 32, 32, 48), (1, 3, 260, 64)])
 def test_thin_layer(N, H, W, K):
     """Rows of whole words take the staged gather, the others the general one; fewer pixels than a tile; 16 to 144 filters."""
