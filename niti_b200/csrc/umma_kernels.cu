@@ -18,6 +18,7 @@
 //            a second 128-wide panel sits `rows * 128` bytes further (leading byte offset).
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 
@@ -145,7 +146,8 @@ struct GemmCfg {
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 };
 
-__device__ __forceinline__ void report_abort(int32_t* status, int code, int role) {
+// a call of its own: its dozen instructions at every wait lay between the ones that a launch fetches and runs once
+__device__ __noinline__ void report_abort(int32_t* status, int code, int role) {
     if (status != nullptr && atomicCAS(status, 0, code) == 0) {
         status[1] = static_cast<int32_t>(blockIdx.x + blockIdx.y * gridDim.x);
         status[2] = role;
@@ -272,12 +274,11 @@ __device__ __forceinline__ int ring_stages(const GemmParams& p, int compiled) { 
 // sources made every other product's issue slower (2048 x 128 x 4096: 20.5 us with the branch, 18.5 without; 8x8x8, 512 -> 256: 20.5, 18.5).
 template <int BN, int STAGES, int STAGE_BYTES, bool TWO, bool ROWS32>
 __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, const CUtensorMap* tmA,
-                                              const CUtensorMap* tmB, const GemmParams& p, volatile int* abort_flag) {
+                                              const CUtensorMap* tmB, const GemmParams& p, const int first, const int step,
+                                              volatile int* abort_flag) {
     const int mn_tiles = p.m_tiles * p.n_tiles;
     const int total_tiles = mn_tiles * p.splits;
     const uint32_t rank = TWO ? __shfl_sync(0xFFFFFFFFu, cluster_ctarank(), 0) : 0u;  // a special register: make it provably uniform
-    const int first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-    const int step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
     constexpr int BNH = TWO ? BN / 2 : BN;  // B columns this CTA loads
     const int nst = ring_stages(p, STAGES);
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
@@ -391,15 +392,14 @@ __device__ __forceinline__ void umma_issue(uint32_t d_tmem, uint64_t a, uint64_t
 }
 template <int BN, int STAGES, int STAGE_BYTES, int NACC, bool TWO, bool ROWS32>
 __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* tfull_bar,
-                                         uint64_t* tempty_bar, uint32_t tmem_base_in, const GemmParams& p, volatile int* abort_flag) {
+                                         uint64_t* tempty_bar, uint32_t tmem_base_in, const GemmParams& p, const int first, const int step,
+                                         volatile int* abort_flag) {
     constexpr bool PARKED = NACC == 0;
     const int rows32 = ROWS32 ? keep_reg(p.rows32) : 0;
     const int mn_tiles = p.m_tiles * p.n_tiles;
     const int total_tiles = mn_tiles * p.splits;
     const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, rows32 == 2 ? 32 : BN, p.a_mn, p.b_mn);
     const int nst = ring_stages(p, STAGES);
-    const int first = TWO ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-    const int step = TWO ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
     const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_in, 0);  // read from shared memory: make it provably uniform
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
     const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
@@ -789,11 +789,11 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // Only one lane of warps 0 and 1 works; the others wait at __syncwarp so that each warp reaches the
     // block-wide barrier of the teardown converged (an aligned barrier executed by a diverged warp is undefined).
     if (warp == 0) {
-        producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, cta_first, cta_step, abort_flag);
         __syncwarp();
     } else if (warp == 1) {
         if (rank == 0)
-            mma_role<BN, STAGES, Cfg::STAGE_BYTES, 2, TWO, ROWS32>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            mma_role<BN, STAGES, Cfg::STAGE_BYTES, 2, TWO, ROWS32>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, cta_first, cta_step, abort_flag);
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue (2 x 4 warps)
@@ -1032,12 +1032,12 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
     if (warp == 0) {
         if constexpr (shares_rows(MODE)) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
-        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, cta_first, cta_step, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if (rank == 0) {
             if constexpr (shares_rows(MODE)) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, tempty_bar, tmem_base, p, abort_flag);
-            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, cta_first, cta_step, abort_flag);
         }
         __syncwarp();
     } else {
@@ -1192,6 +1192,56 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // ------------------------------------------------------------------------------------------------
 constexpr unsigned long long GRID_BARRIER_LIMIT_NS = 500000000ull;  // 0.5 s
 
+// The grid barrier of the kernels below, run by a CTA's epilogue warps (which have left their maxima in warp_max): every CTA
+// has contributed its maximum when it returns the shift that narrows the tensor, the same to all of them; -1 where the others
+// did not arrive or a role of this CTA gave up.
+// One atomic per CTA: atomics on one address serialise at the L2; the waiters poll with plain acquire loads for the same reason.
+// The exit ticket (thread 64's) is drawn as soon as this CTA has read the barrier's words, so that its round trip runs under
+// the narrowing; drawn at the end, behind a barrier of the epilogue warps, it was 0.45 us of every launch.
+__device__ __forceinline__ int parked_grid_shift(const GemmParams& p, const volatile unsigned* warp_max, volatile int* shift_slot,
+                                                 volatile int* abort_flag, int* ticket) {
+    int32_t* st = p.state;
+    named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
+    if (threadIdx.x == 64) {
+        unsigned cta_max = 0;
+#pragma unroll
+        for (int i = 0; i < EPI_WARPS; ++i) cta_max = max(cta_max, warp_max[i]);
+        // The maximum and the arrival count sit side by side (st[6], st[7]): two fire-and-forget reductions on the
+        // way in (the count's release orders the maximum before it), ONE 64-bit acquire load per poll that returns
+        // both -- a fence + atomicAdd + atomicMax read-back would add three round trips to the L2.
+        if (cta_max != 0) red_relaxed_max(reinterpret_cast<unsigned*>(&st[6]), cta_max);
+        red_release_add(&st[7], 1);
+        const unsigned long long t0 = global_timer_ns();
+        bool arrived = false;
+        unsigned m = 0;
+        for (unsigned spin = 0;; ++spin) {
+            const unsigned long long both = ld_acquire_gpu_u64(&st[6]);
+            if (static_cast<int>(both >> 32) >= static_cast<int>(gridDim.x)) { arrived = true; m = static_cast<unsigned>(both); break; }
+            if ((spin & 63) == 63) {
+                if (*abort_flag || global_timer_ns() - t0 > GRID_BARRIER_LIMIT_NS) break;
+            }
+        }
+        bool zero_out;
+        *shift_slot = arrived && !*abort_flag ? shift_for(m, p.kind, p.target_bits, &zero_out) : -1;
+        if (!arrived) { *abort_flag = 1; report_abort(p.status, 5, 2); }
+    }
+    named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
+    if (threadIdx.x == 64) *ticket = atomicAdd(&st[4], 1);
+    return *shift_slot;
+}
+// the CTA that drew the last ticket publishes the shift and clears the words for the next call
+__device__ __forceinline__ void parked_leave(const GemmParams& p, int shift, int ticket) {
+    int32_t* st = p.state;
+    if (threadIdx.x == 64) {
+        if (ticket == static_cast<int>(gridDim.x) - 1) {
+            const int s_out = shift < 0 ? 0 : shift;
+            st[0] = s_out; st[2] = 0; st[1] = 0; st[5] = 0; st[4] = 0; st[6] = 0; st[7] = 0;
+            if (p.exp_out) *p.exp_out = s_out + (p.exp_a ? *p.exp_a : 0) + (p.exp_b ? *p.exp_b : 0);
+            if (p.shift_out) *p.shift_out = s_out;
+        }
+    }
+}
+
 template <int BN, bool TWO, int MODE>
 __global__ void __launch_bounds__(REQUANT_THREADS, 1)
 umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
@@ -1244,12 +1294,12 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 
     if (warp == 0) {
         if constexpr (shares_rows(MODE)) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
-        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, TWO, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, cta_first, cta_step, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if (rank == 0) {
             if constexpr (shares_rows(MODE)) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, 0, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, nullptr, tmem_base, p, abort_flag);
-            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO, false>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, abort_flag);
+            else mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, TWO, false>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, cta_first, cta_step, abort_flag);
         }
         __syncwarp();
     } else {
@@ -1304,38 +1354,10 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             }
         }
         const unsigned local_max = __reduce_max_sync(0xFFFFFFFFu, fold_minmax(vmax, vmin));
-        int32_t* st = p.state;
         if (lane == 0) warp_max[warp - 2] = local_max;
         if (threadIdx.x == 64) PARK_STAMP(5);
-
-        // ---- grid barrier: every CTA has contributed its maximum (one atomic each: atomics on one address
-        //      serialise at the L2; the waiters poll with plain acquire loads for the same reason)
-        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
-        if (threadIdx.x == 64) {
-            unsigned cta_max = 0;
-#pragma unroll
-            for (int i = 0; i < EPI_WARPS; ++i) cta_max = max(cta_max, warp_max[i]);
-            // The maximum and the arrival count sit side by side (st[6], st[7]): two fire-and-forget reductions on the
-            // way in (the count's release orders the maximum before it), ONE 64-bit acquire load per poll that returns
-            // both -- a fence + atomicAdd + atomicMax read-back would add three round trips to the L2.
-            if (cta_max != 0) red_relaxed_max(reinterpret_cast<unsigned*>(&st[6]), cta_max);
-            red_release_add(&st[7], 1);
-            const unsigned long long t0 = global_timer_ns();
-            bool arrived = false;
-            unsigned m = 0;
-            for (unsigned spin = 0;; ++spin) {
-                const unsigned long long both = ld_acquire_gpu_u64(&st[6]);
-                if (static_cast<int>(both >> 32) >= static_cast<int>(gridDim.x)) { arrived = true; m = static_cast<unsigned>(both); break; }
-                if ((spin & 63) == 63) {
-                    if (*abort_flag || global_timer_ns() - t0 > GRID_BARRIER_LIMIT_NS) break;
-                }
-            }
-            bool zero_out;
-            *shift_slot = arrived ? shift_for(m, p.kind, p.target_bits, &zero_out) : -1;
-            if (!arrived) { *abort_flag = 1; report_abort(p.status, 5, 2); }
-        }
-        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
-        const int shift = *shift_slot;
+        int ticket = -1;
+        const int shift = parked_grid_shift(p, warp_max, shift_slot, abort_flag, &ticket);
         if (threadIdx.x == 64) PARK_STAMP(6);
 
         // ---- pass 2: narrow the parked accumulators with the true shift
@@ -1375,17 +1397,7 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             }
         }
         if (threadIdx.x == 64) PARK_STAMP(7);
-        // ---- the CTA that leaves last publishes the shift and clears the words for the next call
-        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
-        if (threadIdx.x == 64) {
-            if (atomicAdd(&st[4], 1) == static_cast<int>(gridDim.x) - 1) {
-                __threadfence();
-                const int s_out = shift < 0 ? 0 : shift;
-                st[0] = s_out; st[2] = 0; st[1] = 0; st[5] = 0; st[4] = 0; st[6] = 0; st[7] = 0;
-                if (p.exp_out) *p.exp_out = s_out + (p.exp_a ? *p.exp_a : 0) + (p.exp_b ? *p.exp_b : 0);
-                if (p.shift_out) *p.shift_out = s_out;
-            }
-        }
+        parked_leave(p, shift, ticket);
     }
 
     tc_fence_before();
@@ -1397,6 +1409,241 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         tc_fence_after();
         __syncwarp();
         if (TWO) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Few output tiles: a cluster of CS thread blocks shares one tile's REDUCTION.
+// A convolution of 16 tiles (512 -> 512 at 4x4, 32 images) kept 16 of the 148 SMs busy with 36 reduction blocks each, a
+// single image one to four of them.  Here CTA r of a cluster contracts its share of the reduction blocks into its own tensor
+// memory, the partial sums meet in distributed shared memory, and CTA r owns rows [r 128/CS, (r + 1) 128/CS) of the tile from
+// there on: it adds the CS partial sums (int32, exact in any order), takes the tensor-wide maximum over the same grid barrier
+// as the parked kernel and narrows its rows, so the epilogue is shared out as well.
+//   exchange  every warp writes its 32 x 32 partial sums into the CTA's (by then idle) operand ring, 128-byte rows with their
+//             16-byte chunks exchanged by the row number (both passes free of bank conflicts), and sends them to the rows'
+//             owners as bulk copies of 2 or 4 KB into their receive slots, counted on their mbarriers, without waiting for the
+//             other warps: (CS - 1) / CS x 64 KB per CTA and direction.
+//   cluster   both cluster-wide barriers (peers exist; peers are done) are arrived at early and waited for late.
+//   rows      a warp works on whole rows from here (lane = four columns): row coordinates are uniform, stores are 128
+//             contiguous bytes, a lane's four outputs are one Philox block.
+// state and grid barrier: as umma_parked_kernel.
+// ------------------------------------------------------------------------------------------------
+template <int CS>
+struct SplitCfg {
+    static constexpr int BN = 128;
+    static constexpr int RPC = 128 / CS;                       // rows of the tile a CTA owns
+    static constexpr int SLOT_BYTES = RPC * BN * 4;            // an owner's rows: four panels of 32 columns
+    static constexpr int RECV_BYTES = (CS - 1) * SLOT_BYTES;
+    static constexpr int STAGE_BYTES = PANEL_BYTES + BN * ROW_BYTES;
+    static constexpr int STAGES = 5;
+    static constexpr int POOL_BYTES = RPC * BN;                // the CTA's int8 rows, for the pooling windows
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + RECV_BYTES + POOL_BYTES + 1024 /*alignment slack*/ + 512 /*barriers*/;
+    static_assert(CS * SLOT_BYTES <= STAGES * STAGE_BYTES, "the partial sums are staged in the ring");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a CTA");
+};
+
+// Four accumulators, any rounding and shift, random words from any element on: a call of its own, so that the rare forms are
+// not fetched on the way to the common ones.
+__device__ __noinline__ uint32_t narrow4_general(uint32_t a, uint32_t b, uint32_t c, uint32_t d, int shift, int mode,
+                                                 unsigned long long seed, unsigned rng_stream, unsigned long long e) {
+    const uint32_t v[4] = {a, b, c, d};
+    uint32_t w = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t rnd = mode == ROUND_STOCHASTIC && shift > 0 ? random_word(seed, rng_stream, e + j) : 0u;
+        w |= static_cast<uint32_t>(static_cast<uint8_t>(narrow(static_cast<int>(v[j]), shift, mode, rnd))) << (8 * j);
+    }
+    return w;
+}
+
+template <int CS>
+__global__ void __launch_bounds__(REQUANT_THREADS, 1)
+umma_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+    using Cfg = SplitCfg<CS>;
+    constexpr int STAGES = Cfg::STAGES, RPC = Cfg::RPC, BN = Cfg::BN;
+    constexpr int ROWS = RPC / EPI_WARPS;  // rows of a warp: 4, 2 or 1
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* recv = smem + STAGES * Cfg::STAGE_BYTES;
+    uint32_t* pool_rows = reinterpret_cast<uint32_t*>(recv + Cfg::RECV_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(recv + Cfg::RECV_BYTES + Cfg::POOL_BYTES);
+    uint64_t* full_bar = bars;
+    uint64_t* empty_bar = bars + STAGES;
+    uint64_t* tfull_bar = bars + 2 * STAGES;
+    uint64_t* recv_bar = bars + 2 * STAGES + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* shift_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);
+    volatile unsigned* warp_max = reinterpret_cast<volatile unsigned*>(tmem_slot + 4);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int rank = static_cast<int>(__shfl_sync(0xFFFFFFFFu, cluster_ctarank(), 0));
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; ++i) { mbar_init(smem_u32(&full_bar[i]), 1); mbar_init(smem_u32(&empty_bar[i]), 1); }
+        mbar_init(smem_u32(tfull_bar), 1);
+        mbar_init(smem_u32(recv_bar), 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+        mbar_arrive_expect_tx(smem_u32(recv_bar), Cfg::RECV_BYTES);  // its one arrival; the peers' copies bring the bytes
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+    }
+    if (warp == 1) { tmem_alloc(smem_u32(tmem_slot), BN); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    cluster_arrive();  // this CTA's barriers exist: peers may send (each warp waits for the others' before it sends)
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // the roles see a split reduction: one work item per CTA, numbered split-major
+    const int mn_tiles = p.m_tiles * p.n_tiles;
+    const int tile = static_cast<int>(blockIdx.x) / CS;
+    const int cta_first = rank * mn_tiles + tile, cta_step = CS * mn_tiles;
+
+    if (warp == 0) {
+        producer_role<BN, STAGES, Cfg::STAGE_BYTES, false, false>(smem, full_bar, empty_bar, &tmA, &tmB, p, cta_first, cta_step, abort_flag);
+        __syncwarp();
+        cluster_wait();
+        cluster_arrive();
+    } else if (warp == 1) {
+        mma_role<BN, STAGES, Cfg::STAGE_BYTES, 0, false, false>(smem, full_bar, empty_bar, tfull_bar, nullptr, tmem_base, p, cta_first, cta_step, abort_flag);
+        __syncwarp();
+        cluster_wait();
+        cluster_arrive();
+    } else {
+        const int ew = warp - 2, grp = ew >> 2, q = warp & 3;
+        int m_t, n_t;
+        tile_coords(p, tile, &m_t, &n_t);
+        const int col0 = n_t * BN + 4 * lane;  // this lane's four columns (N is a multiple of 16)
+        const bool in_cols = col0 < p.N;
+        // where this warp's rows lie in the output (and in the pooled output), and their ReLU masks, while the main loop runs
+        int row[ROWS], prow[ROWS];
+        uint32_t mk[ROWS];
+        {
+            const int q1 = fdiv(m_t, p.fd_tw), tw = m_t - q1 * p.tiles_w, tn = fdiv(q1, p.fd_th), th = q1 - tn * p.tiles_h;
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                const int t = rank * RPC + ew * ROWS + i;  // row of the tile
+                const int w = tw * p.BW + t % p.BW, h = th * p.BH + (t / p.BW) % p.BH, n = tn * p.BI + t / (p.BW * p.BH);
+                const bool valid = t < p.BW * p.BH * p.BI && w < p.W && h < p.H && n < p.Nimg;
+                row[i] = valid ? (n * p.H + h) * p.W + w : -1;
+                prow[i] = (valid && ((w | h) & 1) == 0) ? (n * (p.H >> 1) + (h >> 1)) * (p.W >> 1) + (w >> 1) : -1;
+                mk[i] = 0;
+                if (p.mask != nullptr && valid && in_cols) mk[i] = __ldg(reinterpret_cast<const uint32_t*>(p.mask + static_cast<long long>(row[i]) * p.N + col0));
+            }
+        }
+        // ---- the partial sums: tensor memory -> staging -> the rows' owners
+        cluster_wait();  // every CTA of the cluster has set up its barriers
+        bool up = mbar_wait(smem_u32(tfull_bar), 0, abort_flag);
+        if (!up) report_abort(p.status, 4, 2);
+        if (__all_sync(0xFFFFFFFFu, up)) {
+            tc_fence_after();
+            const int t = q * 32 + lane, lr = t % RPC;  // row of the tile, row of its owner
+            uint32_t v[32];
+            tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(grp * 32), v);
+            tmem_ld_wait();
+            const uint32_t base = smem_u32(smem) + static_cast<uint32_t>(t / RPC) * Cfg::SLOT_BYTES + static_cast<uint32_t>(grp * RPC + lr) * 128u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                st_shared_v4(base + ((static_cast<uint32_t>(j) ^ (static_cast<uint32_t>(lr) & 7u)) << 4), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            fence_proxy_async();
+            __syncwarp();
+            // this warp's rows belong to two owners (16 rows each) or to one
+            constexpr int PIECE = RPC < 32 ? RPC : 32, OWNERS = 32 / PIECE;
+            if (lane < OWNERS) {
+                const int t0 = q * 32 + lane * PIECE, owner = t0 / RPC;
+                if (owner != rank) {
+                    const uint32_t slot = static_cast<uint32_t>(rank - owner - 1) & static_cast<uint32_t>(CS - 1);
+                    const uint32_t at = static_cast<uint32_t>(grp * RPC + t0 % RPC) * 128u;
+                    bulk_copy_cluster(mapa_u32(smem_u32(recv) + slot * Cfg::SLOT_BYTES + at, owner), smem_u32(smem) + owner * Cfg::SLOT_BYTES + at,
+                                      PIECE * 128, mapa_u32(smem_u32(recv_bar), owner));
+                }
+            }
+            __syncwarp();
+        }
+        named_barrier(EPI_BARRIER, 32 * EPI_WARPS);  // this CTA's own rows lie in the staging area
+        up = mbar_wait(smem_u32(recv_bar), 0, abort_flag);
+        if (!up) report_abort(p.status, 4, 2);
+        __syncwarp();
+        cluster_arrive();  // nothing this warp waits for is still on its way
+        // ---- this CTA's rows: the sum of CS partial sums, and their maximum
+        uint32_t acc[ROWS][4];
+        unsigned local_max = 0;
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const int lr = ew * ROWS + i;
+            const uint32_t at = static_cast<uint32_t>((lane >> 3) * RPC + lr) * 128u + (static_cast<uint32_t>((lane ^ lr) & 7) << 4);
+            int4 s = *reinterpret_cast<const int4*>(smem + rank * Cfg::SLOT_BYTES + at);
+#pragma unroll
+            for (int k = 0; k < CS - 1; ++k) {
+                const int4 o = *reinterpret_cast<const int4*>(recv + k * Cfg::SLOT_BYTES + at);
+                s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w;
+            }
+            acc[i][0] = static_cast<uint32_t>(s.x); acc[i][1] = static_cast<uint32_t>(s.y); acc[i][2] = static_cast<uint32_t>(s.z); acc[i][3] = static_cast<uint32_t>(s.w);
+            if (row[i] >= 0 && in_cols)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    local_max = max(local_max, min(acc[i][j], 0u - acc[i][j]));  // |x|
+        }
+        local_max = __reduce_max_sync(0xFFFFFFFFu, local_max);
+        if (lane == 0) warp_max[ew] = local_max;
+        int ticket = -1;
+        const int shift = parked_grid_shift(p, warp_max, shift_slot, abort_flag, &ticket);
+        // ---- narrow, store, pool
+        if (shift >= 0) {
+            const unsigned long long seed = (p.mode == ROUND_STOCHASTIC && shift > 0) ? *p.seed : 0ull;
+            const bool pooling = p.pool_out != nullptr;  // the same for the whole grid
+            const unsigned long long e0 = p.rng_offset + static_cast<unsigned long long>(col0);
+            uint32_t y[ROWS];
+            if (p.mode == ROUND_NEAREST && shift > 0) {
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i) y[i] = narrow4_nearest<false>(acc[i], shift, 1 << (shift - 1));
+            } else if (p.mode == ROUND_STOCHASTIC && shift > 0 && shift < 24 && (e0 & 3ull) == 0) {
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i) {
+                    uint32_t rnd[4];
+                    random_block(seed, p.rng_stream, (e0 + static_cast<unsigned long long>(static_cast<long long>(row[i]) * p.N)) >> 2, rnd);
+                    y[i] = narrow4_stochastic<false>(acc[i], shift, (1u << shift) - 1u, rnd);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i)
+                    y[i] = narrow4_general(acc[i][0], acc[i][1], acc[i][2], acc[i][3], shift, p.mode, seed, p.rng_stream,
+                                           e0 + static_cast<unsigned long long>(static_cast<long long>(row[i]) * p.N));
+            }
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                if (p.relu) y[i] = __vmaxs4(y[i], 0u);
+                if (p.mask != nullptr) y[i] &= __vcmpgts4(mk[i], 0);
+                if (row[i] >= 0 && in_cols) *reinterpret_cast<uint32_t*>(p.out8 + static_cast<long long>(row[i]) * p.N + col0) = y[i];
+                if (pooling) pool_rows[(ew * ROWS + i) * 32 + lane] = y[i];
+            }
+            if (pooling) {
+                // the 2x2 window of local row r is rows r, r + 1, r + BW, r + BW + 1: all in this CTA (split_cluster)
+                named_barrier(EPI_BARRIER, 32 * EPI_WARPS);
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i)
+                    if (prow[i] >= 0 && in_cols) {
+                        const uint32_t* at = pool_rows + (ew * ROWS + i) * 32 + lane;
+                        const uint32_t m = __vmaxs4(__vmaxs4(at[0], at[32]), __vmaxs4(at[p.BW * 32], at[(p.BW + 1) * 32]));
+                        *reinterpret_cast<uint32_t*>(p.pool_out + static_cast<long long>(prow[i]) * p.N + col0) = m;
+                    }
+            }
+        }
+        parked_leave(p, shift, ticket);
+    }
+
+    // ---------------------------------------------------------------------- teardown
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) __nanosleep(200000);  // a block that gave up: let copies in flight, its own and its peers', land
+    cluster_wait();  // no CTA leaves while a peer may still send to it
+    if (warp == 1) {
+        tc_fence_after();
+        __syncwarp();
+        tmem_dealloc(tmem_base, BN);
     }
 }
 
@@ -1772,6 +2019,40 @@ static int launch_requant(int bn, bool pair, int mode, bool parked, const CUtens
     if (bn == 64) return launch_requant_inst<64, false, LOAD_TAPS, false>(a, b, p, st);
     return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, false>(a, b, p, st);
 }
+template <int CS>
+static cudaLaunchConfig_t split_config(int tiles, cudaLaunchAttribute* attr, cudaStream_t st) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative; attr[1].val.cooperative = g_cooperative;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(tiles * CS); cfg.blockDim = dim3(REQUANT_THREADS); cfg.dynamicSmemBytes = SplitCfg<CS>::SMEM_BYTES; cfg.stream = st;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    return cfg;
+}
+template <int CS>
+static int launch_split(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
+    cudaError_t e = cudaFuncSetAttribute(umma_split_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<CS>::SMEM_BYTES);
+    if (e != cudaSuccess) return set_cuda_error(e);
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = split_config<CS>(p.m_tiles * p.n_tiles, attr, st);
+    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_split_kernel<CS>, a, b, p));
+}
+// Clusters of CS CTAs (one CTA per SM) that an idle device holds at a time; 0 where it cannot be asked.  They lie within a
+// GPC each, so that it is less than the number of SMs over CS.
+template <int CS>
+static int split_clusters() {
+    static std::atomic<int> known{-1};
+    int n = known.load(std::memory_order_relaxed);
+    if (n < 0) {
+        cudaLaunchAttribute attr[2];
+        cudaLaunchConfig_t cfg = split_config<CS>(1, attr, nullptr);
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(umma_split_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<CS>::SMEM_BYTES) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, umma_split_kernel<CS>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
+        known.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
 // all accumulators of the problem fit in the tensor memory of one wave of CTAs (units: 128-row tiles,
 // or 256-row pair tiles on sm/2 pairs)
 static bool fits_parked(int bn, int tiles, bool pair) { return tiles <= (pair ? sm_count() / 2 : sm_count()) * (512 / bn); }
@@ -1855,6 +2136,26 @@ static ConvPlan pool_plan(int Nimg, int H, int W, int outc, bool k3) {
     return pool_box_ok(H, W, c.BW, c.BH) ? c : conv_plan(Nimg, H, W, outc, false, 0, 2);
 }
 
+// CTAs that share the reduction of one output tile (umma_split_kernel); 1: none do.  bw: 0, or the width of the tile's pixel
+// box in a call that pools (a CTA's rows are then whole pairs of image rows).
+// Where the line lies: sharing costs about 1.6 us (exchange, cluster) and saves the (1 - 1 / cs) of the main loop that the
+// others take over, 0.21 us per 128-byte reduction block with a box per tap and 0.14 where the rows of three taps come in one
+// (us, before / after, batch x map, channels):
+//   box per tap   32x4x4 512->512 15.3 / 10.6, 12x8x8 256->256 11.8 / 10.1, 32x8x8 256->512 11.7 / 11.0; 64x8x8 128->128 9.9 / 9.9
+//   shared rows   1x8x8 512->512 12.7 / 10.1, 1x16x16 256->256 10.3 / 9.5; 16x16x16 256->256 10.6 / 11.4, 4x32x32 128->128 9.3 / 9.9,
+//                 37x15x13 48->80 10.9 / 12.8
+// and with random words, whose drawing is shared out too, it pays from half of that on: 64x8x8 128->128 11.9 / 10.6, 4x32x32
+// 128->128 11.2 / 10.5; 8x32x32 64->64 10.4 / 12.1.
+static int split_cluster(int tiles, int taps, int red, bool halo, bool stochastic, int bw) {
+    if (tiles > sm_count() / 2 || (g_two_cta & 2)) return 1;
+    const int num_kb = taps * ((red + 127) / 128);
+    const auto fits = [&](int cs, int clusters) { return tiles <= clusters && num_kb >= 2 * cs && (bw == 0 || 128 / cs % (2 * bw) == 0); };
+    const int cs = fits(8, split_clusters<8>()) ? 8 : fits(4, split_clusters<4>()) ? 4 : fits(2, split_clusters<2>()) ? 2 : 1;
+    // reduction steps of 32 channels that the other CTAs take over, in quarters of a block
+    const int saved = taps * ((red + 31) / 32) * (cs - 1) / cs;
+    return saved >= (stochastic ? 24 : halo ? 46 : 30) ? cs : 1;
+}
+
 int umma_gemm_splits(int M, int N, int K) {
     const int bn = (N > 128) ? 256 : 128;
     const int tiles = ((M + 127) / 128) * ((N + bn - 1) / bn);
@@ -1917,8 +2218,15 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     GemmParams p{};
     const bool parked = fused && fused->parked;
     const bool k3 = R == 3 && S == 3 && pad == 1;
-    const ConvPlan plan = fused && fused->pool_out != nullptr ? pool_plan(Nimg, H, W, outc, k3)
-                                                              : conv_plan(Nimg, H, W, outc, k3, flip, !fused ? 0 : parked ? 2 : 1);
+    ConvPlan plan = fused && fused->pool_out != nullptr ? pool_plan(Nimg, H, W, outc, k3)
+                                                        : conv_plan(Nimg, H, W, outc, k3, flip, !fused ? 0 : parked ? 2 : 1);
+    int split = 1;
+    if (parked) {
+        const ConvPlan taps = conv_plan(Nimg, H, W, outc, false, flip, 2);
+        split = split_cluster(taps.m_tiles * ((outc + 127) / 128), R * S, red, plan.halo, fused->mode == NITI_ROUND_STOCHASTIC,
+                              fused->pool_out != nullptr ? taps.BW : 0);
+        if (split > 1) { plan = taps; plan.bn = 128; }
+    }
     const int bn = plan.bn;
     const bool pair = plan.pair;
     p.BW = plan.BW; p.BH = plan.BH; p.BI = plan.BI;
@@ -1937,7 +2245,7 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         uint32_t bc[4] = {32, (uint32_t)p.BW, (uint32_t)p.BH, (uint32_t)p.BI};
         if (!fused) if (int e = encode_map(&mc, out, true, 4, dc, sc, bc)) return e;
     }
-    p.conv = 1; p.flip = flip; p.splits = 1;
+    p.conv = 1; p.flip = flip; p.splits = split;
     p.H = H; p.W = W; p.S = S; p.pad = pad; p.Nimg = Nimg; p.tapstride = C;
     p.tiles_w = plan.tiles_w; p.tiles_h = plan.tiles_h;
     p.cblocks = (red + 127) / 128; p.red = red;
@@ -1955,6 +2263,9 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         p.pool_out = fused->pool_out;
     }
     if (parked && !fits_parked(bn, p.m_tiles * p.n_tiles, pair)) return NITI_ERR_UNSUPPORTED;
+    if (split == 8) return launch_split<8>(ma, mb, p, st);
+    if (split == 4) return launch_split<4>(ma, mb, p, st);
+    if (split == 2) return launch_split<2>(ma, mb, p, st);
     const int mode = !plan.halo ? LOAD_TAPS : p.cblocks == 1 && p.n_tiles == 1 ? LOAD_HALO_RESIDENT : LOAD_HALO;
     if (fused) return launch_requant(bn, pair, mode, parked, ma, mb, p, st);
     return launch_gemm(bn, pair, ma, mb, mc, p, st);

@@ -73,6 +73,38 @@ def test_pooling_in_the_same_launch_on_maps_of_any_even_height(N, H, W, C, K, mo
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("N,H,W,C,K", [
+    (1, 8, 8, 512, 512), (32, 4, 4, 272, 512),    # eight and four thread blocks to a tile; tiles of 64 and of 128 pixels
+    (1, 16, 16, 384, 512),                        # four (16-pixel rows: pooling leaves a block whole pairs of image rows)
+    (20, 8, 8, 144, 272), (70, 10, 10, 240, 112), # four; two, in tiles of 120 pixels
+    (1, 3, 5, 288, 208), (3, 2, 2, 144, 512), (2, 2, 130, 192, 176)])
+@pytest.mark.parametrize("mode,offset", [(0, 0), (1, 0), (1, 5), (2, 0)])
+def test_tiles_that_share_a_reduction(N, H, W, C, K, mode, offset):
+    """So few tiles that a cluster of thread blocks works on each: rows, columns and reduction blocks that do not divide evenly,
+    masks, pooling, every rounding, and random words that start inside a block of four."""
+    rng = np.random.default_rng(N + H + 3 * W + C + K)
+    x, w, err = np.maximum(rnd8(rng, (N, H, W, C)), 0), rnd8(rng, (K, 3, 3, C)), rnd8(rng, (N, H, W, K))
+    seed, ea = ops.seed_tensor(9, DEV), torch.full((), 3, dtype=torch.int32, device=DEV)
+    acc, back = O.conv_fprop(x, w), O.conv_dgrad(err, w)
+    y, _, shift = O.act_calc(acc, 0, mode, philox.random_u32_tensor(9, 3, acc.shape, offset))
+    e, shift_e = O.err_calc(back, mode, philox.random_u32_tensor(9, 4, back.shape, offset))
+    fwd, bwd = ops.new_requant_state(DEV), ops.new_requant_state(DEV)
+    for relu in (False, True):
+        want = O.relu_fwd(y) if relu else y
+        got, exp, _ = ops.conv_fprop_fused(cu(x), cu(w), fwd, 1, mode, seed, 3, offset, relu, ea, ea)
+        same(got, want)
+        assert int(exp) == shift + 6
+        if ops.conv_fprop_pool_fused_supported(N, H, W, C, K, 3, 3, 1):
+            got, pooled, exp, _ = ops.conv_fprop_pool_fused(cu(x), cu(w), fwd, 1, mode, seed, 3, offset, relu, ea, ea)
+            same(got, want)
+            same(pooled, O.maxpool_fwd(want))
+    for mask in (None, cu(x)):
+        got, exp, _ = ops.conv_dgrad_fused(cu(err), cu(w), bwd, 1, mode, seed, 4, offset, ea, ea, relu_mask=mask)
+        same(got, e if mask is None else np.where(x > 0, e, 0).astype(np.int8))
+        assert int(exp) == shift_e + 6
+    ops.check_status(DEV)
+
+
 def test_more_than_2_to_the_31_output_rows():
     """16 channels in and out, 34 GB each: images at both ends and in the middle come out as they do alone, the others stay zero."""
     N, C = (1 << 21) + 5, 16
