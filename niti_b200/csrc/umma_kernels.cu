@@ -21,6 +21,9 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <functional>
+#include <queue>
+#include <vector>
 
 #include "../../include/niti_b200.h"
 #include "internal.h"
@@ -2380,6 +2383,45 @@ int umma_conv_wgrad_batch_inner(const int8_t* x_t, const int8_t* err_t, int32_t*
 
 int umma_wgrad_multi_max() { return WG_MULTI_MAX; }
 
+// Splits for layers whose items alone are more than the SMs: of several ways to cut them, the one whose thread blocks, longest
+// first, are done earliest on `sms` SMs.  A thread block costs its chunks and about twelve chunks' time for its start and its
+// flush.  Left uncut, the four last layers of VGG-13 at batch 1024 (48 + 48 items of 32 chunks, 48 + 24 of 128) were 168 blocks:
+// 20 of 128 chunks started when the first ones were through.
+static void wgrad_deal(WgradMultiParams* mp, const int* items, int count, int sms) {
+    constexpr int OVERHEAD = 12, MAX_BLOCKS = 512;
+    constexpr int CUTS[] = {1, 2, 3, 4, 6, 8};
+    long long best = -1;
+    int splits[WG_MULTI_MAX], chosen[WG_MULTI_MAX];
+    for (int ref = 0; ref < count; ++ref)
+        for (const int cut : CUTS) {
+            const int len = (mp->layer[ref].chunks + cut - 1) / cut;  // chunks of a thread block
+            int order[WG_MULTI_MAX], total = 0;
+            for (int l = 0; l < count; ++l) {
+                splits[l] = (mp->layer[l].chunks + len - 1) / len;
+                total += splits[l] * items[l];
+            }
+            if (total > MAX_BLOCKS && best >= 0) continue;
+            const auto cost = [&](int l) { return (mp->layer[l].chunks + splits[l] - 1) / splits[l] + OVERHEAD; };
+            for (int l = 0; l < count; ++l) {
+                int at = l;
+                for (; at > 0 && cost(order[at - 1]) < cost(l); --at) order[at] = order[at - 1];
+                order[at] = l;
+            }
+            std::priority_queue<long long, std::vector<long long>, std::greater<long long>> busy;  // when each SM is free
+            for (int i = 0; i < sms; ++i) busy.push(0);
+            long long end = 0;
+            for (int o = 0; o < count; ++o)
+                for (int b = 0; b < splits[order[o]] * items[order[o]]; ++b) {
+                    const long long done = busy.top() + cost(order[o]);
+                    busy.pop();
+                    busy.push(done);
+                    if (done > end) end = done;
+                }
+            if (best < 0 || end < best) { best = end; for (int l = 0; l < count; ++l) chosen[l] = splits[l]; }
+        }
+    for (int l = 0; l < count; ++l) mp->layer[l].splits = chosen[l];
+}
+
 // Up to WG_MULTI_MAX layers' gradients added into their (zeroed or accumulating) int32 buffers by one launch.
 int umma_conv_wgrad_multi(const WgradJob* jobs, int count, int32_t* status, cudaStream_t st) {
     if (count < 1 || count > WG_MULTI_MAX) return NITI_ERR_BAD_ARG;
@@ -2405,17 +2447,28 @@ int umma_conv_wgrad_multi(const WgradJob* jobs, int count, int32_t* status, cuda
             mp.layer[l].splits = sp;
             ctas += sp * items[l];
         }
+        if (ctas <= sms) break;
         bool whole = true;  // nothing left to merge: every layer is down to one split
         for (int l = 0; l < count; ++l) whole = whole && mp.layer[l].splits == 1;
-        if (ctas <= sms || whole) break;
+        if (whole) { wgrad_deal(&mp, items, count, sms); break; }
     }
+    // the longest thread blocks first: where there are more than SMs, the short ones fill up behind them
+    int order[WG_MULTI_MAX];
+    for (int l = 0; l < count; ++l) {
+        int at = l;
+        const auto len = [&](int i) { return (mp.layer[i].chunks + mp.layer[i].splits - 1) / mp.layer[i].splits; };
+        for (; at > 0 && len(order[at - 1]) < len(l); --at) order[at] = order[at - 1];
+        order[at] = l;
+    }
+    const WgradMultiParams planned = mp;
     int grid = 0;
     for (int l = 0; l < count; ++l) {
-        const WgradJob& j = jobs[l];
+        const WgradJob& j = jobs[order[l]];
+        mp.layer[l] = planned.layer[order[l]];
         if (int e = wgrad_setup(j.x, j.err, j.g32, 1, j.N, j.H, j.W, j.C, j.K, j.R, j.S, j.pad, status, &mp.layer[l], &maps.err[l],
                                 &maps.x[l], &maps.g[l])) return e;
         mp.first_cta[l] = grid;
-        grid += mp.layer[l].splits * items[l];
+        grid += mp.layer[l].splits * items[order[l]];
     }
     mp.first_cta[count] = grid;
     mp.count = count;
