@@ -488,6 +488,12 @@ NITI_API int niti_fc_head_train_i8(const niti_fc_head_args* args, void* stream);
 NITI_API int niti_quantize_input_f32(const float* x, int8_t* x8, int32_t* exp_out, uint32_t* scratch,
                             int N, int C, int H, int W, void* stream);
 
+/* What a training loop reads back after a step, written to PINNED host memory by one kernel: n int8 logits, their exponent and
+ * the status word (int32[4]).  The three host buffers must be page-locked and mapped (cudaHostAlloc; any pinned allocation under
+ * unified addressing); they are valid once the stream has passed the launch.  The reference copies its outputs one by one. */
+NITI_API int niti_publish_step(const int8_t* out, int64_t n, const int32_t* exp, const int32_t* status, int8_t* host_out,
+                               int32_t* host_exp, int32_t* host_status, void* stream);
+
 /* Self-test of the bounded waits: launches one thread block that waits at a grid barrier expecting two blocks.  The
  * wait gives up after its 0.5 s limit, writes {8, block index, expected arrivals} to status[0..2] (int32[4], zeroed by
  * the caller) and the kernel returns normally: the context stays usable.  scratch: one int32 word. */

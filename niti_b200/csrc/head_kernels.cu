@@ -467,8 +467,7 @@ extern "C" int niti_fc_head_train_i8(const niti_fc_head_args* a, void* stream) {
     const int useful = p.B > p.F / 16 ? p.B : p.F / 16;
     if (grid > useful) grid = useful;
 
-    e = cudaMemsetAsync(p.state, 0, 4 * sizeof(int32_t), st);
-    if (e != cudaSuccess) return set_cuda_error(e);
+    if (int rc = clear_words(p.state, 4, st)) return rc;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid); cfg.blockDim = dim3(HEAD_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];

@@ -66,6 +66,7 @@ int simt_conv_wgrad(const int8_t* x, const int8_t* err, int32_t* g32, unsigned* 
                     int K, int R, int S, int pad, cudaStream_t st);
 int simt_gemm(const int8_t* A, const int8_t* B, int32_t* C32, unsigned* maxabs, int M, int N, int K, int trans_a,
               int trans_b, cudaStream_t st);
+int clear_words(void* p, int n, cudaStream_t st);  // n (few) 32-bit words to zero
 int reduce_partials(const int32_t* partial, int splits, long long n, int32_t* out, unsigned* maxabs, cudaStream_t st);
 int reduce_rows32(const int32_t* partial, int splits, int rows, int cols_out, int32_t* out, unsigned* maxabs, cudaStream_t st);
 // xcol[pixels][32] and wp[K][32] in the order the MMA reads 32-byte rows in (rows32 of umma_gemm).

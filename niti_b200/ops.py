@@ -396,7 +396,7 @@ def fc_head_train(x, exp_x, w, exp_w, target, seed, layer_stream, *, dropout=Tru
                    exps[1:2].data_ptr(), _p(g32), _p(gm), _p(sc), nbytes, B, F, J, int(dropout), bits, act_mode, err_mode,
                    grad_mode, mu, int(update), _p(seed), layer_stream, dropout_stream, loss_stream, sample_offset,
                    _p(status_word(dev)))
-    _call("niti_fc_head_train_i8", 1, 6 * B * F * J, 2 * x.numel() + 6 * w.numel(), lib.niti_fc_head_train_i8,
+    _call("niti_fc_head_train_i8", 2, 6 * B * F * J, 2 * x.numel() + 6 * w.numel(), lib.niti_fc_head_train_i8,
           ctypes.byref(a), _st())
     return out8, exps[0], err8, e8, exps[1], g32, gm
 
@@ -422,7 +422,7 @@ def update_multi(ws, g32s, streams, mu, mode=ROUND_PSEUDO_STOCHASTIC, seed=None,
     nbytes = lib.niti_update_multi_scratch_bytes()
     sc = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     total = sum(w.numel() for w in ws)
-    _call("niti_update_multi_i8", (n + 15) // 16, 0, 10 * total, lib.niti_update_multi_i8, items, n, mu, mode, int(clear), _p(seed),
+    _call("niti_update_multi_i8", 2 * ((n + 15) // 16), 0, 10 * total, lib.niti_update_multi_i8, items, n, mu, mode, int(clear), _p(seed),
           _p(sc), nbytes, _p(status_word(dev)), _st())
     return mx
 
@@ -456,13 +456,23 @@ def peer_copy(dst_ptr, src_ptr, nbytes):
     check(lib.niti_peer_copy(ctypes.c_void_p(dst_ptr), ctypes.c_void_p(src_ptr), nbytes, _st()), "niti_peer_copy")
 
 
+def publish_step(out, exp, status, host_out, host_exp, host_status):
+    """A step's int8 logits, exponent and status word into pinned host tensors by one kernel (valid once the current stream has
+    passed it)."""
+    _need_cuda(out, exp, status)
+    assert out.dtype == torch.int8 and exp.dtype == torch.int32 and out.shape == host_out.shape and exp.numel() == 1
+    assert host_out.is_contiguous() and host_out.dtype == torch.int8
+    _call("niti_publish_step", 1, 0, out.numel() + 20, lib.niti_publish_step, _p(out), out.numel(), _p(exp), _p(status), _p(host_out),
+          _p(host_exp), _p(host_status), _st())
+
+
 def quantize_input(x, reduce_max=None):
     """float32 NCHW -> (int8 NHWC, exponent).  ``reduce_max(t)``: optional hook that replaces the int32[1] word
     holding the bit pattern of max|x| by its maximum over a process group, in place."""
     if reduce_max is None:
         def work(r):
             return 0, 9 * x.numel()
-        return _run("niti_quantize_input_f32", 2, work, native.quantize_input, x)
+        return _run("niti_quantize_input_f32", 3, work, native.quantize_input, x)
     _need_cuda(x)
     assert x.dtype == torch.float32
     N, C, H, W = x.shape

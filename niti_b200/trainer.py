@@ -350,9 +350,13 @@ class Trainer:
         self.run_device_step()
         k = self._res_slot = 1 - self._res_slot
         self.out_host, self.exp_host = self._out_hosts[k], self._exp_hosts[k]
-        self.out_host.copy_(self.model.out, non_blocking=True)
-        self.exp_host.copy_(self.model.out_exp, non_blocking=True)
-        self._status_hosts[k].copy_(ops.status_word(self.device), non_blocking=True)
+        out, exp = self.model.out, self.model.out_exp
+        if out.dtype is torch.int8 and out.is_contiguous() and out.shape == self.out_host.shape and exp.dtype is torch.int32:
+            ops.publish_step(out, exp, ops.status_word(self.device), self.out_host, self.exp_host, self._status_hosts[k])
+        else:
+            self.out_host.copy_(out, non_blocking=True)
+            self.exp_host.copy_(exp, non_blocking=True)
+            self._status_hosts[k].copy_(ops.status_word(self.device), non_blocking=True)
         self._done[k].record(main)
         return StepResult(self.out_host, self.exp_host, self._done[k], self._status_hosts[k], self)
 
