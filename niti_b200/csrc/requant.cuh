@@ -109,14 +109,15 @@ __device__ __forceinline__ uint32_t narrow4_nearest(const uint32_t* v, int shift
 // when lo > r, i.e. when lo + (mask - r) carries into bit `shift`: y = (|x| + (~r & mask)) >> shift.  For x < 0 the
 // negated quotient is the arithmetic shift (x + (r & mask)) >> shift (-floor(a / d) = floor((d - 1 - a) / d)), so both
 // signs are one add and one shift behind a three-input logic operation.  For shifts below 24 and x <= 2^31 - 2^shift, as
-// for the nearest form: negative sums only move towards zero, positive ones must not pass 2^31.
+// for the nearest form: negative sums only move towards zero, positive ones must not pass 2^31.  Under a ReLU the sign is left
+// out: a negative value with any of these bits added stays below 2^shift and comes out as zero or less either way.
 template <bool RELU>
 __device__ __forceinline__ uint32_t narrow4_stochastic(const uint32_t* v, int shift, uint32_t mask, const uint32_t (&rnd)[4]) {
     int y[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int x = static_cast<int>(v[j]);
-        y[j] = (x + static_cast<int>((rnd[j] ^ ~static_cast<uint32_t>(x >> 31)) & mask)) >> shift;
+        y[j] = (x + static_cast<int>((RELU ? ~rnd[j] : rnd[j] ^ ~static_cast<uint32_t>(x >> 31)) & mask)) >> shift;
     }
     if (RELU) return __vminu4(pack2_sat_u8(y[1], y[0], pack2_sat_u8(y[3], y[2], 0u)), 0x7F7F7F7Fu);
     return __vmaxs4(pack2_sat_s8(y[1], y[0], pack2_sat_s8(y[3], y[2], 0u)), 0x81818181u);

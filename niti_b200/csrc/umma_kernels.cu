@@ -661,14 +661,18 @@ __device__ __forceinline__ void narrow32(const uint32_t (&v)[32], uint32_t (&pac
 #pragma unroll
             for (int i = 0; i < 32; i += 4) packed[i >> 2] = narrow4_nearest<false>(&v[i], shift, half);
         }
-    } else if (mode == ROUND_STOCHASTIC && shift > 0 && shift < 24 && (e0 & 3ull) == 0) {
+    } else if (mode == ROUND_STOCHASTIC && shift > 0 && shift < 24 && (e0 & 3ull) == 0 && static_cast<uint32_t>(e0 >> 2) <= 0xFFFFFFF8u) {
         // The random words of four neighbouring outputs come from one Philox block: ten rounds of two wide multiplications,
         // which with the short narrowing is what a stochastic epilogue costs; the general form works value by value.
         const uint32_t mask = (1u << shift) - 1u;
+        // The eight blocks' counters differ in their low words: with the high word a value of its own, what the first rounds make
+        // of it, of the stream and of the keys is worked out once (128->128 at 32x32, 128 images: 31.3 -> 30.6 us; 256->256, 256
+        // 16x16 maps, error-backward: 45.3 -> 42.7).
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
             uint32_t rnd[4];
-            random_block(seed, rng_stream, (e0 + i) >> 2, rnd);
+            philox4x32_10(static_cast<uint32_t>(e0 >> 2) + (i >> 2), static_cast<uint32_t>(e0 >> 34), rng_stream, 0u, static_cast<uint32_t>(seed),
+                          static_cast<uint32_t>(seed >> 32), rnd);
             packed[i >> 2] = relu ? narrow4_stochastic<true>(&v[i], shift, mask, rnd) : narrow4_stochastic<false>(&v[i], shift, mask, rnd);
         }
     } else if (shift == 0) {
