@@ -96,6 +96,7 @@ struct GemmParams {
     int m_tiles, n_tiles;
     int a_mn, b_mn;        // operand majors (0 = K-major, 1 = MN-major)
     int a_bytes;           // bytes one A stage receives from TMA
+    int b_bytes;           // bytes of one tap's B tile (of this CTA's half of it): fewer than the tile where the box is lower
     // Operands of 32-byte rows that lie in memory as the MMA reads them (32-byte swizzle: see patch_half), loaded with
     // one untiled bulk copy instead of a box of 128 rows.  1: A [M][32] and B [N][32], one reduction block;
     // 2: B [reduction][32] as 32 MN-major columns.
@@ -289,7 +290,7 @@ __device__ __forceinline__ void producer_role(uint8_t* smem, uint64_t* full_bar,
     const int conv = keep_reg(p.conv), flip = keep_reg(p.flip), pad = keep_reg(p.pad), S = keep_reg(p.S), cblocks = keep_reg(p.cblocks);
     const int tapstride = keep_reg(p.tapstride), b_mn = keep_reg(p.b_mn), a_mn = keep_reg(p.a_mn);
     const int rows32 = ROWS32 ? keep_reg(p.rows32) : 0;
-    const uint32_t tx_full = static_cast<uint32_t>(keep_reg(TWO ? 2 * (p.a_bytes + BNH * ROW_BYTES) : p.a_bytes + BN * ROW_BYTES));
+    const uint32_t tx_full = static_cast<uint32_t>(keep_reg((TWO ? 2 : 1) * (p.a_bytes + p.b_bytes)));
     int s = 0; uint32_t ph = 0;
     uint32_t sa = smem0, fb_cur = full0, eb_cur = empty0;  // running stage pointers, wrapping with the ring
     DBG_DECL;
@@ -500,7 +501,7 @@ __device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
     const uint32_t smem0 = smem_u32(smem), full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
     const int flip = keep_reg(p.flip), cblocks = keep_reg(p.cblocks), tapstride = keep_reg(p.tapstride), b_mn = keep_reg(p.b_mn);
-    const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg(p.a_bytes + (RESIDENT ? 0 : 3 * BN * ROW_BYTES)));
+    const uint32_t tx_bytes = static_cast<uint32_t>(keep_reg(p.a_bytes + (RESIDENT ? 0 : 3 * p.b_bytes)));
     const uint32_t res0 = smem0 + STAGES * STAGE_BYTES;  // resident weights: [column][filter row]
     bool weights_due = RESIDENT;
     const int nst = ring_stages(p, STAGES);
@@ -519,7 +520,7 @@ __device__ __forceinline__ void producer_halo_role(uint8_t* smem, uint64_t* full
                     if (!RESIDENT || weights_due) {
                         const uint32_t dst = RESIDENT ? res0 + sx * 3 * BN * ROW_BYTES : sa + HALO_A_BYTES;
                         const uint32_t bar = RESIDENT ? weights0 + 8u * sx : fb;
-                        if (RESIDENT) mbar_arrive_expect_tx(bar, 3 * BN * ROW_BYTES);
+                        if (RESIDENT) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(3 * p.b_bytes));
 #pragma unroll
                         for (int r = 0; r < 3; ++r) {
                             const int x = (r * 3 + sx) * tapstride;
@@ -575,7 +576,7 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
                     if (accumulate == 0) b_cur = b_base;
                     if (it == 0) mbar_wait_quiet(weights0 + 8u * sx, 0, abort_addr);
                 }
-                if (left >= 128) {
+                if (left > 96) {
 #pragma unroll
                     for (int r = 0; r < 3; ++r) {
                         umma_seq4(d_tmem, a_cur + r * a_next, b_cur + static_cast<uint64_t>(r * BN * ROW_BYTES >> 4), 2, b_step, idesc, accumulate);
@@ -584,14 +585,12 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
                     if (elect_one()) umma_commit(empty_cur);
                 } else {  // only the MMAs (K = 32 each) that cover real channels; the rest of the rows is TMA zero fill
                     const int nmma = (left + 31) >> 5;
-                    if (elect_one()) {
-                        for (int r = 0; r < 3; ++r)
-                            for (int k = 0; k < nmma; ++k)
-                                umma_i8(d_tmem, a_cur + r * a_next + 2 * k, b_cur + static_cast<uint64_t>(r * BN * ROW_BYTES >> 4) + k * b_step, idesc,
-                                        accumulate | static_cast<uint32_t>(r + k != 0));
-                        umma_commit(empty_cur);
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        umma_seq_upto3(d_tmem, a_cur + r * a_next, b_cur + static_cast<uint64_t>(r * BN * ROW_BYTES >> 4), 2, b_step, idesc, accumulate, nmma);
+                        accumulate = 1;
                     }
-                    accumulate = 1;
+                    if (elect_one()) umma_commit(empty_cur);
                 }
                 a_cur += STAGE_BYTES >> 4; b_cur += (RESIDENT ? 3 * BN * ROW_BYTES : STAGE_BYTES) >> 4; full_cur += 8u; empty_cur += 8u;
                 if (++s == nst) {
@@ -1927,7 +1926,8 @@ static EncodeTiledFn get_encode() {
 // Tensor map with 128-byte swizzle over uint8 (operands) or int32 (outputs) elements; dims/box
 // innermost first, in elements; strides of dims 1.. in bytes.
 static int encode_map(CUtensorMap* map, const void* ptr, bool int32_elems, int rank, const uint64_t* dims,
-                      const uint64_t* strides, const uint32_t* box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+                      const uint64_t* strides, const uint32_t* box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B,
+                      CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_L2_256B) {
     EncodeTiledFn enc = get_encode();
     if (!enc) return set_cuda_error_text("cuTensorMapEncodeTiled is not available from this driver");
     cuuint64_t gdim[4]; cuuint64_t gstr[3]; cuuint32_t bx[4]; cuuint32_t es[4];
@@ -1935,7 +1935,7 @@ static int encode_map(CUtensorMap* map, const void* ptr, bool int32_elems, int r
     for (int i = 0; i + 1 < rank; ++i) gstr[i] = strides[i];
     CUresult r = enc(map, int32_elems ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, rank,
                      const_cast<void*>(ptr), gdim, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     swizzle, promotion, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         char buf[160];
         snprintf(buf, sizeof buf, "cuTensorMapEncodeTiled failed with CUresult %d (rank %d)", static_cast<int>(r), rank);
@@ -2201,7 +2201,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.conv = 0; p.M = M; p.N = N; p.num_kb = (K + 127) / 128; p.splits = splits;
     p.m_tiles = (M + 127) / 128; p.n_tiles = (N + bn - 1) / bn;
     if (pair) p.m_tiles = (p.m_tiles + 1) / 2;
-    p.a_mn = a_mn; p.b_mn = b_mn; p.a_bytes = PANEL_BYTES;
+    p.a_mn = a_mn; p.b_mn = b_mn; p.a_bytes = PANEL_BYTES; p.b_bytes = (pair ? bn / 2 : bn) * ROW_BYTES;
     p.rows32 = rows32; p.a32 = A; p.b32 = B; p.K = K;
     p.maxabs = splits > 1 ? nullptr : maxabs; p.status = status;
     p.split_cols = (bn == 256 && p.m_tiles * p.n_tiles * splits <= 2 * (pair ? sm_count() / 2 : sm_count())) ? 1 : 0;
@@ -2241,11 +2241,19 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         uint64_t dims[4] = {(uint64_t)red, (uint64_t)W, (uint64_t)H, (uint64_t)Nimg};
         uint64_t str[3] = {(uint64_t)red, (uint64_t)W * red, (uint64_t)H * W * red};
         uint32_t box[4] = {128, (uint32_t)p.BW, (uint32_t)(plan.halo ? p.BH + 2 : p.BH), (uint32_t)p.BI};
-        if (int e = encode_map(&ma, x, false, 4, dims, str, box)) return e;
+        // Rows that end inside the box: without promotion (a TMA unit's cycles per row, 128-byte boxes of 16 / 48 / 64 / 80 / 96 / 128
+        // channels: 4.2 / 4.9 / 2.0 / 5.0 / 2.5 / 1.85, with promotion 5.8 / 6.5 / 2.35 / 6.75 / 2.8 / 1.85)
+        if (int e = encode_map(&ma, x, false, 4, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                               red % 128 == 0 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_NONE)) return e;
         uint64_t d2[2] = {(uint64_t)R * S * C, (uint64_t)K};
         uint64_t s2[1] = {(uint64_t)R * S * C};
         const bool narrow_b = flip && bn == 64;  // MN-major rows of 64 bytes
+        // Rows of a weight box: no more than there are output channels (the columns beyond are neither stored nor counted) or, where
+        // they are the reduction, than its MMAs read.
         uint32_t b2[2] = {narrow_b ? 64u : 128u, flip ? 128u : (uint32_t)(pair ? bn / 2 : bn)};
+        if (!pair && !flip && outc < bn) b2[1] = (uint32_t)outc;
+        if (!pair && flip && red < 128) b2[1] = (uint32_t)((red + 31) / 32 * 32);
+        p.b_bytes = flip ? (int)b2[1] * (pair ? bn / 2 : bn) : (int)b2[1] * ROW_BYTES;
         if (int e = encode_map(&mb, w, false, 2, d2, s2, b2, narrow_b ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B)) return e;
         uint64_t dc[4] = {(uint64_t)outc, (uint64_t)W, (uint64_t)H, (uint64_t)Nimg};
         uint64_t sc[3] = {(uint64_t)outc * 4, (uint64_t)W * outc * 4, (uint64_t)H * W * outc * 4};
