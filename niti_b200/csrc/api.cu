@@ -377,7 +377,7 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
     }
     if (pool_out != nullptr && !(g_opt_parking && !thin && !flip && umma_conv_pool_fusable(N, H, W, K))) return NITI_ERR_UNSUPPORTED;
     // Few enough output tiles for every accumulator to stay in tensor memory: one exact launch.
-    if (g_opt_parking && !thin && umma_conv_fits_parked(N, H, W, flip ? C : K, k3(R, S, pad), flip)) {
+    if (g_opt_parking && !thin && umma_conv_fits_parked(N, H, W, flip ? K : C, flip ? C : K, k3(R, S, pad), flip)) {
         f.parked = 1;
         return umma_conv(in, w, out8, nullptr, N, H, W, C, K, R, S, pad, flip, &f, status, st);
     }
@@ -445,7 +445,7 @@ extern "C" int niti_conv_dgrad_requant_i8(const int8_t* err, const int8_t* w, in
 
 extern "C" size_t niti_conv_dgrad_requant_side_bytes(int N, int H, int W, int C, int K, int R, int S, int pad) {
     if (N <= 0 || H <= 0 || W <= 0 || !niti_conv_dgrad_requant_supported(C, K, R, S, pad)) return 0;
-    if (g_opt_parking && umma_conv_fits_parked(N, H, W, C, k3(R, S, pad), 1)) return 0;  // exact in one launch: nothing to predict
+    if (g_opt_parking && umma_conv_fits_parked(N, H, W, K, C, k3(R, S, pad), 1)) return 0;  // exact in one launch: nothing to predict
     return static_cast<size_t>(N) * H * W * C / 4;
 }
 

@@ -39,8 +39,8 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
               int lda = 0, int ldc = 0);  // row pitches of A and of an int32 result in elements (0: dense)
 int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int Nimg, int H, int W, int C, int K,
               int R, int S, int pad, int flip, const FusedArgs* fused, int32_t* status, cudaStream_t st);
-// k3: 3x3 filters, padding 1
-bool umma_conv_fits_parked(int Nimg, int H, int W, int outc, bool k3, int flip);
+// red / outc: reduction channels per tap, output channels; k3: 3x3 filters, padding 1
+bool umma_conv_fits_parked(int Nimg, int H, int W, int red, int outc, bool k3, int flip);
 bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc);  // the fused forward kernel can also emit the 2x2-pooled output
 size_t umma_wgrad_scratch_bytes(int Nimg, int H, int W, int C, int K, int R, int S);
 // max_splits > 0 caps the number of pixel-range splits (and with it the size of `partial`)

@@ -96,6 +96,7 @@ struct GemmParams {
     int m_tiles, n_tiles;
     int a_mn, b_mn;        // operand majors (0 = K-major, 1 = MN-major)
     int a_bytes;           // bytes one A stage receives from TMA
+    int mma_n;             // columns of one MMA: the tile's, or of the only column tile those that exist (in sixteens)
     int b_bytes;           // bytes of one tap's B tile (of this CTA's half of it): fewer than the tile where the box is lower
     // Operands of 32-byte rows that lie in memory as the MMA reads them (32-byte swizzle: see patch_half), loaded with
     // one untiled bulk copy instead of a box of 128 rows.  1: A [M][32] and B [N][32], one reduction block;
@@ -402,7 +403,7 @@ __device__ __forceinline__ void mma_role(uint8_t* smem, uint64_t* full_bar, uint
     const int rows32 = ROWS32 ? keep_reg(p.rows32) : 0;
     const int mn_tiles = p.m_tiles * p.n_tiles;
     const int total_tiles = mn_tiles * p.splits;
-    const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, rows32 == 2 ? 32 : BN, p.a_mn, p.b_mn);
+    const uint32_t idesc = make_idesc_i8(TWO ? 2 * BLOCK_M : BLOCK_M, p.mma_n, p.a_mn, p.b_mn);
     const int nst = ring_stages(p, STAGES);
     const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_in, 0);  // read from shared memory: make it provably uniform
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
@@ -542,7 +543,7 @@ __device__ __forceinline__ void mma_halo_role(uint8_t* smem, uint64_t* full_bar,
     constexpr bool PARKED = NACC == 0;
     constexpr int MOD = PARKED ? 1 : NACC;
     const int total_tiles = p.m_tiles * p.n_tiles;
-    const uint32_t idesc = make_idesc_i8(BLOCK_M, BN, 0, p.b_mn);
+    const uint32_t idesc = make_idesc_i8(BLOCK_M, p.mma_n, 0, p.b_mn);
     const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, tmem_base_in, 0);
     const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
     const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar), s0 = smem_u32(smem);
@@ -2081,6 +2082,8 @@ int g_stage_cap = 0;  // 0: use every compiled stage
 // nothing else occupying the SMs, and a barrier that is not met ends in the bounded wait's error status.
 int g_cooperative = 1;
 
+static int mma_columns(int n, int bn, int n_tiles, bool pair) { return n_tiles == 1 && !pair ? (n + 15) / 16 * 16 : bn; }
+
 static void finish_params(GemmParams* p) {
     p->fd_mn = make_fastdiv(p->m_tiles * p->n_tiles); p->fd_n = make_fastdiv(p->n_tiles);
     p->fd_tw = make_fastdiv(p->tiles_w); p->fd_th = make_fastdiv(p->tiles_h);
@@ -2114,7 +2117,9 @@ static bool pool_box_ok(int H, int W, int bw, int bh);
 
 // Tiles of a convolution.  kernel: 0 = int32 out, 1 = streaming, 2 = parked.
 struct ConvPlan { int BW, BH, BI, tiles_w, tiles_h, m_tiles, bn; bool pair, halo; };
-static ConvPlan conv_plan(int Nimg, int H, int W, int outc, bool k3, int flip, int kernel) {
+// red: reduction channels per tap.  (`stochastic` turns down plans of more tiles only, so what fits in tensor memory does not
+// depend on it.)
+static ConvPlan conv_plan(int Nimg, int H, int W, int red, int outc, bool k3, int flip, int kernel, bool stochastic = false) {
     ConvPlan c{};
     pick_pixel_box(Nimg, H, W, &c.BW, &c.BH, &c.BI);
     c.tiles_w = (W + c.BW - 1) / c.BW; c.tiles_h = (H + c.BH - 1) / c.BH;
@@ -2123,12 +2128,22 @@ static ConvPlan conv_plan(int Nimg, int H, int W, int outc, bool k3, int flip, i
     c.pair = c.bn != 64 && pair_ok(c.m_tiles, c.bn, flip, 1);
     // 8-pixel-wide tiles of one image with the activations of three taps in one load (producer_halo_role): up to 128
     // columns, where the loads and not the MMAs set the pace (128 -> 128 at 32x32, batch 128: 28.0 -> 19.5 us; 64 -> 64,
-    // batch 1024: 157 -> 119).  A tile so loaded takes about 0.7 of the time, so a quarter more of them (maps that 8 x 16
-    // pixels cover badly) is still a gain.
+    // batch 1024: 157 -> 119).
+    // Maps that 8 x 16 pixels cover badly have more of these tiles; a tile takes about two thirds of the time, so up to half as
+    // many more rounds of thread blocks are a gain (190 random layers, both ways timed; us, box per tap / shared rows, batch x map,
+    // channels, rounds: 501x8x25 16->64, 7 / 14: 67 / 29; 437x28x10 32->96, 9 / 12: 42 / 24; 192x25x12 112->128, 4 / 6: 28.4 / 28.5;
+    // 280x10x11 224->112, 2 / 4: 17.2 / 19.7; 154x10x5 48->128, 1 / 2: 10.6 / 11.9); where random words are drawn, for every row of
+    // a tile, only up to a quarter unless the channels are few (300x20x20, 9 / 13: 96->96 37 / 42, 48->48 49 / 32).  Within one round they always are, but for
+    // layers of 16 and 32 channels, whose time is the loading of the weights by every one of the thread blocks (60x28x4 16->128,
+    // 60 / 120 blocks: 11.0 / 12.6; 36x8x26 80->128, 72 / 144: 10.9 / 10.2; 18x24x10 336->16, 36 / 72: 12.9 / 10.2).
     if (k3 && kernel != 0 && !c.pair && c.bn <= 128) {
         const int th = (H + 15) / 16, bh = (H + th - 1) / th, tw = (W + 7) / 8;
         const long long tiles = static_cast<long long>(tw) * th * Nimg;
-        if (4 * tiles <= 5ll * c.m_tiles && (kernel != 2 || fits_parked(c.bn, static_cast<int>(tiles) * ((outc + c.bn - 1) / c.bn), false))) {
+        const long long n_tiles = (outc + c.bn - 1) / c.bn, sms = sm_count();
+        const long long before = (c.m_tiles * n_tiles + sms - 1) / sms, after = (tiles * n_tiles + sms - 1) / sms;
+        const bool gain = after == 1 ? red >= 48 || tiles * n_tiles <= 64 || 4 * tiles <= 5ll * c.m_tiles
+                                     : (stochastic && red > 64 ? 4 * after <= 5 * before : 2 * after <= 3 * before) || (red == 16 && before > 1 && after <= 2 * before);
+        if (gain && (kernel != 2 || fits_parked(c.bn, static_cast<int>(tiles) * ((outc + c.bn - 1) / c.bn), false))) {
             c.halo = true;
             c.BW = 8; c.BH = bh; c.BI = 1; c.tiles_w = tw; c.tiles_h = th; c.m_tiles = static_cast<int>(tiles);
         }
@@ -2138,9 +2153,9 @@ static ConvPlan conv_plan(int Nimg, int H, int W, int outc, bool k3, int flip, i
 
 // The tiles of a call that pools too: with the shared activation rows unless that makes tiles of an odd number of rows
 // (18, 22, 26, 30, 38 image rows), which would tear pooling windows apart; those keep the box per tap.
-static ConvPlan pool_plan(int Nimg, int H, int W, int outc, bool k3) {
-    const ConvPlan c = conv_plan(Nimg, H, W, outc, k3, 0, 2);
-    return pool_box_ok(H, W, c.BW, c.BH) ? c : conv_plan(Nimg, H, W, outc, false, 0, 2);
+static ConvPlan pool_plan(int Nimg, int H, int W, int red, int outc, bool k3) {
+    const ConvPlan c = conv_plan(Nimg, H, W, red, outc, k3, 0, 2);
+    return pool_box_ok(H, W, c.BW, c.BH) ? c : conv_plan(Nimg, H, W, red, outc, false, 0, 2);
 }
 
 // CTAs that share the reduction of one output tile (umma_split_kernel); 1: none do.  bw: 0, or the width of the tile's pixel
@@ -2202,6 +2217,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.m_tiles = (M + 127) / 128; p.n_tiles = (N + bn - 1) / bn;
     if (pair) p.m_tiles = (p.m_tiles + 1) / 2;
     p.a_mn = a_mn; p.b_mn = b_mn; p.a_bytes = PANEL_BYTES; p.b_bytes = (pair ? bn / 2 : bn) * ROW_BYTES;
+    p.mma_n = rows32 == 2 ? 32 : mma_columns(N, bn, p.n_tiles, pair);
     p.rows32 = rows32; p.a32 = A; p.b32 = B; p.K = K;
     p.maxabs = splits > 1 ? nullptr : maxabs; p.status = status;
     p.split_cols = (bn == 256 && p.m_tiles * p.n_tiles * splits <= 2 * (pair ? sm_count() / 2 : sm_count())) ? 1 : 0;
@@ -2225,11 +2241,12 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     GemmParams p{};
     const bool parked = fused && fused->parked;
     const bool k3 = R == 3 && S == 3 && pad == 1;
-    ConvPlan plan = fused && fused->pool_out != nullptr ? pool_plan(Nimg, H, W, outc, k3)
-                                                        : conv_plan(Nimg, H, W, outc, k3, flip, !fused ? 0 : parked ? 2 : 1);
+    ConvPlan plan = fused && fused->pool_out != nullptr ? pool_plan(Nimg, H, W, red, outc, k3)
+                                                        : conv_plan(Nimg, H, W, red, outc, k3, flip, !fused ? 0 : parked ? 2 : 1,
+                                                                    fused && fused->mode == NITI_ROUND_STOCHASTIC);
     int split = 1;
     if (parked) {
-        const ConvPlan taps = conv_plan(Nimg, H, W, outc, false, flip, 2);
+        const ConvPlan taps = conv_plan(Nimg, H, W, red, outc, false, flip, 2);
         split = split_cluster(taps.m_tiles * ((outc + 127) / 128), R * S, red, plan.halo, fused->mode == NITI_ROUND_STOCHASTIC,
                               fused->pool_out != nullptr ? taps.BW : 0);
         if (split > 1) { plan = taps; plan.bn = 128; }
@@ -2267,6 +2284,7 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     p.M = Nimg * H * W; p.N = outc; p.num_kb = R * S * p.cblocks;
     p.m_tiles = plan.m_tiles; p.n_tiles = (outc + bn - 1) / bn;
     if (pair) p.m_tiles = (p.m_tiles + 1) / 2;
+    p.mma_n = mma_columns(outc, bn, p.n_tiles, pair);
     p.a_mn = 0; p.b_mn = flip ? 1 : 0; p.a_bytes = p.BW * (plan.halo ? p.BH + 2 : p.BH) * p.BI * ROW_BYTES;
     p.maxabs = maxabs; p.status = status;
     p.split_cols = (bn == 256 && p.m_tiles * p.n_tiles <= 2 * (pair ? sm_count() / 2 : sm_count())) ? 1 : 0;
@@ -2291,12 +2309,12 @@ static bool pool_box_ok(int H, int W, int bw, int bh) {
     return H % 2 == 0 && W % 2 == 0 && bh % 2 == 0 && (bw == 2 || bw == 4 || bw == 8 || bw == 16);
 }
 bool umma_conv_pool_fusable(int Nimg, int H, int W, int outc) {
-    const ConvPlan c = conv_plan(Nimg, H, W, outc, false, 0, 2);
-    return pool_box_ok(H, W, c.BW, c.BH) && umma_conv_fits_parked(Nimg, H, W, outc, false, 0);
+    const ConvPlan c = conv_plan(Nimg, H, W, 0, outc, false, 0, 2);
+    return pool_box_ok(H, W, c.BW, c.BH) && umma_conv_fits_parked(Nimg, H, W, 0, outc, false, 0);
 }
 
-bool umma_conv_fits_parked(int Nimg, int H, int W, int outc, bool k3, int flip) {
-    const ConvPlan c = conv_plan(Nimg, H, W, outc, k3, flip, 2);
+bool umma_conv_fits_parked(int Nimg, int H, int W, int red, int outc, bool k3, int flip) {
+    const ConvPlan c = conv_plan(Nimg, H, W, red, outc, k3, flip, 2);
     return fits_parked(c.bn, (c.pair ? (c.m_tiles + 1) / 2 : c.m_tiles) * ((outc + c.bn - 1) / c.bn), c.pair);
 }
 
