@@ -369,6 +369,13 @@ NITI_API int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int32
                        int N, int H, int W, int C, int K, int R, int S, int pad,
                        int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream, int32_t* status, void* stream);
 
+/* The same with `state`, int32[4], 16-byte aligned, owned by the layer: zero before the first call, left zero by every call (calls that
+ * share it must be stream-ordered).  Where one wave of thread blocks holds the layer, the (cooperative) launch of the gradient clears it
+ * too, and for layers of up to 200000 weights also finds the maximum and updates; elsewhere it is the call above. */
+NITI_API int niti_conv_wgrad_update_state_i8(const int8_t* x, const int8_t* err, int32_t* g32, int8_t* w, int32_t* state, int N, int H,
+                       int W, int C, int K, int R, int S, int pad, int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream,
+                       int32_t* status, void* stream);
+
 /* niti_gemm_i8 with scratch of niti_gemm_scratch_bytes() bytes (0: none needed): shapes whose row pitches the tensor-core
  * kernels do not take (A rows that are not whole 16-byte groups, results of any width) then run on them all the same. */
 NITI_API size_t niti_gemm_scratch_bytes(int M, int N, int K, int trans_a, int trans_b);

@@ -65,6 +65,7 @@ SIGNATURES = {
     "niti_quantize_input_with_max_f32": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "niti_conv_wgrad_update_elems": (_sz, [_i] * 5),
     "niti_conv_wgrad_update_i8": (_i, [_p] * 4 + [_i] * 10 + [_p, _u32, _p, _p]),
+    "niti_conv_wgrad_update_state_i8": (_i, [_p] * 5 + [_i] * 10 + [_p, _u32, _p, _p]),
     "niti_gemm_scratch_bytes": (_sz, [_i] * 5),
     "niti_gemm_scratch_i8": (_i, [_p] * 5 + [_sz] + [_i] * 5 + [_p, _p]),
     "niti_update_multi_scratch_bytes": (_sz, []),

@@ -48,6 +48,12 @@ size_t umma_wgrad_scratch_bytes(int Nimg, int H, int W, int C, int K, int R, int
 int umma_conv_wgrad_partials(const int8_t* x, const int8_t* err, int32_t* partial, int* splits_out, int max_splits,
                              int Nimg, int H, int W, int C, int K, int R, int S, int pad, int32_t* status, cudaStream_t st,
                              int direct = 0);
+// gradient, cleared by the launch, and for small layers (*updated) the update, in one (cooperative) launch of one wave of thread
+// blocks; state: int32[4], zero between calls; words: cleared, the first is max |g| of an update
+bool umma_conv_wgrad_update_fits(int Nimg, int H, int W, int C, int K, int R);
+int umma_conv_wgrad_update(const int8_t* x, const int8_t* err, int32_t* out, int8_t* w, uint32_t* words, int num_words, int32_t* state,
+                           int Nimg, int H, int W, int C, int K, int R, int S, int pad, int mu, int mode, const unsigned long long* seed,
+                           unsigned rng_stream, bool* updated, int32_t* status, cudaStream_t st);
 // operands with the batch innermost ([channels][H][W][N]) -> out [C][R][S][K] (zeroed by the caller)
 int umma_conv_wgrad_batch_inner(const int8_t* x_t, const int8_t* err_t, int32_t* out, int Nimg, int H, int W, int C, int K, int R,
                                 int S, int pad, int32_t* status, cudaStream_t st);

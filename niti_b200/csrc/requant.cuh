@@ -54,6 +54,11 @@ __host__ __device__ __forceinline__ int shift_for(uint32_t m, int kind, int targ
     return s > 0 ? s : 0;
 }
 
+__device__ __forceinline__ unsigned iabs_u(int x) { return static_cast<unsigned>(x < 0 ? -x : x); }
+__device__ __forceinline__ unsigned absmax4(const int4 v) {
+    return max(max(iabs_u(v.x), iabs_u(v.y)), max(iabs_u(v.z), iabs_u(v.w)));
+}
+
 __device__ __forceinline__ int clamp127(int v) { return max(-127, min(127, v)); }
 
 // One element: shift == 0 wraps like `.type(torch.int8)`; shift > 0 rounds then clamps to +-127.
@@ -130,6 +135,19 @@ __device__ __forceinline__ int narrow_pseudo(int x, int shift) {
     const uint32_t up = (lo >> h) > ((lo & ((1u << h) - 1u)) << (shift & 1)) ? 1u : 0u;
     const int v = static_cast<int>(min((a >> shift) + up, 127u));
     return x < 0 ? -v : v;
+}
+
+// Four weights less their narrowed gradients.  Pseudo-stochastic rounding, the gradients' own mode, has a short form.
+__device__ __forceinline__ uint32_t update_word(const int4 gv, const uint32_t wv, const uint32_t (&rnd)[4], int shift, int mode,
+                                                bool zero_out) {
+    const int gx[4] = {gv.x, gv.y, gv.z, gv.w};
+    int y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int g8 = zero_out ? 0 : mode == ROUND_PSEUDO_STOCHASTIC && shift > 0 ? narrow_pseudo(gx[j], shift) : narrow(gx[j], shift, mode, rnd[j]);
+        y[j] = static_cast<int8_t>(wv >> (8 * j)) - g8;
+    }
+    return __vmaxs4(pack2_sat_s8(y[1], y[0], pack2_sat_s8(y[3], y[2], 0u)), 0x81818181u);
 }
 
 }  // namespace niti

@@ -33,7 +33,6 @@ static int sm_count_simt() {
     return n;
 }
 
-__device__ __forceinline__ unsigned iabs_u(int x) { return static_cast<unsigned>(x < 0 ? -x : x); }
 
 __device__ __forceinline__ void warp_atomic_max(unsigned* dst, unsigned v) {
     v = __reduce_max_sync(0xFFFFFFFFu, v);
@@ -625,18 +624,6 @@ __global__ void loss_kernel(const int8_t* __restrict__ out8, const int32_t* __re
 // ------------------------------------------------------------------------------------------------
 // weight update and the flipped / transposed filter bank the error-backward convolution reads
 // ------------------------------------------------------------------------------------------------
-// Four weights less their narrowed gradients.  Pseudo-stochastic rounding, the gradients' own mode, has a short form.
-__device__ __forceinline__ uint32_t update_word(const int4 gv, const uint32_t wv, const uint32_t (&rnd)[4], int shift, int mode,
-                                                bool zero_out) {
-    const int gx[4] = {gv.x, gv.y, gv.z, gv.w};
-    int y[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int g8 = zero_out ? 0 : mode == ROUND_PSEUDO_STOCHASTIC && shift > 0 ? narrow_pseudo(gx[j], shift) : narrow(gx[j], shift, mode, rnd[j]);
-        y[j] = static_cast<int8_t>(wv >> (8 * j)) - g8;
-    }
-    return __vmaxs4(pack2_sat_s8(y[1], y[0], pack2_sat_s8(y[3], y[2], 0u)), 0x81818181u);
-}
 __global__ void __launch_bounds__(256)
 update_kernel(int8_t* __restrict__ w, const int32_t* __restrict__ g32, const unsigned* __restrict__ maxabs, long long n,
               int mu, int mode, const unsigned long long* seed_p, unsigned rng_stream) {
@@ -673,9 +660,6 @@ struct UpdateMultiParams {
     int32_t* state;  // [count] maxima, [UPDATE_MULTI_MAX] barrier arrivals; zero at launch
     int32_t* status;
 };
-__device__ __forceinline__ unsigned absmax4(const int4 v) {
-    return max(max(iabs_u(v.x), iabs_u(v.y)), max(iabs_u(v.z), iabs_u(v.w)));
-}
 // Every block works on ONE layer (blocks are dealt to the layers in proportion to their sizes on the host), so a
 // block has one chain of loads -> maximum -> atomic before the barrier and one read of its layer's maximum after it.
 __global__ void __launch_bounds__(256)
@@ -1567,6 +1551,18 @@ extern "C" int niti_update_multi_i8(const niti_update_item* items, int count, in
     return NITI_OK;
 }
 
+// One layer's update; words: zero, the first ends up as the maximum.
+static int update_after_gradient(int8_t* w, int32_t* g32, int32_t* words, long long n, int mu, int round_mode, const uint64_t* seed,
+                                 uint32_t rng_stream, int32_t* status, cudaStream_t st) {
+    UpdateMultiParams p;
+    p.count = 1; p.mu = mu; p.mode = round_mode; p.clear = 0;
+    p.item[0] = UpdateItem{w, g32, nullptr, n, rng_stream};
+    p.seed = reinterpret_cast<const unsigned long long*>(seed);
+    p.state = words;
+    p.status = status;
+    return launch_update(p, st);
+}
+
 // The gradient's zeroing, its tail's and nothing else in front of the contraction; the maximum is found by the update
 // itself (grid barrier).  Per convolution that is three launches instead of the five of niti_conv_wgrad_i8 +
 // niti_update_i8 (two memsets, contraction, maximum, update), and a small layer's step is launches.
@@ -1589,13 +1585,27 @@ extern "C" int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int e = set_cuda_error(cudaMemsetAsync(g32, 0, elems * 4, st))) return e;
     if (int e = niti_conv_wgrad_accumulate_i8(x, err, g32, N, H, W, C, K, R, S, pad, status, stream)) return e;
-    UpdateMultiParams p;
-    p.count = 1; p.mu = mu; p.mode = round_mode; p.clear = 0;
-    p.item[0] = UpdateItem{w, g32, nullptr, static_cast<long long>(K) * R * S * C, rng_stream};
-    p.seed = reinterpret_cast<const unsigned long long*>(seed);
-    p.state = g32 + elems - niti_update_multi_scratch_bytes() / 4;  // its first word ends up as the maximum
-    p.status = status;
-    return launch_update(p, st);
+    return update_after_gradient(w, g32, g32 + elems - niti_update_multi_scratch_bytes() / 4, static_cast<long long>(K) * R * S * C, mu, round_mode,
+                                 seed, rng_stream, status, st);
+}
+
+extern "C" int niti_conv_wgrad_update_state_i8(const int8_t* x, const int8_t* err, int32_t* g32, int8_t* w, int32_t* state, int N, int H,
+                                               int W, int C, int K, int R, int S, int pad, int mu, int round_mode, const uint64_t* seed,
+                                               uint32_t rng_stream, int32_t* status, void* stream) {
+    NITI_REQUIRE(x && err && g32 && w && state && N > 0 && H > 0 && W > 0 && round_mode >= 0 && round_mode <= 2);
+    NITI_REQUIRE((seed || round_mode != NITI_ROUND_STOCHASTIC) && reinterpret_cast<uintptr_t>(state) % 16 == 0);
+    NITI_REQUIRE(reinterpret_cast<uintptr_t>(w) % 4 == 0 && reinterpret_cast<uintptr_t>(g32) % 16 == 0);
+    const size_t elems = niti_conv_wgrad_update_elems(C, K, R, S, pad);
+    if (elems == 0) return NITI_ERR_UNSUPPORTED;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(err)) % 16 != 0 || !umma_conv_wgrad_update_fits(N, H, W, C, K, R))
+        return niti_conv_wgrad_update_i8(x, err, g32, w, N, H, W, C, K, R, S, pad, mu, round_mode, seed, rng_stream, status, stream);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int words = static_cast<int>(niti_update_multi_scratch_bytes() / 4);
+    int32_t* tail = g32 + elems - words;
+    bool updated = false;
+    if (int e = umma_conv_wgrad_update(x, err, g32, w, reinterpret_cast<uint32_t*>(tail), words, state, N, H, W, C, K, R, S, pad, mu, round_mode,
+                                       reinterpret_cast<const unsigned long long*>(seed), rng_stream, &updated, status, st)) return e;
+    return updated ? NITI_OK : update_after_gradient(w, g32, tail, static_cast<long long>(K) * R * S * C, mu, round_mode, seed, rng_stream, status, st);
 }
 
 extern "C" size_t niti_dp_exchange_bytes(void) { return DPX_WORDS * sizeof(int32_t); }

@@ -345,8 +345,10 @@ PyObject* conv_wgrad_update(Args& a) {
     const int pad = a.i32(), mu = a.i32(), mode = a.i32();
     const Tensor* seed = a.maybe();
     const uint32_t stream = a.u32();
-    need_cuda({&x, &err, &w});
+    const Tensor* state = a.maybe();
+    need_cuda({&x, &err, &w, state});
     require(x.dim() == 4 && err.dim() == 4 && w.scalar_type() == at::kChar);
+    require(state == nullptr || (state->scalar_type() == at::kInt && state->numel() >= 4));
     const Conv s = conv_shape(x, w);
     require(w.size(3) == s.C && err.size(3) == s.K && err.size(0) == s.N && err.size(1) == s.H && err.size(2) == s.W);
     Tensor g32, mx;
@@ -354,6 +356,11 @@ PyObject* conv_wgrad_update(Args& a) {
         Launch l(x);
         const int64_t elems = static_cast<int64_t>(niti_conv_wgrad_update_elems(s.C, s.K, s.R, s.S, pad));
         const Tensor both = l.empty({elems}, at::kInt);
+        if (state != nullptr)
+            check(niti_conv_wgrad_update_state_i8(cptr<int8_t>(x), cptr<int8_t>(err), mptr<int32_t>(both), mptr<int8_t>(w), mptr<int32_t>(state), s.N,
+                                                  s.H, s.W, s.C, s.K, s.R, s.S, pad, mu, mode, cptr<uint64_t>(seed), stream, l.status(), l.stream),
+                  "niti_conv_wgrad_update_state_i8");
+        else
         check(niti_conv_wgrad_update_i8(cptr<int8_t>(x), cptr<int8_t>(err), mptr<int32_t>(both), mptr<int8_t>(w), s.N, s.H, s.W, s.C, s.K, s.R,
                                         s.S, pad, mu, mode, cptr<uint64_t>(seed), stream, l.status(), l.stream), "niti_conv_wgrad_update_i8");
         auto view = [&](int64_t at_, at::IntArrayRef shape) {

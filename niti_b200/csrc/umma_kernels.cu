@@ -1694,11 +1694,25 @@ constexpr int WG_STAGES = 3;
 constexpr int WG_SMEM_BYTES = WG_STAGES * WG_STAGE_BYTES + 1024 + 256;
 constexpr int WG_TMEM_COLS = 512;
 
+// What surrounds the contraction in umma_wgrad_update_kernel.
+struct WgradUpdate {
+    int32_t* g32;
+    int8_t* w;             // null: the update is a launch of its own, which counts in `words`
+    unsigned* maxabs;
+    uint32_t* words; int num_words;  // cleared
+    long long n;           // gradient elements, a multiple of 4
+    int mu, mode;
+    const unsigned long long* seed;
+    unsigned rng_stream;
+    int32_t* state;        // {zeroed, barrier arrivals, max |g|, exit ticket}: zero between calls
+};
+
 // One CTA's share of one layer's weight gradient: work item `item` (filter row, k tile, c tile) over the pixel chunks of
 // split `split`.  The tensor maps live in kernel parameter space (grid constants of the calling kernel).
-template <bool KMAJ>
+template <bool KMAJ, bool UPDATE = false>
 __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUtensorMap& tmX, const CUtensorMap& tmP,
-                                           const WgradParams& p, const int split, const int item, const bool probe_cta) {
+                                           const WgradParams& p, const int split, const int item, const bool probe_cta,
+                                           const WgradUpdate* u = nullptr) {
     if (threadIdx.x == 0 && probe_cta) PARK_STAMP(10);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1834,12 +1848,32 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUten
         const int q = warp & 3;
         const int row_in_tile = q * 32 + lane;
         const bool leader = threadIdx.x == 64;
+        const int ctas = static_cast<int>(gridDim.x * gridDim.y);
+        if (UPDATE && p.splits > 1) {
+            // the gradient is cleared here, under the contraction; nobody adds to it before every CTA has cleared its part
+            int4* g = reinterpret_cast<int4*>(u->g32);
+            const long long groups = u->n >> 2;
+            for (long long i = static_cast<long long>(blockIdx.y * gridDim.x + blockIdx.x) * 128 + row_in_tile; i < groups; i += 128ll * ctas)
+                g[i] = make_int4(0, 0, 0, 0);
+            fence_proxy_async_global();
+            __threadfence();
+            named_barrier(EPI_BARRIER, 128);
+            if (leader) red_release_add(&u->state[0], 1);
+        }
         const uint32_t failed = mbar_wait(smem_u32(&tfull_bar[0]), 0, abort_flag) ? 0u : 1u;
         if (barrier_or(EPI_BARRIER, 128, failed)) {
             if (failed) report_abort(p.status, 14, 2);
         } else {
             tc_fence_after();
             if (leader && probe_cta) PARK_STAMP(14);
+            bool cleared = true;
+            if (UPDATE && p.splits > 1 && leader) {
+                const unsigned long long t0 = global_timer_ns();
+                for (unsigned spin = 0; ld_acquire_gpu(&u->state[0]) < ctas; ++spin)
+                    if ((spin & 63) == 63 && global_timer_ns() - t0 > GRID_BARRIER_LIMIT_NS) { cleared = false; break; }
+                if (!cleared) { *abort_flag = 1; report_abort(p.status, 15, 2); }
+                fence_proxy_async_global();
+            }
             for (int sx = 0; sx < p.S; ++sx) {
                 const uint32_t buf = smem_u32(smem + sx * WG_STAGE_BYTES);
                 uint32_t v[4][32];
@@ -1850,7 +1884,7 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUten
                 for (int j = 0; j < 4; ++j) stage_row(buf + j * EPI_CHUNK_BYTES, row_in_tile, v[j]);
                 fence_proxy_async();
                 named_barrier(EPI_BARRIER, 128);
-                if (leader) {
+                if (leader && cleared) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         if (ct * 128 + j * 32 < p.C) {
@@ -1861,7 +1895,8 @@ __device__ __forceinline__ void wgrad_body(const CUtensorMap& tmErr, const CUten
                 }
             }
             if (leader && probe_cta) PARK_STAMP(15);
-            if (leader) bulk_wait_read<0>();
+            if (leader) { if (UPDATE) bulk_wait<0>(); else bulk_wait_read<0>(); }  // UPDATE: the sums are in memory
+            if (UPDATE && leader) fence_proxy_async_global();
             if (leader && probe_cta) PARK_STAMP(16);
         }
     }
@@ -1880,6 +1915,82 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1)
 umma_wgrad_kernel(const __grid_constant__ CUtensorMap tmErr, const __grid_constant__ CUtensorMap tmX,
                   const __grid_constant__ CUtensorMap tmP, const __grid_constant__ WgradParams p) {
     wgrad_body<false>(tmErr, tmX, tmP, p, blockIdx.x, blockIdx.y, blockIdx.y == 0);
+}
+// The same with the gradient cleared under the contraction, and for small layers followed by the update (UpdateWeight.weight_update)
+// in the same launch: a grid barrier when every CTA's sums are in memory, max |g|, a second one, the update.  A single layer's
+// backward is launches: 48 -> 80 on 37 15x13 maps took 14.5 us with a memset, the contraction and the update in a row (and a gap of 1
+// to 2 us behind each) and takes 11 as one.  Cooperative; one wave of CTAs, whose six warps are too few for the update of a large
+// layer (589 thousand weights: even; 2.4 million: 44 us against 27).
+constexpr long long WG_UPDATE_MAX = 200000;
+__global__ void __launch_bounds__(UMMA_THREADS, 1)
+umma_wgrad_update_kernel(const __grid_constant__ CUtensorMap tmErr, const __grid_constant__ CUtensorMap tmX,
+                         const __grid_constant__ CUtensorMap tmP, const __grid_constant__ WgradParams p, const __grid_constant__ WgradUpdate u) {
+    __shared__ int flag;
+    __shared__ unsigned part[UMMA_THREADS / 32];
+    if (blockIdx.x + blockIdx.y == 0)
+        for (int i = threadIdx.x; i < u.num_words; i += UMMA_THREADS) u.words[i] = 0;
+    wgrad_body<false, true>(tmErr, tmX, tmP, p, blockIdx.x, blockIdx.y, blockIdx.y == 0, &u);
+    const int ctas = static_cast<int>(gridDim.x * gridDim.y);
+    if (u.w == nullptr) {
+        if (p.splits > 1 && threadIdx.x == 0 && atomicAdd(&u.state[3], 1) == ctas - 1) { u.state[0] = 0; u.state[3] = 0; }
+        return;
+    }
+    const long long groups = u.n >> 2, step = static_cast<long long>(ctas) * UMMA_THREADS;
+    const long long tid = static_cast<long long>(blockIdx.y * gridDim.x + blockIdx.x) * UMMA_THREADS + threadIdx.x;
+    const int4* g4 = reinterpret_cast<const int4*>(u.g32);
+    uint32_t* w4 = reinterpret_cast<uint32_t*>(u.w);
+    // gradients and weights of a thread's first word groups stay in registers from the maximum to the update
+    constexpr int KEEP = 2;
+    int4 gv[KEEP];
+    uint32_t wv[KEEP];
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k)
+        if (tid + k * step < groups) wv[k] = w4[tid + k * step];  // does not depend on the sums
+    bool ok = bounded_grid_barrier(&u.state[1], ctas, p.status, 7, &flag);
+    if (ok) {
+        unsigned m = 0;
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k)
+            if (tid + k * step < groups) gv[k] = __ldcg(g4 + tid + k * step);
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k)
+            if (tid + k * step < groups) m = max(m, absmax4(gv[k]));
+        for (long long g = tid + KEEP * step; g < groups; g += step) m = max(m, absmax4(__ldcg(g4 + g)));
+        m = __reduce_max_sync(0xFFFFFFFFu, m);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int i = 0; i < UMMA_THREADS / 32; ++i) m = max(m, part[i]);
+            if (m != 0) red_relaxed_max(reinterpret_cast<unsigned*>(&u.state[2]), m);
+        }
+        ok = bounded_grid_barrier(&u.state[1], 2 * ctas, p.status, 7, &flag);
+    }
+    const unsigned mx = static_cast<unsigned>(ld_acquire_gpu(&u.state[2]));
+    int ticket = -1;
+    if (ok) {
+        bool zero_out;
+        const int shift = shift_for(mx, CALC_GRAD, u.mu, &zero_out);
+        const bool stochastic = u.mode == ROUND_STOCHASTIC && shift > 0;
+        const unsigned long long seed = stochastic ? *u.seed : 0ull;
+        const auto one = [&](long long g, const int4 gvv, const uint32_t wvv) {
+            uint32_t rnd[4] = {0, 0, 0, 0};
+            if (stochastic) random_block(seed, u.rng_stream, static_cast<unsigned long long>(g), rnd);
+            w4[g] = update_word(gvv, wvv, rnd, shift, u.mode, zero_out);
+        };
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k)
+            if (tid + k * step < groups) one(tid + k * step, gv[k], wv[k]);
+        for (long long g = tid + KEEP * step; g < groups; g += step) one(g, __ldcg(g4 + g), w4[g]);
+    }
+    __syncthreads();  // every thread has read the maximum
+    if (threadIdx.x == 0) {
+        ticket = atomicAdd(&u.state[3], 1);
+        if (ticket == ctas - 1) {
+            *u.maxabs = mx;
+            u.state[0] = 0; u.state[1] = 0; u.state[2] = 0; u.state[3] = 0;
+        }
+    }
 }
 __global__ void __launch_bounds__(UMMA_THREADS, 1)
 umma_wgrad_kmajor_kernel(const __grid_constant__ CUtensorMap tmErr, const __grid_constant__ CUtensorMap tmX,
@@ -2375,6 +2486,33 @@ int umma_conv_wgrad_partials(const int8_t* x, const int8_t* err, int32_t* partia
     dim3 grid(p.splits, R * p.k_tiles * p.c_tiles);
     umma_wgrad_kernel<<<grid, UMMA_THREADS, WG_SMEM_BYTES, st>>>(me, mx, mp, p);
     return set_cuda_error(cudaGetLastError());
+}
+
+// The gradient into `out`, cleared by the launch, and where *updated says so the update of `w`; state: int32[4], zero between calls.
+// words: cleared too, and the first becomes max |g| of an update.
+bool umma_conv_wgrad_update_fits(int Nimg, int H, int W, int C, int K, int R) {
+    WgradParams p{};
+    wgrad_plan(Nimg, H, W, C, K, R, 0, &p);
+    return p.splits * R * p.k_tiles * p.c_tiles <= sm_count();
+}
+int umma_conv_wgrad_update(const int8_t* x, const int8_t* err, int32_t* out, int8_t* w, uint32_t* words, int num_words, int32_t* state,
+                           int Nimg, int H, int W, int C, int K, int R, int S, int pad, int mu, int mode, const unsigned long long* seed,
+                           unsigned rng_stream, bool* updated, int32_t* status, cudaStream_t st) {
+    WgradParams p{};
+    wgrad_plan(Nimg, H, W, C, K, R, 0, &p);
+    CUtensorMap me, mx, mp;
+    if (int e = wgrad_setup(x, err, out, p.splits > 1 ? 1 : 0, Nimg, H, W, C, K, R, S, pad, status, &p, &me, &mx, &mp)) return e;
+    const long long n = static_cast<long long>(K) * R * S * C;
+    *updated = n <= WG_UPDATE_MAX;
+    const WgradUpdate u{out, *updated ? w : nullptr, words, words, num_words, n, mu, mode, seed, rng_stream, state};
+    cudaError_t e = cudaFuncSetAttribute(umma_wgrad_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM_BYTES);
+    if (e != cudaSuccess) return set_cuda_error(e);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.splits, R * p.k_tiles * p.c_tiles); cfg.blockDim = dim3(UMMA_THREADS); cfg.dynamicSmemBytes = WG_SMEM_BYTES; cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_wgrad_update_kernel, me, mx, mp, p, u));
 }
 
 // x_t [C][H][W][N], err_t [K][H][W][N] (batch innermost, N a multiple of 16) -> out [C][R][S][K], zeroed by the caller:

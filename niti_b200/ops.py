@@ -218,9 +218,15 @@ def conv_wgrad_acc(x, err, R=3, S=3, pad=1, out=None, want_max=True):
     return _run("niti_conv_wgrad_i8", 2 if x.size(3) % 16 == 0 else 3, work, native.conv_wgrad_acc, x, err, R, S, pad, out, want_max)
 
 
-def conv_wgrad_update(x, err, w, pad=1, mu=5, mode=ROUND_PSEUDO_STOCHASTIC, seed=None, rng_stream=0):
+def new_update_state(device):
+    """The words a layer lends to conv_wgrad_update (zero between calls)."""
+    return torch.zeros(4, dtype=torch.int32, device=device)
+
+
+def conv_wgrad_update(x, err, w, pad=1, mu=5, mode=ROUND_PSEUDO_STOCHASTIC, seed=None, rng_stream=0, state=None):
     """conv_wgrad_acc followed by update of the filters w, in fewer launches: (gradient int32, max|gradient|).  For the
-    shapes of conv_wgrad_accumulate_supported; with NITI_OPT_WGRAD_TMA_REDUCE off it is those two calls."""
+    shapes of conv_wgrad_accumulate_supported; with NITI_OPT_WGRAD_TMA_REDUCE off it is those two calls.  ``state``
+    (new_update_state, owned by the layer): one launch for small layers, two for larger ones."""
     K, R, S, C = w.shape
     if not native.conv_wgrad_update_supported(C, K, R, S, pad):
         g32, mx = conv_wgrad_acc(x, err, R, S, pad)
@@ -229,7 +235,7 @@ def conv_wgrad_update(x, err, w, pad=1, mu=5, mode=ROUND_PSEUDO_STOCHASTIC, seed
 
     def work(r):
         return 2 * err.numel() * w[0].numel(), x.numel() + err.numel() + 10 * w.numel()
-    return _run("niti_conv_wgrad_update_i8", 2, work, native.conv_wgrad_update, x, err, w, pad, mu, mode, seed, rng_stream)
+    return _run("niti_conv_wgrad_update_i8", 2, work, native.conv_wgrad_update, x, err, w, pad, mu, mode, seed, rng_stream, state)
 
 
 def conv_wgrad_batch_inner_supported(N, C, K, R, S, pad):

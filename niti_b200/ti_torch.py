@@ -380,6 +380,14 @@ class TiConv2d(UpdateWeight):
         self._bwd_state = None
         self._bwd_side, self._bwd_side_shape = None, None
         self._patches, self._patches_of = None, None
+        self._update_state = None  # words of the gradient-and-update launch
+
+    def _new_states(self, dev):
+        """The device words of this layer's launches that are not there yet, from one allocation."""
+        words = torch.zeros(20, dtype=torch.int32, device=dev)
+        for name, part in (('_fwd_state', words[:8]), ('_bwd_state', words[8:16]), ('_update_state', words[16:])):
+            if self.__dict__[name] is None:
+                self.__dict__[name] = part
 
     def forward(self, input):
         act, exp_in = input
@@ -390,7 +398,7 @@ class TiConv2d(UpdateWeight):
             # conv2d_int8 + act_calc (:393-395) in one kernel; see ops.conv_fprop_fused
             dev = act.device
             if self._fwd_state is None:
-                self._fwd_state = ops.new_requant_state(dev)
+                self._new_states(dev)
             mode, seed, stream, exp_in = _mode(ACT_ROUND_METHOD), RNG_SEED(dev), 16 * self.layer_id, exp_tensor(exp_in, dev)
             pool = self.pool_layer
             if (pool is not None and FUSE_POOL and self.fuse_relu and pool.kernel_size == 2 and pool.stride == 2
@@ -434,7 +442,7 @@ class TiConv2d(UpdateWeight):
             offset = SAMPLE_OFFSET * h * w_ * C
             if FUSE_REQUANT and GLOBAL_MAX_GROUP is None and ops.conv_dgrad_fused_supported(C, K, R, S, self.padding):
                 if self._bwd_state is None:
-                    self._bwd_state = ops.new_requant_state(dev)
+                    self._new_states(dev)
                 if STEP_DOWN_CODES and (self._bwd_side is None or self._bwd_side_shape != (n, h, w_)):
                     # layers whose output does not fit in tensor memory guess their shift; two more bits per output
                     # make a guess one too high a cheap repair instead of a second contraction
@@ -468,8 +476,10 @@ class TiConv2d(UpdateWeight):
         elif (not self.defer_update and self.grad_buffer is None and self.grad_ready is None
                 and self.plain_update() and ops.conv_wgrad_accumulate_supported(C, K, R, S, self.padding)):
             # nobody looks at the gradient between its computation and the update: both in one call
+            if self._update_state is None:
+                self._new_states(dev)
             g32, g_max = ops.conv_wgrad_update(act, err_in, self.weight, self.padding, GRAD_BITWIDTH, _mode(GRAD_ROUND_METHOD),
-                                               RNG_SEED(dev), 16 * self.layer_id + 2)
+                                               RNG_SEED(dev), 16 * self.layer_id + 2, self._update_state)
             updated = True
         elif self._patches_of is act and self._patches is not None:
             # the patch matrix of this step's forward pass is still there

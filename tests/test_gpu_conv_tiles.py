@@ -232,7 +232,8 @@ def test_input_quantisation_of_three_planes(N, H, W):
     assert int(e) == want_e
 
 
-@pytest.mark.parametrize("N,H,W,C,K,mode", [(2, 5, 7, 16, 16, 2), (3, 8, 8, 48, 80, 2), (1, 4, 4, 144, 128, 1)])
+@pytest.mark.parametrize("N,H,W,C,K,mode", [(2, 5, 7, 16, 16, 2), (3, 8, 8, 48, 80, 2), (1, 4, 4, 144, 128, 1),
+                                            (7, 4, 4, 512, 528, 2), (1, 2, 2, 1040, 1024, 2)])  # more weights than stay in registers; two waves
 def test_gradient_and_update_in_one_call(N, H, W, C, K, mode):
     rng = np.random.default_rng(N + C + K)
     x, w, err = rnd8(rng, (N, H, W, C)), rnd8(rng, (K, 3, 3, C)), rnd8(rng, (N, H, W, K))
@@ -242,6 +243,14 @@ def test_gradient_and_update_in_one_call(N, H, W, C, K, mode):
     same(g32, g)
     assert int(mx) == int(np.abs(g).max())
     same(wd, O.weight_update(w, g, 5, mode, philox.random_u32_tensor(7, 18, g.shape))[0])
+    # the same in one launch, over the layer's own words, which every call leaves zero
+    st = ops.new_update_state(DEV)
+    for _ in range(2):
+        w1 = cu(w)
+        g1, m1 = ops.conv_wgrad_update(cu(x), cu(err), w1, 1, 5, mode, ops.seed_tensor(7, DEV), 18, st)
+        same(g1, g)
+        assert torch.equal(w1, wd) and int(m1) == int(mx) and not bool(st.any())
+    ops.check_status(DEV)
     # operands that do not start on a 16-byte boundary are served too, as by the separate calls
     odd = torch.empty(x.size + 1, dtype=torch.int8, device=DEV)[1:].view(x.shape)
     odd.copy_(cu(x))
