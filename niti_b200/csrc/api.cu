@@ -365,7 +365,10 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
                       const uint64_t* seed, uint32_t rng_stream, uint64_t rng_offset, int relu, const int32_t* exp_a,
                       const int32_t* exp_b, int32_t* exp_out, int32_t* shift_out, int32_t* status, cudaStream_t st,
                       const int8_t* relu_mask = nullptr, int8_t* pool_out = nullptr, void* side = nullptr) {
-    FusedArgs f{state, 0, 0, round_mode, relu, reinterpret_cast<const unsigned long long*>(seed), rng_stream, rng_offset,
+    // Narrow with the predicted shift, reduce max|acc|, verify, narrow again where it was wrong: forward layers in one launch, the
+    // thin layer, the error's way back and CTA pairs with a conditional second one.
+    const bool one = !flip && fprop_path(C, K, R, S, pad) != CONV_THIN && !(g_two_cta & 2) && relu_mask == nullptr && side == nullptr;
+    FusedArgs f{state, 0, one ? 1 : 0, 0, round_mode, relu, reinterpret_cast<const unsigned long long*>(seed), rng_stream, rng_offset,
                 kind, 7, exp_a, exp_b, exp_out, shift_out, relu_mask, pool_out, side};
     const bool thin = !flip && fprop_path(C, K, R, S, pad) == CONV_THIN;
     const size_t m = static_cast<size_t>(N) * H * W;
@@ -381,8 +384,7 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
         f.parked = 1;
         return umma_conv(in, w, out8, nullptr, N, H, W, C, K, R, S, pad, flip, &f, status, st);
     }
-    // first launch: narrow with the predicted shift, reduce max|acc|, verify; second launch: redo if it was wrong
-    for (int pass = 0; pass < 2; ++pass) {
+    for (int pass = 0; pass < (one ? 1 : 2); ++pass) {
         f.only_if_redo = pass;
         int rc = thin ? umma_gemm(xcol, wp, out8, nullptr, static_cast<int>(m), K, 32, 0, 1, 1, &f, status, st, 1)
                       : umma_conv(in, w, out8, nullptr, N, H, W, C, K, R, S, pad, flip, &f, status, st);

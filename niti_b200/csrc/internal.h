@@ -15,6 +15,7 @@ int set_cuda_error_text(const char* text);
 struct FusedArgs {
     int32_t* state;        // {shift, max|acc|, redo flag, redo count, exit ticket, barrier arrivals, -, -}
     int only_if_redo;
+    int one;               // 1: the streaming kernel narrows again in the same launch where its guess was wrong (forward layers)
     int parked;            // 1: accumulator-parking kernel (exact in one launch; needs umma_conv_fits_parked)
     int mode, relu;
     const unsigned long long* seed;

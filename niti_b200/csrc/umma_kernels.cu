@@ -959,6 +959,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // 18 warps (five on one scheduler) leave 96 registers per thread, which 32 accumulators at a time fit into.
 // ------------------------------------------------------------------------------------------------
 constexpr int EPI_WARPS = 16;
+constexpr unsigned long long GRID_BARRIER_LIMIT_NS = 500000000ull;  // 0.5 s
 constexpr int REQUANT_THREADS = 64 + 32 * EPI_WARPS;  // producer warp, MMA warp, epilogue warps
 template <int BN>
 struct EpiSplit {
@@ -1197,7 +1198,6 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // no int32 in memory.  state = {shift out, max|acc|, redo flag (cleared), redo count, exit ticket,
 // -, max|acc| and barrier arrivals (adjacent: read with one 64-bit load)}; words 1, 4, 5, 6 and 7 are zero between calls.
 // ------------------------------------------------------------------------------------------------
-constexpr unsigned long long GRID_BARRIER_LIMIT_NS = 500000000ull;  // 0.5 s
 
 // The grid barrier of the kernels below, run by a CTA's epilogue warps (which have left their maxima in warp_max): every CTA
 // has contributed its maximum when it returns the shift that narrows the tensor, the same to all of them; -1 where the others
@@ -1246,6 +1246,180 @@ __device__ __forceinline__ void parked_leave(const GemmParams& p, int shift, int
             if (p.exp_out) *p.exp_out = s_out + (p.exp_a ? *p.exp_a : 0) + (p.exp_b ? *p.exp_b : 0);
             if (p.shift_out) *p.shift_out = s_out;
         }
+    }
+}
+
+// Forward layers: a cooperative launch, whose CTAs meet at a grid barrier behind their last tile, know the true shift and where the
+// guess was wrong contract and narrow again.  The conditional second launch of the kernel above cost a layer whose guess was right
+// 1 us in a graph and 2 to 4 in a stream, and without masks and side codes the epilogue needs no spills (us, before / after: 64 ->
+// 128 on 400 16x16 maps 17.9 / 15.6, 128 -> 128 at 32x32, 128 images 20.8 / 19.3 and stochastic 30.2 / 27.0, 500 8x8 maps of 512
+// channels 54.8 / 51.9).  The error's way back keeps the kernel above: with the ReLU mask in the epilogue a second pass in the same
+// kernel costs large layers up to 16 %, and a guess one shift too high is repaired from the side codes there.
+// One pass of a CTA over its tiles, all warps; AGAIN: the second one, whose shift is known.  (A pass number in a loop around the
+// body cost it 170 bytes of spills and up to 20 % of the time.)
+template <int BN, int MODE, bool AGAIN>
+__device__ __forceinline__ void requant_pass(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, uint8_t* smem, uint64_t* bars,
+                                             uint32_t* tmem_slot) {
+    using Cfg = RequantCfg<BN, false, MODE>;
+    using Split = EpiSplit<BN>;
+    constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC;
+    const uint32_t tmem_base = *tmem_slot;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    volatile int* again_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);
+    volatile int* shift_slot = reinterpret_cast<volatile int*>(tmem_slot + 3);
+    volatile unsigned* warp_max = reinterpret_cast<volatile unsigned*>(tmem_slot + 4);  // one word per epilogue warp
+    uint64_t* full_bar = bars;
+    uint64_t* empty_bar = bars + STAGES;
+    uint64_t* tfull_bar = bars + 2 * STAGES;
+    uint64_t* tempty_bar = bars + 2 * STAGES + NACC;
+    uint64_t* weights_bar = bars + 2 * STAGES + 2 * NACC;
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int total_tiles = p.m_tiles * p.n_tiles;
+    const int cta_first = static_cast<int>(blockIdx.x), cta_step = static_cast<int>(gridDim.x);
+
+    if (warp == 0) {
+        if constexpr (shares_rows(MODE)) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, false, false>(smem, full_bar, empty_bar, &tmA, &tmB, p, cta_first, cta_step, abort_flag);
+        __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
+    } else if (warp == 1) {
+        if constexpr (shares_rows(MODE)) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, tempty_bar, tmem_base, p, abort_flag);
+        else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, false, false>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, cta_first, cta_step, abort_flag);
+        __syncwarp();
+    } else {
+        const int grp = (warp - 2) >> 2;
+        const int q = warp & 3;  // TMEM lanes [32q, 32q+32) are the ones this warp may read
+        const int row_in_tile = q * 32 + lane;
+        const int cg = (grp % Split::GROUPS) * Split::COLS;
+        const int shift = AGAIN ? *shift_slot : p.state[0];
+        const unsigned long long seed = (p.mode == ROUND_STOCHASTIC && shift > 0) ? *p.seed : 0ull;
+        const bool wide = rows_of_32(p.out8, p.N);
+        int vmax[4] = {0, 0, 0, 0}, vmin[4] = {0, 0, 0, 0};
+        // this thread's row inside a tile never changes: pixel offsets within the tile's box
+        int row_w = 0, row_h = 0, row_n = 0;
+        bool row_in_box = true;
+        if (p.conv) {
+            const int t_ = row_in_tile / p.BW;
+            row_w = row_in_tile - t_ * p.BW; row_n = t_ / p.BH; row_h = t_ - row_n * p.BH;
+            row_in_box = row_in_tile < p.BW * p.BH * p.BI;
+        }
+        int it = grp / Split::GROUPS;
+        for (int tile = cta_first + it * cta_step; tile < total_tiles; tile += Split::TILES * cta_step, it += Split::TILES) {
+            const int acc = it & (NACC - 1); const uint32_t aph = (it / NACC) & 1u;
+            // where the tile lies, before waiting for its accumulator
+            int m_t, n_t;
+            tile_coords(p, tile, &m_t, &n_t);
+            bool valid; long long row;  // row of the output tensor (there may be more than 2^31)
+            if (p.conv) {
+                const int q1 = fdiv(m_t, p.fd_tw), tw = m_t - q1 * p.tiles_w, tn = fdiv(q1, p.fd_th), th = q1 - tn * p.tiles_h;
+                const int w = tw * p.BW + row_w, h = th * p.BH + row_h, n = tn * p.BI + row_n;
+                valid = row_in_box && w < p.W && h < p.H && n < p.Nimg;
+                row = (static_cast<long long>(n) * p.H + h) * p.W + w;
+            } else {
+                row = static_cast<long long>(m_t) * BLOCK_M + row_in_tile;
+                valid = row < p.M;
+            }
+            const int col0 = n_t * BN + cg;
+            const long long off = row * p.N + col0;  // of this thread's first output
+            const bool up = mbar_wait(smem_u32(&tfull_bar[acc]), aph, abort_flag);
+            if (!__all_sync(0xFFFFFFFFu, up)) { if (!up) report_abort(p.status, 4, 2); break; }
+            tc_fence_after();
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(acc * BN + cg);
+#pragma unroll 1
+            for (int c = 0; c < Split::CHUNKS; ++c) {
+                const int cols = p.N - col0 - 32 * c;  // columns of the tensor from here on
+                uint32_t v[32], packed[8];
+                tmem_ld_32x32(taddr + 32 * c, v);
+                tmem_ld_wait();
+                if (c == Split::CHUNKS - 1) {  // this warp's last columns sit in registers: hand the accumulator back
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[acc]));
+                }
+                if (cols <= 0) continue;
+                if (!AGAIN && valid) minmax32(v, cols, vmax, vmin);
+                narrow32(v, packed, shift, p.mode, p.relu, seed, p.rng_stream, p.rng_offset + static_cast<unsigned long long>(off) + 32 * c);
+                store_piece(valid ? p.out8 + off + 32 * c : nullptr, cols, packed, wide);
+            }
+        }
+        if (AGAIN) return;
+        const unsigned local_max = __reduce_max_sync(0xFFFFFFFFu, fold_minmax(vmax, vmin));
+        if (lane == 0) warp_max[warp - 2] = local_max;
+        int ticket = -1;
+        const int true_shift = parked_grid_shift(p, warp_max, shift_slot, abort_flag, &ticket);  // (releases the CTA's outputs too)
+        if (threadIdx.x == 64) {
+            *again_slot = true_shift >= 0 && true_shift != shift ? 1 : 0;
+            if (ticket == static_cast<int>(gridDim.x) - 1) {  // every CTA has read its guess and the barrier's words
+                int32_t* st = p.state;
+                const int s_out = true_shift < 0 ? 0 : true_shift;
+                const bool again = true_shift >= 0 && true_shift != shift;
+                if (again) { st[3] += 1; st[0] = true_shift; }
+                st[2] = again ? 1 : 0; st[1] = 0; st[4] = 0; st[5] = 0; st[6] = 0; st[7] = 0;  // ready for the next call
+                if (p.exp_out) *p.exp_out = s_out + (p.exp_a ? *p.exp_a : 0) + (p.exp_b ? *p.exp_b : 0);
+                if (p.shift_out) *p.shift_out = s_out;
+            }
+        }
+    }
+}
+
+// What a CTA keeps in shared memory behind the operand ring: the barriers of one pass, of a second, and a few words.
+template <int BN, int MODE>
+struct RequantShared {
+    static constexpr int BARS = 2 * RequantCfg<BN, false, MODE>::STAGES + 2 * RequantCfg<BN, false, MODE>::NACC + 3;  // stages full and free, accumulators, weights
+    uint8_t* smem; uint64_t* bars; uint32_t* tmem_slot;
+    __device__ __forceinline__ explicit RequantShared(uint8_t* raw) {
+        using Cfg = RequantCfg<BN, false, MODE>;
+        smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+        bars = reinterpret_cast<uint64_t*>(smem + Cfg::STAGES * Cfg::STAGE_BYTES + Cfg::RESIDENT_BYTES);
+        tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * BARS);
+    }
+    // The same addresses worked out anew behind a pass instead of kept through it: its epilogue has no register to spare.
+    static __device__ __forceinline__ RequantShared again(uint8_t* raw) {
+        int zero;
+        asm volatile("mov.u32 %0, 0;" : "=r"(zero));
+        return RequantShared(raw + zero);
+    }
+};
+
+template <int BN, int MODE>
+__global__ void __launch_bounds__(REQUANT_THREADS, 1)
+umma_requant_once_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+    using Cfg = RequantCfg<BN, false, MODE>;
+    constexpr int NACC = Cfg::NACC, BARS = RequantShared<BN, MODE>::BARS;
+    extern __shared__ uint8_t smem_raw[];
+    {
+        const RequantShared<BN, MODE> sh(smem_raw);
+        if (threadIdx.x == 0) {
+            for (int b = 0; b < 2; ++b)
+                for (int i = 0; i < BARS; ++i)  // the accumulators come back from the warps that share a tile
+                    mbar_init(smem_u32(&sh.bars[b * BARS + i]), i >= BARS - 3 - NACC && i < BARS - 3 ? 4 * EpiSplit<BN>::GROUPS : 1);
+            sh.tmem_slot[1] = 0;  // abort flag
+            sh.tmem_slot[2] = 0;  // a second pass
+            fence_barrier_init();
+            tma_prefetch_desc(&tmA);
+            tma_prefetch_desc(&tmB);
+        }
+        if (threadIdx.x >> 5 == 1) { tmem_alloc(smem_u32(sh.tmem_slot), NACC * BN); tmem_relinquish(); }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        requant_pass<BN, MODE, false>(tmA, tmB, p, sh.smem, sh.bars, sh.tmem_slot);
+    }
+    const auto sh = RequantShared<BN, MODE>::again(smem_raw);
+    tc_fence_before();
+    __syncthreads();
+    if (static_cast<volatile uint32_t*>(sh.tmem_slot)[2] != 0) {  // with barriers of its own: commits of the first pass may still be on their way to theirs
+        tc_fence_after();
+        requant_pass<BN, MODE, true>(tmA, tmB, p, sh.smem, sh.bars + BARS, sh.tmem_slot);
+        tc_fence_before();
+        __syncthreads();
+    }
+    if (threadIdx.x >> 5 == 1) {
+        const uint32_t tmem_base = *sh.tmem_slot;
+        if (static_cast<volatile uint32_t*>(sh.tmem_slot)[1]) __nanosleep(200000);  // let copies and MMAs already in flight land
+        tc_fence_after();
+        __syncwarp();
+        tmem_dealloc(tmem_base, NACC * BN);
     }
 }
 
@@ -2097,12 +2271,12 @@ int g_two_cta = 1;
 static bool pair_ok(int m_tiles, int bn, int b_mn, int conv) {
     return (g_two_cta & (conv ? 2 : 1)) && m_tiles >= 2 && (!b_mn || bn == 256);
 }
-// PARKED: the kernel with the grid barrier (cooperative launch: every CTA must be resident at the same time)
-template <int BN, bool TWO, int MODE, bool PARKED>
+// Kernels with a grid barrier are cooperative launches: every CTA must be resident at the same time
+template <int BN, bool TWO, int MODE, bool PARKED, bool ONE = false>
 static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
     using Cfg = RequantCfg<BN, TWO, MODE>;
     void (*kernel)(CUtensorMap, CUtensorMap, GemmParams);
-    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, MODE>; else kernel = umma_requant_kernel<BN, TWO, MODE>;
+    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, MODE>; else if constexpr (ONE) kernel = umma_requant_once_kernel<BN, MODE>; else kernel = umma_requant_kernel<BN, TWO, MODE>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     int tiles = p.m_tiles * p.n_tiles;
@@ -2111,7 +2285,7 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
     cfg.gridDim = dim3(TWO ? 2 * tiles : tiles); cfg.blockDim = dim3(REQUANT_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM_BYTES; cfg.stream = st;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (PARKED) { attr[n].id = cudaLaunchAttributeCooperative; attr[n].val.cooperative = g_cooperative; ++n; }
+    if (PARKED || ONE) { attr[n].id = cudaLaunchAttributeCooperative; attr[n].val.cooperative = g_cooperative; ++n; }
     if (TWO) {
         attr[n].id = cudaLaunchAttributeClusterDimension;
         attr[n].val.clusterDim.x = 2; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1; ++n;
@@ -2119,7 +2293,15 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
     cfg.attrs = attr; cfg.numAttrs = n;
     return set_cuda_error(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
 }
-static int launch_requant(int bn, bool pair, int mode, bool parked, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p,
+template <bool ONE>
+static int launch_streaming(int bn, int mode, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
+    if (mode == LOAD_HALO_RESIDENT)
+        return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO_RESIDENT, false, ONE>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO_RESIDENT, false, ONE>(a, b, p, st);
+    if (mode == LOAD_HALO) return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO, false, ONE>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO, false, ONE>(a, b, p, st);
+    if (bn == 64) return launch_requant_inst<64, false, LOAD_TAPS, false, ONE>(a, b, p, st);
+    return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, false, ONE>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, false, ONE>(a, b, p, st);
+}
+static int launch_requant(int bn, bool pair, int mode, bool parked, bool one, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p,
                           cudaStream_t st) {
     if (parked) {
         if (pair) return bn == 256 ? launch_requant_inst<256, true, LOAD_TAPS, true>(a, b, p, st) : launch_requant_inst<128, true, LOAD_TAPS, true>(a, b, p, st);
@@ -2127,16 +2309,13 @@ static int launch_requant(int bn, bool pair, int mode, bool parked, const CUtens
         if (mode == LOAD_HALO) return launch_requant_inst<128, false, LOAD_HALO, true>(a, b, p, st);
         return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, true>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, true>(a, b, p, st);
     }
+    if (one) return launch_streaming<true>(bn, mode, a, b, p, st);
     if (pair) return bn == 256 ? launch_requant_inst<256, true, LOAD_TAPS, false>(a, b, p, st) : launch_requant_inst<128, true, LOAD_TAPS, false>(a, b, p, st);
-    if (mode == LOAD_HALO_RESIDENT)
-        return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO_RESIDENT, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO_RESIDENT, false>(a, b, p, st);
-    if (mode == LOAD_HALO) return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO, false>(a, b, p, st);
     if (mode == LOAD_ROWS32)
         return bn == 64    ? launch_requant_inst<64, false, LOAD_ROWS32, false>(a, b, p, st)
                : bn == 256 ? launch_requant_inst<256, false, LOAD_ROWS32, false>(a, b, p, st)
                            : launch_requant_inst<128, false, LOAD_ROWS32, false>(a, b, p, st);
-    if (bn == 64) return launch_requant_inst<64, false, LOAD_TAPS, false>(a, b, p, st);
-    return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, false>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, false>(a, b, p, st);
+    return launch_streaming<false>(bn, mode, a, b, p, st);
 }
 template <int CS>
 static cudaLaunchConfig_t split_config(int tiles, cudaLaunchAttribute* attr, cudaStream_t st) {
@@ -2336,7 +2515,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.group_m = (static_cast<long long>(M) + N) * K > (48ll << 20) ? 8 : 0;
     set_fused(&p, fused);
     finish_params(&p);
-    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, rows32 ? LOAD_ROWS32 : LOAD_TAPS, false, ma, mb, p, st); }
+    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, rows32 ? LOAD_ROWS32 : LOAD_TAPS, false, false, ma, mb, p, st); }
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
@@ -2411,7 +2590,7 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
     if (split == 4) return launch_split<4>(ma, mb, p, st);
     if (split == 2) return launch_split<2>(ma, mb, p, st);
     const int mode = !plan.halo ? LOAD_TAPS : p.cblocks == 1 && p.n_tiles == 1 ? LOAD_HALO_RESIDENT : LOAD_HALO;
-    if (fused) return launch_requant(bn, pair, mode, parked, ma, mb, p, st);
+    if (fused) return launch_requant(bn, pair, mode, parked, fused->one && !pair, ma, mb, p, st);
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
