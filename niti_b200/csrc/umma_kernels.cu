@@ -984,7 +984,9 @@ struct RequantCfg {
 };
 
 // Streaming kernel: narrows with the shift in state[0]; the last CTA derives the true one from max|acc|.
-template <int BN, bool TWO, int MODE>
+// CODES: with the side codes, where the call has room for them.  Without them the registers suffice (128 -> 128 at 32x32, 128 images,
+// stochastic: 33.3 -> 32.1 us, at 80 images 28.2 -> 26.5); 64-column tiles are 3 % slower like that and keep them.
+template <int BN, bool TWO, int MODE, bool CODES>
 __global__ void __launch_bounds__(REQUANT_THREADS, 1)
 umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
     using Cfg = RequantCfg<BN, TWO, MODE>;
@@ -993,7 +995,7 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (p.only_if_redo) {
         const int verdict = p.state[2] & 3;
         if (verdict == 0) return;  // the prediction was right: nothing to redo
-        if (verdict == 2) {        // one bit too many was shifted out and the side codes hold what is missing
+        if (CODES && verdict == 2) {  // one bit too many was shifted out and the side codes hold what is missing
             requant_step_down(p.out8, p.side, p.mask, static_cast<long long>(p.M) * p.N / 16);
             return;
         }
@@ -1056,8 +1058,8 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const int shift = p.state[0];
         const unsigned long long seed = (p.mode == ROUND_STOCHASTIC && shift > 0) ? *p.seed : 0ull;
         // a first launch also keeps what the next lower shift would need (see narrow16_nearest_codes)
-        const bool with_codes = p.mode == ROUND_NEAREST && shift >= 2 && !p.relu && p.side != nullptr && !p.only_if_redo;
-        const int half = shift > 0 ? 1 << (shift - 1) : 0;
+        const bool with_codes = CODES && p.mode == ROUND_NEAREST && shift >= 2 && !p.relu && p.side != nullptr && !p.only_if_redo;
+        const int half = CODES && shift > 0 ? 1 << (shift - 1) : 0;
         const bool wide = rows_of_32(p.out8, p.N);
         int vmax[4] = {0, 0, 0, 0}, vmin[4] = {0, 0, 0, 0};
         // this thread's row inside a tile never changes: pixel offsets within the tile's box
@@ -1154,7 +1156,7 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 int verdict = 0;
                 if (true_shift == pred) {
                     run = 0;
-                } else if (p.side != nullptr && p.mode == ROUND_NEAREST && !p.relu && pred >= 2 && true_shift == pred - 1) {
+                } else if (CODES && p.side != nullptr && p.mode == ROUND_NEAREST && !p.relu && pred >= 2 && true_shift == pred - 1) {
                     // the prediction stays: a layer whose maximum hovers around a power of two keeps the upper
                     // shift as its guess and pays the cheap pass when the lower one applies; after
                     // STEP_DOWN_RUN lower ones in a row the guess follows
@@ -2272,11 +2274,11 @@ static bool pair_ok(int m_tiles, int bn, int b_mn, int conv) {
     return (g_two_cta & (conv ? 2 : 1)) && m_tiles >= 2 && (!b_mn || bn == 256);
 }
 // Kernels with a grid barrier are cooperative launches: every CTA must be resident at the same time
-template <int BN, bool TWO, int MODE, bool PARKED, bool ONE = false>
+template <int BN, bool TWO, int MODE, bool PARKED, bool ONE = false, bool CODES = false>
 static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
     using Cfg = RequantCfg<BN, TWO, MODE>;
     void (*kernel)(CUtensorMap, CUtensorMap, GemmParams);
-    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, MODE>; else if constexpr (ONE) kernel = umma_requant_once_kernel<BN, MODE>; else kernel = umma_requant_kernel<BN, TWO, MODE>;
+    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, MODE>; else if constexpr (ONE) kernel = umma_requant_once_kernel<BN, MODE>; else kernel = umma_requant_kernel<BN, TWO, MODE, CODES>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     int tiles = p.m_tiles * p.n_tiles;
@@ -2293,13 +2295,13 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
     cfg.attrs = attr; cfg.numAttrs = n;
     return set_cuda_error(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
 }
-template <bool ONE>
+template <bool ONE, bool CODES>
 static int launch_streaming(int bn, int mode, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
     if (mode == LOAD_HALO_RESIDENT)
-        return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO_RESIDENT, false, ONE>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO_RESIDENT, false, ONE>(a, b, p, st);
-    if (mode == LOAD_HALO) return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO, false, ONE>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO, false, ONE>(a, b, p, st);
-    if (bn == 64) return launch_requant_inst<64, false, LOAD_TAPS, false, ONE>(a, b, p, st);
-    return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, false, ONE>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, false, ONE>(a, b, p, st);
+        return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO_RESIDENT, false, ONE, CODES>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO_RESIDENT, false, ONE, CODES>(a, b, p, st);
+    if (mode == LOAD_HALO) return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO, false, ONE, CODES>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO, false, ONE, CODES>(a, b, p, st);
+    if (bn == 64) return launch_requant_inst<64, false, LOAD_TAPS, false, ONE, CODES>(a, b, p, st);
+    return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, false, ONE, CODES>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, false, ONE, CODES>(a, b, p, st);
 }
 static int launch_requant(int bn, bool pair, int mode, bool parked, bool one, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p,
                           cudaStream_t st) {
@@ -2309,13 +2311,14 @@ static int launch_requant(int bn, bool pair, int mode, bool parked, bool one, co
         if (mode == LOAD_HALO) return launch_requant_inst<128, false, LOAD_HALO, true>(a, b, p, st);
         return bn == 256 ? launch_requant_inst<256, false, LOAD_TAPS, true>(a, b, p, st) : launch_requant_inst<128, false, LOAD_TAPS, true>(a, b, p, st);
     }
-    if (one) return launch_streaming<true>(bn, mode, a, b, p, st);
-    if (pair) return bn == 256 ? launch_requant_inst<256, true, LOAD_TAPS, false>(a, b, p, st) : launch_requant_inst<128, true, LOAD_TAPS, false>(a, b, p, st);
+    if (one) return launch_streaming<true, false>(bn, mode, a, b, p, st);
+    if (pair) return bn == 256 ? launch_requant_inst<256, true, LOAD_TAPS, false, false, true>(a, b, p, st) : launch_requant_inst<128, true, LOAD_TAPS, false, false, true>(a, b, p, st);
     if (mode == LOAD_ROWS32)
         return bn == 64    ? launch_requant_inst<64, false, LOAD_ROWS32, false>(a, b, p, st)
                : bn == 256 ? launch_requant_inst<256, false, LOAD_ROWS32, false>(a, b, p, st)
                            : launch_requant_inst<128, false, LOAD_ROWS32, false>(a, b, p, st);
-    return launch_streaming<false>(bn, mode, a, b, p, st);
+    return bn == 64 || (p.side != nullptr && p.mode == NITI_ROUND_NEAREST && !p.relu) ? launch_streaming<false, true>(bn, mode, a, b, p, st)
+                                                                         : launch_streaming<false, false>(bn, mode, a, b, p, st);
 }
 template <int CS>
 static cudaLaunchConfig_t split_config(int tiles, cudaLaunchAttribute* attr, cudaStream_t st) {
