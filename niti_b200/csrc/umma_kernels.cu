@@ -1556,7 +1556,7 @@ umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             for (int it = 0; it < my_tiles; ++it) {
                 const int tile = cta_first + it * cta_step, col0 = (tile - fdiv(tile, p.fd_n) * p.n_tiles) * BN + cg;
                 const int row = out_row[it * 128 + row_in_tile], prow = pool_row[it * 128 + row_in_tile];
-                const long long off = static_cast<long long>(row) * p.N + col0;
+                const long long off = static_cast<long long>(max(row, 0)) * p.N + col0;  // rows outside the tensor go through the same form as the others
                 const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(it * BN + cg);
 #pragma unroll 1
                 for (int c = 0; c < Split::CHUNKS; ++c) {
