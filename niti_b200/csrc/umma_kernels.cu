@@ -2232,6 +2232,20 @@ static int encode_map(CUtensorMap* map, const void* ptr, bool int32_elems, int r
     return 0;
 }
 
+// The dynamic shared memory of a kernel, granted once per device: asked for at every launch it was about a microsecond of the host's
+// time, and a single image's layers are bound by that.
+template <auto KERNEL>
+static cudaError_t allow_shared(int bytes) {
+    static std::atomic<unsigned long long> done{0};  // one bit per device
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+
 static int sm_count() {
     static int n = 0;
     if (n == 0) {
@@ -2247,7 +2261,7 @@ static int sm_count() {
 template <int BN, bool TWO, bool ROWS32 = false>
 static int launch_gemm_inst(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p, cudaStream_t st) {
     using Cfg = GemmCfg<BN, TWO>;
-    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN, TWO, ROWS32>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+    cudaError_t e = allow_shared<umma_gemm_kernel<BN, TWO, ROWS32>>(Cfg::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     int tiles = p.m_tiles * p.n_tiles * p.splits;
     if (tiles > sm_count() / (TWO ? 2 : 1)) tiles = sm_count() / (TWO ? 2 : 1);
@@ -2278,8 +2292,10 @@ template <int BN, bool TWO, int MODE, bool PARKED, bool ONE = false, bool CODES 
 static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
     using Cfg = RequantCfg<BN, TWO, MODE>;
     void (*kernel)(CUtensorMap, CUtensorMap, GemmParams);
-    if constexpr (PARKED) kernel = umma_parked_kernel<BN, TWO, MODE>; else if constexpr (ONE) kernel = umma_requant_once_kernel<BN, MODE>; else kernel = umma_requant_kernel<BN, TWO, MODE, CODES>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+    cudaError_t e;
+    if constexpr (PARKED) { kernel = umma_parked_kernel<BN, TWO, MODE>; e = allow_shared<umma_parked_kernel<BN, TWO, MODE>>(Cfg::SMEM_BYTES); }
+    else if constexpr (ONE) { kernel = umma_requant_once_kernel<BN, MODE>; e = allow_shared<umma_requant_once_kernel<BN, MODE>>(Cfg::SMEM_BYTES); }
+    else { kernel = umma_requant_kernel<BN, TWO, MODE, CODES>; e = allow_shared<umma_requant_kernel<BN, TWO, MODE, CODES>>(Cfg::SMEM_BYTES); }
     if (e != cudaSuccess) return set_cuda_error(e);
     int tiles = p.m_tiles * p.n_tiles;
     if (tiles > sm_count() / (TWO ? 2 : 1)) tiles = sm_count() / (TWO ? 2 : 1);
@@ -2332,7 +2348,7 @@ static cudaLaunchConfig_t split_config(int tiles, cudaLaunchAttribute* attr, cud
 }
 template <int CS>
 static int launch_split(const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(umma_split_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<CS>::SMEM_BYTES);
+    cudaError_t e = allow_shared<umma_split_kernel<CS>>(SplitCfg<CS>::SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t cfg = split_config<CS>(p.m_tiles * p.n_tiles, attr, st);
@@ -2348,7 +2364,7 @@ static int split_clusters() {
         cudaLaunchAttribute attr[2];
         cudaLaunchConfig_t cfg = split_config<CS>(1, attr, nullptr);
         cfg.numAttrs = 1;
-        if (cudaFuncSetAttribute(umma_split_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<CS>::SMEM_BYTES) != cudaSuccess ||
+        if (allow_shared<umma_split_kernel<CS>>(SplitCfg<CS>::SMEM_BYTES) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, umma_split_kernel<CS>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
         known.store(n, std::memory_order_relaxed);
     }
@@ -2663,7 +2679,7 @@ int umma_conv_wgrad_partials(const int8_t* x, const int8_t* err, int32_t* partia
     CUtensorMap me, mx, mp;
     if (int e = wgrad_setup(x, err, partial, direct, Nimg, H, W, C, K, R, S, pad, status, &p, &me, &mx, &mp)) return e;
     *splits_out = p.splits;
-    cudaError_t e = cudaFuncSetAttribute(umma_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM_BYTES);
+    cudaError_t e = allow_shared<umma_wgrad_kernel>(WG_SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     dim3 grid(p.splits, R * p.k_tiles * p.c_tiles);
     umma_wgrad_kernel<<<grid, UMMA_THREADS, WG_SMEM_BYTES, st>>>(me, mx, mp, p);
@@ -2687,7 +2703,7 @@ int umma_conv_wgrad_update(const int8_t* x, const int8_t* err, int32_t* out, int
     const long long n = static_cast<long long>(K) * R * S * C;
     *updated = n <= WG_UPDATE_MAX;
     const WgradUpdate u{out, *updated ? w : nullptr, words, words, num_words, n, mu, mode, seed, rng_stream, state};
-    cudaError_t e = cudaFuncSetAttribute(umma_wgrad_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM_BYTES);
+    cudaError_t e = allow_shared<umma_wgrad_update_kernel>(WG_SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(p.splits, R * p.k_tiles * p.c_tiles); cfg.blockDim = dim3(UMMA_THREADS); cfg.dynamicSmemBytes = WG_SMEM_BYTES; cfg.stream = st;
@@ -2725,7 +2741,7 @@ int umma_conv_wgrad_batch_inner(const int8_t* x_t, const int8_t* err_t, int32_t*
     const uint64_t sc[3] = {(uint64_t)K * 4, (uint64_t)R * S * K * 4, (uint64_t)C * R * S * K * 4};
     const uint32_t bc[4] = {32, 1, 128, 1};
     if (int e = encode_map(&mc, out, true, 4, dc, sc, bc)) return e;
-    cudaError_t e = cudaFuncSetAttribute(umma_wgrad_kmajor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM_BYTES);
+    cudaError_t e = allow_shared<umma_wgrad_kmajor_kernel>(WG_SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     umma_wgrad_kmajor_kernel<<<dim3(p.splits, R * p.k_tiles * p.c_tiles), UMMA_THREADS, WG_SMEM_BYTES, st>>>(ma, mb, mc, p);
     return set_cuda_error(cudaGetLastError());
@@ -2822,7 +2838,7 @@ int umma_conv_wgrad_multi(const WgradJob* jobs, int count, int32_t* status, cuda
     }
     mp.first_cta[count] = grid;
     mp.count = count;
-    cudaError_t e = cudaFuncSetAttribute(umma_wgrad_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM_BYTES);
+    cudaError_t e = allow_shared<umma_wgrad_multi_kernel>(WG_SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     umma_wgrad_multi_kernel<<<grid, UMMA_THREADS, WG_SMEM_BYTES, st>>>(maps, mp);
     return set_cuda_error(cudaGetLastError());

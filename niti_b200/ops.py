@@ -168,7 +168,8 @@ def conv_fprop_fused(x, w, state, pad=1, mode=ROUND_NEAREST, seed=None, rng_stre
     then survives in its first N*H*W*32 bytes for conv_wgrad_from_patches."""
     def work(r):
         return 2 * r[0].numel() * w[0].numel(), x.numel() + w.numel() + r[0].numel()
-    # contraction and conditional second launch; a thin layer gathers its patches first
+    # at most: contraction and conditional second launch (one launch where the kernel narrows again itself); a thin layer gathers
+    # its patches first
     return _run("niti_conv_fprop_requant_i8", 3 if w.numel() <= 32 * w.size(0) else 2, work, native.conv_fprop_fused, x, w, state, pad,
                 mode, seed, rng_stream, rng_offset, relu, exp_a, exp_b, scratch_buf)
 

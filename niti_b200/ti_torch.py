@@ -362,6 +362,8 @@ class TiConv2d(UpdateWeight):
     """3x3 (or RxR) convolution, stride 1, NHWC (:379-437).  ``fuse_relu`` applies the following
     TiReLU inside the requantisation kernel (pair it with ``TiReLU(fused=True)``)."""
 
+    _update_state = None  # words of the gradient-and-update launch (layers pickled without them get theirs too)
+
     def __init__(self, in_channels, out_channels, kernel_size=3, stride=1, padding=1, first_layer=False, fuse_relu=False):
         super(TiConv2d, self).__init__()
         self.weight, self.weight_exp = WEIGHT_INIT_METHOD(torch.Size([out_channels, kernel_size, kernel_size, in_channels]))
@@ -380,29 +382,30 @@ class TiConv2d(UpdateWeight):
         self._bwd_state = None
         self._bwd_side, self._bwd_side_shape = None, None
         self._patches, self._patches_of = None, None
-        self._update_state = None  # words of the gradient-and-update launch
 
     def _new_states(self, dev):
-        """The device words of this layer's launches that are not there yet, from one allocation."""
-        words = torch.zeros(20, dtype=torch.int32, device=dev)
-        for name, part in (('_fwd_state', words[:8]), ('_bwd_state', words[8:16]), ('_update_state', words[16:])):
-            if self.__dict__[name] is None:
-                self.__dict__[name] = part
+        """The device words of the backward's launches that are not there yet, from one allocation."""
+        words = torch.zeros(12, dtype=torch.int32, device=dev)
+        if self._bwd_state is None:
+            self._bwd_state = words[:8]
+        if self._update_state is None:
+            self._update_state = words[8:]
 
     def forward(self, input):
         act, exp_in = input
         self.__dict__.update(act=act, act_in_exp=exp_in)
         K, R, S, C = self.weight.shape
-        offset = SAMPLE_OFFSET * act.shape[1] * act.shape[2] * K
+        shape = act.shape
+        offset = SAMPLE_OFFSET * shape[1] * shape[2] * K if SAMPLE_OFFSET else 0
         if FUSE_REQUANT and GLOBAL_MAX_GROUP is None and self.stride == 1 and ops.conv_fprop_fused_supported(C, K, R, S, self.padding):
             # conv2d_int8 + act_calc (:393-395) in one kernel; see ops.conv_fprop_fused
             dev = act.device
             if self._fwd_state is None:
-                self._new_states(dev)
+                self._fwd_state = ops.new_requant_state(dev)
             mode, seed, stream, exp_in = _mode(ACT_ROUND_METHOD), RNG_SEED(dev), 16 * self.layer_id, exp_tensor(exp_in, dev)
             pool = self.pool_layer
             if (pool is not None and FUSE_POOL and self.fuse_relu and pool.kernel_size == 2 and pool.stride == 2
-                    and ops.conv_fprop_pool_fused_supported(*act.shape, K, R, S, self.padding)):
+                    and ops.conv_fprop_pool_fused_supported(*shape, K, R, S, self.padding)):
                 # conv2d_int8 + act_calc + ReLU (:393-395, :268-277) and the pool's forward (:302-307) in one kernel
                 out, pooled, exp_out, _ = ops.conv_fprop_pool_fused(act, self.weight, self._fwd_state, self.padding, mode, seed,
                                                                     stream, offset, True, exp_in, self.weight_exp)
@@ -412,7 +415,7 @@ class TiConv2d(UpdateWeight):
             if TRAINING and KEEP_PATCHES and self.first_layer:
                 # a thin layer runs as a GEMM over a patch matrix; kept in memory of its own it also serves the weight
                 # gradient of this step (the reference gathers its first-layer operands twice, :412-428)
-                nbytes = ops.conv_fprop_scratch_bytes(*act.shape, K, R, S)
+                nbytes = ops.conv_fprop_scratch_bytes(*shape, K, R, S)
                 if nbytes:
                     patches = self._patches
                     if patches is None or patches.numel() < nbytes or patches.device != dev:
