@@ -1255,7 +1255,7 @@ __device__ __forceinline__ void parked_leave(const GemmParams& p, int shift, int
 // guess was wrong contract and narrow again.  The conditional second launch of the kernel above cost a layer whose guess was right
 // 1 us in a graph and 2 to 4 in a stream, and without masks and side codes the epilogue needs no spills (us, before / after: 64 ->
 // 128 on 400 16x16 maps 17.9 / 15.6, 128 -> 128 at 32x32, 128 images 20.8 / 19.3 and stochastic 30.2 / 27.0, 500 8x8 maps of 512
-// channels 54.8 / 51.9).  The error's way back keeps the kernel above: with the ReLU mask in the epilogue a second pass in the same
+// channels 54.8 / 51.9; the first layer's product the same way: evaluation of 500 images 397 / 392).  The error's way back keeps the kernel above: with the ReLU mask in the epilogue a second pass in the same
 // kernel costs large layers up to 16 %, and a guess one shift too high is repaired from the side codes there.
 // One pass of a CTA over its tiles, all warps; AGAIN: the second one, whose shift is known.  (A pass number in a loop around the
 // body cost it 170 bytes of spills and up to 20 % of the time.)
@@ -1282,11 +1282,11 @@ __device__ __forceinline__ void requant_pass(const CUtensorMap& tmA, const CUten
 
     if (warp == 0) {
         if constexpr (shares_rows(MODE)) producer_halo_role<BN, STAGES, Cfg::STAGE_BYTES, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), &tmA, &tmB, p, abort_flag);
-        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, false, false>(smem, full_bar, empty_bar, &tmA, &tmB, p, cta_first, cta_step, abort_flag);
+        else producer_role<BN, STAGES, Cfg::STAGE_BYTES, false, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, &tmA, &tmB, p, cta_first, cta_step, abort_flag);
         __syncwarp();  // reach the teardown's block-wide barrier as a converged warp
     } else if (warp == 1) {
         if constexpr (shares_rows(MODE)) mma_halo_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, MODE == LOAD_HALO_RESIDENT>(smem, full_bar, empty_bar, smem_u32(weights_bar), tfull_bar, tempty_bar, tmem_base, p, abort_flag);
-        else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, false, false>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, cta_first, cta_step, abort_flag);
+        else mma_role<BN, STAGES, Cfg::STAGE_BYTES, NACC, false, MODE == LOAD_ROWS32>(smem, full_bar, empty_bar, tfull_bar, tempty_bar, tmem_base, p, cta_first, cta_step, abort_flag);
         __syncwarp();
     } else {
         const int grp = (warp - 2) >> 2;
@@ -2313,6 +2313,11 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
 }
 template <bool ONE, bool CODES>
 static int launch_streaming(int bn, int mode, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
+    if constexpr (!CODES)
+        if (mode == LOAD_ROWS32)
+            return bn == 64    ? launch_requant_inst<64, false, LOAD_ROWS32, false, ONE>(a, b, p, st)
+                   : bn == 256 ? launch_requant_inst<256, false, LOAD_ROWS32, false, ONE>(a, b, p, st)
+                               : launch_requant_inst<128, false, LOAD_ROWS32, false, ONE>(a, b, p, st);
     if (mode == LOAD_HALO_RESIDENT)
         return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO_RESIDENT, false, ONE, CODES>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO_RESIDENT, false, ONE, CODES>(a, b, p, st);
     if (mode == LOAD_HALO) return bn == 64 ? launch_requant_inst<64, false, LOAD_HALO, false, ONE, CODES>(a, b, p, st) : launch_requant_inst<128, false, LOAD_HALO, false, ONE, CODES>(a, b, p, st);
@@ -2329,10 +2334,7 @@ static int launch_requant(int bn, bool pair, int mode, bool parked, bool one, co
     }
     if (one) return launch_streaming<true, false>(bn, mode, a, b, p, st);
     if (pair) return bn == 256 ? launch_requant_inst<256, true, LOAD_TAPS, false, false, true>(a, b, p, st) : launch_requant_inst<128, true, LOAD_TAPS, false, false, true>(a, b, p, st);
-    if (mode == LOAD_ROWS32)
-        return bn == 64    ? launch_requant_inst<64, false, LOAD_ROWS32, false>(a, b, p, st)
-               : bn == 256 ? launch_requant_inst<256, false, LOAD_ROWS32, false>(a, b, p, st)
-                           : launch_requant_inst<128, false, LOAD_ROWS32, false>(a, b, p, st);
+    if (mode == LOAD_ROWS32) return launch_streaming<false, false>(bn, mode, a, b, p, st);
     return bn == 64 || (p.side != nullptr && p.mode == NITI_ROUND_NEAREST && !p.relu) ? launch_streaming<false, true>(bn, mode, a, b, p, st)
                                                                          : launch_streaming<false, false>(bn, mode, a, b, p, st);
 }
@@ -2534,7 +2536,7 @@ int umma_gemm(const int8_t* A, const int8_t* B, void* out, unsigned* maxabs, int
     p.group_m = (static_cast<long long>(M) + N) * K > (48ll << 20) ? 8 : 0;
     set_fused(&p, fused);
     finish_params(&p);
-    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, rows32 ? LOAD_ROWS32 : LOAD_TAPS, false, false, ma, mb, p, st); }
+    if (fused) { p.out8 = static_cast<int8_t*>(out); return launch_requant(bn, false, rows32 ? LOAD_ROWS32 : LOAD_TAPS, false, fused->one, ma, mb, p, st); }
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
 }
 
