@@ -620,6 +620,21 @@ PyObject* quantize_input(Args& a) {
     return tuple(x8, e.first);
 }
 
+// A step's results into pinned host tensors, on the device and the stream of `out`: a replayed step runs there whatever device is
+// current, and the event behind the launch is recorded there.
+PyObject* publish_step(Args& a) {
+    const Tensor &out = a.tensor(), &exp = a.tensor(), &status = a.tensor(), &host_out = a.tensor(), &host_exp = a.tensor(), &host_status = a.tensor();
+    need_cuda({&out, &exp, &status});
+    require(out.scalar_type() == at::kChar && exp.scalar_type() == at::kInt && exp.numel() == 1 && out.device() == exp.device() && out.device() == status.device());
+    require(host_out.is_contiguous() && host_out.scalar_type() == at::kChar && host_out.sizes() == out.sizes());
+    {
+        Launch l(out);
+        check(niti_publish_step(cptr<int8_t>(out), out.numel(), cptr<int32_t>(exp), cptr<int32_t>(status), mptr<int8_t>(host_out),
+                                mptr<int32_t>(host_exp), mptr<int32_t>(host_status), l.stream), "niti_publish_step");
+    }
+    Py_RETURN_NONE;
+}
+
 #define NITI_ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<&name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     NITI_ENTRY(set_error_type), NITI_ENTRY(status_word), NITI_ENTRY(conv_fprop_fused_supported),
@@ -630,7 +645,7 @@ PyMethodDef methods[] = {
     NITI_ENTRY(conv_wgrad_batch_inner_supported), NITI_ENTRY(conv_wgrad_batch_inner), NITI_ENTRY(maxpool_bwd_f16),
     NITI_ENTRY(conv_wgrad_from_patches), NITI_ENTRY(conv_wgrad_update), NITI_ENTRY(conv_wgrad_accumulate), NITI_ENTRY(gemm_acc), NITI_ENTRY(requant),
     NITI_ENTRY(absmax), NITI_ENTRY(maxpool_fwd), NITI_ENTRY(maxpool_bwd), NITI_ENTRY(relu_fwd), NITI_ENTRY(relu_bwd),
-    NITI_ENTRY(dropout), NITI_ENTRY(loss_err), NITI_ENTRY(update), NITI_ENTRY(quantize_input),
+    NITI_ENTRY(dropout), NITI_ENTRY(loss_err), NITI_ENTRY(update), NITI_ENTRY(quantize_input), NITI_ENTRY(publish_step),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_torch_ops", "native torch front end of libniti_b200 (" NITI_OPS_TAG ")", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -464,13 +464,11 @@ def peer_copy(dst_ptr, src_ptr, nbytes):
 
 
 def publish_step(out, exp, status, host_out, host_exp, host_status):
-    """A step's int8 logits, exponent and status word into pinned host tensors by one kernel (valid once the current stream has
-    passed it)."""
-    _need_cuda(out, exp, status)
-    assert out.dtype == torch.int8 and exp.dtype == torch.int32 and out.shape == host_out.shape and exp.numel() == 1
-    assert host_out.is_contiguous() and host_out.dtype == torch.int8
-    _call("niti_publish_step", 1, 0, out.numel() + 20, lib.niti_publish_step, _p(out), out.numel(), _p(exp), _p(status), _p(host_out),
-          _p(host_exp), _p(host_status), _st())
+    """A step's int8 logits, exponent and status word into pinned host tensors by one kernel on the current stream of their
+    device (valid once that stream has passed it)."""
+    def work(r):
+        return 0, out.numel() + 20
+    _run("niti_publish_step", 1, work, native.publish_step, out, exp, status, host_out, host_exp, host_status)
 
 
 def quantize_input(x, reduce_max=None):

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 if not torch.cuda.is_available():
     pytest.skip("needs a CUDA device", allow_module_level=True)
 
-from niti_b200 import ti_torch, ti_vgg  # noqa: E402
+from niti_b200 import ops, ti_torch, ti_vgg  # noqa: E402
 from niti_b200.trainer import Trainer  # noqa: E402
 
 DEV = "cuda:0"
@@ -308,3 +308,40 @@ def test_a_reported_wait_expiry_is_sticky():
         tr.step(xh, th).wait()
     finally:
         ops.status_word(DEV).zero_()
+
+
+def pinned_results(n):
+    return (torch.zeros(n, dtype=torch.int8).pin_memory(), torch.zeros((), dtype=torch.int32).pin_memory(),
+            torch.zeros(4, dtype=torch.int32).pin_memory())
+
+
+@pytest.mark.parametrize("n,offset,host_offset", [(1280, 0, 0), (30, 0, 0), (770, 3, 0), (770, 0, 5), (1, 0, 0)])
+def test_results_go_out_on_the_device_and_stream_of_their_tensors(n, offset, host_offset, monkeypatch):
+    """Not on the current device's: a captured trainer's step runs on its own device whatever device is current.  (Here the
+    current device's stream may simply not be asked for; with two GPUs see the test below.)  Logits and host buffers may start
+    at any byte."""
+    def no_current_device():
+        raise AssertionError("the current device's stream")
+    rng = np.random.default_rng(n + offset)
+    out = torch.from_numpy(rng.integers(-127, 128, n + offset).astype(np.int8)).to(DEV)[offset:]
+    exp, status = torch.tensor([-7], dtype=torch.int32, device=DEV), torch.tensor([0, 5, -6, 7], dtype=torch.int32, device=DEV)
+    host, host_exp, host_status = pinned_results(n + host_offset)
+    side = torch.cuda.Stream(device=DEV)
+    side.wait_stream(torch.cuda.current_stream())
+    monkeypatch.setattr(ops, "_st", no_current_device)
+    with torch.cuda.stream(side):
+        ops.publish_step(out, exp, status, host[host_offset:], host_exp, host_status)
+    side.synchronize()
+    assert torch.equal(host[host_offset:], out.cpu()) and not bool(host[:host_offset].any())
+    assert int(host_exp) == -7 and host_status.tolist() == [0, 5, -6, 7]
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_results_of_a_device_that_is_not_current():
+    host, host_exp, host_status = pinned_results(1000)
+    out = torch.randint(-127, 128, (1000,), dtype=torch.int8, device="cuda:1")
+    exp, status = torch.tensor([4], dtype=torch.int32, device="cuda:1"), torch.arange(4, dtype=torch.int32, device="cuda:1")
+    with torch.cuda.device(0):
+        ops.publish_step(out, exp, status, host, host_exp, host_status)
+        torch.cuda.synchronize("cuda:1")
+    assert torch.equal(host, out.cpu()) and int(host_exp) == 4 and host_status.tolist() == [0, 1, 2, 3]
