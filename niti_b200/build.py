@@ -76,7 +76,7 @@ def build_ops(force=False):
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     incs = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
             sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
-    subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+    subprocess.run(["g++", "-O2", "-std=c++17", "-Wno-interference-size", "-fPIC", "-shared", "-fvisibility=hidden",
                     f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DNITI_OPS_TAG="{ops_tag()}"', *["-I" + d for d in incs], src, "-o", OPS,
                     "-L" + PKG, "-l:libniti_b200.so", "-L" + os.path.join(base, "lib"), "-lc10", "-ltorch_cpu", "-ltorch_python",
                     "-lc10_cuda", "-ltorch_cuda", "-Wl,-rpath,$ORIGIN"], check=True)

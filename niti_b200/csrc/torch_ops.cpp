@@ -11,6 +11,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/ATen.h>
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -631,6 +632,12 @@ PyObject* publish_step(Args& a) {
         Launch l(out);
         check(niti_publish_step(cptr<int8_t>(out), out.numel(), cptr<int32_t>(exp), cptr<int32_t>(status), mptr<int8_t>(host_out),
                                 mptr<int32_t>(host_exp), mptr<int32_t>(host_status), l.stream), "niti_publish_step");
+        // as a copy does: whoever drops a host tensor before the kernel has run does not free memory that is still to be written
+        const c10::Stream used = c10::cuda::getCurrentCUDAStream(l.dev.index()).unwrap();
+        for (const Tensor* t : {&host_out, &host_exp, &host_status}) {
+            const c10::DataPtr& p = t->storage().data_ptr();
+            at::getHostAllocator(at::kCUDA)->record_event(p.get(), p.get_context(), used);
+        }
     }
     Py_RETURN_NONE;
 }

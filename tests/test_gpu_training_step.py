@@ -345,3 +345,20 @@ def test_results_of_a_device_that_is_not_current():
         ops.publish_step(out, exp, status, host, host_exp, host_status)
         torch.cuda.synchronize("cuda:1")
     assert torch.equal(host, out.cpu()) and int(host_exp) == 4 and host_status.tolist() == [0, 1, 2, 3]
+
+
+def test_a_result_dropped_before_its_kernel_has_run_keeps_its_memory():
+    """The pinned buffers go back to the host allocator only when the publishing kernel is through, as behind a copy."""
+    n = 3 << 20
+    out = torch.full((n,), 5, dtype=torch.int8, device=DEV)
+    exp, status = torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+    host, host_exp, host_status = pinned_results(n)
+    at = host.data_ptr()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(400_000_000)  # about 0.2 s in front of the kernel
+    ops.publish_step(out, exp, status, host, host_exp, host_status)
+    del host
+    other = torch.zeros(n, dtype=torch.int8, pin_memory=True)
+    assert other.data_ptr() != at
+    torch.cuda.synchronize()
+    assert not bool(other.any())
