@@ -625,9 +625,15 @@ PyObject* quantize_input(Args& a) {
 // current, and the event behind the launch is recorded there.
 PyObject* publish_step(Args& a) {
     const Tensor &out = a.tensor(), &exp = a.tensor(), &status = a.tensor(), &host_out = a.tensor(), &host_exp = a.tensor(), &host_status = a.tensor();
+    // the kernel stores through the host addresses: one exponent, four status words, as many logits as there are
+    for (const Tensor* t : {&host_out, &host_exp, &host_status})
+        if (!(t->is_cpu() && t->is_contiguous() && t->is_pinned()))
+            throw c10::Error({__func__, __FILE__, __LINE__}, "niti_publish_step writes to contiguous pinned host tensors");
+    require(host_out.scalar_type() == at::kChar && host_out.sizes() == out.sizes() && host_exp.scalar_type() == at::kInt && host_exp.numel() == 1 &&
+            host_status.scalar_type() == at::kInt && host_status.numel() >= 4);
     need_cuda({&out, &exp, &status});
-    require(out.scalar_type() == at::kChar && exp.scalar_type() == at::kInt && exp.numel() == 1 && out.device() == exp.device() && out.device() == status.device());
-    require(host_out.is_contiguous() && host_out.scalar_type() == at::kChar && host_out.sizes() == out.sizes());
+    require(out.scalar_type() == at::kChar && exp.scalar_type() == at::kInt && exp.numel() == 1 && status.scalar_type() == at::kInt &&
+            status.numel() >= 4 && out.device() == exp.device() && out.device() == status.device());
     {
         Launch l(out);
         check(niti_publish_step(cptr<int8_t>(out), out.numel(), cptr<int32_t>(exp), cptr<int32_t>(status), mptr<int8_t>(host_out),

@@ -362,3 +362,21 @@ def test_a_result_dropped_before_its_kernel_has_run_keeps_its_memory():
     assert other.data_ptr() != at
     torch.cuda.synchronize()
     assert not bool(other.any())
+
+
+@pytest.mark.parametrize("which", ["logits", "exponent", "status"])
+@pytest.mark.parametrize("wrong", ["pageable", "short", "type", "strided", "device"])
+def test_results_go_to_pinned_buffers_of_the_right_size_only(which, wrong, monkeypatch):
+    """Refused before anything is launched: the kernel stores one exponent, four status words and all logits."""
+    out = torch.zeros(10, dtype=torch.int8, device=DEV)
+    exp, status = torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+    host = dict(zip(("logits", "exponent", "status"), pinned_results(10)))
+    t = host[which]
+    if wrong == "strided" and t.dim() == 0:
+        pytest.skip("one element is contiguous")
+    host[which] = {"pageable": lambda: t.clone(), "short": lambda: t.new_zeros(t.numel() - 1).pin_memory(),
+                   "type": lambda: t.to(torch.int64).pin_memory(), "strided": lambda: t.new_zeros(2 * t.numel()).pin_memory()[::2],
+                   "device": lambda: t.to(DEV)}[wrong]()
+    with pytest.raises((RuntimeError, AssertionError)):
+        ops.publish_step(out, exp, status, *host.values())
+    torch.cuda.synchronize()
