@@ -76,9 +76,11 @@ extern "C" {
  * operand, which cuts the L2 -> shared-memory traffic per output; 0: one thread block per 128-row tile. */
 #define NITI_OPT_CTA_PAIRS 4
 /* NITI_OPT_COOPERATIVE_LAUNCH (default 1): the kernels that contain a grid barrier (accumulator parking,
- * classifier head, multi-layer update) are launched cooperatively, i.e. the driver guarantees that all their
- * thread blocks are resident together.  0: plain launches of the same one-wave grids; a barrier that is not met
- * (something else held SMs for more than 0.5 s) then ends in the status word's error, never in a hang. */
+ * classifier head, multi-layer update, forward layers beyond tensor memory, layers of few tiles, a layer's gradient and
+ * update) are launched cooperatively, i.e. the driver guarantees that all their thread blocks are resident together.
+ * 0: plain launches.  Parking, head and update keep their one-wave grids; a barrier that is not met (something else held SMs
+ * for more than 0.5 s) then ends in the status word's error, never in a hang.  The others take their forms without a barrier:
+ * a conditional second launch, one thread block to a tile, gradient and update apart. */
 #define NITI_OPT_COOPERATIVE_LAUNCH 5
 NITI_API int niti_set_option(int option, int value);
 
@@ -371,7 +373,8 @@ NITI_API int niti_conv_wgrad_update_i8(const int8_t* x, const int8_t* err, int32
 
 /* The same with `state`, int32[4], 16-byte aligned, owned by the layer: zero before the first call, left zero by every call (calls that
  * share it must be stream-ordered).  Where one wave of thread blocks holds the layer, the (cooperative) launch of the gradient clears it
- * too, and for layers of up to 200000 weights also finds the maximum and updates; elsewhere it is the call above. */
+ * too, and for layers of up to 200000 weights also finds the maximum and updates; elsewhere, and with cooperative launches off,
+ * it is the call above. */
 NITI_API int niti_conv_wgrad_update_state_i8(const int8_t* x, const int8_t* err, int32_t* g32, int8_t* w, int32_t* state, int N, int H,
                        int W, int C, int K, int R, int S, int pad, int mu, int round_mode, const uint64_t* seed, uint32_t rng_stream,
                        int32_t* status, void* stream);

@@ -366,8 +366,9 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
                       const int32_t* exp_b, int32_t* exp_out, int32_t* shift_out, int32_t* status, cudaStream_t st,
                       const int8_t* relu_mask = nullptr, int8_t* pool_out = nullptr, void* side = nullptr) {
     // Narrow with the predicted shift, reduce max|acc|, verify, narrow again where it was wrong: forward layers in one launch, the
-    // error's way back and CTA pairs with a conditional second one.
-    const bool one = !flip && !(g_two_cta & 2) && relu_mask == nullptr && side == nullptr;
+    // error's way back and CTA pairs with a conditional second one.  So do forward layers where launches are not cooperative: these
+    // grids fill the device, and beside another kernel their barrier would not be met.
+    const bool one = g_cooperative && !flip && !(g_two_cta & 2) && relu_mask == nullptr && side == nullptr;
     FusedArgs f{state, 0, one ? 1 : 0, 0, round_mode, relu, reinterpret_cast<const unsigned long long*>(seed), rng_stream, rng_offset,
                 kind, 7, exp_a, exp_b, exp_out, shift_out, relu_mask, pool_out, side};
     const bool thin = !flip && fprop_path(C, K, R, S, pad) == CONV_THIN;

@@ -1597,7 +1597,7 @@ extern "C" int niti_conv_wgrad_update_state_i8(const int8_t* x, const int8_t* er
     NITI_REQUIRE(reinterpret_cast<uintptr_t>(w) % 4 == 0 && reinterpret_cast<uintptr_t>(g32) % 16 == 0);
     const size_t elems = niti_conv_wgrad_update_elems(C, K, R, S, pad);
     if (elems == 0) return NITI_ERR_UNSUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(err)) % 16 != 0 || !umma_conv_wgrad_update_fits(N, H, W, C, K, R))
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(err)) % 16 != 0 || !g_cooperative || !umma_conv_wgrad_update_fits(N, H, W, C, K, R))
         return niti_conv_wgrad_update_i8(x, err, g32, w, N, H, W, C, K, R, S, pad, mu, round_mode, seed, rng_stream, status, stream);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int words = static_cast<int>(niti_update_multi_scratch_bytes() / 4);

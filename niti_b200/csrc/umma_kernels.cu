@@ -2480,7 +2480,7 @@ static ConvPlan pool_plan(int Nimg, int H, int W, int red, int outc, bool k3) {
 // and with random words, whose drawing is shared out too, it pays from half of that on: 64x8x8 128->128 11.9 / 10.6, 4x32x32
 // 128->128 11.2 / 10.5; 8x32x32 64->64 10.4 / 12.1.
 static int split_cluster(int tiles, int taps, int red, bool halo, bool stochastic, int bw) {
-    if (tiles > sm_count() / 2 || (g_two_cta & 2)) return 1;
+    if (tiles > sm_count() / 2 || (g_two_cta & 2) || !g_cooperative) return 1;  // without the guarantee a cluster more is a barrier that may not be met
     const int num_kb = taps * ((red + 127) / 128);
     const auto fits = [&](int cs, int clusters) { return tiles <= clusters && num_kb >= 2 * cs && (bw == 0 || 128 / cs % (2 * bw) == 0); };
     const int cs = fits(8, split_clusters<8>()) ? 8 : fits(4, split_clusters<4>()) ? 4 : fits(2, split_clusters<2>()) ? 2 : 1;

@@ -1,0 +1,107 @@
+"""Which launches serve a call, as a captured graph shows them (kernels, cooperative or not, thread blocks of a cluster), and that
+every form gives the same bits: cooperative launches switched off, refused, in a second context."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from cuda.bindings import runtime as rt  # noqa: E402
+
+from niti_b200 import ops  # noqa: E402
+from oracle import niti_oracle as O  # noqa: E402
+
+DEV = "cuda:0"
+
+
+def rnd8(rng, shape, lo=-127):
+    return rng.integers(lo, 128, size=shape).astype(np.int8)
+
+
+def cu(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+
+
+def same(got, want):
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
+def kernels(fn):
+    """(cooperative, thread blocks of a cluster) of every kernel that fn() enqueues, and whatever else it does once."""
+    fn()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
+        return r[1:]
+    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+    n = ok(rt.cudaGraphGetNodes(raw))[1]
+    found = []
+    for node in ok(rt.cudaGraphGetNodes(raw, n))[0]:
+        if ok(rt.cudaGraphNodeGetType(node))[0] != rt.cudaGraphNodeType.cudaGraphNodeTypeKernel:
+            continue
+        value = lambda attr: ok(rt.cudaGraphKernelNodeGetAttribute(node, attr))[0]  # noqa: E731
+        found.append((bool(value(rt.cudaLaunchAttributeID.cudaLaunchAttributeCooperative).cooperative),
+                      max(1, value(rt.cudaLaunchAttributeID.cudaLaunchAttributeClusterDimension).clusterDim.x)))
+    return found
+
+
+class Layer:
+    """One convolution layer's three calls, each with words of its own, and what they must give."""
+
+    def __init__(self, N, H, W, C, K):
+        rng = np.random.default_rng(N + H + W + C + K)
+        self.x, self.w, self.err = rnd8(rng, (N, H, W, C), 0), rnd8(rng, (K, 3, 3, C)), rnd8(rng, (N, H, W, K))
+        self.dx, self.dw, self.derr = cu(self.x), cu(self.w), cu(self.err)
+        self.z = torch.zeros((), dtype=torch.int32, device=DEV)
+        self.fwd, self.bwd, self.upd = ops.new_requant_state(DEV), ops.new_requant_state(DEV), ops.new_update_state(DEV)
+
+    def forward(self):
+        return ops.conv_fprop_fused(self.dx, self.dw, self.fwd, 1, 0, None, 0, 0, False, self.z, self.z)[0]
+
+    def backward(self):
+        return ops.conv_dgrad_fused(self.derr, self.dw, self.bwd, 1, 0, None, 0, 0, self.z, self.z)[0]
+
+    def update(self):
+        w = self.dw.clone()
+        return ops.conv_wgrad_update(self.dx, self.derr, w, 1, 5, 2, None, 18, self.upd)[0], w
+
+    def check(self):
+        for _ in range(2):
+            same(self.forward(), O.act_calc(O.conv_fprop(self.x, self.w), 0, 0)[0])
+            same(self.backward(), O.err_calc(O.conv_dgrad(self.err, self.w), 0)[0])
+            g, w = self.update()
+            want = O.conv_wgrad(self.x, self.err, 3, 3, 1)
+            same(g, want)
+            same(w, O.weight_update(self.w, want, 5, 2)[0])
+        ops.check_status(DEV)
+
+
+@pytest.fixture
+def no_cooperative_launches():
+    old = ops.set_cooperative_launch(False)
+    yield
+    ops.set_cooperative_launch(old)
+
+
+def test_without_cooperative_launches_only_the_parked_layers_meet_at_a_barrier(no_cooperative_launches):
+    """NITI_OPT_COOPERATIVE_LAUNCH = 0: a layer whose tiles do not fit in tensor memory, a layer of few tiles and the weight gradient run
+    without any thread block waiting for another: prediction and conditional second launch, one thread block to a tile, gradient
+    and update apart."""
+    large, few = Layer(75, 32, 32, 16, 128), Layer(1, 8, 8, 512, 512)
+    assert kernels(large.forward) == [(False, 1)] * 2
+    assert kernels(few.forward) == kernels(few.backward) == [(False, 1)]
+    copy_and_update = kernels(few.update)  # the copy of the weights is a kernel or a copy node, as torch likes it
+    assert copy_and_update[-2:] == [(False, 1)] * 2
+    large.check()
+    few.check()
+    old = ops.set_accumulator_parking(False)
+    try:
+        assert kernels(few.forward) == [(False, 1)] * 2
+        few.check()
+    finally:
+        ops.set_accumulator_parking(old)
