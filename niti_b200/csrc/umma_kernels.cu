@@ -2197,18 +2197,20 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+static void* driver_entry(const char* name) {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    return cudaGetDriverEntryPoint(name, &sym, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess ? sym : nullptr;
+}
 static EncodeTiledFn get_encode() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-            qres == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(sym);
-    }
+    static const EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(driver_entry("cuTensorMapEncodeTiled"));
     return fn;
+}
+// A number for the current context that no other one has had or will have; 0: not known.
+static unsigned long long context_number() {
+    static const auto get_id = reinterpret_cast<CUresult (*)(CUcontext, unsigned long long*)>(driver_entry("cuCtxGetId"));
+    unsigned long long id = 0;
+    return get_id != nullptr && get_id(nullptr, &id) == CUDA_SUCCESS ? id + 1 : 0;
 }
 
 // Tensor map with 128-byte swizzle over uint8 (operands) or int32 (outputs) elements; dims/box
@@ -2232,17 +2234,17 @@ static int encode_map(CUtensorMap* map, const void* ptr, bool int32_elems, int r
     return 0;
 }
 
-// The dynamic shared memory of a kernel, granted once per device: asked for at every launch it was about a microsecond of the host's
-// time, and a single image's layers are bound by that.
+// The dynamic shared memory of a kernel, granted once per context: asked for at every launch it was about a microsecond of the host's
+// time, and a single image's layers are bound by that.  Not once per device: a second context of a device, or its first one after a
+// reset, starts without the grant, and a launch there would be refused.
 template <auto KERNEL>
 static cudaError_t allow_shared(int bytes) {
-    static std::atomic<unsigned long long> done{0};  // one bit per device
-    int dev = 0;
-    if (cudaError_t e = cudaGetDevice(&dev)) return e;
-    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
-    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    static std::atomic<unsigned long long> granted[16];  // context numbers; two that share a place ask in turn
+    const unsigned long long now = context_number();
+    std::atomic<unsigned long long>& place = granted[now % 16];
+    if (now != 0 && place.load(std::memory_order_acquire) == now) return cudaSuccess;
     const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    if (e == cudaSuccess && now != 0) place.store(now, std::memory_order_release);
     return e;
 }
 

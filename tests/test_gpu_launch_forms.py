@@ -1,5 +1,9 @@
 """Which launches serve a call, as a captured graph shows them (kernels, cooperative or not, thread blocks of a cluster), and that
 every form gives the same bits: cooperative launches switched off, refused, in a second context."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -105,3 +109,65 @@ def test_without_cooperative_launches_only_the_parked_layers_meet_at_a_barrier(n
         few.check()
     finally:
         ops.set_accumulator_parking(old)
+
+
+CONTEXTS = """
+import ctypes as C, sys
+import numpy as np
+from niti_b200._lib import lib
+cu = C.CDLL("libcuda.so.1")
+def ok(r):
+    assert r == 0, r
+ok(cu.cuInit(0))
+dev, ctx = C.c_int(), C.c_void_p()
+ok(cu.cuDeviceGet(C.byref(dev), 0))
+rng = np.random.default_rng(3)
+N, H, W, C_, K = 2, 8, 8, 144, 128
+x, w, err = (rng.integers(-127, 128, n).astype(np.int8) for n in (N * H * W * C_, K * 9 * C_, N * H * W * K))
+def put(a):
+    p = C.c_uint64()
+    ok(cu.cuMemAlloc_v2(C.byref(p), C.c_size_t(a.nbytes)))
+    ok(cu.cuMemcpyHtoD_v2(p, a.ctypes.data_as(C.c_void_p), C.c_size_t(a.nbytes)))
+    return p.value
+def get(p, shape, type):
+    a = np.empty(shape, type)
+    ok(cu.cuCtxSynchronize())
+    ok(cu.cuMemcpyDtoH_v2(a.ctypes.data_as(C.c_void_p), C.c_uint64(p), C.c_size_t(a.nbytes)))
+    return a
+def calls():
+    dx, dw, de = put(x), put(w), put(err)
+    y, g, c = (put(np.zeros(n, t)) for n, t in ((N * H * W * K, np.int8), (K * 9 * C_, np.int32), (K * K, np.int32)))
+    words, status, mx = put(np.zeros(8, np.int32)), put(np.zeros(4, np.int32)), put(np.zeros(1, np.int32))
+    assert lib.niti_conv_fprop_requant_i8(dx, dw, y, words, None, 0, N, H, W, C_, K, 3, 3, 1, 0, None, 0, 0, 0, None, None, None, None, status, None) == 0, lib.niti_last_cuda_error()
+    assert lib.niti_conv_wgrad_accumulate_i8(dx, de, g, N, H, W, C_, K, 3, 3, 1, status, None) == 0, lib.niti_last_cuda_error()
+    assert lib.niti_gemm_i8(de, de, c, mx, K, K, N * H * W, 1, 0, status, None) == 0, lib.niti_last_cuda_error()
+    r = [get(y, N * H * W * K, np.int8), get(g, K * 9 * C_, np.int32), get(c, K * K, np.int32)]
+    assert not get(status, 4, np.int32).any()
+    return r
+ok(cu.cuDevicePrimaryCtxRetain(C.byref(ctx), dev))
+ok(cu.cuCtxSetCurrent(ctx))
+first = calls()
+assert all(a.any() for a in first)
+def same(r):
+    assert all(np.array_equal(a, b) for a, b in zip(first, r))
+same(calls())
+if sys.argv[1] == "second":
+    other = C.c_void_p()
+    ok(cu.cuCtxCreate_v2(C.byref(other), 0, dev))
+    same(calls())
+    ok(cu.cuCtxDestroy_v2(other))
+else:
+    ok(cu.cuDevicePrimaryCtxReset_v2(dev))
+    ok(cu.cuDevicePrimaryCtxRetain(C.byref(ctx), dev))
+ok(cu.cuCtxSetCurrent(ctx))
+same(calls())
+"""
+
+
+@pytest.mark.parametrize("what", ["second", "reset"])
+def test_contexts_after_the_first(what):
+    """What a kernel is granted belongs to a context: the calls work in a second context of the device, and in the primary one after
+    a reset.  In a process of its own, without torch."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CONTEXTS, what], cwd=root, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
