@@ -370,7 +370,7 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
     // grids fill the device, and beside another kernel their barrier would not be met.
     const bool one = g_cooperative && !flip && !(g_two_cta & 2) && relu_mask == nullptr && side == nullptr;
     FusedArgs f{state, 0, one ? 1 : 0, 0, round_mode, relu, reinterpret_cast<const unsigned long long*>(seed), rng_stream, rng_offset,
-                kind, 7, exp_a, exp_b, exp_out, shift_out, relu_mask, pool_out, side};
+                kind, 7, exp_a, exp_b, exp_out, shift_out, relu_mask, pool_out, side, 0};
     const bool thin = !flip && fprop_path(C, K, R, S, pad) == CONV_THIN;
     const size_t m = static_cast<size_t>(N) * H * W;
     int8_t* xcol = static_cast<int8_t*>(scratch);
@@ -385,13 +385,17 @@ static int fused_conv(const int8_t* in, const int8_t* w, int8_t* out8, int32_t* 
         f.parked = 1;
         return umma_conv(in, w, out8, nullptr, N, H, W, C, K, R, S, pad, flip, &f, status, st);
     }
-    for (int pass = 0; pass < (one ? 1 : 2); ++pass) {
-        f.only_if_redo = pass;
-        int rc = thin ? umma_gemm(xcol, wp, out8, nullptr, static_cast<int>(m), K, 32, 0, 1, 1, &f, status, st, 1)
-                      : umma_conv(in, w, out8, nullptr, N, H, W, C, K, R, S, pad, flip, &f, status, st);
-        if (rc) return rc;
+    const auto launch = [&](int only_if_redo) {
+        f.only_if_redo = only_if_redo;
+        return thin ? umma_gemm(xcol, wp, out8, nullptr, static_cast<int>(m), K, 32, 0, 1, 1, &f, status, st, 1)
+                    : umma_conv(in, w, out8, nullptr, N, H, W, C, K, R, S, pad, flip, &f, status, st);
+    };
+    int rc = launch(0);
+    if (rc == LAUNCH_REFUSED) {  // not every SM of the device is there: the two launches run on any number of them
+        f.one = 0;
+        rc = launch(0);
     }
-    return NITI_OK;
+    return rc != NITI_OK || f.one ? rc : launch(1);
 }
 
 extern "C" int niti_conv_fprop_requant_supported(int C, int K, int R, int S, int pad) {

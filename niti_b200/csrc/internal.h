@@ -10,6 +10,10 @@ namespace niti {
 int set_cuda_error(cudaError_t e);
 int set_cuda_error_text(const char* text);
 
+// What a launcher returns (never the library) where the driver has fewer SMs or clusters for a launch than its thread blocks, which
+// wait for one another, need at a time: on a stream or in a context that is held to part of the device.  Nothing has been enqueued.
+constexpr int LAUNCH_REFUSED = -1000;
+
 // Requantisation fused into a contraction's epilogue: the kernel narrows with the shift it finds in
 // state[0] and its last CTA verifies that shift; `only_if_redo` launches are no-ops unless state[2] is set.
 struct FusedArgs {
@@ -26,6 +30,7 @@ struct FusedArgs {
     const int8_t* relu_mask;  // optional, same shape as the output: zero the output where this tensor is <= 0
     int8_t* pool_out;         // optional (forward, parked kernel): 2x2 / stride-2 max-pooled copy of the output
     void* side;               // optional (streaming kernel, round-to-nearest, no ReLU): outputs / 4 bytes of side codes
+    int whole;                // 1: one thread block to a tile, however few there are
 };
 
 extern int g_two_cta;    // CTA pairs (cta_group::2) where the shape allows: bit 0 for GEMMs, bit 1 for convolutions
@@ -50,7 +55,7 @@ int umma_conv_wgrad_partials(const int8_t* x, const int8_t* err, int32_t* partia
                              int Nimg, int H, int W, int C, int K, int R, int S, int pad, int32_t* status, cudaStream_t st,
                              int direct = 0);
 // gradient, cleared by the launch, and for small layers (*updated) the update, in one (cooperative) launch of one wave of thread
-// blocks; state: int32[4], zero between calls; words: cleared, the first is max |g| of an update
+// blocks; state: int32[4], zero between calls; words: cleared, the first is max |g| of an update; may return LAUNCH_REFUSED
 bool umma_conv_wgrad_update_fits(int Nimg, int H, int W, int C, int K, int R);
 int umma_conv_wgrad_update(const int8_t* x, const int8_t* err, int32_t* out, int8_t* w, uint32_t* words, int num_words, int32_t* state,
                            int Nimg, int H, int W, int C, int K, int R, int S, int pad, int mu, int mode, const unsigned long long* seed,

@@ -1603,8 +1603,11 @@ extern "C" int niti_conv_wgrad_update_state_i8(const int8_t* x, const int8_t* er
     const int words = static_cast<int>(niti_update_multi_scratch_bytes() / 4);
     int32_t* tail = g32 + elems - words;
     bool updated = false;
-    if (int e = umma_conv_wgrad_update(x, err, g32, w, reinterpret_cast<uint32_t*>(tail), words, state, N, H, W, C, K, R, S, pad, mu, round_mode,
-                                       reinterpret_cast<const unsigned long long*>(seed), rng_stream, &updated, status, st)) return e;
+    const int e = umma_conv_wgrad_update(x, err, g32, w, reinterpret_cast<uint32_t*>(tail), words, state, N, H, W, C, K, R, S, pad, mu, round_mode,
+                                         reinterpret_cast<const unsigned long long*>(seed), rng_stream, &updated, status, st);
+    if (e == LAUNCH_REFUSED)  // not every SM of the device is there
+        return niti_conv_wgrad_update_i8(x, err, g32, w, N, H, W, C, K, R, S, pad, mu, round_mode, seed, rng_stream, status, stream);
+    if (e) return e;
     return updated ? NITI_OK : update_after_gradient(w, g32, tail, static_cast<long long>(K) * R * S * C, mu, round_mode, seed, rng_stream, status, st);
 }
 

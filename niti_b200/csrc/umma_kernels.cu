@@ -2248,6 +2248,13 @@ static cudaError_t allow_shared(int bytes) {
     return e;
 }
 
+// The result of a launch whose thread blocks have to be resident together: see LAUNCH_REFUSED.
+static int launched_together(cudaError_t e) {
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorInvalidClusterSize && e != cudaErrorLaunchOutOfResources) return set_cuda_error(e);
+    cudaGetLastError();
+    return LAUNCH_REFUSED;
+}
+
 static int sm_count() {
     static int n = 0;
     if (n == 0) {
@@ -2311,7 +2318,8 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
         attr[n].val.clusterDim.x = 2; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1; ++n;
     }
     cfg.attrs = attr; cfg.numAttrs = n;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, kernel, a, b, p));
+    const cudaError_t r = cudaLaunchKernelEx(&cfg, kernel, a, b, p);
+    return ONE ? launched_together(r) : set_cuda_error(r);
 }
 template <bool ONE, bool CODES>
 static int launch_streaming(int bn, int mode, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
@@ -2356,22 +2364,22 @@ static int launch_split(const CUtensorMap& a, const CUtensorMap& b, const GemmPa
     if (e != cudaSuccess) return set_cuda_error(e);
     cudaLaunchAttribute attr[2];
     const cudaLaunchConfig_t cfg = split_config<CS>(p.m_tiles * p.n_tiles, attr, st);
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_split_kernel<CS>, a, b, p));
+    return launched_together(cudaLaunchKernelEx(&cfg, umma_split_kernel<CS>, a, b, p));
 }
-// Clusters of CS CTAs (one CTA per SM) that an idle device holds at a time; 0 where it cannot be asked.  They lie within a
-// GPC each, so that it is less than the number of SMs over CS.
+// Clusters of CS CTAs (one CTA per SM) that the context holds at a time when idle; 0 where it cannot be asked (now: the next call
+// asks again).  They lie within a GPC each, so that it is less than the number of SMs over CS.
 template <int CS>
 static int split_clusters() {
-    static std::atomic<int> known{-1};
-    int n = known.load(std::memory_order_relaxed);
-    if (n < 0) {
-        cudaLaunchAttribute attr[2];
-        cudaLaunchConfig_t cfg = split_config<CS>(1, attr, nullptr);
-        cfg.numAttrs = 1;
-        if (allow_shared<umma_split_kernel<CS>>(SplitCfg<CS>::SMEM_BYTES) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, umma_split_kernel<CS>, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
-        known.store(n, std::memory_order_relaxed);
-    }
+    static std::atomic<unsigned long long> known{0};  // the context's number, and the clusters in the low 16 bits
+    const unsigned long long now = context_number(), was = known.load(std::memory_order_relaxed);
+    if (now != 0 && was >> 16 == now) return static_cast<int>(was & 0xFFFF);
+    int n = 0;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = split_config<CS>(1, attr, nullptr);
+    cfg.numAttrs = 1;
+    if (allow_shared<umma_split_kernel<CS>>(SplitCfg<CS>::SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, umma_split_kernel<CS>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    known.store(now << 16 | static_cast<unsigned>(n), std::memory_order_relaxed);
     return n;
 }
 // all accumulators of the problem fit in the tensor memory of one wave of CTAs (units: 128-row tiles,
@@ -2558,7 +2566,7 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
                                                         : conv_plan(Nimg, H, W, red, outc, k3, flip, !fused ? 0 : parked ? 2 : 1,
                                                                     fused && fused->mode == NITI_ROUND_STOCHASTIC);
     int split = 1;
-    if (parked) {
+    if (parked && !fused->whole) {
         const ConvPlan taps = conv_plan(Nimg, H, W, red, outc, false, flip, 2);
         split = split_cluster(taps.m_tiles * ((outc + 127) / 128), R * S, red, plan.halo, fused->mode == NITI_ROUND_STOCHASTIC,
                               fused->pool_out != nullptr ? taps.BW : 0);
@@ -2609,9 +2617,13 @@ int umma_conv(const int8_t* x, const int8_t* w, void* out, unsigned* maxabs, int
         p.pool_out = fused->pool_out;
     }
     if (parked && !fits_parked(bn, p.m_tiles * p.n_tiles, pair)) return NITI_ERR_UNSUPPORTED;
-    if (split == 8) return launch_split<8>(ma, mb, p, st);
-    if (split == 4) return launch_split<4>(ma, mb, p, st);
-    if (split == 2) return launch_split<2>(ma, mb, p, st);
+    if (split > 1) {
+        const int rc = split == 8 ? launch_split<8>(ma, mb, p, st) : split == 4 ? launch_split<4>(ma, mb, p, st) : launch_split<2>(ma, mb, p, st);
+        if (rc != LAUNCH_REFUSED) return rc;
+        FusedArgs whole = *fused;  // fewer SMs than the device has: a CS-th of them may do
+        whole.whole = 1;
+        return umma_conv(x, w, out, maxabs, Nimg, H, W, C, K, R, S, pad, flip, &whole, status, st);
+    }
     const int mode = !plan.halo ? LOAD_TAPS : p.cblocks == 1 && p.n_tiles == 1 ? LOAD_HALO_RESIDENT : LOAD_HALO;
     if (fused) return launch_requant(bn, pair, mode, parked, fused->one && !pair, ma, mb, p, st);
     return launch_gemm(bn, pair, ma, mb, mc, p, st);
@@ -2714,7 +2726,7 @@ int umma_conv_wgrad_update(const int8_t* x, const int8_t* err, int32_t* out, int
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_wgrad_update_kernel, me, mx, mp, p, u));
+    return launched_together(cudaLaunchKernelEx(&cfg, umma_wgrad_update_kernel, me, mx, mp, p, u));
 }
 
 // x_t [C][H][W][N], err_t [K][H][W][N] (batch innermost, N a multiple of 16) -> out [C][R][S][K], zeroed by the caller:

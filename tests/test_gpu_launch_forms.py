@@ -171,3 +171,36 @@ def test_contexts_after_the_first(what):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", CONTEXTS, what], cwd=root, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+SOME_SMS = """
+import sys
+from torch.cuda.green_contexts import GreenContext
+import tests.test_gpu_launch_forms as T
+large, few, one, ragged = T.Layer(75, 32, 32, 16, 128), T.Layer(32, 4, 4, 512, 512), T.Layer(1, 8, 8, 512, 512), T.Layer(37, 15, 13, 48, 80)
+T.torch.cuda.synchronize()
+part = GreenContext.create(32, 0)
+part.set_context()
+for _ in range(2):
+    T.same(large.forward(), T.O.act_calc(T.O.conv_fprop(large.x, large.w), 0, 0)[0])
+    T.same(large.backward(), T.O.err_calc(T.O.conv_dgrad(large.err, large.w), 0)[0])
+    for l in (few, one):
+        T.same(l.forward(), T.O.act_calc(T.O.conv_fprop(l.x, l.w), 0, 0)[0])
+        T.same(l.backward(), T.O.err_calc(T.O.conv_dgrad(l.err, l.w), 0)[0])
+    g, w = ragged.update()
+    T.same(g, T.O.conv_wgrad(ragged.x, ragged.err, 3, 3, 1))
+    T.same(w, T.O.weight_update(ragged.w, T.O.conv_wgrad(ragged.x, ragged.err, 3, 3, 1), 5, 2)[0])
+T.torch.cuda.synchronize()
+part.pop_context()
+assert T.kernels(one.forward) == T.kernels(one.backward) == [(True, 8)], T.kernels(one.forward)
+assert T.kernels(large.forward) == [(True, 1)]
+large.check(), few.check()
+"""
+
+
+def test_calls_on_part_of_the_device():
+    """A context of 32 SMs: a launch whose thread blocks have to be resident together and are too many is refused, and the layer goes
+    through the form that takes any number of SMs; the whole device afterwards has its own forms.  In a process of its own."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", SOME_SMS], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
