@@ -77,3 +77,29 @@ def test_the_reference_arm_without_the_reference_says_so():
     out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference"], capture_output=True, text=True, timeout=300, check=True)
     line = json.loads(out.stdout.strip().splitlines()[-1])
     assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
+
+
+def test_dealing_thread_blocks_to_layers_is_no_work_for_the_host():
+    """Weight gradients whose items are more than the SMs are dealt by simulated schedules in every call that is not captured: within a
+    few times the call's other host work (a schedule block by block was 25 to 60 times).  Without a GPU the call ends
+    behind the deal with an error; its addresses are never used."""
+    import time
+
+    import pytest
+    import torch
+    from niti_b200._lib import WgradItem, lib
+    if torch.cuda.is_available():
+        pytest.skip("would launch on addresses that are none")
+
+    def least(shapes):
+        items = (WgradItem * len(shapes))(*[WgradItem(1 << 20, 1 << 21, 1 << 22, *s, 3, 3, 1) for s in shapes])
+        best = 1.0
+        for _ in range(500):
+            t = time.perf_counter()
+            assert lib.niti_conv_wgrad_accumulate_multi_i8(items, len(shapes), None, None) == -3
+            best = min(best, time.perf_counter() - t)
+        return best
+    plain = least([(128, 8, 8, 512, 512), (128, 8, 8, 256, 512)])
+    for shapes in ([(1024, 4, 4, 512, 512), (1024, 4, 4, 512, 512), (1024, 8, 8, 512, 512), (1024, 8, 8, 256, 512)],
+                   [(2, 4, 4, 1024, 1024), (16, 8, 8, 512, 512)]):
+        assert least(shapes) < 15 * plain

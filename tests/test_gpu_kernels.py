@@ -749,3 +749,13 @@ def test_single_conv_layer_step_full_size_stochastic():
         assert_same(w2, O.weight_update(w, gacc, 5, O.STOCHASTIC, philox.random_u32_tensor(42, 34, gacc.shape))[0], "update")
     finally:
         O.set_backend("int64")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shapes", [
+    [(2, 4, 4, 1024, 1024), (16, 8, 8, 512, 512)],                         # 192 items of one chunk, 48 of eight: cut and uncut
+    [(9, 8, 8, 784, 912), (3, 16, 16, 16, 32), (1, 2, 2, 16, 16)],         # 168 items and two layers that fill up behind them
+    [(5, 4, 12, 1040, 656), (40, 4, 4, 400, 528), (7, 8, 8, 272, 144)]])
+def test_weight_gradients_of_more_items_than_sms(shapes):
+    """Layers whose items alone are more than the SMs: cut so that the blocks' schedule ends earliest, longest blocks first."""
+    test_weight_gradients_of_several_layers_in_one_launch(shapes)
