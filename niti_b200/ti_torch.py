@@ -384,12 +384,15 @@ class TiConv2d(UpdateWeight):
         self._patches, self._patches_of = None, None
 
     def _new_states(self, dev):
-        """The device words of the backward's launches that are not there yet, from one allocation."""
-        words = torch.zeros(12, dtype=torch.int32, device=dev)
+        """The device words of the layer's launches that are not there yet, from one allocation (two and two slices of them were 5
+        to 10 us more of a new layer's first pass)."""
+        fwd, bwd, update = torch.zeros(20, dtype=torch.int32, device=dev).split_with_sizes((8, 8, 4))
+        if self._fwd_state is None:
+            self._fwd_state = fwd
         if self._bwd_state is None:
-            self._bwd_state = words[:8]
+            self._bwd_state = bwd
         if self._update_state is None:
-            self._update_state = words[8:]
+            self._update_state = update
 
     def forward(self, input):
         act, exp_in = input
@@ -401,7 +404,10 @@ class TiConv2d(UpdateWeight):
             # conv2d_int8 + act_calc (:393-395) in one kernel; see ops.conv_fprop_fused
             dev = act.device
             if self._fwd_state is None:
-                self._fwd_state = ops.new_requant_state(dev)
+                if TRAINING and not self.first_layer:
+                    self._new_states(dev)  # its backward follows
+                else:
+                    self._fwd_state = ops.new_requant_state(dev)
             mode, seed, stream, exp_in = _mode(ACT_ROUND_METHOD), RNG_SEED(dev), 16 * self.layer_id, exp_tensor(exp_in, dev)
             pool = self.pool_layer
             if (pool is not None and FUSE_POOL and self.fuse_relu and pool.kernel_size == 2 and pool.stride == 2

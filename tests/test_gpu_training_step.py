@@ -380,3 +380,34 @@ def test_results_go_to_pinned_buffers_of_the_right_size_only(which, wrong, monke
     with pytest.raises((RuntimeError, AssertionError)):
         ops.publish_step(out, exp, status, *host.values())
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("training,trained", [(True, True), (False, False), (False, True)])
+def test_a_new_layer_gets_its_device_words_at_once(training, trained, monkeypatch):
+    """One allocation for a layer that trains (the forward's, the backward's and the update's words), the forward's words alone for
+    one that does not; a layer that evaluated first and trains later gets the others then."""
+    made, zeros = [], torch.zeros
+    def counted(*shape, **kw):
+        made.append(shape)
+        return zeros(*shape, **kw)
+    ti_torch.GRAD_BITWIDTH, ti_torch.SAMPLE_OFFSET = 5, 0
+    ti_torch.set_seed(3, DEV)
+    layer = ti_torch.TiConv2d(16, 32)
+    rng = np.random.default_rng(5)
+    w = rng.integers(-127, 128, (32, 3, 3, 16)).astype(np.int8)
+    layer.weight, layer.weight_exp = torch.from_numpy(w).to(DEV), ti_torch.exp_tensor(-9, DEV)
+    x, err = rng.integers(0, 128, (2, 8, 8, 16)).astype(np.int8), rng.integers(-127, 128, (2, 8, 8, 32)).astype(np.int8)
+    exp = ti_torch.exp_tensor(-7, DEV)
+    monkeypatch.setattr(ti_torch, "TRAINING", training)
+    monkeypatch.setattr(torch, "zeros", counted)
+    for _ in range(2):
+        out, _ = layer.forward((torch.from_numpy(x).to(DEV), exp))
+        assert np.array_equal(out.cpu().numpy(), O.act_calc(O.conv_fprop(x, w), 0, 0)[0])
+    assert len(made) == 1
+    if trained:
+        monkeypatch.setattr(ti_torch, "TRAINING", True)
+        back, _ = layer.backward((torch.from_numpy(err).to(DEV), exp))
+        assert np.array_equal(back.cpu().numpy(), O.err_calc(O.conv_dgrad(err, w), 0)[0])
+        assert np.array_equal(layer.weight.cpu().numpy(), O.weight_update(w, O.conv_wgrad(x, err, 3, 3, 1), 5, 2)[0])
+    assert len(made) == (1 if training or not trained else 2)
+    ops.check_status(DEV)
