@@ -444,12 +444,12 @@ def run_ours(args):
     # --- per-kernel timing of one eager step (before graph capture)
     trainer.step(*batches[0])
     trainer.sync()
-    launches0 = ops.LAUNCHES
+    launches0 = ops.lib.niti_launch_count()
     ops.PROFILE = []
     trainer.step(*batches[1])
     trainer.sync()
     prof, ops.PROFILE = ops.PROFILE, None
-    launches_per_step = ops.LAUNCHES - launches0
+    launches_per_step = ops.lib.niti_launch_count() - launches0
     per_kernel = {}
     for name, aops, abytes, a, b in prof:
         d = per_kernel.setdefault(name, [0, 0.0, 0, 0])
@@ -601,14 +601,14 @@ def run_ours(args):
             "e2e": {"value": images / e2e_s, "unit": UNIT, "h2d_bytes_per_step": trainer.h2d_bytes,
                     "d2h_bytes_per_step": trainer.d2h_bytes, "ms_per_step": e2e_s / args.steps * 1e3},
             "gpu_launches": launches_per_step * args.steps,
-            "roofline": {"bound": "tensor", "kernel": "umma_parked_kernel / umma_requant_kernel (conv forward + error-backward, "
+            "roofline": {"bound": "tensor", "kernel": "umma_parked_kernel / umma_split_kernel / umma_requant_once_kernel / umma_requant_kernel (conv forward + error-backward, "
                                                        f"requantisation in the kernel, tcgen05 kind::i8), all {tc_calls} such calls of a step",
                          "achieved": achieved, "peak": peak_tops, "unit": "TOP/s", "frac": achieved / peak_tops,
                          "frac_of_2x_bf16_sustained": achieved / (2.0 * bf16_sus), "frac_of_nominal_4500": achieved / NOMINAL_INT8_TOPS,
                          "traffic": NCU_TRAFFIC_BYTES, "traffic_of": NCU_TRAFFIC_OF, "traffic_source": "recorded ncu capture (constant)",
                          "launches_timed": tc_calls * 10, "avg_launch_us": tc_time / max(tc_calls, 1) * 1e6,
                          "per_layer": per_layer,
-                         "timing": "each call (one launch; two for the layers whose tiles do not fit in tensor memory) x10 in a CUDA graph, CUDA events around the replay",
+                         "timing": "each call (one launch; two on the way back through layers whose tiles do not fit in tensor memory) x10 in a CUDA graph, CUDA events around the replay",
                          "peak_source": f"2 x bf16_tflops burst ({src}): each call is timed alone; dense int8 rate is twice bf16 on this part"},
             "kernels_eager_step": {k: {"launches": v[0], "ms": v[1] * 1e3,
                                        "tops": (v[2] / v[1] / 1e12 if v[1] > 0 and v[2] else None),

@@ -86,6 +86,9 @@ NITI_API int niti_set_option(int option, int value);
 
 NITI_API int niti_version(void);
 NITI_API const char* niti_strerror(int code);
+/* kernels this process has launched through the library so far (into streams or into graphs under capture; a graph's replays are
+ * not seen) */
+NITI_API unsigned long long niti_launch_count(void);
 /* text of the last CUDA error seen by this thread inside the library ("" if none) */
 NITI_API const char* niti_last_cuda_error(void);
 

@@ -60,6 +60,7 @@ SIGNATURES = {
     "niti_update_i8": (_i, [_p, _p, _p, _i64, _i, _i, _p, _u32, _p]),
     "niti_quantize_input_f32": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "niti_publish_step": (_i, [_p, _i64] + [_p] * 6),
+    "niti_launch_count": (C.c_uint64, []),
     "niti_selftest_barrier_timeout": (_i, [_p, _p, _p]),
     "niti_absmax_f32": (_i, [_p, _i64, _p, _p]),
     "niti_quantize_input_with_max_f32": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _p]),

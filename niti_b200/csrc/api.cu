@@ -23,6 +23,12 @@ int set_cuda_error(cudaError_t e) {
     return NITI_ERR_CUDA;
 }
 
+static std::atomic<unsigned long long> g_launches{0};
+int launched(cudaError_t e) {
+    if (e == cudaSuccess) g_launches.fetch_add(1, std::memory_order_relaxed);
+    return set_cuda_error(e);
+}
+
 static bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 }  // namespace niti
@@ -32,6 +38,8 @@ using namespace niti;
 #define NITI_REQUIRE(cond) do { if (!(cond)) return NITI_ERR_BAD_ARG; } while (0)
 
 extern "C" int niti_version(void) { return 100; }
+
+extern "C" unsigned long long niti_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 extern "C" const char* niti_strerror(int code) {
     switch (code) {

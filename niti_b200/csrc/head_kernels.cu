@@ -473,5 +473,5 @@ extern "C" int niti_fc_head_train_i8(const niti_fc_head_args* a, void* stream) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;  // the grid is at most one block per SM
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, fc_head_kernel, p));
+    return launched(cudaLaunchKernelEx(&cfg, fc_head_kernel, p));
 }

@@ -9,6 +9,7 @@ namespace niti {
 // error plumbing: both return NITI_ERR_CUDA (or 0 for cudaSuccess) and remember the text
 int set_cuda_error(cudaError_t e);
 int set_cuda_error_text(const char* text);
+int launched(cudaError_t e);  // the result of one kernel launch: as set_cuda_error, and counts those that went through (niti_launch_count)
 
 // What a launcher returns (never the library) where the driver has fewer SMs or clusters for a launch than its thread blocks, which
 // wait for one another, need at a time: on a stream or in a context that is held to part of the device.  Nothing has been enqueued.

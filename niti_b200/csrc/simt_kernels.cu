@@ -63,7 +63,7 @@ __global__ void clear_words_kernel(uint32_t* p, int n) {
 }
 int clear_words(void* p, int n, cudaStream_t st) {
     clear_words_kernel<<<1, 32, 0, st>>>(static_cast<uint32_t*>(p), n);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -186,7 +186,7 @@ absmax_kernel(const int32_t* __restrict__ acc, long long n, unsigned* maxabs) {
 
 int absmax_i32(const int32_t* acc, long long n, unsigned* maxabs, cudaStream_t st) {
     absmax_kernel<<<blocks_for(n / 4 + 1, 256, sm_count_simt() * 8), 256, 0, st>>>(acc, n, maxabs);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // out[i] = sum over splits of partial[s][i]; max|out| reduced into *maxabs.
@@ -225,7 +225,7 @@ reduce_partials_kernel(const int32_t* __restrict__ partial, int splits, long lon
 int reduce_partials(const int32_t* partial, int splits, long long n, int32_t* out, unsigned* maxabs, cudaStream_t st) {
     if (n % 4 != 0) return NITI_ERR_UNSUPPORTED;
     reduce_partials_kernel<<<blocks_for((n / 4 + 63) / 64, 1, sm_count_simt() * 8), 256, 0, st>>>(partial, splits, n, out, maxabs);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // Same fold for row-padded partials: partial[s][row][cols_in] -> out[row][cols_out] (cols_out <= cols_in = 32).
@@ -251,7 +251,7 @@ reduce_rows_kernel(const int32_t* __restrict__ partial, int splits, int rows, in
 
 int reduce_rows32(const int32_t* partial, int splits, int rows, int cols_out, int32_t* out, unsigned* maxabs, cudaStream_t st) {
     reduce_rows_kernel<<<rows, 256, 0, st>>>(partial, splits, rows, cols_out, out, maxabs);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // Thin convolutions (R*S*C <= 32, the 3-channel first layer) run as GEMMs over an explicit patch
@@ -346,12 +346,12 @@ int im2col32(const int8_t* x, int8_t* xcol, int Nimg, int H, int W, int C, int R
         const int bands = (H + band - 1) / band;
         if (static_cast<long long>(Nimg) * bands < (1ll << 31)) {
             im2col32_rgb_kernel<<<Nimg * bands, 256, (band + 2) * (3 * W / 4 + 3) * 4, st>>>(x, reinterpret_cast<uint4*>(xcol), H, W, band, bands, w, wp, K);
-            return set_cuda_error(cudaGetLastError());
+            return launched(cudaGetLastError());
         }
     }
     im2col32_kernel<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, st>>>(x, reinterpret_cast<uint4*>(xcol), Nimg, H, W, C, R, S, pad,
                                                                                  w, wp, K);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1017,7 +1017,7 @@ static int launch_quantize(const float* x, int8_t* x8, int32_t* exp_out, const u
     const int rgb4 = C == 3 && static_cast<long long>(H) * W % 4 == 0 && static_cast<long long>(H) * W < (1ll << 31) &&
                      reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(x8) % 4 == 0;
     quantize_input_kernel<<<blocks_for(rgb4 ? n / 12 : n, 256, sm_count_simt() * 8), 256, 0, st>>>(x, x8, exp_out, bits, N, C, H, W, rgb4);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1090,14 +1090,14 @@ int simt_conv_fprop(const int8_t* x, const int8_t* w, int32_t* y32, unsigned* ma
     const long long total = static_cast<long long>(Nimg) * P * Q * K;
     conv_fprop_direct_kernel<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, st>>>(x, w, y32, maxabs, Nimg, H, W, C, K,
                                                                                          R, S, pad, P, Q);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 int simt_conv_dgrad(const int8_t* err, const int8_t* w, int32_t* e32, unsigned* maxabs, int Nimg, int H, int W, int C,
                     int K, int R, int S, int pad, cudaStream_t st) {
     const long long total = static_cast<long long>(Nimg) * H * W * C;
     conv_dgrad_direct_kernel<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, st>>>(err, w, e32, maxabs, Nimg, H, W, C,
                                                                                          K, R, S, pad);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // Weight gradient, any shape: one thread per gradient element, summing over all pixels.
@@ -1134,7 +1134,7 @@ int simt_conv_wgrad(const int8_t* x, const int8_t* err, int32_t* g32, unsigned* 
     const int P = H + 2 * pad - R + 1, Q = W + 2 * pad - S + 1;
     const long long total = static_cast<long long>(K) * R * S * C;
     conv_wgrad_direct_kernel<<<blocks_for(total, 128, 1 << 20), 128, 0, st>>>(x, err, g32, maxabs, Nimg, H, W, C, K, R, S, pad, P, Q);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // GEMM, both operands contiguous along the reduction (trans_a = 0, trans_b = 1): one warp per
@@ -1297,7 +1297,7 @@ int simt_gemm(const int8_t* A, const int8_t* B, int32_t* C32, unsigned* maxabs, 
         gemm_bn4_kernel<<<blocks_for(outs / 4, 128, sm_count_simt() * 32), 128, 0, st>>>(A, B, C32, maxabs, M, N, K, trans_a);
     else
         gemm_generic_kernel<<<blocks_for(outs, 256, sm_count_simt() * 32), 256, 0, st>>>(A, B, C32, maxabs, M, N, K, trans_a, trans_b);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 }  // namespace niti
@@ -1318,7 +1318,7 @@ extern "C" int niti_requant_i8(const int32_t* acc, int8_t* out, const uint32_t* 
     NITI_REQUIRE(reinterpret_cast<uintptr_t>(acc) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0);
     requant_kernel<<<blocks_for(n / 16 + 1, 256, sm_count_simt() * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         acc, out, maxabs, n, kind, target_bits, round_mode, reinterpret_cast<const unsigned long long*>(seed), rng_stream, rng_offset, relu, exp_a, exp_b, exp_out, shift_out);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_absmax_i32(const int32_t* acc, int64_t n, uint32_t* maxabs, void* stream) {
@@ -1326,7 +1326,7 @@ extern "C" int niti_absmax_i32(const int32_t* acc, int64_t n, uint32_t* maxabs, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int e = set_cuda_error(cudaMemsetAsync(maxabs, 0, 4, st))) return e;
     absmax_kernel<<<blocks_for(n / 4 + 1, 256, sm_count_simt() * 8), 256, 0, st>>>(acc, n, maxabs);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // Two signed 4-bit values per byte, element 2i in the low nibble (the packing of CUTLASS' int4b_t arrays), to int8.
@@ -1354,11 +1354,11 @@ int copy_rows(const void* src, long long src_pitch, void* dst, long long dst_pit
         copy_rows_kernel<<<grid, 256, 0, st>>>(static_cast<const int32_t*>(src), src_pitch / 4, static_cast<int32_t*>(dst), dst_pitch / 4, static_cast<int>(bytes / 4), rows);
     else
         copy_rows_kernel<<<grid, 256, 0, st>>>(static_cast<const int8_t*>(src), src_pitch, static_cast<int8_t*>(dst), dst_pitch, static_cast<int>(bytes), rows);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 int unpack_i4(const uint8_t* in, int8_t* out, long long nbytes, cudaStream_t st) {
     unpack_i4_kernel<<<blocks_for(nbytes, 256, sm_count_simt() * 16), 256, 0, st>>>(in, out, nbytes);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 }  // namespace niti
 
@@ -1399,7 +1399,7 @@ extern "C" int niti_group_conv1_i8(const int8_t* in, const int8_t* wt, int32_t* 
     const long long chans = static_cast<long long>(G) * Kg;
     group_conv1_kernel<<<blocks_for(chans * 32, 256, sm_count_simt() * 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         in, wt, out32, H, W, G, Kg, R, S, pad, P, Q);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_maxpool_fwd_i8(const int8_t* x, int8_t* y, int N, int H, int W, int C, int k, int stride, void* stream) {
@@ -1414,7 +1414,7 @@ extern "C" int niti_maxpool_fwd_i8(const int8_t* x, int8_t* y, int N, int H, int
         const long long total = static_cast<long long>(N) * P * Q * C;
         maxpool_fwd_generic<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, st>>>(x, y, N, H, W, C, k, stride, P, Q);
     }
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_maxpool_bwd_i8(const int8_t* x, const int8_t* dy, int8_t* dx, int N, int H, int W, int C, int k,
@@ -1431,7 +1431,7 @@ extern "C" int niti_maxpool_bwd_i8(const int8_t* x, const int8_t* dy, int8_t* dx
         const long long total = static_cast<long long>(N) * H * W * C;
         maxpool_bwd_generic<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, st>>>(x, dy, dx, N, H, W, C, k, stride, P, Q, relu_mask);
     }
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_maxpool_bwd_f16(const void* x, const void* dy, void* dx, int N, int H, int W, int C, int k, int stride, void* stream) {
@@ -1441,19 +1441,19 @@ extern "C" int niti_maxpool_bwd_f16(const void* x, const void* dy, void* dx, int
     const long long total = static_cast<long long>(N) * (H / 2) * (W / 2) * (C / 8);
     maxpool2_bwd_f16_kernel<<<blocks_for(total, 256, sm_count_simt() * 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<uint4*>(dx), N, H, W, C / 8, H / 2, W / 2);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_relu_fwd_i8(const int8_t* x, int8_t* y, int64_t n, void* stream) {
     NITI_REQUIRE(x && y && n >= 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16 == 0);
     relu_fwd_kernel<<<blocks_for(n / 16 + 1, 256, sm_count_simt() * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, y, n);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 extern "C" int niti_relu_bwd_i8(const int8_t* act, const int8_t* err, int8_t* out, int64_t n, void* stream) {
     NITI_REQUIRE(act && err && out && n >= 0);
     NITI_REQUIRE((reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(err) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);
     relu_bwd_kernel<<<blocks_for(n / 16 + 1, 256, sm_count_simt() * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(act, err, out, n);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 extern "C" int niti_dropout_i8(const int8_t* x, int8_t* y, int64_t rows, int64_t features, const uint64_t* seed,
                                uint32_t rng_stream, void* stream) {
@@ -1467,7 +1467,7 @@ extern "C" int niti_dropout_i8(const int8_t* x, int8_t* y, int64_t rows, int64_t
         dropout_kernel<<<blocks_for(rows * features, 256, sm_count_simt() * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
             x, y, rows, features, reinterpret_cast<const unsigned long long*>(seed), rng_stream);
     }
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_loss_i8(const int8_t* out8, const int32_t* out_exp, const int64_t* target, int8_t* err8, int B,
@@ -1477,7 +1477,7 @@ extern "C" int niti_loss_i8(const int8_t* out8, const int32_t* out_exp, const in
     loss_kernel<<<(B + 63) / 64, 64, 0, static_cast<cudaStream_t>(stream)>>>(
         out8, out_exp, reinterpret_cast<const long long*>(target), err8, B, classes,
         reinterpret_cast<const unsigned long long*>(seed), rng_stream, sample_offset);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_update_i8(int8_t* w, const int32_t* g32, const uint32_t* maxabs, int64_t n, int mu, int round_mode,
@@ -1487,7 +1487,7 @@ extern "C" int niti_update_i8(int8_t* w, const int32_t* g32, const uint32_t* max
     NITI_REQUIRE(reinterpret_cast<uintptr_t>(w) % 4 == 0 && reinterpret_cast<uintptr_t>(g32) % 16 == 0);
     update_kernel<<<blocks_for(n / 4 + 1, 256, sm_count_simt() * 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         w, g32, maxabs, n, mu, round_mode, reinterpret_cast<const unsigned long long*>(seed), rng_stream);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" size_t niti_update_multi_scratch_bytes(void) { return 2 * UPDATE_MULTI_MAX * sizeof(int32_t); }
@@ -1521,7 +1521,7 @@ static int launch_update(UpdateMultiParams& p, cudaStream_t st) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;  // the grid fits in one wave
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, update_multi_kernel, p));
+    return launched(cudaLaunchKernelEx(&cfg, update_multi_kernel, p));
 }
 
 extern "C" int niti_update_multi_i8(const niti_update_item* items, int count, int mu, int round_mode, int clear_gradients,
@@ -1676,7 +1676,7 @@ extern "C" int niti_dp_update_i8(const niti_dp_update_args* a, void* stream) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = g_cooperative;  // the grid fits in one wave
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, dp_update_kernel, p));
+    return launched(cudaLaunchKernelEx(&cfg, dp_update_kernel, p));
 }
 
 // A step's results into pinned host memory the kernel writes over PCIe: logits, exponent and status word together.  Three
@@ -1698,7 +1698,7 @@ extern "C" int niti_publish_step(const int8_t* out, int64_t n, const int32_t* ex
                                  int32_t* host_exp, int32_t* host_status, void* stream) {
     NITI_REQUIRE(out && n > 0 && exp && status && host_out && host_exp && host_status);
     publish_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(out, n, exp, status, host_out, host_exp, host_status);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // Self-test of the bounded grid barrier: ONE block waits at a barrier that expects two.  Nothing else will ever arrive,
@@ -1712,7 +1712,7 @@ extern "C" int niti_selftest_barrier_timeout(int32_t* scratch, int32_t* status, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int e = set_cuda_error(cudaMemsetAsync(scratch, 0, 4, st))) return e;
     barrier_timeout_selftest_kernel<<<1, 32, 0, st>>>(scratch, status);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_absmax_f32(const float* x, int64_t n, uint32_t* maxbits, void* stream) {
@@ -1720,7 +1720,7 @@ extern "C" int niti_absmax_f32(const float* x, int64_t n, uint32_t* maxbits, voi
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int e = set_cuda_error(cudaMemsetAsync(maxbits, 0, 4, st))) return e;
     absmax_f32_kernel<<<blocks_for(n, 256, sm_count_simt() * 4), 256, 0, st>>>(x, n, maxbits);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 extern "C" int niti_quantize_input_with_max_f32(const float* x, int8_t* x8, int32_t* exp_out, const uint32_t* maxbits, int N,
@@ -1736,5 +1736,6 @@ extern "C" int niti_quantize_input_f32(const float* x, int8_t* x8, int32_t* exp_
     const long long n = static_cast<long long>(N) * C * H * W;
     if (int e = clear_words(scratch, 1, st)) return e;
     absmax_f32_kernel<<<blocks_for(n, 256, sm_count_simt() * 4), 256, 0, st>>>(x, n, scratch);
+    if (int e = launched(cudaGetLastError())) return e;
     return launch_quantize(x, x8, exp_out, scratch, N, C, H, W, st);
 }

@@ -2247,7 +2247,7 @@ static cudaError_t allow_shared(int bytes) {
 
 // The result of a launch whose thread blocks have to be resident together: see LAUNCH_REFUSED.
 static int launched_together(cudaError_t e) {
-    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorInvalidClusterSize && e != cudaErrorLaunchOutOfResources) return set_cuda_error(e);
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorInvalidClusterSize && e != cudaErrorLaunchOutOfResources) return launched(e);
     cudaGetLastError();
     return LAUNCH_REFUSED;
 }
@@ -2277,7 +2277,7 @@ static int launch_gemm_inst(const CUtensorMap& a, const CUtensorMap& b, const CU
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = TWO ? 1 : 0;
-    return set_cuda_error(cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BN, TWO, ROWS32>, a, b, c, p));
+    return launched(cudaLaunchKernelEx(&cfg, umma_gemm_kernel<BN, TWO, ROWS32>, a, b, c, p));
 }
 static int launch_gemm(int bn, bool pair, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const GemmParams& p,
                        cudaStream_t st) {
@@ -2316,7 +2316,7 @@ static int launch_requant_inst(const CUtensorMap& a, const CUtensorMap& b, const
     }
     cfg.attrs = attr; cfg.numAttrs = n;
     const cudaError_t r = cudaLaunchKernelEx(&cfg, kernel, a, b, p);
-    return ONE ? launched_together(r) : set_cuda_error(r);
+    return ONE ? launched_together(r) : launched(r);
 }
 template <bool ONE, bool CODES>
 static int launch_streaming(int bn, int mode, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p, cudaStream_t st) {
@@ -2696,7 +2696,7 @@ int umma_conv_wgrad_partials(const int8_t* x, const int8_t* err, int32_t* partia
     if (e != cudaSuccess) return set_cuda_error(e);
     dim3 grid(p.splits, R * p.k_tiles * p.c_tiles);
     umma_wgrad_kernel<<<grid, UMMA_THREADS, WG_SMEM_BYTES, st>>>(me, mx, mp, p);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 // The gradient into `out`, cleared by the launch, and where *updated says so the update of `w`; state: int32[4], zero between calls.
@@ -2757,7 +2757,7 @@ int umma_conv_wgrad_batch_inner(const int8_t* x_t, const int8_t* err_t, int32_t*
     cudaError_t e = allow_shared<umma_wgrad_kmajor_kernel>(WG_SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     umma_wgrad_kmajor_kernel<<<dim3(p.splits, R * p.k_tiles * p.c_tiles), UMMA_THREADS, WG_SMEM_BYTES, st>>>(ma, mb, mc, p);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 int umma_wgrad_multi_max() { return WG_MULTI_MAX; }
@@ -2869,7 +2869,7 @@ int umma_conv_wgrad_multi(const WgradJob* jobs, int count, int32_t* status, cuda
     cudaError_t e = allow_shared<umma_wgrad_multi_kernel>(WG_SMEM_BYTES);
     if (e != cudaSuccess) return set_cuda_error(e);
     umma_wgrad_multi_kernel<<<grid, UMMA_THREADS, WG_SMEM_BYTES, st>>>(maps, mp);
-    return set_cuda_error(cudaGetLastError());
+    return launched(cudaGetLastError());
 }
 
 }  // namespace niti

@@ -17,7 +17,8 @@ native.set_error_type(NitiError)
 ROUND_NEAREST, ROUND_STOCHASTIC, ROUND_PSEUDO_STOCHASTIC = 0, 1, 2
 CALC_ACT, CALC_ERR, CALC_GRAD = 0, 1, 2
 
-# Launch accounting.  LAUNCHES counts kernels of this library enqueued through this module.
+# Launch accounting.  LAUNCHES counts kernels of this library enqueued through this module: at most, where the form a call takes
+# is decided behind it (lib.niti_launch_count() is what really went out).
 # PROFILE, when set to a list (eager execution only, never under graph capture), makes every
 # call record (name, algorithmic ops, algorithmic bytes, start event, end event) on the
 # launching stream.

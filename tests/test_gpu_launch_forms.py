@@ -204,3 +204,34 @@ def test_calls_on_part_of_the_device():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", SOME_SMS], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_the_library_counts_its_launches():
+    """niti_launch_count against the kernels of a captured graph: gather and product of a thin layer, one launch of a parked, a
+    streaming and a shared layer, the conditional second one on the way back, gradient and update in one and in two, an update of two
+    layers, a head's step, the input."""
+    def counted(fn, torch_kernels=0):
+        n = len(kernels(fn)) - torch_kernels
+        before = ops.lib.niti_launch_count()
+        fn()
+        assert ops.lib.niti_launch_count() - before == n, (fn, n)
+        return n
+
+    large, few, small = Layer(75, 32, 32, 16, 128), Layer(1, 8, 8, 512, 512), Layer(37, 15, 13, 48, 80)
+    assert counted(large.forward) == 1 and counted(few.forward) == 1 and counted(small.forward) == 1
+    wide = Layer(75, 32, 32, 128, 16)
+    assert counted(wide.backward) == 2 and counted(few.backward) == 1
+    g32 = [torch.zeros((n,), dtype=torch.int32, device=DEV) for n in (4096, 512)]
+    ws = [torch.zeros((n,), dtype=torch.int8, device=DEV) for n in (4096, 512)]
+    assert counted(lambda: ops.update_multi(ws, g32, [1, 2], 5)) == 2
+    assert counted(lambda: ops.conv_wgrad_update(small.dx, small.derr, small.dw, 1, 5, 2, None, 18, small.upd)) == 1
+    assert counted(lambda: ops.conv_wgrad_update(few.dx, few.derr, few.dw, 1, 5, 2, None, 18, few.upd)) == 2
+    rng = np.random.default_rng(1)
+    x, w = cu(rnd8(rng, (2, 32, 32, 3))), cu(rnd8(rng, (64, 3, 3, 3)))
+    st = ops.new_requant_state(DEV)
+    assert counted(lambda: ops.conv_fprop_fused(x, w, st, 1, 0, None, 0, 0, True, small.z, small.z)) == 2
+    images = torch.randn(4, 3, 32, 32, device=DEV)
+    assert counted(lambda: ops.quantize_input(images)) == 3
+    a, b = cu(rnd8(rng, (64, 256))), cu(rnd8(rng, (256, 10)))
+    assert counted(lambda: ops.gemm_acc(a, b)) == 1
+    ops.check_status(DEV)
