@@ -15,6 +15,7 @@ from niti_b200._lib import lib  # noqa: E402
 from niti_b200.compat import cutlassconv_cuda  # noqa: E402
 from oracle import niti_oracle as O  # noqa: E402
 from oracle import philox  # noqa: E402
+from tests.test_gpu_launch_forms import Layer, kernels  # noqa: E402
 
 DEV = "cuda:0"
 
@@ -76,7 +77,7 @@ def test_pooling_in_the_same_launch_on_maps_of_any_even_height(N, H, W, C, K, mo
 @pytest.mark.parametrize("N,H,W,C,K", [
     (1, 8, 8, 512, 512), (32, 4, 4, 272, 512),    # eight and four thread blocks to a tile; tiles of 64 and of 128 pixels
     (1, 16, 16, 384, 512),                        # four (16-pixel rows: pooling leaves a block whole pairs of image rows)
-    (20, 8, 8, 144, 272), (70, 10, 10, 240, 112), # four; two, in tiles of 120 pixels
+    (20, 8, 8, 144, 272), (70, 10, 10, 240, 112), # four; two, in tiles of 100 pixels
     (1, 3, 5, 288, 208), (3, 2, 2, 144, 512), (2, 2, 130, 192, 176)])
 @pytest.mark.parametrize("mode,offset", [(0, 0), (1, 0), (1, 5), (2, 0)])
 def test_tiles_that_share_a_reduction(N, H, W, C, K, mode, offset):
@@ -345,3 +346,51 @@ def test_partial_sums_instead_of_reductions_in_every_weight_gradient(N, H, W, C,
     assert int(mx) == int(np.abs(g).max())
     same(wd, O.weight_update(w, g, 5, 2)[0])
     same(dis, g.transpose(3, 1, 2, 0))
+
+
+@pytest.mark.parametrize("N,H,W,C,K,forward,pooled,backward", [
+    (1, 8, 8, 512, 512, 8, 8, 8), (1, 16, 16, 384, 512, 8, 4, 8),  # 16-pixel rows: a block of a pooling call keeps pairs of them
+    (12, 8, 8, 256, 512, 4, 4, 8), (20, 8, 8, 400, 512, 2, 2, 2),
+    (75, 4, 4, 384, 496, 2, 2, 4), (44, 5, 7, 400, 272, 2, 0, 2)])  # tiles of 105 pixels, maps that no pool divides
+def test_as_many_thread_blocks_to_a_tile_as_the_rule_says(N, H, W, C, K, forward, pooled, backward):
+    """Eight, four and two thread blocks to a tile, in both directions and with pooling, whatever the rounding; results as above."""
+    seed, layer = ops.seed_tensor(9, DEV), Layer(N, H, W, C, K)
+    O.set_backend("int_mm")
+    try:
+        for mode in (0, 1, 2):
+            def call(fn, x, *more):
+                st = ops.new_requant_state(DEV)
+                return kernels(lambda: fn(x, layer.dw, st, 1, mode, seed, 3, 0, *more))
+            assert call(ops.conv_fprop_fused, layer.dx, False, layer.z, layer.z) == [(True, forward)]
+            assert call(ops.conv_dgrad_fused, layer.derr, layer.z, layer.z) == [(True, backward)]
+            if pooled:
+                assert call(ops.conv_fprop_pool_fused, layer.dx, False, layer.z, layer.z) == [(True, pooled)]
+            else:
+                assert not ops.conv_fprop_pool_fused_supported(N, H, W, C, K, 3, 3, 1)
+            test_tiles_that_share_a_reduction(N, H, W, C, K, mode, 0)
+    finally:
+        O.set_backend("int64")
+
+
+@pytest.mark.parametrize("offset", [(1 << 34) - 16, (1 << 34) + 64, (1 << 34) - 16 * 1001, (1 << 36) - 32, 3 << 40])
+@pytest.mark.parametrize("N,H,W,C,K,parking", [(2, 9, 7, 48, 80, False), (2, 9, 7, 48, 80, True), (3, 8, 8, 128, 256, True),
+                                               (3, 8, 8, 144, 64, False), (1, 8, 8, 512, 512, True)])
+def test_random_words_where_their_block_number_leaves_32_bits(N, H, W, C, K, parking, offset):
+    """A sample offset may put a tensor's elements anywhere in 64 bits: block numbers (four elements each) that carry into their high
+    word inside a row of outputs, inside the tensor and before it, in the streaming, the parked and the shared kernels."""
+    rng = np.random.default_rng(N + H + C + K)
+    x, w, err = np.maximum(rnd8(rng, (N, H, W, C)), 0), rnd8(rng, (K, 3, 3, C)), rnd8(rng, (N, H, W, K))
+    seed, z = ops.seed_tensor(9, DEV), torch.zeros((), dtype=torch.int32, device=DEV)
+    acc, back = O.conv_fprop(x, w), O.conv_dgrad(err, w)
+    want = O.act_calc(acc, 0, 1, philox.random_u32_tensor(9, 3, acc.shape, offset))[0]
+    want_e = O.err_calc(back, 1, philox.random_u32_tensor(9, 4, back.shape, offset))[0]
+    old = ops.set_accumulator_parking(parking)
+    try:
+        fwd, bwd = ops.new_requant_state(DEV), ops.new_requant_state(DEV)
+        for _ in range(2):
+            for relu in (False, True):
+                same(ops.conv_fprop_fused(cu(x), cu(w), fwd, 1, 1, seed, 3, offset, relu, z, z)[0], np.maximum(want, 0) if relu else want)
+            same(ops.conv_dgrad_fused(cu(err), cu(w), bwd, 1, 1, seed, 4, offset, z, z)[0], want_e)
+    finally:
+        ops.set_accumulator_parking(old)
+    ops.check_status(DEV)
