@@ -235,3 +235,13 @@ def test_the_library_counts_its_launches():
     a, b = cu(rnd8(rng, (64, 256))), cu(rnd8(rng, (256, 10)))
     assert counted(lambda: ops.gemm_acc(a, b)) == 1
     ops.check_status(DEV)
+
+
+def test_the_smoke_step_holds_no_cluster_launch():
+    """Its convolutions (128 channels, batch 4, 16x16 and 8x8 maps) keep one thread block to a tile, in every form the step uses."""
+    for hw in (16, 8):
+        l = Layer(4, hw, hw, 128, 128)
+        assert ops.conv_fprop_pool_fused_supported(4, hw, hw, 128, 128, 3, 3, 1)
+        pooled = kernels(lambda: ops.conv_fprop_pool_fused(l.dx, l.dw, l.fwd, 1, 0, None, 0, 0, True, l.z, l.z))
+        back = kernels(lambda: ops.conv_dgrad_fused(l.derr, l.dw, l.bwd, 1, 0, None, 0, 0, l.z, l.z, relu_mask=l.dx))
+        assert pooled + kernels(l.forward) + back == [(True, 1)] * 3
