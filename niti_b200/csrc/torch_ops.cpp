@@ -362,8 +362,8 @@ PyObject* conv_wgrad_update(Args& a) {
                                                   s.H, s.W, s.C, s.K, s.R, s.S, pad, mu, mode, cptr<uint64_t>(seed), stream, l.status(), l.stream),
                   "niti_conv_wgrad_update_state_i8");
         else
-        check(niti_conv_wgrad_update_i8(cptr<int8_t>(x), cptr<int8_t>(err), mptr<int32_t>(both), mptr<int8_t>(w), s.N, s.H, s.W, s.C, s.K, s.R,
-                                        s.S, pad, mu, mode, cptr<uint64_t>(seed), stream, l.status(), l.stream), "niti_conv_wgrad_update_i8");
+            check(niti_conv_wgrad_update_i8(cptr<int8_t>(x), cptr<int8_t>(err), mptr<int32_t>(both), mptr<int8_t>(w), s.N, s.H, s.W, s.C, s.K, s.R,
+                                            s.S, pad, mu, mode, cptr<uint64_t>(seed), stream, l.status(), l.stream), "niti_conv_wgrad_update_i8");
         auto view = [&](int64_t at_, at::IntArrayRef shape) {
             Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(both.storage()), both.key_set(), both.dtype());
             t.unsafeGetTensorImpl()->set_storage_offset(at_);

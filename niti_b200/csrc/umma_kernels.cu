@@ -1187,20 +1187,9 @@ umma_requant_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
 }
 
-
-// ------------------------------------------------------------------------------------------------
-// Exact single-pass requantisation for problems whose accumulators all fit in tensor memory:
-// every CTA owns at most 512 / BN output tiles and PARKS their int32 accumulators in TMEM.  After
-// its main loops a CTA reduces max|acc| of its tiles into the global word, all CTAs meet at a grid
-// barrier (cooperative launch: all resident; bounded spin), read the now final max, derive the true
-// shift and only then narrow their parked accumulators to int8.  No prediction, no second launch,
-// no int32 in memory.  state = {shift out, max|acc|, redo flag (cleared), redo count, exit ticket,
-// -, max|acc| and barrier arrivals (adjacent: read with one 64-bit load)}; words 1, 4, 5, 6 and 7 are zero between calls.
-// ------------------------------------------------------------------------------------------------
-
-// The grid barrier of the kernels below, run by a CTA's epilogue warps (which have left their maxima in warp_max): every CTA
-// has contributed its maximum when it returns the shift that narrows the tensor, the same to all of them; -1 where the others
-// did not arrive or a role of this CTA gave up.
+// The grid barrier of the narrowing kernels below (streaming in one launch, parked, shared tiles), run by a CTA's epilogue
+// warps (which have left their maxima in warp_max): every CTA has contributed its maximum when it returns the shift that
+// narrows the tensor, the same to all of them; -1 where the others did not arrive or a role of this CTA gave up.
 // One atomic per CTA: atomics on one address serialise at the L2; the waiters poll with plain acquire loads for the same reason.
 // The exit ticket (thread 64's) is drawn as soon as this CTA has read the barrier's words, so that its round trip runs under
 // the narrowing; drawn at the end, behind a barrier of the epilogue warps, it was 0.45 us of every launch.
@@ -1422,6 +1411,15 @@ umma_requant_once_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Exact single-pass requantisation for problems whose accumulators all fit in tensor memory:
+// every CTA owns at most 512 / BN output tiles and PARKS their int32 accumulators in TMEM.  After
+// its main loops a CTA reduces max|acc| of its tiles into the global word, all CTAs meet at a grid
+// barrier (cooperative launch: all resident; bounded spin), read the now final max, derive the true
+// shift and only then narrow their parked accumulators to int8.  No prediction, no second launch,
+// no int32 in memory.  state = {shift out, max|acc|, redo flag (cleared), redo count, exit ticket,
+// -, max|acc| and barrier arrivals (adjacent: read with one 64-bit load)}; words 1, 4, 5, 6 and 7 are zero between calls.
+// ------------------------------------------------------------------------------------------------
 template <int BN, bool TWO, int MODE>
 __global__ void __launch_bounds__(REQUANT_THREADS, 1)
 umma_parked_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
