@@ -223,7 +223,8 @@ NITI_API int niti_conv_wgrad_builtin_scratch_i8(const int8_t* x, const int8_t* e
  * is only known when the contraction has finished, so the kernel narrows with a PREDICTED shift
  * (the one this layer needed last time, state[0]) while it reduces the true max|acc|; the thread
  * block that finishes last derives the true shift, and only if the prediction was wrong the
- * contraction is launched again (that second launch returns at once otherwise).  The result is
+ * contraction is launched again (that second launch returns at once otherwise); forward layers do
+ * the same within one cooperative launch where they may.  The result is
  * always the exact one; the int32 tensor never touches memory.  When the whole output is at most
  * 148 x (512 / tile width) tiles, all accumulators fit in tensor memory at once and a single
  * cooperative launch does it without any prediction: reduce max, grid barrier, narrow (state[0]
@@ -231,7 +232,7 @@ NITI_API int niti_conv_wgrad_builtin_scratch_i8(const int8_t* x, const int8_t* e
  *   state: device int32[8], 8-byte aligned, owned by the caller, one per layer and direction, zeroed once:
  *          [0] shift (in: prediction, out: true value), [1] max|acc| (zero between calls), [2] 1 if
  *          the last call had to redo (bits 0-1; see niti_conv_dgrad_requant_side_i8), [3] number of redos so far, [4] block ticket, [5..7] grid-barrier
- *          words of the single-launch kernel (all zero between calls).
+ *          words of the single-launch kernels (all zero between calls).
  *   kind is ACT for fprop (exp_out = shift + *exp_a + *exp_b) and ERR for dgrad; target 7 bits.
  * Shapes: niti_conv_*_requant_supported() != 0 (the tensor-core shapes of the entry points above
  * with 16-byte-multiple output channels); otherwise NITI_ERR_UNSUPPORTED and the caller uses
